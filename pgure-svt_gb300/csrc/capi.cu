@@ -1432,10 +1432,9 @@ int pgsvt_hot_pixel_filter(uint16_t* frames, uint32_t nrows, uint32_t ncols, uin
     uint16_t* colmed = mem.arr<uint16_t>((size_t)ncols * nframes);
     uint32_t* med = mem.arr<uint32_t>(nframes);
     uint32_t* madm = mem.arr<uint32_t>(nframes);
-    uint8_t* flag = mem.arr<uint8_t>(n);
     PGSVT_CK(cudaMemcpyAsync(seq, frames, n * 2, cudaMemcpyHostToDevice, s));
     check_launch(launch_hot_pixel(seq, (int)nrows, (int)ncols, (int)nframes, threshold, colmed,
-                                  med, madm, flag, s), stats, 6);
+                                  med, madm, s), stats, 5);
     PGSVT_CK(cudaMemcpyAsync(frames, seq, n * 2, cudaMemcpyDeviceToHost, s));
     PGSVT_CK(cudaStreamSynchronize(s));
   });

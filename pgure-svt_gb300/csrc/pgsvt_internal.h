@@ -278,7 +278,7 @@ cudaError_t launch_noise_apply(const Problem& pb, const DeviceBuffers& d, const 
 
 // hot-pixel filter (hotpixel.cu)
 cudaError_t launch_hot_pixel(uint16_t* seq, int nr, int nc, int nimg, double thr, uint16_t* colmed,
-                             uint32_t* med, uint32_t* madm, uint8_t* flag, cudaStream_t s);
+                             uint32_t* med, uint32_t* madm, cudaStream_t s);
 
 // learned lambda proposal (lambda.cu)
 struct LambdaTrain {

@@ -1,0 +1,21 @@
+"""Kernel forms at the sizes where they can go wrong: edges of tiles and
+stripes, remainders, the smallest and the largest of a form's range.  Each is
+held to the oracle, or bit for bit to the general form of the same kernel."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nr,nc", [(1, 1), (2, 5), (3, 3), (5, 1), (9, 33), (40, 31), (64, 32),
+                                   (7, 512), (11, 513), (6, 1061)])
+@pytest.mark.parametrize("thr", [0.0, 3.0])
+def test_hot_pixel_wavefront(capi, oracle, nr, nc, thr):
+    """Column stripes of 512 and their remainders; dense outliers (threshold 0,
+    and every value below the median), so replacements feed one another."""
+    rng = np.random.default_rng(nr * 4099 + nc)
+    a = rng.integers(0, 65536, (nr, nc, 2), dtype=np.uint16)
+    a[..., 1] = rng.integers(900, 1000, (nr, nc))
+    a[rng.random(a.shape) < 0.02] = 65535
+    a = np.asfortranarray(a)
+    np.testing.assert_array_equal(capi.hot_pixel_filter(a, thr), oracle.hot_pixel_filter(a, thr))
