@@ -643,7 +643,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
   int nfslots = 0;
   if (use_model) {
     dmodel = mem.arr<float>(PGSVT_LAMBDA_MODEL_FLOATS);
-    dmodel_bf = mem.get(PGSVT_LAMBDA_MODEL_FLOATS * 2);
+    dmodel_bf = mem.get(PGSVT_LAMBDA_SHADOW_BYTES);
     PGSVT_CK(cudaMemcpyAsync(dmodel, p.lambda_model, sizeof(float) * PGSVT_LAMBDA_MODEL_FLOATS,
                              cudaMemcpyHostToDevice, s));
     stats.h2d += sizeof(float) * PGSVT_LAMBDA_MODEL_FLOATS;
@@ -1244,7 +1244,7 @@ int pgsvt_lambda_predict(const float* model, const float* features, uint32_t n, 
     PGSVT_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
     float* m = mem.arr<float>(PGSVT_LAMBDA_MODEL_FLOATS);
-    void* wbf = mem.get(PGSVT_LAMBDA_MODEL_FLOATS * 2);
+    void* wbf = mem.get(PGSVT_LAMBDA_SHADOW_BYTES);
     float* f = mem.arr<float>((size_t)n * PGSVT_LAMBDA_FEATURES);
     float* yd = mem.arr<float>(n);
     PGSVT_CK(cudaMemcpyAsync(m, model, sizeof(float) * PGSVT_LAMBDA_MODEL_FLOATS, cudaMemcpyHostToDevice, s));
@@ -1270,10 +1270,10 @@ int pgsvt_lambda_grad(const float* model, const float* features, const float* ta
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
     const int nblk = ((int)n + 31) / 32;
     float* m = mem.arr<float>(PGSVT_LAMBDA_MODEL_FLOATS);
-    void* wbf = mem.get(PGSVT_LAMBDA_MODEL_FLOATS * 2);
+    void* wbf = mem.get(PGSVT_LAMBDA_SHADOW_BYTES);
     float* f = mem.arr<float>((size_t)n * PGSVT_LAMBDA_FEATURES);
     float* t = mem.arr<float>(n);
-    float* part = mem.arr<float>((size_t)nblk * PGSVT_LAMBDA_PARAMS);
+    float* act = mem.arr<float>(lambda_act_floats((int)n));
     float* pl = mem.arr<float>(nblk);
     float* g = mem.arr<float>(PGSVT_LAMBDA_PARAMS);
     PGSVT_CK(cudaMemcpyAsync(m, model, sizeof(float) * PGSVT_LAMBDA_MODEL_FLOATS, cudaMemcpyHostToDevice, s));
@@ -1282,7 +1282,7 @@ int pgsvt_lambda_grad(const float* model, const float* features, const float* ta
     PGSVT_CK(cudaMemcpyAsync(t, targets, sizeof(float) * n, cudaMemcpyHostToDevice, s));
     PGSVT_CK(lambda_attrs());
     check_launch(lambda_shadow(m, wbf, s), stats);
-    check_launch(lambda_grad(m, wbf, f, t, (int)n, part, pl, g, s), stats, 2);
+    check_launch(lambda_grad(m, wbf, f, t, (int)n, act, pl, g, s), stats, 2);
     std::vector<float> hl(nblk);
     PGSVT_CK(cudaMemcpyAsync(grad, g, sizeof(float) * PGSVT_LAMBDA_PARAMS, cudaMemcpyDeviceToHost, s));
     PGSVT_CK(cudaMemcpyAsync(hl.data(), pl, sizeof(float) * nblk, cudaMemcpyDeviceToHost, s));
@@ -1323,7 +1323,7 @@ int pgsvt_lambda_train(float* model, const float* features, const float* targets
     t.eps = tp->eps;
     const int nblk = batch / 32;
     t.m = mem.arr<float>(PGSVT_LAMBDA_MODEL_FLOATS);
-    t.wbf = mem.get(PGSVT_LAMBDA_MODEL_FLOATS * 2);
+    t.wbf = mem.get(PGSVT_LAMBDA_SHADOW_BYTES);
     t.mom1 = mem.arr<float>(PGSVT_LAMBDA_PARAMS);
     t.mom2 = mem.arr<float>(PGSVT_LAMBDA_PARAMS);
     float* feat = mem.arr<float>((size_t)n * PGSVT_LAMBDA_FEATURES);
@@ -1333,7 +1333,7 @@ int pgsvt_lambda_train(float* model, const float* features, const float* targets
     t.target = target;
     t.perm = perm;
     t.epoch = mem.arr<int>(1);
-    t.part = mem.arr<float>((size_t)nblk * PGSVT_LAMBDA_PARAMS);
+    t.act = mem.arr<float>(lambda_act_floats(batch));
     t.loss_acc = mem.arr<float>((size_t)t.steps * nblk);
     t.epoch_loss = mem.arr<float>(tp->epochs);
     // sample order of every epoch: Fisher-Yates shuffles from a pcg64 stream

@@ -4,12 +4,17 @@
 // histogram of log singular values) to y = log10(lambda/upper); the proposal
 // starts a narrow PGURE search (eval.cu, phase 1) that falls back to the plain
 // search.  The network is tiny (67 -> 128 -> 128 -> 128 -> 1, 41,857
-// parameters), so every pass is one CUDA-core kernel over blocks of 32
-// samples: weights are read as bf16 from global memory (they stay in L1),
-// activations live in shared memory, sums are FP32.  Training keeps FP32
-// master weights and a bf16 shadow that the passes read; per-block gradient
-// partials are summed in a fixed order, so training is deterministic.
+// parameters), far too small to fill a tensor-core tile per step, so every pass
+// runs on CUDA cores with FP32 sums.  Training keeps FP32 master weights and a
+// bf16 shadow that the passes read.  What bounds a step is latency: 14 MFLOP
+// over chains of 128 dependent FMAs per layer.  So it is spread thin: k_mlp_pass
+// runs four samples per block (the samples are independent), with the weights in
+// shared memory, and k_mlp_update forms every weight's gradient, sums it in
+// a fixed order (chains of 32 samples, then the chains) and applies AdamW in
+// the same thread, so training is deterministic.
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "pgsvt.h"
 #include "pgsvt_internal.h"
@@ -19,9 +24,6 @@ namespace lam {
 
 constexpr int NF = PGSVT_LAMBDA_FEATURES;   // 67
 constexpr int H = PGSVT_LAMBDA_HIDDEN;      // 128
-constexpr int SB = 32;                      // samples per block
-constexpr int LD0 = NF + 2;                 // 69: odd row strides keep the
-constexpr int LDH = H + 1;                  // column reads conflict-free
 constexpr int OFF_MEAN = 0, OFF_SCALE = NF, OFF_W1 = 2 * NF;
 constexpr int OFF_B1 = OFF_W1 + H * NF, OFF_W2 = OFF_B1 + H, OFF_B2 = OFF_W2 + H * H;
 constexpr int OFF_W3 = OFF_B2 + H, OFF_B3 = OFF_W3 + H * H, OFF_W4 = OFF_B3 + H;
@@ -32,14 +34,29 @@ static_assert(TOTAL == PGSVT_LAMBDA_MODEL_FLOATS, "model layout");
 static_assert(NPARAM == PGSVT_LAMBDA_PARAMS, "parameter count");
 static_assert(OFF_W1 == PGSVT_LAMBDA_PARAM_OFFSET, "parameter offset");
 
-struct Smem {
-  float x0[SB * LD0];
-  float z[3][SB * LDH];   // pre-activations, then their gradients
-  float a[3][SB * LDH];   // activations
-  float o[SB];            // network outputs (before y_scale / y_mean)
-  float dO[SB];
-  float red[4];
+constexpr int GS = 4;         // samples of a pass at a time
+constexpr int PT = 256;       // its threads: one output of two samples each
+constexpr int LDA = 132;      // row stride of the activations in shared memory
+constexpr int WS1 = 72, WS2 = 136;  // weight row strides (bf16): 16-byte rows that
+                                    // start four banks apart
+// The bf16 shadow of the model, laid out as the passes hold it in shared memory
+// (one straight copy): padded weight rows, then the output row as floats.
+struct __align__(16) Shadow {
+  __nv_bfloat16 w1[H * WS1], w2[H * WS2], w3[H * WS2];
+  float w4[H];
 };
+static_assert(sizeof(Shadow) <= PGSVT_LAMBDA_SHADOW_BYTES, "shadow allocation");
+struct Smem {
+  Shadow w;
+  float x0[GS * LDA];
+  float z[3][GS * LDA];   // pre-activations, then their gradients
+  float a[3][GS * LDA];   // activations
+  float o[GS], dO[GS];    // network outputs (before y_scale / y_mean), their gradients
+};
+
+// Rows of a training pass in device memory, kept for the weight gradients:
+// [row][128] each, row r the r-th sample of the batch
+enum { ACT_X0, ACT_A1, ACT_A2, ACT_A3, ACT_Z1, ACT_Z2, ACT_Z3, ACT_N };
 
 __device__ __forceinline__ float gelu(float z) {
   return 0.5f * z * (1.f + erff(z * 0.70710678118654752f));
@@ -48,173 +65,207 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.f + erff(z * 0.70710678118654752f)) +
          z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
-__device__ __forceinline__ float wb(const __nv_bfloat16* W, int i) {
-  return __bfloat162float(W[i]);
+// Parameter at model offset i (value v) into the shadow, rounded to bf16.
+__device__ __forceinline__ void to_shadow(Shadow* sh, int i, float v) {
+  const __nv_bfloat16 b = __float2bfloat16_rn(v);
+  if (i >= OFF_W1 && i < OFF_B1) sh->w1[(i - OFF_W1) / NF * WS1 + (i - OFF_W1) % NF] = b;
+  else if (i >= OFF_W2 && i < OFF_B2) sh->w2[(i - OFF_W2) / H * WS2 + (i - OFF_W2) % H] = b;
+  else if (i >= OFF_W3 && i < OFF_B3) sh->w3[(i - OFF_W3) / H * WS2 + (i - OFF_W3) % H] = b;
+  else if (i >= OFF_W4 && i < OFF_B4) sh->w4[i - OFF_W4] = __bfloat162float(b);
 }
 
-// One dense layer plus GELU: thread j computes output j for every sample.
-template <int KIN>
-__device__ void dense_gelu(const __nv_bfloat16* W, const float* b, const float* in, int ld_in,
-                           float* z, float* a) {
-  const int j = threadIdx.x;
-  float acc[SB];
-  const float bj = b[j];
+// The weights into shared memory.
+__device__ void load_weights(const Shadow* __restrict__ sh, Smem& sm) {
+  const uint4* g = reinterpret_cast<const uint4*>(sh);
+  uint4* o = reinterpret_cast<uint4*>(&sm.w);
+  constexpr int N = (int)(sizeof(Shadow) / 16);
+#pragma unroll 11
+  for (int i = threadIdx.x; i < N; i += PT) o[i] = g[i];
+}
+
+__device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+
+// One dense layer plus GELU: thread (j, h) computes output j of samples 2h
+// and 2h + 1, each sum in input order.
+template <int KIN, int WS>
+__device__ __forceinline__ void dense_gelu(const __nv_bfloat16* W, float bj, const float* in,
+                                           float* z, float* a) {
+  const int j = threadIdx.x & (H - 1), s0 = (threadIdx.x >> 7) * 2;
+  const float* p = in + s0 * LDA;
+  const __nv_bfloat16* wr = W + j * WS;
+  float c0 = bj, c1 = bj;
+  constexpr int K8 = KIN / 8 * 8;
+#pragma unroll 4
+  for (int k = 0; k < K8; k += 8) {
+    const uint4 wv = *reinterpret_cast<const uint4*>(wr + k);
+    const uint32_t wu[4] = {wv.x, wv.y, wv.z, wv.w};
+    float u[8], v[8];
+    *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(p + k);
+    *reinterpret_cast<float4*>(u + 4) = *reinterpret_cast<const float4*>(p + k + 4);
+    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p + LDA + k);
+    *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(p + LDA + k + 4);
 #pragma unroll
-  for (int s = 0; s < SB; ++s) acc[s] = bj;
-  for (int k = 0; k < KIN; ++k) {
-    const float w = wb(W, j * KIN + k);
-#pragma unroll
-    for (int s = 0; s < SB; ++s) acc[s] = fmaf(w, in[s * ld_in + k], acc[s]);
+    for (int q = 0; q < 8; ++q) {
+      const float w = (q & 1) ? bf_hi(wu[q >> 1]) : bf_lo(wu[q >> 1]);
+      c0 = fmaf(w, u[q], c0);
+      c1 = fmaf(w, v[q], c1);
+    }
   }
 #pragma unroll
-  for (int s = 0; s < SB; ++s) {
-    z[s * LDH + j] = acc[s];
-    a[s * LDH + j] = gelu(acc[s]);
+  for (int k = K8; k < KIN; ++k) {
+    const float w = __bfloat162float(wr[k]);
+    c0 = fmaf(w, p[k], c0);
+    c1 = fmaf(w, p[LDA + k], c1);
+  }
+  z[s0 * LDA + j] = c0;
+  z[(s0 + 1) * LDA + j] = c1;
+  a[s0 * LDA + j] = gelu(c0);
+  a[(s0 + 1) * LDA + j] = gelu(c1);
+}
+
+// Gradient of a layer's input through the GELU before it: thread (k, h),
+// samples 2h and 2h + 1, each sum in output order; zprev holds the previous
+// pre-activations and receives their gradients.
+__device__ __forceinline__ void dense_back(const __nv_bfloat16* W, const float* dz, float* zprev) {
+  const int k = threadIdx.x & (H - 1), s0 = (threadIdx.x >> 7) * 2;
+  const float* p = dz + s0 * LDA;
+  float c0 = 0.f, c1 = 0.f;
+#pragma unroll 4
+  for (int j = 0; j < H; j += 4) {
+    float u[4], v[4];
+    *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(p + j);
+    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p + LDA + j);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float w = __bfloat162float(W[(j + q) * WS2 + k]);
+      c0 = fmaf(w, u[q], c0);
+      c1 = fmaf(w, v[q], c1);
+    }
+  }
+  float* zp = zprev + s0 * LDA + k;
+  zp[0] = c0 * gelu_grad(zp[0]);
+  zp[LDA] = c1 * gelu_grad(zp[LDA]);
+}
+
+// Stage the features of samples [b0, b0 + GS) of [0, n) as (f - mean) * scale,
+// the others as zeros.  `rows` maps a sample to a feature row (or null).
+__device__ void load_inputs(const float* m, const float* feat, const int32_t* rows, int b0, int n,
+                            Smem& sm) {
+  for (int i = threadIdx.x; i < GS * NF; i += PT) {
+    const int s = i / NF, k = i % NF;
+    float v = 0.f;
+    if (b0 + s < n) {
+      const int r = rows ? rows[b0 + s] : b0 + s;
+      v = (feat[(size_t)r * NF + k] - m[OFF_MEAN + k]) * m[OFF_SCALE + k];
+    }
+    sm.x0[s * LDA + k] = v;
   }
 }
 
-// Forward pass of samples [0, ns) held in sm.x0 (already normalised); the
-// outputs land in sm.o.  128 threads.
-__device__ void forward(const float* m, const __nv_bfloat16* wbf, Smem& sm) {
-  dense_gelu<NF>(wbf + OFF_W1, m + OFF_B1, sm.x0, LD0, sm.z[0], sm.a[0]);
+// Forward pass of the GS samples in sm.x0; the outputs land in sm.o.
+__device__ void forward(const float* m, Smem& sm) {
+  const int j = threadIdx.x & (H - 1);
   __syncthreads();
-  dense_gelu<H>(wbf + OFF_W2, m + OFF_B2, sm.a[0], LDH, sm.z[1], sm.a[1]);
+  dense_gelu<NF, WS1>(sm.w.w1, m[OFF_B1 + j], sm.x0, sm.z[0], sm.a[0]);
   __syncthreads();
-  dense_gelu<H>(wbf + OFF_W3, m + OFF_B3, sm.a[1], LDH, sm.z[2], sm.a[2]);
+  dense_gelu<H, WS2>(sm.w.w2, m[OFF_B2 + j], sm.a[0], sm.z[1], sm.a[1]);
   __syncthreads();
-  if (threadIdx.x < SB) {
+  dense_gelu<H, WS2>(sm.w.w3, m[OFF_B3 + j], sm.a[1], sm.z[2], sm.a[2]);
+  __syncthreads();
+  if (threadIdx.x < GS) {
     const int s = threadIdx.x;
     float acc = m[OFF_B4];
-    for (int k = 0; k < H; ++k) acc = fmaf(wb(wbf, OFF_W4 + k), sm.a[2][s * LDH + k], acc);
+#pragma unroll 16
+    for (int k = 0; k < H; ++k) acc = fmaf(sm.w.w4[k], sm.a[2][s * LDA + k], acc);
     sm.o[s] = acc;
   }
   __syncthreads();
 }
 
-// Stage features rows [r0, r0+ns) into sm.x0 as (f - mean) * scale, rows
-// beyond ns as zeros.  `rows` maps a block row to a feature row (or null).
-__device__ void load_inputs(const float* m, const float* feat, const int32_t* rows, int r0,
-                            int ns, Smem& sm) {
-  for (int i = threadIdx.x; i < SB * NF; i += blockDim.x) {
-    const int s = i / NF, k = i % NF;
-    float v = 0.f;
-    if (s < ns) {
-      const int r = rows ? rows[r0 + s] : r0 + s;
-      v = (feat[(size_t)r * NF + k] - m[OFF_MEAN + k]) * m[OFF_SCALE + k];
-    }
-    sm.x0[s * LD0 + k] = v;
-  }
-  __syncthreads();
-}
-
-// Weight gradients of one layer (thread k owns input column k) and the
-// gradient of its input, through GELU when `zprev` is given.
-template <int KIN>
-__device__ void dense_backward(const __nv_bfloat16* W, const float* dz, const float* in,
-                               int ld_in, float* gW, float* gb, float* zprev) {
-  const int k = threadIdx.x;
-  float acol[SB];
-#pragma unroll
-  for (int s = 0; s < SB; ++s) acol[s] = (k < KIN) ? in[s * ld_in + k] : 0.f;
-  float din[SB];
-#pragma unroll
-  for (int s = 0; s < SB; ++s) din[s] = 0.f;
-  for (int j = 0; j < H; ++j) {
-    float g = 0.f;
-    const float w = (k < KIN) ? wb(W, j * KIN + k) : 0.f;
-#pragma unroll
-    for (int s = 0; s < SB; ++s) {
-      const float d = dz[s * LDH + j];
-      g = fmaf(d, acol[s], g);
-      din[s] = fmaf(w, d, din[s]);
-    }
-    if (k < KIN) gW[j * KIN + k] = g;
-  }
-  {
-    const int j = threadIdx.x;  // H threads: bias gradient of output j
-    float g = 0.f;
-#pragma unroll
-    for (int s = 0; s < SB; ++s) g += dz[s * LDH + j];
-    gb[j] = g;
-  }
-  __syncthreads();  // every read of dz and of the previous z is done
-  if (zprev && k < KIN) {
-#pragma unroll
-    for (int s = 0; s < SB; ++s) zprev[s * LDH + k] = din[s] * gelu_grad(zprev[s * LDH + k]);
-  }
-  __syncthreads();
-}
-
-// Forward + backward of one block of samples; writes the block's gradient
-// partial (NPARAM floats, already divided by `norm`) and its squared-error sum.
-__global__ void __launch_bounds__(H) k_mlp_grad(const float* __restrict__ m,
-                                                const __nv_bfloat16* __restrict__ wbf,
-                                                const float* __restrict__ feat,
-                                                const float* __restrict__ target,
-                                                const int32_t* __restrict__ perm,
-                                                const int* __restrict__ epoch, int64_t perm_stride,
-                                                int r0, int n, float norm, float* __restrict__ part,
-                                                float* __restrict__ part_loss) {
-  extern __shared__ float smraw[];
+// Forward pass and the gradients of the pre-activations of the samples of one
+// batch (r0 .. n of the permuted order, rows padded to a multiple of 32): the
+// activations, gradients, output gradients and errors of every row to device
+// memory.  One block per GS rows; a batch of 256 fills 64 of the 152 SMs, and
+// its chains of dependent FMAs, not its 14 MFLOP, are what takes the time.
+// One training step (batch 256), GB300: 177 -> 11.7 us here and 8.5 us in
+// k_mlp_update (before, one block of 128 threads did everything for 32 samples).
+__global__ void __launch_bounds__(PT) k_mlp_pass(const float* __restrict__ m,
+                                                 const Shadow* __restrict__ wbf,
+                                                 const float* __restrict__ feat,
+                                                 const float* __restrict__ target,
+                                                 const int32_t* __restrict__ perm,
+                                                 const int* __restrict__ epoch, int64_t perm_stride,
+                                                 int r0, int n, int rows_pad, float norm,
+                                                 float* __restrict__ act, float* __restrict__ dO,
+                                                 float* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
   Smem& sm = *reinterpret_cast<Smem*>(smraw);
-  const int b0 = r0 + blockIdx.x * SB;
-  const int ns = max(0, min(SB, n - b0));
   const int32_t* rows = perm ? perm + (epoch ? (int64_t)(*epoch) * perm_stride : 0) : nullptr;
-  load_inputs(m, feat, rows, b0, ns, sm);
-  forward(m, wbf, sm);
+  load_weights(wbf, sm);
   const float ym = m[OFF_YMEAN], ysi = 1.f / m[OFF_YSCALE];
-  if (threadIdx.x < SB) {
-    const int s = threadIdx.x;
-    float e = 0.f;
-    if (s < ns) {
-      const int r = rows ? rows[b0 + s] : b0 + s;
-      e = sm.o[s] - (target[r] - ym) * ysi;
+  const size_t plane = (size_t)rows_pad * H;
+  for (int g0 = blockIdx.x * GS; g0 < rows_pad; g0 += gridDim.x * GS) {
+    const int b0 = r0 + g0;
+    load_inputs(m, feat, rows, b0, n, sm);
+    forward(m, sm);
+    if (threadIdx.x < GS) {
+      const int s = threadIdx.x;
+      float e = 0.f;
+      if (b0 + s < n) {
+        const int r = rows ? rows[b0 + s] : b0 + s;
+        e = sm.o[s] - (target[r] - ym) * ysi;
+      }
+      sm.dO[s] = 2.f * e * norm;
+      dO[g0 + s] = sm.dO[s];
+      err[g0 + s] = e;
     }
-    sm.dO[s] = 2.f * e * norm;
-    float sq = e * e;
+    __syncthreads();
+    // dz3 = dO W4 gelu'(z3)
+    const int j = threadIdx.x & (H - 1), s0 = (threadIdx.x >> 7) * 2;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if (s == 0) part_loss[blockIdx.x] = sq;
-  }
-  __syncthreads();
-  float* g = part + (size_t)blockIdx.x * NPARAM;
-  // output layer: dW4[k] = sum_s dO a3, da3 = dO W4, dz3 = da3 gelu'(z3)
-  {
-    const int k = threadIdx.x;
-    float gw = 0.f, gbias = 0.f;
-    const float w4 = wb(wbf, OFF_W4 + k);
-#pragma unroll
-    for (int s = 0; s < SB; ++s) {
-      gw = fmaf(sm.dO[s], sm.a[2][s * LDH + k], gw);
-      gbias += sm.dO[s];
+    for (int q = 0; q < 2; ++q) {
+      float* z = &sm.z[2][(s0 + q) * LDA + j];
+      *z = sm.dO[s0 + q] * sm.w.w4[j] * gelu_grad(*z);
     }
-    g[OFF_W4 - OFF_W1 + k] = gw;
-    if (k == 0) g[OFF_B4 - OFF_W1] = gbias;
     __syncthreads();
+    dense_back(sm.w.w3, sm.z[2], sm.z[1]);
+    __syncthreads();
+    dense_back(sm.w.w2, sm.z[1], sm.z[0]);
 #pragma unroll
-    for (int s = 0; s < SB; ++s)
-      sm.z[2][s * LDH + k] = sm.dO[s] * w4 * gelu_grad(sm.z[2][s * LDH + k]);
-    __syncthreads();
+    for (int q = 0; q < 2; ++q) {  // (own elements only: no barrier needed)
+      const size_t o = (size_t)(g0 + s0 + q) * H + j;
+      const int l = (s0 + q) * LDA + j;
+      if (j < NF) act[ACT_X0 * plane + o] = sm.x0[l];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        act[(ACT_A1 + t) * plane + o] = sm.a[t][l];
+        act[(ACT_Z1 + t) * plane + o] = sm.z[t][l];
+      }
+    }
+    __syncthreads();  // the next group overwrites the rows
   }
-  dense_backward<H>(wbf + OFF_W3, sm.z[2], sm.a[1], LDH, g + (OFF_W3 - OFF_W1),
-                    g + (OFF_B3 - OFF_W1), sm.z[1]);
-  dense_backward<H>(wbf + OFF_W2, sm.z[1], sm.a[0], LDH, g + (OFF_W2 - OFF_W1),
-                    g + (OFF_B2 - OFF_W1), sm.z[0]);
-  dense_backward<NF>(wbf + OFF_W1, sm.z[0], sm.x0, LD0, g + 0, g + (OFF_B1 - OFF_W1), nullptr);
 }
 
 // Network outputs y (after y_scale / y_mean) of n feature rows.
-__global__ void __launch_bounds__(H) k_mlp_forward(const float* __restrict__ m,
-                                                   const __nv_bfloat16* __restrict__ wbf,
-                                                   const float* __restrict__ feat, int n,
-                                                   float* __restrict__ y) {
-  extern __shared__ float smraw[];
+__global__ void __launch_bounds__(PT) k_mlp_forward(const float* __restrict__ m,
+                                                    const Shadow* __restrict__ wbf,
+                                                    const float* __restrict__ feat, int n,
+                                                    float* __restrict__ y, float* __restrict__ y2) {
+  extern __shared__ __align__(16) unsigned char smraw[];
   Smem& sm = *reinterpret_cast<Smem*>(smraw);
-  const int b0 = blockIdx.x * SB;
-  const int ns = max(0, min(SB, n - b0));
-  load_inputs(m, feat, nullptr, b0, ns, sm);
-  forward(m, wbf, sm);
-  if (threadIdx.x < ns) y[b0 + threadIdx.x] = sm.o[threadIdx.x] * m[OFF_YSCALE] + m[OFF_YMEAN];
+  load_weights(wbf, sm);
+  for (int b0 = blockIdx.x * GS; b0 < n; b0 += gridDim.x * GS) {
+    load_inputs(m, feat, nullptr, b0, n, sm);
+    forward(m, sm);
+    const int r = b0 + threadIdx.x;
+    if (threadIdx.x < GS && r < n) {
+      const float v = sm.o[threadIdx.x] * m[OFF_YSCALE] + m[OFF_YMEAN];
+      y[r] = v;
+      if (y2) y2[r] = v;
+    }
+    __syncthreads();
+  }
 }
 
 __device__ __forceinline__ bool is_weight(int i) {  // i: offset in the model
@@ -222,19 +273,10 @@ __device__ __forceinline__ bool is_weight(int i) {  // i: offset in the model
          (i >= OFF_W3 && i < OFF_B3) || (i >= OFF_W4 && i < OFF_B4);
 }
 
-// bf16 shadow of the whole model (only the weight ranges are read as bf16).
-__global__ void k_mlp_shadow(const float* __restrict__ m, __nv_bfloat16* __restrict__ wbf) {
+// bf16 shadow of the weights.
+__global__ void k_mlp_shadow(const float* __restrict__ m, Shadow* __restrict__ wbf) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < TOTAL; i += gridDim.x * blockDim.x)
-    wbf[i] = __float2bfloat16_rn(m[i]);
-}
-
-// Sum of the block partials in block order (gradient entry point).
-__global__ void k_mlp_gsum(const float* __restrict__ part, int nblk, float* __restrict__ grad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NPARAM) return;
-  float g = 0.f;
-  for (int b = 0; b < nblk; ++b) g += part[(size_t)b * NPARAM + i];
-  grad[i] = g;
+    to_shadow(wbf, i, m[i]);
 }
 
 struct AdamCfg {
@@ -242,19 +284,12 @@ struct AdamCfg {
   int steps_per_epoch, total_steps;
 };
 
-// AdamW step `step` of the epoch in *epoch: gradient = sum of the block
-// partials in block order; FP32 master and moments, bf16 shadow refreshed.
-__global__ void k_mlp_adam(float* __restrict__ m, __nv_bfloat16* __restrict__ wbf,
-                           float* __restrict__ mom1, float* __restrict__ mom2,
-                           const float* __restrict__ part, int nblk,
-                           const int* __restrict__ epoch, int step, AdamCfg c) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NPARAM) return;
-  const int t = *epoch * c.steps_per_epoch + step + 1;  // 1-based step count
+// AdamW step t (1-based) of parameter i with gradient g: FP32 master and
+// moments, bf16 shadow refreshed.
+__device__ __forceinline__ void adam(float* m, Shadow* wbf, float* mom1, float* mom2, int i,
+                                     float g, int t, const AdamCfg& c) {
   const float prog = (float)(t - 1) / (float)max(1, c.total_steps - 1);
   const float lr = c.lr_final + 0.5f * (c.lr - c.lr_final) * (1.f + cospif(prog));
-  float g = 0.f;
-  for (int b = 0; b < nblk; ++b) g += part[(size_t)b * NPARAM + i];
   const float m1 = c.b1 * mom1[i] + (1.f - c.b1) * g;
   const float m2 = c.b2 * mom2[i] + (1.f - c.b2) * g * g;
   mom1[i] = m1;
@@ -265,7 +300,98 @@ __global__ void k_mlp_adam(float* __restrict__ m, __nv_bfloat16* __restrict__ wb
   if (is_weight(mi)) w -= lr * c.wd * w;
   w -= lr * (m1 / bc1) / (sqrtf(m2 / bc2) + c.eps);
   m[mi] = w;
-  wbf[mi] = __float2bfloat16_rn(w);
+  to_shadow(wbf, mi, w);
+}
+
+// Gradients from the rows of a pass, summed in a fixed order (a chain of FMAs
+// over each 32 rows, then the chains in order), and with ADAM the parameter
+// update; without it the gradients go to `grad`.  A block of 128 inputs x NCH
+// chains takes JB outputs of one layer: the chains run side by side (what
+// bounds the kernel is their latency) and are added in order from shared
+// memory.  The last blocks take the biases, the output layer and the squared
+// errors.
+constexpr int JB = 2;                    // outputs per block
+constexpr int NCH = 8;                   // chains at a time
+constexpr int UB = H / JB;               // blocks of one layer
+constexpr int kUpdateBlocks = 3 * UB + 5;
+
+template <bool ADAM>
+__global__ void __launch_bounds__(H * NCH) k_mlp_update(
+    float* __restrict__ m, Shadow* __restrict__ wbf, float* __restrict__ mom1,
+    float* __restrict__ mom2, const float* __restrict__ act, const float* __restrict__ dO,
+    const float* __restrict__ err, int rows_pad, const int* __restrict__ epoch, int step,
+    AdamCfg c, float* __restrict__ grad, float* __restrict__ loss) {
+  __shared__ float part[JB][NCH][H];
+  const int bi = blockIdx.x, tid = threadIdx.x & (H - 1), ch = threadIdx.x >> 7;
+  const size_t plane = (size_t)rows_pad * H;
+  const int t = ADAM ? *epoch * c.steps_per_epoch + step + 1 : 0;  // 1-based step count
+  // kinds of block: layer weights, bias, output row, output bias + errors
+  const bool weights = bi < 3 * UB;
+  const int rest = bi - 3 * UB;
+  const int layer = weights ? bi / UB : rest;
+  const int j0 = weights ? (bi % UB) * JB : 0;
+  const int kin = weights && layer == 0 ? NF : H;
+  float g[JB];
+#pragma unroll
+  for (int q = 0; q < JB; ++q) g[q] = 0.f;
+  for (int b0 = 0; b0 < rows_pad; b0 += 32 * NCH) {
+    const int r = b0 + 32 * ch;
+    float p[JB];
+#pragma unroll
+    for (int q = 0; q < JB; ++q) p[q] = 0.f;
+    if (r < rows_pad && tid < kin) {
+      if (weights) {
+        const float* in = act + (ACT_X0 + layer) * plane + (size_t)r * H + tid;
+        const float* dz = act + (ACT_Z1 + layer) * plane + (size_t)r * H + j0;
+        static_assert(JB == 2, "two outputs per thread");
+#pragma unroll
+        for (int s = 0; s < 32; ++s) {
+          const float x = in[s * H];
+          const float2 d = *reinterpret_cast<const float2*>(dz + s * H);
+          p[0] = fmaf(d.x, x, p[0]);
+          p[1] = fmaf(d.y, x, p[1]);
+        }
+      } else if (rest < 3) {
+        const float* dz = act + (ACT_Z1 + layer) * plane + (size_t)r * H + tid;
+#pragma unroll
+        for (int s = 0; s < 32; ++s) p[0] += dz[s * H];
+      } else if (rest == 3) {
+        const float* in = act + ACT_A3 * plane + (size_t)r * H + tid;
+#pragma unroll
+        for (int s = 0; s < 32; ++s) p[0] = fmaf(dO[r + s], in[s * H], p[0]);
+      } else {
+        if (tid == 0) {
+#pragma unroll
+          for (int s = 0; s < 32; ++s) p[0] += dO[r + s];
+        }
+        if (tid < 32) {
+          const float e = err[r + tid];
+          float sq = e * e;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+          if (tid == 0) loss[r >> 5] = sq;
+        }
+      }
+    }
+    if (b0 > 0) __syncthreads();
+#pragma unroll
+    for (int q = 0; q < JB; ++q) part[q][ch][tid] = p[q];
+    __syncthreads();
+    if (ch < JB)
+      for (int k = 0; k < NCH && b0 + 32 * k < rows_pad; ++k) g[0] += part[ch][k][tid];
+  }
+  // thread (tid, ch < JB) holds the gradient of output j0 + ch
+  int i;
+  if (weights) {
+    if (ch >= JB || tid >= kin) return;
+    i = (layer == 0 ? OFF_W1 : (layer == 1 ? OFF_W2 : OFF_W3)) + (j0 + ch) * kin + tid;
+  } else {
+    if (ch > 0 || (rest == 4 && tid > 0)) return;
+    i = (rest == 0 ? OFF_B1 : rest == 1 ? OFF_B2 : rest == 2 ? OFF_B3 : rest == 3 ? OFF_W4 : OFF_B4) + tid;
+  }
+  i -= OFF_W1;
+  if constexpr (ADAM) adam(m, wbf, mom1, mom2, i, g[0], t, c);
+  else grad[i] = g[0];
 }
 
 // Mean loss of the epoch; advances the device epoch counter.
@@ -313,24 +439,6 @@ __global__ void __launch_bounds__(256) k_lambda_features(Problem pb, DeviceBuffe
   }
 }
 
-// Proposals of the batch's windows (W <= 32: one block) into d.prop; the
-// narrow search of each window starts from them (launch_search_hint).
-__global__ void __launch_bounds__(lam::H) k_lambda_propose(Problem pb, DeviceBuffers d) {
-  extern __shared__ float smraw[];
-  lam::Smem& sm = *reinterpret_cast<lam::Smem*>(smraw);
-  const float* m = d.model;
-  const __nv_bfloat16* wbf = (const __nv_bfloat16*)d.model_bf16;
-  const int ns = min(pb.W, lam::SB);
-  lam::load_inputs(m, d.feat, nullptr, 0, ns, sm);
-  lam::forward(m, wbf, sm);
-  if (threadIdx.x < ns) {
-    const int w = threadIdx.x;
-    const float y = sm.o[w] * m[lam::OFF_YSCALE] + m[lam::OFF_YMEAN];
-    d.prop[w] = y;
-    if (d.prop_out) d.prop_out[d.win0 + w] = y;
-  }
-}
-
 size_t lambda_smem() { return sizeof(lam::Smem); }
 
 cudaError_t launch_lambda_features(const Problem& pb, const DeviceBuffers& d, cudaStream_t s) {
@@ -338,67 +446,70 @@ cudaError_t launch_lambda_features(const Problem& pb, const DeviceBuffers& d, cu
   return cudaGetLastError();
 }
 
+// Proposals of the batch's windows into d.prop; the narrow search of each
+// window starts from them (launch_search_hint).
 cudaError_t launch_lambda_propose(const Problem& pb, const DeviceBuffers& d, cudaStream_t s) {
-  const size_t shm = lambda_smem();
-  cudaError_t e = cudaFuncSetAttribute(k_lambda_propose, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)shm);
-  if (e != cudaSuccess) return e;
-  k_lambda_propose<<<1, lam::H, shm, s>>>(pb, d);
+  lam::k_mlp_forward<<<(pb.W + lam::GS - 1) / lam::GS, lam::PT, lambda_smem(), s>>>(
+      d.model, (const lam::Shadow*)d.model_bf16, d.feat, pb.W, d.prop,
+      d.prop_out ? d.prop_out + d.win0 : nullptr);
   return cudaGetLastError();
 }
 
 // ---- training / inference launchers (device buffers)
 cudaError_t lambda_shadow(const float* m, void* wbf, cudaStream_t s) {
-  lam::k_mlp_shadow<<<64, 256, 0, s>>>(m, (__nv_bfloat16*)wbf);
+  lam::k_mlp_shadow<<<64, 256, 0, s>>>(m, (lam::Shadow*)wbf);
   return cudaGetLastError();
 }
+
+// blocks of a pass over n rows: at most two per SM (their shared memory)
+static int pass_blocks(int n) { return std::min((n + lam::GS - 1) / lam::GS, 2 * 152); }
+
+size_t lambda_rows(int n) { return ((size_t)n + 31) / 32 * 32; }
+size_t lambda_act_floats(int n) { return lambda_rows(n) * (lam::ACT_N * lam::H + 2); }
 
 cudaError_t lambda_forward(const float* m, const void* wbf, const float* feat, int n, float* y,
                            cudaStream_t s) {
-  const size_t shm = lambda_smem();
-  cudaError_t e = cudaFuncSetAttribute(lam::k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)shm);
-  if (e != cudaSuccess) return e;
-  lam::k_mlp_forward<<<(n + lam::SB - 1) / lam::SB, lam::H, shm, s>>>(
-      m, (const __nv_bfloat16*)wbf, feat, n, y);
+  lam::k_mlp_forward<<<pass_blocks(n), lam::PT, lambda_smem(), s>>>(
+      m, (const lam::Shadow*)wbf, feat, n, y, nullptr);
   return cudaGetLastError();
 }
 
+// Gradient over n samples: act holds lambda_act_floats(n) floats, part_loss
+// the squared error of each 32 samples.
 cudaError_t lambda_grad(const float* m, const void* wbf, const float* feat, const float* target,
-                        int n, float* part, float* part_loss, float* grad, cudaStream_t s) {
-  const size_t shm = lambda_smem();
-  cudaError_t e = cudaFuncSetAttribute(lam::k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)shm);
-  if (e != cudaSuccess) return e;
-  const int nblk = (n + lam::SB - 1) / lam::SB;
-  lam::k_mlp_grad<<<nblk, lam::H, shm, s>>>(m, (const __nv_bfloat16*)wbf, feat, target, nullptr,
-                                            nullptr, 0, 0, n, 1.f / (float)n, part, part_loss);
-  lam::k_mlp_gsum<<<(lam::NPARAM + 255) / 256, 256, 0, s>>>(part, nblk, grad);
+                        int n, float* act, float* part_loss, float* grad, cudaStream_t s) {
+  const int rp = (int)lambda_rows(n);
+  float* dO = act + (size_t)rp * lam::ACT_N * lam::H;
+  lam::k_mlp_pass<<<pass_blocks(rp), lam::PT, lambda_smem(), s>>>(
+      m, (const lam::Shadow*)wbf, feat, target, nullptr, nullptr, 0, 0, n, rp, 1.f / (float)n, act,
+      dO, dO + rp);
+  lam::k_mlp_update<false><<<lam::kUpdateBlocks, lam::H * lam::NCH, 0, s>>>(
+      nullptr, nullptr, nullptr, nullptr, act, dO, dO + rp, rp, nullptr, 0, lam::AdamCfg{}, grad,
+      part_loss);
   return cudaGetLastError();
 }
 
 cudaError_t lambda_attrs() {
   const int shm = (int)lambda_smem();
-  cudaError_t e = cudaFuncSetAttribute(lam::k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
+  cudaError_t e = cudaFuncSetAttribute(lam::k_mlp_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(lam::k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_lambda_propose, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
   return e;
 }
 
 // One epoch of training (stream-capturable: launches only; lambda_attrs()
 // must have run).
 cudaError_t lambda_train_epoch(const LambdaTrain& t, cudaStream_t s) {
-  const size_t shm = lambda_smem();
-  const int nblk = t.batch / lam::SB;
+  const int nblk = t.batch / 32;
+  float* dO = t.act + (size_t)t.batch * lam::ACT_N * lam::H;
   lam::AdamCfg c{t.lr, t.lr_final, t.wd, t.b1, t.b2, t.eps, t.steps, t.total_steps};
   for (int st = 0; st < t.steps; ++st) {
-    lam::k_mlp_grad<<<nblk, lam::H, shm, s>>>(
-        t.m, (const __nv_bfloat16*)t.wbf, t.feat, t.target, t.perm, t.epoch, t.n, st * t.batch,
-        t.n, 1.f / (float)t.batch, t.part, t.loss_acc + (size_t)st * nblk);
-    lam::k_mlp_adam<<<(lam::NPARAM + 255) / 256, 256, 0, s>>>(t.m, (__nv_bfloat16*)t.wbf, t.mom1,
-                                                            t.mom2, t.part, nblk, t.epoch, st, c);
+    lam::k_mlp_pass<<<pass_blocks(t.batch), lam::PT, lambda_smem(), s>>>(
+        t.m, (const lam::Shadow*)t.wbf, t.feat, t.target, t.perm, t.epoch, t.n, st * t.batch,
+        t.n, t.batch, 1.f / (float)t.batch, t.act, dO, dO + t.batch);
+    lam::k_mlp_update<true><<<lam::kUpdateBlocks, lam::H * lam::NCH, 0, s>>>(
+        t.m, (lam::Shadow*)t.wbf, t.mom1, t.mom2, t.act, dO, dO + t.batch, t.batch, t.epoch, st, c,
+        nullptr, t.loss_acc + (size_t)st * nblk);
   }
   lam::k_mlp_epoch_end<<<1, 32, 0, s>>>(t.loss_acc, t.steps, nblk, t.steps * t.batch, t.epoch,
                                         t.epoch_loss);

@@ -281,6 +281,7 @@ cudaError_t launch_hot_pixel(uint16_t* seq, int nr, int nc, int nimg, double thr
                              uint32_t* med, uint32_t* madm, cudaStream_t s);
 
 // learned lambda proposal (lambda.cu)
+constexpr size_t PGSVT_LAMBDA_SHADOW_BYTES = 88704;  // bf16 shadow of the weights
 struct LambdaTrain {
   float* m;            // FP32 model (PGSVT_LAMBDA_MODEL_FLOATS)
   void* wbf;           // bf16 shadow
@@ -289,7 +290,7 @@ struct LambdaTrain {
   const float* target; // [n]
   const int32_t* perm; // [epochs][n] sample order
   int* epoch;          // device epoch counter
-  float* part;         // [batch/32][PGSVT_LAMBDA_PARAMS] gradient partials
+  float* act;          // lambda_act_floats(batch): the rows of a pass
   float* loss_acc;     // [steps][batch/32]
   float* epoch_loss;   // [epochs]
   int n, batch, steps, total_steps;
@@ -302,7 +303,8 @@ cudaError_t lambda_shadow(const float* m, void* wbf, cudaStream_t s);
 cudaError_t lambda_forward(const float* m, const void* wbf, const float* feat, int n, float* y,
                            cudaStream_t s);
 cudaError_t lambda_grad(const float* m, const void* wbf, const float* feat, const float* target,
-                        int n, float* part, float* part_loss, float* grad, cudaStream_t s);
+                        int n, float* act, float* part_loss, float* grad, cudaStream_t s);
+size_t lambda_act_floats(int n);
 cudaError_t lambda_train_epoch(const LambdaTrain& t, cudaStream_t s);
 cudaError_t lambda_attrs();
 

@@ -19,3 +19,21 @@ def test_hot_pixel_wavefront(capi, oracle, nr, nc, thr):
     a[rng.random(a.shape) < 0.02] = 65535
     a = np.asfortranarray(a)
     np.testing.assert_array_equal(capi.hot_pixel_filter(a, thr), oracle.hot_pixel_filter(a, thr))
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 32, 33, 255, 256, 257, 2500])
+def test_mlp_gradient_rows(capi, pkg, oracle, n):
+    """Groups of 4 samples, chains of 32 rows, 8 chains at a time and more
+    groups than blocks; the tolerances are those of the fixed-size test."""
+    import lambda_mlp as lm
+    rng = np.random.default_rng(n)
+    f = rng.normal(size=(max(n, 2), 67)).astype(np.float32)
+    t = rng.uniform(-6, 0, max(n, 2)).astype(np.float32)
+    m = pkg.learned.init_model(f, t, seed=n)
+    f, t = f[:n], t[:n]
+    loss, g = capi.lambda_grad(m, f, t)
+    loss0, g0 = lm.loss_and_grad(m, f, t)
+    assert abs(loss - loss0) <= 1e-5 * loss0
+    assert np.abs(g - g0).max() <= 1e-4 * np.abs(g0).max()
+    y0 = lm.predict(m, f)
+    assert np.abs(capi.lambda_predict(m, f) - y0).max() <= 1e-4 * (1 + np.abs(y0).max())
