@@ -182,7 +182,7 @@ struct DeviceBuffers {
   float* sv;
   float* hv;
   float* xq;               // split SVD forms' scratch: [items][NC][X rows] (svd_split.cu)
-  float* xqn;              // its column norms [items][NC]
+  float* xqn;              // surviving triplets of each item (ints; [items])
   int32_t* nlive0;         // [W][NP] singular triplets of copy 0 that can survive
   void* acc;               // [W][K][nwin][S*S] int32 or int64 fixed point
   double* part_lin;        // [W][K][nblk_eval]

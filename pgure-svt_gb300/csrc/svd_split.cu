@@ -15,8 +15,8 @@
 //             reflections in a runtime loop; X = R^T to a scratch array
 //   k_xsweep  4 lanes x (NC/4) rows per patch, eight patches per warp: the
 //             register-form Jacobi sweeps of svd_kernel.cuh (same rotations,
-//             same convergence rules) on X; rotated columns and their norms
-//             back to the scratch
+//             same convergence rules) on X; the singular values, sorted, and
+//             the rotated columns that can survive back to the scratch
 //   k_qr_out  16 lanes x 4 rows per patch: u_t = B v_t / s_t, the stored
 //             factors and the risk projections h_t = u_t^T G v_t.
 //
@@ -101,7 +101,7 @@ __device__ __forceinline__ float half_sum(float v) {  // over the 16 lanes of a 
   return v;
 }
 
-// ---- TMA staging of frame tiles (k_bout<NC, true>)
+// ---- TMA staging of frame tiles (k_bout_tma)
 //
 // The 32 patches of a factors block are 8 x 4 neighbouring grid positions
 // (the tile order of the kept patches), so in every slice of the window their
@@ -238,6 +238,105 @@ __global__ void __launch_bounds__(128) k_qr(Problem pb, DeviceBuffers d, int nit
   }
 }
 
+// ---- end of a sweep kernel: the column norms (the singular values) of one
+// patch per lane group, sorted, and the rotated columns of the triplets that
+// can survive the threshold, in that order: xq [item][rank][XR], the count in
+// xqn [item].  Lane q takes columns 4n + q: their sums come from a
+// reduce-scatter (the lanes added in lanes_sum's order), their ranks from
+// comparisons with every column (ties by index); sorting in the factors
+// kernels took more instructions there than the factors themselves.  `get`:
+// this lane's row r of column k; `slot`: the lane group's scratch (32 floats).
+template <int NC, int RX, int XR, class Get>
+__device__ __forceinline__ void store_sorted(const Problem& pb, const DeviceBuffers& d, Get get,
+                                             float* slot, int q, int gid, bool live) {
+  constexpr int N4 = (NC + 3) / 4;
+  const Geometry& g = pb.g;
+  const int gbase = (threadIdx.x & 31) & ~3;
+  const bool b0 = (q & 1) != 0, b1 = (q & 2) != 0;
+  float s[N4];
+  float smax = 0.f;
+#pragma unroll
+  for (int n = 0; n < N4; ++n) {
+    float t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int k = 4 * n + j;
+      t[j] = 0.f;
+      if (k < NC - 1)
+#pragma unroll
+        for (int r = 0; r < RX; ++r) t[j] = fmaf(get(r, k), get(r, k), t[j]);
+    }
+    const float u0 = (b0 ? t[1] : t[0]) + __shfl_xor_sync(0xffffffffu, b0 ? t[0] : t[1], 1);
+    const float u1 = (b0 ? t[3] : t[2]) + __shfl_xor_sync(0xffffffffu, b0 ? t[2] : t[3], 1);
+    s[n] = sqrtf((b1 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b1 ? u0 : u1, 2));
+    smax = fmaxf(smax, s[n]);
+  }
+  smax = fmaxf(smax, __shfl_xor_sync(0xffffffffu, smax, 1));
+  smax = fmaxf(smax, __shfl_xor_sync(0xffffffffu, smax, 2));
+  int p = 0, c = 0, w = 0;
+  if (live) {
+    p = gid % g.NP;
+    const int r = gid / g.NP;
+    c = r % d.ncopies;
+    w = r / d.ncopies;
+  }
+  const float upper = (float)d.wc[w].upper;
+  int nl = 0, rank[N4];
+#pragma unroll
+  for (int n = 0; n < N4; ++n) {
+    nl += 4 * n + q < NC && can_survive(pb, s[n], smax, upper);
+    rank[n] = 0;
+  }
+  nl += __shfl_xor_sync(0xffffffffu, nl, 1);
+  nl += __shfl_xor_sync(0xffffffffu, nl, 2);
+#pragma unroll
+  for (int j = 0; j < NC; ++j) {
+    const float sj = __shfl_sync(0xffffffffu, s[j >> 2], gbase | (j & 3));
+#pragma unroll
+    for (int n = 0; n < N4; ++n) rank[n] += sj > s[n] || (sj == s[n] && j < 4 * n + q);
+  }
+  __syncwarp();
+  int* ir = reinterpret_cast<int*>(slot + 16);
+#pragma unroll
+  for (int n = 0; n < N4; ++n)
+    if (4 * n + q < NC) {
+      slot[rank[n]] = s[n];
+      ir[4 * n + q] = rank[n];
+    }
+  __syncwarp();
+  if (live) {
+    const size_t NP = g.NP;
+    float* svo = d.sv + (((size_t)w * 4 + c) * g.NC) * NP + p;
+    float* hvo = d.hv + (((size_t)w * 4 + c) * g.NC) * NP + p;
+#pragma unroll
+    for (int n = 0; n < N4; ++n) {
+      const int t = 4 * n + q;
+      if (t < NC) {
+        svo[(size_t)t * NP] = slot[t];
+        if (t >= nl) hvo[(size_t)t * NP] = 0.f;
+      }
+    }
+    if (q == 0) {
+      reinterpret_cast<int*>(d.xqn)[gid] = nl;
+      if (c == 0) d.nlive0[(size_t)w * NP + p] = nl;
+    }
+    float* xo = d.xq + (size_t)gid * NC * XR + q * RX;
+#pragma unroll
+    for (int k = 0; k < NC - 1; ++k) {
+      const int t = ir[k];
+      if (t >= nl) continue;
+      if constexpr (RX == 4) {
+        *reinterpret_cast<float4*>(xo + t * XR) =
+            make_float4(get(0, k), get(1, k), get(2, k), get(3, k));
+      } else {
+#pragma unroll
+        for (int r = 0; r < RX; ++r) xo[t * XR + r] = get(r, k);
+      }
+    }
+  }
+  __syncwarp();
+}
+
 // ---- Jacobi sweeps on X, four lanes per patch, eight patches per warp
 template <int NC>
 __global__ void __launch_bounds__(128, 4) k_xsweep(Problem pb, DeviceBuffers d, int nitems) {
@@ -259,40 +358,30 @@ __global__ void __launch_bounds__(128, 4) k_xsweep(Problem pb, DeviceBuffers d, 
   const int sweeps = register_sweeps<RX, 4, NC, CS, 1>(A, X, q, pb.g.nwin, fp64_tests);
   if (lane == 0) atomicAdd(d.counters + 1, (unsigned long long)(sweeps + 1));
   if (q == 0 && fp64_tests) atomicAdd(d.counters + 2, (unsigned long long)fp64_tests);
-  // column norms (the singular values), then the rotated columns of those
-  // triplets that can survive the threshold (the only ones k_qr_out reads)
-  float sv[NC];
-#pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    float t = 0.f;
-#pragma unroll
-    for (int r = 0; r < RX; ++r) t = fmaf(A(r, k), A(r, k), t);
-    sv[k] = sqrtf(lanes_sum<4>(t));  // every lane takes part
-  }
-  if (!live) return;
-  float smax = sv[0];
-#pragma unroll
-  for (int k = 1; k < NC; ++k) smax = fmaxf(smax, sv[k]);
-  const float upper = (float)d.wc[(gid / pb.g.NP) / d.ncopies].upper;
-  float* xo = d.xq + (size_t)gid * NC * D::XR;
-#pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    if (q == 0) d.xqn[(size_t)gid * NC + k] = sv[k];
-    if (can_survive(pb, sv[k], smax, upper))
-#pragma unroll
-      for (int r = 0; r < RX; ++r) xo[k * D::XR + q * RX + r] = A(r, k);
-  }
+  store_sorted<NC, RX, D::XR>(pb, d, [&](int r, int k) { return A(r, k); }, X, q, gid, live);
 }
 
-// ---- the factors: u_t = B v_t / s_t, h_t = u_t^T G v_t, sorted by s
+// ---- the factors: u_t = B v_t / s_t, h_t = u_t^T G v_t, for the nl triplets
+// that can survive (already sorted, see store_sorted).  Few of them can (about
+// 5 of 15 at 8 x 8 patches), so up to kQT are formed side by side while one
+// slice of B, then of G, is in registers: nothing is held across slices and
+// the loads of many warps overlap.  256 x 256 x 24, 8 x 8 patches, GB300: 56.2 ->
+// 22.6 ms in 3 launches (before, B held in registers and the columns sorted here).
+constexpr int kQT = 8;
+
 template <int NC>
-__global__ void __launch_bounds__(128) k_qr_out(Problem pb, DeviceBuffers d, int nitems) {
+__global__ void __launch_bounds__(128, 5) k_qr_out(Problem pb, DeviceBuffers d, int nitems) {
   using D = QrDims<NC>;
   const Geometry& g = pb.g;
   const int lane = threadIdx.x & 31, l16 = lane & (kQL - 1);
-  const int gid = blockIdx.x * 8 + (threadIdx.x >> 4);
+  const int slot = threadIdx.x >> 4;
+  const int gid = blockIdx.x * 8 + slot;
   const bool live = gid < nitems;
   const int nwin = g.nwin, M = g.M;
+  __shared__ __align__(16) float Vs[8][NC][kQT];  // v_t of the triplets at hand
+  const int nl = live ? reinterpret_cast<const int*>(d.xqn)[gid] : 0;
+  const int nl_max = max(nl, __shfl_xor_sync(0xffffffffu, nl, 16));
+  if (nl_max == 0) return;  // warp-uniform
   int p, c, w;
   {
     const int gg = live ? gid : 0;
@@ -301,7 +390,6 @@ __global__ void __launch_bounds__(128) k_qr_out(Problem pb, DeviceBuffers d, int
     c = r % d.ncopies;
     w = r / d.ncopies;
   }
-  const WinConst& wc = d.wc[w];
   const float* X = d.xq + (size_t)(live ? gid : 0) * NC * D::XR;
   int roff[kQR];
 #pragma unroll
@@ -309,96 +397,97 @@ __global__ void __launch_bounds__(128) k_qr_out(Problem pb, DeviceBuffers d, int
     const int e = l16 * kQR + r;
     roff[r] = e < M ? (e % g.bs) + (e / g.bs) * g.S : -1;
   }
-  float sv[NC];
-#pragma unroll
-  for (int k = 0; k < NC; ++k) sv[k] = live ? __ldg(d.xqn + (size_t)gid * NC + k) : 0.f;
-  float smax = sv[0];
-#pragma unroll
-  for (int k = 1; k < NC; ++k) smax = fmaxf(smax, sv[k]);
   const size_t NP = g.NP;
   const int NCg = g.NC;
-  float* svo = d.sv + (((size_t)w * 4 + c) * NCg) * NP + p;
+  const float* svo = d.sv + (((size_t)w * 4 + c) * NCg) * NP + p;
   float* hvo = d.hv + (((size_t)w * 4 + c) * NCg) * NP + p;
-  int nl = 0;
-#pragma unroll
-  for (int k = 0; k < NC; ++k) nl += can_survive(pb, sv[k], smax, (float)wc.upper);
-  int nl_max = nl;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) nl_max = max(nl_max, __shfl_xor_sync(0xffffffffu, nl_max, o));
-  if (c == 0 && live && l16 == 0) d.nlive0[(size_t)w * NP + p] = nl;
   const float* fld = (c == 0) ? d.fld0 : (c == 3 ? d.fld1 : d.fld2);
   const float* fw_ = (pb.optimize && fld) ? fld + (size_t)w * g.cube() : nullptr;
   PatchSrc src;
   src.init(pb, d, p, c, w);
-  float B[kQR][NC];
+  const bool keep = c == 0 && live && d.U0 && d.V0;
+  for (int t0 = 0; t0 < nl_max; t0 += kQT) {
+    const int nt = min(kQT, nl_max - t0);  // warp-uniform
+    float inv[kQT];
+    __syncwarp();
 #pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    const bool colok = live && k < nwin && nl_max > 0;
-    const size_t b = colok ? src.base(k) : 0;
-#pragma unroll
-    for (int r = 0; r < kQR; ++r)
-      B[r][k] = (colok && roff[r] >= 0) ? src.value(b + roff[r]) : 0.f;
-  }
-  int prev = -1;
-  float prev_s = INFINITY;
-  for (int t = 0; t < NC; ++t) {
-    // next column in decreasing singular-value order (ties by index)
-    int ct = 0;
-    float st = -1.f;
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      const float sk = sv[k];
-      const bool after = (sk < prev_s) || (sk == prev_s && k > prev);
-      if (after && (sk > st)) {
-        st = sk;
-        ct = k;
+    for (int t = 0; t < kQT; ++t) {
+      inv[t] = 0.f;
+      if (t < nt) {
+        const float st = t0 + t < nl ? svo[(size_t)(t0 + t) * NP] : 0.f;
+        inv[t] = st > 0.f ? 1.f / st : 0.f;
+        // v_t = X's rotated column t times inv
+        if (l16 < NC) {
+          const float v = (t0 + t < nl && l16 < nwin) ? X[(t0 + t) * D::XR + l16] * inv[t] : 0.f;
+          Vs[slot][l16][t] = v;
+          if (keep && t0 + t < nl && l16 < nwin)
+            d.V0[(((size_t)w * NCg + t0 + t) * nwin + l16) * NP + p] = v;
+        }
+      } else if (l16 < NC) {
+        Vs[slot][l16][t] = 0.f;
       }
     }
-    prev = ct;
-    prev_s = st;
-    const bool use = t < nl;
-    if (live && l16 == 0) {
-      svo[(size_t)t * NP] = st;
-      if (!use) hvo[(size_t)t * NP] = 0.f;
+    __syncwarp();
+    float a[kQT][kQR];  // u_t rows
+#pragma unroll
+    for (int t = 0; t < kQT; ++t)
+#pragma unroll
+      for (int r = 0; r < kQR; ++r) a[t][r] = 0.f;
+#pragma unroll 3
+    for (int k = 0; k < nwin; ++k) {
+      float B[kQR];
+      const size_t b = live ? src.base(k) : 0;
+#pragma unroll
+      for (int r = 0; r < kQR; ++r) B[r] = (live && roff[r] >= 0) ? src.value(b + roff[r]) : 0.f;
+      float v[kQT];
+#pragma unroll
+      for (int t = 0; t < kQT; t += 4)
+        *reinterpret_cast<float4*>(v + t) = *reinterpret_cast<const float4*>(&Vs[slot][k][t]);
+#pragma unroll
+      for (int t = 0; t < kQT; ++t)
+        if (t < nt)
+#pragma unroll
+          for (int r = 0; r < kQR; ++r) a[t][r] = fmaf(B[r], v[t], a[t][r]);
     }
-    if (t >= nl_max) continue;  // warp-uniform
-    const float inv = st > 0.f ? 1.f / st : 0.f;
-    const float* xc = X + ct * D::XR;  // v_t = X's rotated column ct times inv
-    float a[kQR];                      // u_t rows
 #pragma unroll
-    for (int r = 0; r < kQR; ++r) a[r] = 0.f;
+    for (int t = 0; t < kQT; ++t) {
 #pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      const float vk = (live && k < nwin) ? __ldg(xc + k) * inv : 0.f;
-#pragma unroll
-      for (int r = 0; r < kQR; ++r) a[r] = fmaf(B[r][k], vk, a[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < kQR; ++r) a[r] *= inv;
-    if (c == 0 && live && use && d.U0 && d.V0) {
-#pragma unroll
-      for (int r = 0; r < kQR; ++r)
-        if (roff[r] >= 0) d.U0[(((size_t)w * NCg + t) * g.M + l16 * kQR + r) * NP + p] = a[r];
-      if (l16 < nwin)
-        d.V0[(((size_t)w * NCg + t) * nwin + l16) * NP + p] = __ldg(xc + l16) * inv;
+      for (int r = 0; r < kQR; ++r) {
+        a[t][r] *= inv[t];
+        if (keep && t0 + t < nl && roff[r] >= 0)
+          d.U0[(((size_t)w * NCg + t0 + t) * g.M + l16 * kQR + r) * NP + p] = a[t][r];
+      }
     }
     if (fw_) {
       // h_t = sum_k v_k (G_k . u_t): the lanes' partial sums, one reduction
-      float h = 0.f;
-      if (live && use) {
+      float h[kQT];
 #pragma unroll
-        for (int k = 0; k < NC; ++k) {
-          if (k >= nwin) break;
-          const size_t b = src.base(k);
-          float gu = 0.f;
+      for (int t = 0; t < kQT; ++t) h[t] = 0.f;
+#pragma unroll 3
+      for (int k = 0; k < nwin; ++k) {
+        float G[kQR];
+        const size_t b = live ? src.base(k) : 0;
 #pragma unroll
-          for (int r = 0; r < kQR; ++r)
-            if (roff[r] >= 0) gu = fmaf(__ldg(fw_ + b + roff[r]), a[r], gu);
-          h = fmaf(__ldg(xc + k) * inv, gu, h);
-        }
+        for (int r = 0; r < kQR; ++r) G[r] = (live && roff[r] >= 0) ? __ldg(fw_ + b + roff[r]) : 0.f;
+        float v[kQT];
+#pragma unroll
+        for (int t = 0; t < kQT; t += 4)
+          *reinterpret_cast<float4*>(v + t) = *reinterpret_cast<const float4*>(&Vs[slot][k][t]);
+#pragma unroll
+        for (int t = 0; t < kQT; ++t)
+          if (t < nt) {
+            float gu = 0.f;
+#pragma unroll
+            for (int r = 0; r < kQR; ++r) gu = fmaf(G[r], a[t][r], gu);
+            h[t] = fmaf(v[t], gu, h[t]);
+          }
       }
-      h = half_sum(h);
-      if (live && use && l16 == 0) hvo[(size_t)t * NP] = h;
+#pragma unroll
+      for (int t = 0; t < kQT; ++t)
+        if (t < nt) {
+          const float hs = half_sum(h[t]);
+          if (live && t0 + t < nl && l16 == 0) hvo[(size_t)(t0 + t) * NP] = hs;
+        }
     }
   }
 }
@@ -419,16 +508,11 @@ __global__ void __launch_bounds__(128, 4) k_bsweep(Problem pb, DeviceBuffers d, 
   const int nwin = g.nwin, M = g.M;
   __shared__ float Xs[32][NC * CS];
   float* X = Xs[slot];
-  int p, c, w;
-  {
-    const int gg = live ? gid : 0;
-    p = gg % g.NP;
-    const int r = gg / g.NP;
-    c = r % d.ncopies;
-    w = r / d.ncopies;
-  }
   PatchSrc src;
-  src.init(pb, d, p, c, w);
+  {
+    const int gg = live ? gid : 0, r = gg / g.NP;
+    src.init(pb, d, gg % g.NP, r % d.ncopies, r / d.ncopies);
+  }
   int roff[RX];
 #pragma unroll
   for (int r = 0; r < RX; ++r) {
@@ -447,34 +531,112 @@ __global__ void __launch_bounds__(128, 4) k_bsweep(Problem pb, DeviceBuffers d, 
   const int sweeps = register_sweeps<RX, 4, NC, CS, 1>(A, X, q, nwin, fp64_tests);
   if (lane == 0) atomicAdd(d.counters + 1, (unsigned long long)(sweeps + 1));
   if (q == 0 && fp64_tests) atomicAdd(d.counters + 2, (unsigned long long)fp64_tests);
-  // column norms (the singular values), then the rotated columns of those
-  // triplets that can survive the threshold (the only ones k_bout reads)
-  float sv[NC];
-#pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    float t = 0.f;
-#pragma unroll
-    for (int r = 0; r < RX; ++r) t = fmaf(A(r, k), A(r, k), t);
-    sv[k] = sqrtf(lanes_sum<4>(t));  // every lane takes part
+  store_sorted<NC, RX, XR>(pb, d, [&](int r, int k) { return A(r, k); }, X, q, gid, live);
+}
+
+// The factors of the nl triplets that can survive (already sorted, see
+// store_sorted): one or two of 15 as a rule, so up to kBT are formed side by
+// side while one slice of B and G is in registers.  Nothing is held across
+// slices (the earlier form kept all of B and G, at 16 warps per SM, and was
+// bound by the latency of its loads and by sorting the columns).  256 x 256 x
+// 100, GB300: 35.0 -> 15.1 ms in 13 launches, still bound by the latency of the
+// gathers.
+constexpr int kBT = 4;
+
+template <int NC>
+__global__ void __launch_bounds__(128, 8) k_bout(Problem pb, DeviceBuffers d, int nitems) {
+  constexpr int RX = 4, XR = 16;
+  const Geometry& g = pb.g;
+  const int lane = threadIdx.x & 31, q = lane & 3;
+  const int gid = blockIdx.x * 32 + (threadIdx.x >> 2);
+  const bool live = gid < nitems;
+  const int nwin = g.nwin, M = g.M;
+  const int nl = live ? reinterpret_cast<const int*>(d.xqn)[gid] : 0;
+  const int nl_max = __reduce_max_sync(0xffffffffu, nl);
+  if (nl_max == 0) return;  // warp-uniform
+  int p, c, w;
+  {
+    const int gg = live ? gid : 0;
+    p = gg % g.NP;
+    const int r = gg / g.NP;
+    c = r % d.ncopies;
+    w = r / d.ncopies;
   }
-  if (!live) return;
-  float smax = sv[0];
+  const float* X = d.xq + (size_t)(live ? gid : 0) * NC * XR + q * RX;
+  int roff[RX];
 #pragma unroll
-  for (int k = 1; k < NC; ++k) smax = fmaxf(smax, sv[k]);
-  const float upper = (float)d.wc[w].upper;
-  float* xo = d.xq + (size_t)gid * NC * XR;
+  for (int r = 0; r < RX; ++r) {
+    const int e = q * RX + r;
+    roff[r] = (live && e < M) ? (e % g.bs) + (e / g.bs) * g.S : -1;
+  }
+  const size_t NP = g.NP;
+  const int NCg = g.NC;
+  const float* svo = d.sv + (((size_t)w * 4 + c) * NCg) * NP + p;
+  float* hvo = d.hv + (((size_t)w * 4 + c) * NCg) * NP + p;
+  const float* fld = (c == 0) ? d.fld0 : (c == 3 ? d.fld1 : d.fld2);
+  const float* fw_ = (pb.optimize && fld) ? fld + (size_t)w * g.cube() : nullptr;
+  PatchSrc src;
+  src.init(pb, d, p, c, w);
+  const bool keep = c == 0 && live && d.U0 && d.V0;
+  for (int t0 = 0; t0 < nl_max; t0 += kBT) {
+    const int nt = min(kBT, nl_max - t0);  // warp-uniform
+    float a[kBT][RX], inv[kBT], h[kBT];    // u_t rows, 1 / s_t
 #pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    if (q == 0) d.xqn[(size_t)gid * NC + k] = sv[k];
-    if (can_survive(pb, sv[k], smax, upper))
+    for (int t = 0; t < kBT; ++t) {
+      const bool use = t0 + t < nl;
+      const float st = use ? svo[(size_t)(t0 + t) * NP] : 0.f;
+      inv[t] = st > 0.f ? 1.f / st : 0.f;
+      const float4 x = use ? *reinterpret_cast<const float4*>(X + (t0 + t) * XR)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float* xp = &x.x;
+      h[t] = 0.f;
 #pragma unroll
-      for (int r = 0; r < RX; ++r) xo[k * XR + q * RX + r] = A(r, k);
+      for (int r = 0; r < RX; ++r) {
+        a[t][r] = xp[r] * inv[t];
+        if (keep && use && roff[r] >= 0)
+          d.U0[(((size_t)w * NCg + t0 + t) * g.M + q * RX + r) * NP + p] = a[t][r];
+      }
+    }
+    // v_t = B^T u_t / s_t and h_t = u_t^T G v_t = sum_k v_k (G_k . u_t)
+#pragma unroll 3
+    for (int k = 0; k < nwin; ++k) {
+      const size_t b = live ? src.base(k) : 0;
+      float B[RX], G[RX];
+#pragma unroll
+      for (int r = 0; r < RX; ++r) {
+        B[r] = roff[r] >= 0 ? src.value(b + roff[r]) : 0.f;
+        G[r] = fw_ && roff[r] >= 0 ? __ldg(fw_ + b + roff[r]) : 0.f;
+      }
+#pragma unroll
+      for (int t = 0; t < kBT; ++t) {
+        if (t >= nt) break;
+        float bu = 0.f;
+#pragma unroll
+        for (int r = 0; r < RX; ++r) bu = fmaf(B[r], a[t][r], bu);
+        const float vk = lanes_sum<4>(bu) * inv[t];
+        if (keep && t0 + t < nl && (k & 3) == q)
+          d.V0[(((size_t)w * NCg + t0 + t) * nwin + k) * NP + p] = vk;
+        float gu = 0.f;
+#pragma unroll
+        for (int r = 0; r < RX; ++r) gu = fmaf(G[r], a[t][r], gu);
+        h[t] = fmaf(vk, gu, h[t]);
+      }
+    }
+    if (fw_) {
+#pragma unroll
+      for (int t = 0; t < kBT; ++t)
+        if (t < nt) {
+          const float hs = lanes_sum<4>(h[t]);
+          if (live && t0 + t < nl && q == 0) hvo[(size_t)(t0 + t) * NP] = hs;
+        }
+    }
   }
 }
 
-template <int NC, bool TMA>
+// The same from TMA-staged frame tiles (see above).
+template <int NC>
 __global__ void __launch_bounds__(128, 4)
-    k_bout(Problem pb, DeviceBuffers d, int nitems, const __grid_constant__ BoutMaps tm) {
+    k_bout_tma(Problem pb, DeviceBuffers d, int nitems, const __grid_constant__ BoutMaps tm) {
   constexpr int RX = 4, XR = 16;
   const Geometry& g = pb.g;
   const int lane = threadIdx.x & 31, q = lane & 3;
@@ -489,7 +651,6 @@ __global__ void __launch_bounds__(128, 4)
     c = r % d.ncopies;
     w = r / d.ncopies;
   }
-  const WinConst& wc = d.wc[w];
   const float* X = d.xq + (size_t)(live ? gid : 0) * NC * XR;
   int roff[RX];
 #pragma unroll
@@ -497,50 +658,21 @@ __global__ void __launch_bounds__(128, 4)
     const int e = q * RX + r;
     roff[r] = (live && e < M) ? (e % g.bs) + (e / g.bs) * g.S : -1;
   }
-  float sv[NC];
-#pragma unroll
-  for (int k = 0; k < NC; ++k) sv[k] = live ? __ldg(d.xqn + (size_t)gid * NC + k) : 0.f;
-  float smax = sv[0];
-#pragma unroll
-  for (int k = 1; k < NC; ++k) smax = fmaxf(smax, sv[k]);
   const size_t NP = g.NP;
   const int NCg = g.NC;
-  float* svo = d.sv + (((size_t)w * 4 + c) * NCg) * NP + p;
+  const float* svo = d.sv + (((size_t)w * 4 + c) * NCg) * NP + p;
   float* hvo = d.hv + (((size_t)w * 4 + c) * NCg) * NP + p;
-  int nl = 0;
-#pragma unroll
-  for (int k = 0; k < NC; ++k) nl += can_survive(pb, sv[k], smax, (float)wc.upper);
-  int nl_max = nl;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) nl_max = max(nl_max, __shfl_xor_sync(0xffffffffu, nl_max, o));
-  if (c == 0 && live && q == 0) d.nlive0[(size_t)w * NP + p] = nl;
+  const int nl = live ? reinterpret_cast<const int*>(d.xqn)[gid] : 0;
+  const int nl_max = __reduce_max_sync(0xffffffffu, nl);
   const float* fld = (c == 0) ? d.fld0 : (c == 3 ? d.fld1 : d.fld2);
   const float* fw_ = (pb.optimize && fld) ? fld + (size_t)w * g.cube() : nullptr;
   PatchSrc src;
   src.init(pb, d, p, c, w);
-  // B again and, in shared memory, this lane's rows of the field G along the
-  // trajectory (each lane reads back only what it wrote)
+  // B in registers and, in shared memory, this lane's rows of the field G along
+  // the trajectory (each lane reads back only what it wrote)
   float B[RX][NC];
   float* gs;
-  if constexpr (!TMA) {
-    __shared__ __align__(16) float Gs[32][NC][4 * RX];
-    gs = &Gs[threadIdx.x >> 2][0][q * RX];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      const bool colok = live && k < nwin && nl_max > 0;
-      const size_t b = colok ? src.base(k) : 0;
-#pragma unroll
-      for (int r = 0; r < RX; ++r) B[r][k] = (colok && roff[r] >= 0) ? src.value(b + roff[r]) : 0.f;
-      if (fw_) {
-        float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        float* gp = &g4.x;
-#pragma unroll
-        for (int r = 0; r < RX; ++r)
-          if (colok && roff[r] >= 0) gp[r] = __ldg(fw_ + b + roff[r]);
-        *reinterpret_cast<float4*>(gs + k * 4 * RX) = g4;
-      }
-    }
-  } else {
+  {
     // dynamic shared memory: [Gs (padded rows) | field tiles]; the window
     // and probe tiles share the Gs region, which is written only after
     // every lane has assembled B
@@ -683,33 +815,13 @@ __global__ void __launch_bounds__(128, 4)
       }
     }
   }
-  int prev = -1;
-  float prev_s = INFINITY;
-  for (int t = 0; t < NC; ++t) {
-    // next column in decreasing singular-value order (ties by index)
-    int ct = 0;
-    float st = -1.f;
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      const float sk = sv[k];
-      const bool after = (sk < prev_s) || (sk == prev_s && k > prev);
-      if (after && (sk > st)) {
-        st = sk;
-        ct = k;
-      }
-    }
-    prev = ct;
-    prev_s = st;
+  for (int t = 0; t < nl_max; ++t) {
     const bool use = t < nl;
-    if (live && q == 0) {
-      svo[(size_t)t * NP] = st;
-      if (!use) hvo[(size_t)t * NP] = 0.f;
-    }
-    if (t >= nl_max) continue;  // warp-uniform
+    const float st = use ? svo[(size_t)t * NP] : 0.f;
     const float inv = st > 0.f ? 1.f / st : 0.f;
     float a[RX];  // u_t rows
 #pragma unroll
-    for (int r = 0; r < RX; ++r) a[r] = (live ? __ldg(X + ct * XR + q * RX + r) : 0.f) * inv;
+    for (int r = 0; r < RX; ++r) a[r] = (use ? X[t * XR + q * RX + r] : 0.f) * inv;
     if (c == 0 && live && use && d.U0 && d.V0) {
 #pragma unroll
       for (int r = 0; r < RX; ++r)
@@ -821,12 +933,11 @@ cudaError_t run_svd_split(const Problem& pb, const DeviceBuffers& d, cudaStream_
     constexpr int GSS = NC * 16 + 16;
     const size_t shm = (size_t)32 * GSS * 4 + (size_t)NC * kTile * 4 + 128;
     const cudaError_t e = cudaFuncSetAttribute(
-        k_bout<NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+        k_bout_tma<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
     if (e != cudaSuccess) return e;
-    k_bout<NC, true><<<(nitems + 31) / 32, 128, shm, s>>>(pb, d, nitems, tm);
+    k_bout_tma<NC><<<(nitems + 31) / 32, 128, shm, s>>>(pb, d, nitems, tm);
   } else {
-    std::memset(&tm, 0, sizeof(tm));
-    k_bout<NC, false><<<(nitems + 31) / 32, 128, 0, s>>>(pb, d, nitems, tm);
+    k_bout<NC><<<(nitems + 31) / 32, 128, 0, s>>>(pb, d, nitems);
   }
   return cudaGetLastError();
 }

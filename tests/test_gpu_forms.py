@@ -37,3 +37,38 @@ def test_mlp_gradient_rows(capi, pkg, oracle, n):
     assert np.abs(g - g0).max() <= 1e-4 * np.abs(g0).max()
     y0 = lm.predict(m, f)
     assert np.abs(capi.lambda_predict(m, f) - y0).max() <= 1e-4 * (1 + np.abs(y0).max())
+
+
+def _noisy(pkg, side, nt, seed):
+    return pkg.synth.workload("arps_256", seed=seed, side=side, nt=nt)
+
+
+@pytest.mark.parametrize("bs,T", [(2, 3), (3, 7), (4, 9), (4, 11), (4, 15)])
+@pytest.mark.parametrize("expw", [0, 1])
+def test_sorted_factors_are_identical(capi, pkg, bs, T, expw):
+    """The two-kernel SVD form (columns sorted by the sweeps, factors of four
+    triplets at a time) against the shared-memory form, bit for bit; without
+    exponential weighting every triplet survives, more than four."""
+    noisy, _, (a, m, s) = _noisy(pkg, 37, T + 3, 40 + bs)
+    out = []
+    for form in (0, 3):
+        p = capi.default_params(traj_length=T, block_size=bs, motion_window=5, median_size=-1,
+                                random_seed=3, alpha=a / 300, mu=m / 300, sigma=s / 300,
+                                exp_weighting=expw, autotune=form)
+        Y, est, _, ex = capi.denoise_ex(noisy, p)
+        out.append((Y, est, ex["risk"]))
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("bs,T", [(5, 7), (6, 9), (7, 11), (8, 15)])
+def test_qr_factors_of_every_triplet(capi, pkg, oracle, bs, T):
+    """More surviving triplets than the QR form's factors take at a time, against
+    the oracle at a fixed threshold (the whole-sequence tolerance at fixed
+    lambda)."""
+    noisy, _, _ = _noisy(pkg, 33, T + 2, 50 + bs)
+    kw = dict(traj_length=T, block_size=bs, motion_window=5, median_size=-1, random_seed=3,
+              optimize_pgure=0, exp_weighting=0, lambda_=0.002)
+    Y, _, _ = capi.denoise(noisy, capi.default_params(autotune=5, **kw))
+    Yo, _, _ = oracle.denoise(noisy, n_jobs=4, **kw)
+    assert np.abs(Y - Yo).max() <= 2e-5 * np.abs(Yo).max()
