@@ -358,10 +358,10 @@ size_t window_bytes(const Problem& pb) {
   b += (size_t)g.nwin * g.P * 4;    // pos
   b += C * 4;                       // cnt
   b += C * 4 * 3;                   // fields
-  b += NC * g.M * NP * 4;           // U0
-  b += NC * g.nwin * NP * 4;        // V0
-  b += 2 * 4 * NC * NP * 4 + NP * 4;  // sv, hv, nlive0
-  if (svd_split_scratch(g.M, g.NC)) b += 4 * NP * NC * (16 + 1) * 4;  // xq, xqn
+  b += NC * g.M * (NP + 31) * 4;    // U0
+  b += NC * g.nwin * (NP + 31) * 4; // V0
+  b += 2 * 4 * NC * NP * 4 + 4 * NP * 4;  // sv, hv, nlive
+  if (svd_split_scratch(g.M, g.NC)) b += 4 * NP * NC * 16 * 4;  // xq
   b += (size_t)pb.K * C * (pb.acc64 ? 8 : 4);  // acc
   b += (size_t)pb.K * ((NP + 31) / 32 + mse_blocks(g)) * 8 + 256 * 8;  // partials
   b += sizeof(WinConst) + sizeof(SearchState) + 2 * (size_t)g.fw * sizeof(ArpsChain);
@@ -712,15 +712,14 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
       d.fld2 = mem.arr<float>((size_t)W * C);
       d.fld1 = (ncopies == 4) ? mem.arr<float>((size_t)W * C) : nullptr;
     }
-    d.U0 = mem.arr<float>((size_t)W * g.NC * g.M * g.NP);
-    d.V0 = mem.arr<float>((size_t)W * g.NC * g.nwin * g.NP);
+    d.U0 = mem.arr<float>((size_t)W * g.NC * g.M * g.NPB() * 32);
+    d.V0 = mem.arr<float>((size_t)W * g.NC * g.nwin * g.NPB() * 32);
     d.sv = mem.arr<float>((size_t)W * 4 * g.NC * g.NP);
     d.hv = mem.arr<float>((size_t)W * 4 * g.NC * g.NP);
-    d.nlive0 = mem.arr<int32_t>((size_t)W * g.NP);
+    d.nlive = mem.arr<int32_t>((size_t)W * 4 * g.NP);
     if (svd_split_scratch(g.M, g.NC)) {
       const size_t items = (size_t)W * ncopies * g.NP;
       d.xq = mem.arr<float>(items * g.NC * 16);
-      d.xqn = mem.arr<float>(items * g.NC);
     }
     PGSVT_CK(cudaMemsetAsync(d.hv, 0, sizeof(float) * (size_t)W * 4 * g.NC * g.NP, L.s));
     const size_t accb = (size_t)W * pb.K * C * (pb.acc64 ? 8 : 4);
@@ -1055,14 +1054,13 @@ struct OneWindow {
   void alloc_factors(int ncopies) {
     const Geometry& g = pb.g;
     d.ncopies = ncopies;
-    d.U0 = mem.arr<float>((size_t)g.NC * g.M * g.NP);
-    d.V0 = mem.arr<float>((size_t)g.NC * g.nwin * g.NP);
+    d.U0 = mem.arr<float>((size_t)g.NC * g.M * g.NPB() * 32);
+    d.V0 = mem.arr<float>((size_t)g.NC * g.nwin * g.NPB() * 32);
     d.sv = mem.arr<float>((size_t)4 * g.NC * g.NP);
     d.hv = mem.arr<float>((size_t)4 * g.NC * g.NP);
-    d.nlive0 = mem.arr<int32_t>(g.NP);
+    d.nlive = mem.arr<int32_t>((size_t)4 * g.NP);
     if (svd_split_scratch(g.M, g.NC)) {
       d.xq = mem.arr<float>((size_t)ncopies * g.NP * g.NC * 16);
-      d.xqn = mem.arr<float>((size_t)ncopies * g.NP * g.NC);
     }
     PGSVT_CK(cudaMemsetAsync(d.hv, 0, sizeof(float) * 4 * g.NC * g.NP, s));
     pb.acc64 = 1;  // a caller-given trajectory table may stack any number of patches

@@ -379,33 +379,166 @@ struct Acc<unsigned long long> {  // 2^-32
   }
 };
 
-// ---- one evaluation round: shrink, linear terms, rebuild + scatter of copy 0
+// ---- overlap sums of rebuilt blocks
 //
-// Block = 32 kept patches (an 8 x 4 half of an 8 x 8 tile of grid positions,
-// see the patch order in capi.cu; one per lane) x nwin warps, small enough
-// (at most about 100 KB of shared memory, 64 registers) for two blocks per
-// SM when nwin <= 16.  Phase A spreads the (lambda, copy) pairs over all
-// warps: the shrunk singular values g_i (svt.hpp:135-143) of copy 0 go to
-// shared memory and sum_i g_i h_i of every copy to per-lane partials.
-// Phase B: warp k rebuilds column k (trajectory slice k) of its lanes'
-// patches from the live singular triplets.  The 32 rebuilt blocks of one
-// slice overlap heavily, so each warp sums them into a shared-memory tile in
+// A warp holds 32 kept patches (an 8 x 4 half of an 8 x 8 tile of grid positions,
+// see the patch order in capi.cu; one per lane).  Their rebuilt blocks in one
+// slice overlap heavily, so the warp sums them in a shared-memory tile in
 // int32 fixed point (2^-20, order-free) and adds the tile to the accumulator
 // with one atomic per touched pixel.
+// Pixels of a tile: the 32 blocks of an 8 x 4 half tile cover (7 + side) x (3 +
+// side) pixels when they move together, and a few more rows and columns as a
+// rule (simulated on the benchmark's trajectories: 4 x 4 patches fit 256 pixels
+// in 85% of the cases and 384 in 98%, 8 x 8 ones 256 in 62% and 512 in 97%; the
+// rest straddle two columns of tiles).  A footprint that does not fit costs a
+// global atomic per pixel and patch.  The int64 accumulators round values of the
+// tile and others differently, so they keep one size.
+// Patches of at most 16 rows with more than 8 lambda values in a round have no
+// room for more than 256 at two blocks per SM.
+template <int BS, typename AccT>
+__host__ __device__ constexpr int tile_pixels(int nl) {
+  return sizeof(AccT) == 8 ? 256 : (BS >= 1 && BS <= 4 ? (nl <= 8 ? 384 : 256) : 512);
+}
+constexpr float kTileBound = 60.f;  // |value| above this bypasses the tile (32 x 60 < 2048)
+constexpr float kMagicBound = 4.f;  // and below this value * 2^20 + 1.5 * 2^23 is exact
 
-constexpr int kTileMax = 512;      // pixels of a warp's shared-memory tile
-constexpr float kTileBound = 60.f; // |value| above this bypasses the tile (32 x 60 < 2048)
+// The warp's footprint in one slice.  The tile's column stride is padded to 8
+// (mod 16) where the footprint allows it, so that the warp's four 8-row lane
+// groups (one grid column each) start 0, 8, 16, 24 (or 0, 24, 16, 8) banks apart.
+struct Footprint {
+  int y0, x0, th, ths, area;  // corner, rows, column stride, pixels
+  bool tile;              // it fits the tile
+  __device__ __forceinline__ void init(bool live, int y, int x, int nb, int tile_max) {
+    y0 = __reduce_min_sync(0xffffffffu, live ? y : 1 << 30);
+    x0 = __reduce_min_sync(0xffffffffu, live ? x : 1 << 30);
+    const int y1 = __reduce_max_sync(0xffffffffu, live ? y : -1);
+    const int x1 = __reduce_max_sync(0xffffffffu, live ? x : -1);
+    const int tw = x1 - x0 + nb;
+    th = y1 - y0 + nb;
+    ths = th <= 8 ? 8 : 8 + 16 * ((th - 8 + 15) / 16);
+    if (y1 >= 0 && ths * tw > tile_max) ths = th;
+    tile = y1 >= 0 && ths * tw <= tile_max;
+    area = th * tw;
+  }
+};
+
+// Add one lane's rebuilt rows e0 .. e0 + CH - 1 (column-major in the nb x nb
+// block at (y, x)) to the tile or, where they do not fit, to the accumulator
+// slice acc.  A value below kMagicBound becomes its fixed-point integer with
+// one FMA (rounding to nearest even, as __float2int_rn rounds it).
+template <int BS, int CH, typename AccT>
+__device__ __forceinline__ void scatter(const float (&col)[CH], int e0, int nb, const Footprint& f,
+                                        int* tile, AccT* acc, int S, int y, int x) {
+  const int M = nb * nb;
+  float mx = 0.f;
+#pragma unroll
+  for (int e = 0; e < CH; ++e)  // NaN stays NaN, and takes the second path
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(mx) : "f"(mx), "f"(fabsf(col[e])));
+  if (mx == 0.f) return;
+  if (f.tile && mx <= kMagicBound) {
+    int* t = tile + (y - f.y0) + (x - f.x0) * f.ths;
+#pragma unroll
+    for (int e = 0; e < CH; ++e) {
+      const int ee = e0 + e;
+      if (ee >= M) continue;
+      const int v = __float_as_int(fmaf(col[e], 1048576.f, 12582912.f)) - 0x4B400000;
+      atomicAdd(t + ee % nb + (ee / nb) * f.ths, v);
+    }
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < CH; ++e) {
+    const int ee = e0 + e;
+    const float val = col[e];
+    if (ee >= M || val == 0.f) continue;
+    const int er = ee % nb, ec = ee / nb;
+    if (f.tile && fabsf(val) <= kTileBound)
+      atomicAdd(tile + (y - f.y0 + er) + (x - f.x0 + ec) * f.ths, __float2int_rn(val * 1048576.f));
+    else
+      Acc<AccT>::add(acc + (y + er) + (size_t)(x + ec) * S, Acc<AccT>::fix(val));
+  }
+}
+
+// Add n <= N tiles (T pixels each) to their accumulator slices (acc, acc +
+// jstride) and clear them.
+template <int N, typename AccT>
+__device__ __forceinline__ void flush(const Footprint& f, int* tile, int T, AccT* acc,
+                                      size_t jstride, int n, int S, int lane) {
+  // the lane's entries are row r of a column, 32 entries of the footprint apart:
+  // divided once, then stepped
+  int r = lane % f.th, ti = r + lane / f.th * f.ths;
+  AccT* a = acc + (size_t)(f.y0 + r) + (size_t)(f.x0 + lane / f.th) * S;
+  const int dr = 32 % f.th, dc = 32 / f.th;
+  const int dti = dr + dc * f.ths, da = dr + dc * S;
+  const int wti = f.ths - f.th, wa = S - f.th;
+  for (int t = lane; t < f.area; t += 32) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if (j >= n) break;
+      const int v = tile[j * T + ti];
+      if (v != 0) {
+        tile[j * T + ti] = 0;
+        Acc<AccT>::add(a + j * jstride, Acc<AccT>::from_tile(v));
+      }
+    }
+    r += dr;
+    ti += dti;
+    a += da;
+    if (r >= f.th) {
+      r -= f.th;
+      ti += wti;
+      a += wa;
+    }
+  }
+}
+
+// shrunk singular value (svt.hpp:135-143)
+__device__ __forceinline__ float shrink(int expw, float s, float smax, float lam) {
+  float th;
+  if (expw) th = fabsf(smax * expf(-0.5f * lam * (s * s)));  // svt.hpp:137
+  else th = lam;                                             // svt.hpp:142
+  return fmaxf(fabsf(s) - th, 0.f);
+}
+
+// ---- one evaluation round: shrink, linear terms, rebuild + scatter of copy 0
+//
+// Block = 32 kept patches x nwin warps, small enough (at most about 110 KB of
+// shared memory, 64 registers) for two blocks per SM when nwin <= 16.  Phase A
+// spreads the (lambda, copy) pairs over all warps: the shrunk singular values
+// g_i of copy 0 go to shared memory and sum_i g_i h_i of every copy to per-lane
+// partials, over the triplets that can survive (one or two of 15 as a rule; the
+// others have g = 0 or h = 0).  Phase B: warp k rebuilds column k (trajectory
+// slice k) of its lanes' patches, two lambda values per pass (they share every
+// load of the left and right vectors), and scatters them.  What bounds it is
+// the instructions and shared-memory atomics of the scatter, 16 per patch,
+// slice and lambda, and the flush of the tiles (72% of the shared-memory
+// pipe's peak).  GB300, the rounds of one call: 256 x 256 x 100, 4 x 4 patches, 117
+// -> 58 ms; 256 x 256 x 24, 8 x 8 patches, 127 -> 34 ms (before: tiles of 256
+// pixels, divisions in the flush, conversions on the XU pipe, every triplet
+// shrunk, one lambda value per pass for the larger patches).
+
+// left vectors staged in shared memory for patches of at most 16 rows:
+// [triplet][lane][e], a lane's rows as 16-byte vectors that start on
+// different banks
+template <int M>
+constexpr int kUStride = M == 16 ? 20 : M;
+
+// Rows of a patch rebuilt per pass: all of a small patch, else whole columns, few
+// enough that the left vectors of a pass are loaded together within 64 registers
+// (16 rows of an 8 x 8 patch: the loads were made one by one, 62 instead of 34 ms).
+template <int BS>
+__host__ __device__ constexpr int chunk_rows() {
+  return BS >= 1 && BS <= 4 ? BS * BS : (BS == 5 ? 5 : (BS == 6 ? 12 : (BS == 7 ? 7 : 8)));
+}
 
 // launch bounds of k_eval: a block is 32 x nwin threads, nwin <= MAXW;
 // windows up to 16 frames run two blocks per SM
-
-template <int BS, typename AccT, bool STAGE = false, int MAXW = 21>
+template <int BS, typename AccT, int MAXW>
 __global__ void __launch_bounds__(32 * MAXW, MAXW <= 16 ? 2 : 1)
     k_eval(Problem pb, DeviceBuffers d, int final_pass) {
   const int nb = BS > 0 ? BS : pb.g.bs;  // BS == 0: any side (9..16)
   const int M = nb * nb;
   constexpr int PB = kEvalPatches;  // patches per block
-  constexpr int H = PB / 32;         // patches per lane
   const Geometry& g = pb.g;
   const int w = blockIdx.y;
   const SearchState& st = d.st[w];
@@ -417,196 +550,188 @@ __global__ void __launch_bounds__(32 * MAXW, MAXW <= 16 ? 2 : 1)
   const size_t NP = g.NP;
   const bool lin_terms = pb.optimize && !final_pass;
   const int ncp = lin_terms ? d.ncopies : 1;
-  extern __shared__ float sg[];  // g of copy 0 [nl][NC][PB], lin [nl][4][PB], tiles
-  float* slin = sg + (size_t)nl * NC * PB;
+  extern __shared__ __align__(16) float sg[];  // left vectors, g of copy 0 [nl][NC][PB],
+                                               // lin [nl][4][PB], tiles
+  constexpr bool kStage = BS > 0 && BS * BS <= 16;
+  constexpr int US = kUStride<BS * BS>;
+  float* Us = sg;
+  float* sgv = kStage ? sg + NC * PB * US : sg;
+  const int T = tile_pixels<BS, AccT>(nl);
+  float* slin = sgv + (size_t)nl * NC * PB;
   int* tiles = (int*)(slin + (size_t)nl * 4 * PB);
   __shared__ int srmax[kMaxK];
-  const WinConst& wc = d.wc[w];
-  int* tile = tiles + (size_t)k * kTileMax;
-  for (int i = lane; i < kTileMax; i += 32) tile[i] = 0;
+  int* tile = tiles + (size_t)k * (2 * T);
+  for (int i = lane * 4; i < 2 * T; i += 128) *reinterpret_cast<int4*>(tile + i) = make_int4(0, 0, 0, 0);
   if (threadIdx.x < kMaxK) srmax[threadIdx.x] = 0;
   __syncthreads();
-  // phase A: (lambda, copy, half) tasks over all warps
-  for (int task = k; task < nl * ncp * H; task += nwarps) {
-    const int h = task % H, jc = task / H;
-    const int j = jc / ncp, c = jc % ncp;
-    const int slot = h * 32 + lane;
-    const int p = blockIdx.x * PB + slot;
-    const bool live = p < g.NP;
+  const int p = blockIdx.x * PB + lane;
+  const bool live = p < g.NP;
+  // phase A: (lambda, copy) tasks over all warps
+  for (int task = k; task < nl * ncp; task += nwarps) {
+    const int j = task / ncp, c = task % ncp;
     const float lam = (float)(final_pass ? st.final_lambda : st.next[j]);
     const float* sv = d.sv + ((size_t)w * 4 + c) * NC * NP;
     const float* hv = d.hv + ((size_t)w * 4 + c) * NC * NP;
+    const int nv = live ? d.nlive[((size_t)w * 4 + c) * NP + p] : 0;
+    const int nvmax = __reduce_max_sync(0xffffffffu, nv);
     const float smax = live ? sv[p] : 0.f;  // sorted: column 0 is the largest
     float lin = 0.f;
     int r0 = 0;
-    for (int i = 0; i < NC; ++i) {
+    for (int i = 0; i < nvmax; ++i) {
       const float s = live ? sv[(size_t)i * NP + p] : 0.f;
-      float th;
-      if (pb.expw) th = fabsf(smax * expf(-0.5f * lam * (s * s)));  // svt.hpp:137
-      else th = lam;                                                // svt.hpp:142
-      const float gi = fmaxf(fabsf(s) - th, 0.f);
+      const float gi = shrink(pb.expw, s, smax, lam);
       if (c == 0) {
-        sg[((size_t)j * NC + i) * PB + slot] = gi;
+        sgv[((size_t)j * NC + i) * PB + lane] = gi;
         r0 += gi > 0.f;
       }
       if (lin_terms && live) lin = fmaf(gi, hv[(size_t)i * NP + p], lin);
     }
-    slin[((size_t)j * 4 + c) * PB + slot] = lin;
+    slin[((size_t)j * 4 + c) * PB + lane] = lin;
     if (c == 0) {
-      for (int o = 16; o > 0; o >>= 1) r0 = max(r0, __shfl_xor_sync(0xffffffffu, r0, o));
+      r0 = __reduce_max_sync(0xffffffffu, r0);
       if (lane == 0) atomicMax(&srmax[j], r0);
     }
   }
   __syncthreads();
   // patches of at most 16 rows: the left singular vectors of the block's
   // patches, up to the largest rank any lambda of the round keeps, staged in
-  // shared memory once ([i][e][PB]); every slice warp and every lambda reads
-  // them there instead of through L1
-  constexpr bool kStage = STAGE && BS > 0 && BS * BS <= 16;
-  float* Us = (float*)(tiles + (size_t)nwarps * kTileMax);
+  // shared memory once; every slice warp and every lambda reads them there
   if constexpr (kStage) {
     int R = 0;
     for (int j = 0; j < nl; ++j) R = max(R, srmax[j]);
-    const float* U0w = d.U0 + (size_t)w * NC * M * NP;
-    for (int t = threadIdx.x; t < R * M * PB; t += blockDim.x) {
-      const int slot = t % PB, ie = t / PB;  // ie = i * M + e
-      const int p = blockIdx.x * PB + slot;
-      Us[t] = p < g.NP ? __ldg(U0w + (size_t)ie * NP + p) : 0.f;
-    }
+    const float* U0p = d.U0 + g.u_at(w, p);
+    for (int t = k; t < R * M; t += nwarps)  // t = i * M + e
+      Us[((t / M) * PB + lane) * US + t % M] = live ? __ldg(U0p + t * 32) : 0.f;
     __syncthreads();
   }
   if (lin_terms)
     for (int j = k; j < nl; j += nwarps) {
       float lin = 0.f;
-      for (int h = 0; h < H; ++h)
-        for (int c = 0; c < ncp; ++c) lin += slin[((size_t)j * 4 + c) * PB + h * 32 + lane];
+      for (int c = 0; c < ncp; ++c) lin += slin[((size_t)j * 4 + c) * PB + lane];
       const double t = warp_sum_d((double)lin);
       if (lane == 0) d.part_lin[((size_t)w * pb.K + j) * d.nblk_eval + blockIdx.x] = t;
     }
   if (k >= g.nwin) return;
-  if (final_pass == 1 && k != wc.out_slice) return;  // 2: every slice
-  int y[H], x[H], nlive[H];
-  bool live[H];
-  int y0 = 1 << 30, y1 = -1, x0 = 1 << 30, x1 = -1;
-#pragma unroll
-  for (int h = 0; h < H; ++h) {
-    const int p = blockIdx.x * PB + h * 32 + lane;
-    live[h] = p < g.NP;
-    y[h] = x[h] = nlive[h] = 0;
-    if (live[h]) {
-      const uint32_t pc = d.pos[((size_t)w * g.nwin + k) * g.P + d.plist[p]];
-      y[h] = pc & 0xffffu;
-      x[h] = pc >> 16;
-      nlive[h] = d.nlive0[(size_t)w * NP + p];
-      y0 = min(y0, y[h]);
-      y1 = max(y1, y[h]);
-      x0 = min(x0, x[h]);
-      x1 = max(x1, x[h]);
-    }
+  int y = 0, x = 0, nlive = 0;
+  if (live) {
+    const uint32_t pc = d.pos[((size_t)w * g.nwin + k) * g.P + d.plist[p]];
+    y = pc & 0xffffu;
+    x = pc >> 16;
+    nlive = d.nlive[(size_t)w * 4 * NP + p];
   }
-  // the warp's footprint in this slice
-  for (int o = 16; o > 0; o >>= 1) {
-    y0 = min(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-    y1 = max(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-    x0 = min(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-    x1 = max(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-  }
-  // Two lambda values per pass share every load of the left and right
-  // vectors (patches of at most 16 rows, whose left vectors are staged in
-  // shared memory; the larger forms keep one value per pass within their
-  // registers); each has its own half of the warp's tile.  The tile's column
-  // stride is padded to 8 (mod 16) where the footprint allows it, so that
-  // the warp's four 8-row lane groups (one grid column each) start 0, 8, 16,
-  // 24 (or 0, 24, 16, 8) banks apart.
-  const int th = y1 - y0 + nb, tw = x1 - x0 + nb;
-  constexpr int kHalfTile = kTileMax / 2;
-  int ths = th <= 8 ? 8 : 8 + 16 * ((th - 8 + 15) / 16);
-  if (ths * tw > kHalfTile) ths = th;
-  const bool use_tile = (y1 >= 0) && ths * tw <= kHalfTile;
-  const float* U0 = d.U0 + (size_t)w * NC * M * NP;
-  const float* V0 = d.V0 + (size_t)w * NC * g.nwin * NP;
-  AccT* accw = (AccT*)d.acc;
-  constexpr int CH = (BS > 0 && BS * BS < 16) ? BS * BS : 16;  // rows rebuilt per pass
-  constexpr bool kPair = kStage;
-  for (int j0 = 0; j0 < nl; j0 += kPair ? 2 : 1) {
-    const bool two = kPair && j0 + 1 < nl;
-    AccT* acc[2];
-    int* tl[2] = {tile, tile + kHalfTile};
-#pragma unroll
-    for (int jj = 0; jj < 2; ++jj)
-      acc[jj] = accw + (((size_t)w * pb.K + (two ? j0 + jj : j0)) * g.nwin + k) * g.F();
-    const int rj = max(srmax[j0], two ? srmax[j0 + 1] : 0);
-#pragma unroll 1
-    for (int h = 0; h < H; ++h) {
-      if (!live[h]) continue;
-      const int p = blockIdx.x * PB + h * 32 + lane;
-      const int rm = min(rj, nlive[h]);
-      const float* sg0 = sg + (size_t)j0 * NC * PB + h * 32 + lane;
-      const float* sg1 = sg + (size_t)(two ? j0 + 1 : j0) * NC * PB + h * 32 + lane;
+  Footprint f;
+  f.init(live, y, x, nb, T);
+  const float* U0 = d.U0 + g.u_at(w, p);
+  const float* V0 = d.V0 + g.v_at(w, p) + k * 32;
+  AccT* accw = (AccT*)d.acc + ((size_t)w * pb.K * g.nwin + k) * g.F();
+  const size_t jstride = (size_t)g.nwin * g.F();  // accumulators of one lambda
+  constexpr int CH = chunk_rows<BS>();
+  for (int j0 = 0; j0 < nl; j0 += 2) {
+    const bool two = j0 + 1 < nl;
+    const int rm = min(max(srmax[j0], two ? srmax[j0 + 1] : 0), nlive);
+    if (rm > 0) {
+      const float* sg0 = sgv + (size_t)j0 * NC * PB + lane;
+      const float* sg1 = sgv + (size_t)(two ? j0 + 1 : j0) * NC * PB + lane;
 #pragma unroll 1
       for (int e0 = 0; e0 < M; e0 += CH) {
         float col[2][CH];
 #pragma unroll
         for (int e = 0; e < CH; ++e) col[0][e] = col[1][e] = 0.f;
         for (int i = 0; i < rm; ++i) {
-          const float v = V0[((size_t)i * g.nwin + k) * NP + p];
-          const float c0 = sg0[(size_t)i * PB] * v;
-          const float c1 = two ? sg1[(size_t)i * PB] * v : 0.f;
+          const float v = V0[i * g.nwin * 32];
+          const float c0 = sg0[i * PB] * v;
+          const float c1 = two ? sg1[i * PB] * v : 0.f;
           if (c0 == 0.f && c1 == 0.f) continue;
+          float u[CH];
           if constexpr (kStage) {
-            const float* ui = Us + ((size_t)i * M + e0) * PB + h * 32 + lane;
+            const float* ui = Us + (i * PB + lane) * US;
+            if constexpr (CH % 4 == 0) {
 #pragma unroll
-            for (int e = 0; e < CH; ++e)
-              if (e0 + e < M) {
-                const float u = ui[e * PB];
-                col[0][e] = fmaf(c0, u, col[0][e]);
-                col[1][e] = fmaf(c1, u, col[1][e]);
-              }
+              for (int e = 0; e < CH; e += 4)
+                *reinterpret_cast<float4*>(u + e) = *reinterpret_cast<const float4*>(ui + e);
+            } else {
+#pragma unroll
+              for (int e = 0; e < CH; ++e) u[e] = ui[e];
+            }
           } else {
-            const float* ui = U0 + ((size_t)i * M + e0) * NP + p;
+            const float* ui = U0 + (i * M + e0) * 32;
 #pragma unroll
-            for (int e = 0; e < CH; ++e)
-              if (e0 + e < M) {
-                const float u = __ldg(ui + (size_t)e * NP);
-                col[0][e] = fmaf(c0, u, col[0][e]);
-                col[1][e] = fmaf(c1, u, col[1][e]);
-              }
+            for (int e = 0; e < CH; ++e) u[e] = e0 + e < M ? __ldg(ui + e * 32) : 0.f;
           }
-        }
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          if (jj == 1 && !two) break;
 #pragma unroll
           for (int e = 0; e < CH; ++e) {
-            const int ee = e0 + e;
-            const float val = col[jj][e];
-            if (ee >= M || val == 0.f) continue;
-            const int er = ee % nb, ec = ee / nb;
-            if (use_tile && fabsf(val) <= kTileBound)
-              atomicAdd(tl[jj] + (y[h] - y0 + er) + (x[h] - x0 + ec) * ths,
-                        __float2int_rn(val * 1048576.f));
-            else
-              Acc<AccT>::add(acc[jj] + (y[h] + er) + (size_t)(x[h] + ec) * g.S, Acc<AccT>::fix(val));
+            col[0][e] = fmaf(c0, u[e], col[0][e]);
+            col[1][e] = fmaf(c1, u[e], col[1][e]);
           }
         }
+        scatter<BS, CH>(col[0], e0, nb, f, tile, accw + j0 * jstride, g.S, y, x);
+        if (two)
+          scatter<BS, CH>(col[1], e0, nb, f, tile + T, accw + (j0 + 1) * jstride, g.S, y, x);
       }
     }
-    if (use_tile) {
+    if (f.tile) {
       __syncwarp();
+      flush<2>(f, tile, T, accw + j0 * jstride, jstride, two ? 2 : 1, g.S, lane);
+      __syncwarp();
+    }
+  }
+}
+
+// ---- the output slice alone, at the chosen lambda: one warp per 32 patches
+// (a block of k_eval would keep one of its nwin warps)
+template <int BS, typename AccT>
+__global__ void __launch_bounds__(128) k_eval_out(Problem pb, DeviceBuffers d) {
+  const int nb = BS > 0 ? BS : pb.g.bs;
+  const int M = nb * nb;
+  const Geometry& g = pb.g;
+  const int w = blockIdx.y;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  constexpr int T = tile_pixels<BS, AccT>(1);
+  __shared__ int tiles[4][T];
+  int* tile = tiles[wib];
+  for (int i = lane; i < T; i += 32) tile[i] = 0;
+  __syncwarp();
+  const size_t NP = g.NP;
+  const int NC = g.NC, k = d.wc[w].out_slice;
+  const int p = (blockIdx.x * 4 + wib) * kEvalPatches + lane;
+  const bool live = p < g.NP;
+  int y = 0, x = 0, nlive = 0;
+  if (live) {
+    const uint32_t pc = d.pos[((size_t)w * g.nwin + k) * g.P + d.plist[p]];
+    y = pc & 0xffffu;
+    x = pc >> 16;
+    nlive = d.nlive[(size_t)w * 4 * NP + p];
+  }
+  Footprint f;
+  f.init(live, y, x, nb, T);
+  const float lam = (float)d.st[w].final_lambda;
+  const float* sv = d.sv + (size_t)w * 4 * NC * NP + p;
+  const float* U0 = d.U0 + g.u_at(w, p);
+  const float* V0 = d.V0 + g.v_at(w, p) + k * 32;
+  AccT* acc = (AccT*)d.acc + ((size_t)w * pb.K * g.nwin + k) * g.F();
+  constexpr int CH = chunk_rows<BS>();
+  if (nlive > 0) {
+    const float smax = sv[0];
+#pragma unroll 1
+    for (int e0 = 0; e0 < M; e0 += CH) {
+      float col[CH];
 #pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        if (jj == 1 && !two) break;
-        for (int t = lane; t < ths * tw; t += 32) {
-          const int v = tl[jj][t];
-          if (v != 0) {
-            tl[jj][t] = 0;
-            Acc<AccT>::add(acc[jj] + (y0 + t % ths) + (size_t)(x0 + t / ths) * g.S,
-                           Acc<AccT>::from_tile(v));
-          }
-        }
+      for (int e = 0; e < CH; ++e) col[e] = 0.f;
+      for (int i = 0; i < nlive; ++i) {
+        const float gi = shrink(pb.expw, sv[(size_t)i * NP], smax, lam);
+        const float c0 = gi * V0[i * g.nwin * 32];
+        if (c0 == 0.f) continue;
+        const float* ui = U0 + (i * M + e0) * 32;
+#pragma unroll
+        for (int e = 0; e < CH; ++e)
+          col[e] = fmaf(c0, e0 + e < M ? __ldg(ui + e * 32) : 0.f, col[e]);
       }
-      __syncwarp();
+      scatter<BS, CH>(col, e0, nb, f, tile, acc, g.S, y, x);
     }
+  }
+  if (f.tile) {
+    __syncwarp();
+    flush<1>(f, tile, T, acc, 0, 1, g.S, lane);
   }
 }
 
@@ -732,13 +857,12 @@ __global__ void k_risk_collect(Problem pb, DeviceBuffers d, double* out) {
   }
 }
 
-// shared memory of a k_eval block; stage: the left vectors fit beside it
-size_t eval_smem(const Geometry& g, int nl, int& stage) {
-  const size_t base = (size_t)nl * (g.NC + 4) * kEvalPatches * sizeof(float) +
-                      (size_t)g.nwin * kTileMax * sizeof(int);
-  const size_t staged = g.bs <= 4 ? (size_t)g.NC * g.M * kEvalPatches * sizeof(float) : 0;
-  stage = (staged > 0 && base + staged <= 227 * 1024) ? 1 : 0;
-  return base + (stage ? staged : 0);
+// shared memory of a k_eval block (110 KB at most for windows up to 16 frames)
+template <int BS, typename AccT>
+size_t eval_smem(const Geometry& g, int nl) {
+  const int us = BS >= 1 && BS <= 4 ? g.NC * kUStride<BS * BS> : 0;  // staged left vectors
+  return ((size_t)nl * (g.NC + 4) + us) * kEvalPatches * sizeof(float) +
+         (size_t)g.nwin * 2 * tile_pixels<BS, AccT>(nl) * sizeof(int);
 }
 
 // Raise, never lower, a kernel's dynamic shared-memory limit on the current
@@ -758,53 +882,58 @@ void allow_dynamic_smem(const void* kernel, size_t shm) {
 }
 
 template <int BS, typename AccT>
-void launch_k_eval_bs(dim3 grid, int threads, size_t shm, cudaStream_t s, const Problem& pb,
-                      const DeviceBuffers& d, int final_pass, int stage) {
-  if constexpr (BS > 0 && BS * BS <= 16) {
-    if (stage && threads <= 32 * 16) {  // two blocks per SM
-      allow_dynamic_smem((const void*)k_eval<BS, AccT, true, 16>, shm);
-      k_eval<BS, AccT, true, 16><<<grid, threads, shm, s>>>(pb, d, final_pass);
-      return;
-    }
-    if (stage) {  // the left vectors staged in shared memory
-      allow_dynamic_smem((const void*)k_eval<BS, AccT, true>, shm);
-      k_eval<BS, AccT, true><<<grid, threads, shm, s>>>(pb, d, final_pass);
-      return;
-    }
+void launch_k_eval_bs(dim3 grid, int threads, int nl, cudaStream_t s, const Problem& pb,
+                      const DeviceBuffers& d, int final_pass) {
+  const size_t shm = eval_smem<BS, AccT>(pb.g, nl);
+  if constexpr (BS > 0 && BS * BS <= 16) {  // windows of at most 15 frames
+    allow_dynamic_smem((const void*)k_eval<BS, AccT, 16>, shm);
+    k_eval<BS, AccT, 16><<<grid, threads, shm, s>>>(pb, d, final_pass);
+  } else if (threads <= 32 * 16) {  // two blocks per SM
+    allow_dynamic_smem((const void*)k_eval<BS, AccT, 16>, shm);
+    k_eval<BS, AccT, 16><<<grid, threads, shm, s>>>(pb, d, final_pass);
+  } else {
+    allow_dynamic_smem((const void*)k_eval<BS, AccT, 21>, shm);
+    k_eval<BS, AccT, 21><<<grid, threads, shm, s>>>(pb, d, final_pass);
   }
-  if (threads <= 32 * 16) {  // two blocks per SM
-    allow_dynamic_smem((const void*)k_eval<BS, AccT, false, 16>, shm);
-    k_eval<BS, AccT, false, 16><<<grid, threads, shm, s>>>(pb, d, final_pass);
-    return;
-  }
-  allow_dynamic_smem((const void*)k_eval<BS, AccT>, shm);
-  k_eval<BS, AccT><<<grid, threads, shm, s>>>(pb, d, final_pass);
 }
 
 template <typename AccT>
-void launch_k_eval_t(int bs, dim3 grid, int threads, size_t shm, cudaStream_t s,
-                     const Problem& pb, const DeviceBuffers& d, int final_pass, int stage) {
+void launch_k_eval_t(int bs, dim3 grid, int threads, int nl, cudaStream_t s,
+                     const Problem& pb, const DeviceBuffers& d, int final_pass) {
   switch (bs) {
-    case 2: launch_k_eval_bs<2, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
-    case 3: launch_k_eval_bs<3, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
-    case 4: launch_k_eval_bs<4, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
-    case 5: launch_k_eval_bs<5, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
-    case 6: launch_k_eval_bs<6, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
-    case 7: launch_k_eval_bs<7, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
-    case 8: launch_k_eval_bs<8, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
-    default: launch_k_eval_bs<0, AccT>(grid, threads, shm, s, pb, d, final_pass, stage); break;
+    case 2: launch_k_eval_bs<2, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
+    case 3: launch_k_eval_bs<3, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
+    case 4: launch_k_eval_bs<4, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
+    case 5: launch_k_eval_bs<5, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
+    case 6: launch_k_eval_bs<6, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
+    case 7: launch_k_eval_bs<7, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
+    case 8: launch_k_eval_bs<8, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
+    default: launch_k_eval_bs<0, AccT>(grid, threads, nl, s, pb, d, final_pass); break;
   }
 }
 
 void launch_k_eval(const Problem& pb, const DeviceBuffers& d, int final_pass, int nl,
                    cudaStream_t s) {
   const Geometry& g = pb.g;
-  int stage = 0;
-  const size_t shm = eval_smem(g, nl, stage);
   const dim3 grid(d.nblk_eval, pb.W);
   if (pb.acc64)
-    launch_k_eval_t<unsigned long long>(g.bs, grid, 32 * g.nwin, shm, s, pb, d, final_pass, stage);
-  else launch_k_eval_t<int>(g.bs, grid, 32 * g.nwin, shm, s, pb, d, final_pass, stage);
+    launch_k_eval_t<unsigned long long>(g.bs, grid, 32 * g.nwin, nl, s, pb, d, final_pass);
+  else launch_k_eval_t<int>(g.bs, grid, 32 * g.nwin, nl, s, pb, d, final_pass);
+}
+
+template <typename AccT>
+void launch_k_eval_out_t(const Problem& pb, const DeviceBuffers& d, cudaStream_t s) {
+  const dim3 grid((pb.g.NP + 4 * kEvalPatches - 1) / (4 * kEvalPatches), pb.W);
+  switch (pb.g.bs) {
+    case 2: k_eval_out<2, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+    case 3: k_eval_out<3, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+    case 4: k_eval_out<4, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+    case 5: k_eval_out<5, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+    case 6: k_eval_out<6, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+    case 7: k_eval_out<7, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+    case 8: k_eval_out<8, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+    default: k_eval_out<0, AccT><<<grid, 128, 0, s>>>(pb, d); break;
+  }
 }
 
 void launch_k_mse(const Problem& pb, const DeviceBuffers& d, cudaStream_t s) {
@@ -848,8 +977,13 @@ cudaError_t launch_search_hint(const Problem& pb, const DeviceBuffers& d, cudaSt
 
 cudaError_t launch_eval_round(const Problem& pb, const DeviceBuffers& d, int final_pass,
                               cudaStream_t s) {
+  if (final_pass == 1) {  // the output slice alone
+    if (pb.acc64) launch_k_eval_out_t<unsigned long long>(pb, d, s);
+    else launch_k_eval_out_t<int>(pb, d, s);
+    return cudaGetLastError();
+  }
   launch_k_eval(pb, d, final_pass, final_pass ? 1 : pb.K, s);
-  if (final_pass) return cudaGetLastError();
+  if (final_pass) return cudaGetLastError();  // 2: every slice
   launch_k_mse(pb, d, s);
   k_search_step<<<pb.W, 256, 0, s>>>(pb, d);
   return cudaGetLastError();

@@ -182,7 +182,7 @@ extern "C" int pgsvt_svd_window_noalloc(const float* u_dev, uint32_t nrows, uint
   d.plist = (const int32_t*)(sb + kOffPlist);
   d.sv = (float*)(sb + kOffSv);
   d.hv = (float*)(sb + kOffHv);
-  d.nlive0 = (int32_t*)(sb + kOffNlive);
+  d.nlive = (int32_t*)(sb + kOffNlive);
   d.wc = (WinConst*)(sb + kOffWc);
   d.counters = (unsigned long long*)(sb + kOffCnt);
   int* err = (int*)(sb + kOffErr);

@@ -14,9 +14,10 @@
 //                                 P = (S-bs+1)^2 ARPS positions (arps.hpp:42)
 //   cnt     i32 [W][nwin][S*S]    patch coverage per voxel (svt.hpp:157-159)
 //   fld0,2  f32 [W][nwin][S*S]    lambda-independent risk fields (see eval.cu)
-//   U0      f32 [W][NC][M][NP]    left singular vectors of copy 0 (patch
+//   U0      f32 [W][NPB][NC][M][32]  left singular vectors of copy 0 (blocks
+//                                 of 32 patches, patch
 //                                 fastest), columns sorted by singular value
-//   V0      f32 [W][NC][N][NP]    right singular vectors of copy 0
+//   V0      f32 [W][NPB][NC][N][32]  right singular vectors of copy 0
 //   sv,hv   f32 [W][4][NC][NP]    singular values and risk projections of
 //                                 copies 0 (clean), 1 (+eps2*delta2),
 //                                 2 (-eps2*delta2), 3 (+eps1*delta1)
@@ -135,6 +136,15 @@ struct Geometry {
   int nimg;
   __host__ __device__ size_t F() const { return (size_t)S * S; }
   __host__ __device__ size_t cube() const { return F() * nwin; }
+  // factor arrays: blocks of 32 patches; element (triplet t, row e) of patch p
+  // of window w at u_at(w, p) + (t * M + e) * 32, V's at v_at(w, p) + (t * nwin + k) * 32
+  __host__ __device__ int NPB() const { return (NP + 31) / 32; }
+  __host__ __device__ size_t u_at(int w, int p) const {
+    return ((size_t)w * NPB() + (p >> 5)) * NC * M * 32 + (p & 31);
+  }
+  __host__ __device__ size_t v_at(int w, int p) const {
+    return ((size_t)w * NPB() + (p >> 5)) * NC * nwin * 32 + (p & 31);
+  }
 };
 
 struct Problem {
@@ -182,8 +192,7 @@ struct DeviceBuffers {
   float* sv;
   float* hv;
   float* xq;               // split SVD forms' scratch: [items][NC][X rows] (svd_split.cu)
-  float* xqn;              // surviving triplets of each item (ints; [items])
-  int32_t* nlive0;         // [W][NP] singular triplets of copy 0 that can survive
+  int32_t* nlive;          // [W][4][NP] singular triplets that can survive
   void* acc;               // [W][K][nwin][S*S] int32 or int64 fixed point
   double* part_lin;        // [W][K][nblk_eval]
   double* part_mse;        // [W][K][nblk_mse]
@@ -318,7 +327,7 @@ constexpr int kSvdVariants = 6;
 int svd_variants(int M, int NC);
 bool svd_qr_form(int M, int NC);  // the QR-preconditioned SVD applies (its scratch is needed)
 int svd_default_variant(int M, int NC);
-bool svd_split_scratch(int M, int NC);  // a split SVD form applies (xq, xqn needed)
+bool svd_split_scratch(int M, int NC);  // a split SVD form applies (xq needed)
 bool svd_variant_ok(int M, int NC, int v);
 bool svd_supported(int bs, int nwin);
 

@@ -99,7 +99,7 @@ cudaError_t launch_svd(const Problem& pb, const DeviceBuffers& d, cudaStream_t s
     if (NC == 10) return run_svd_qr<10>(pb, d, s);
     if (NC == 16) return run_svd_qr<16>(pb, d, s);
   }
-  if ((pb.svd_variant == 0 || pb.svd_variant == 5) && M <= 16 && d.xq && d.xqn) {
+  if ((pb.svd_variant == 0 || pb.svd_variant == 5) && M <= 16 && d.xq) {
     // sweeps and factors in two kernels; variant 5 stages the factors' frame
     // tiles with TMA
     if (NC == 10) return run_svd_split<10>(pb, d, s, pb.svd_variant == 5);

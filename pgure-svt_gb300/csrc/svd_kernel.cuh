@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(128, (svd_minblocks<RPL, NC, SM>()))
   int nl_max = nl;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) nl_max = max(nl_max, __shfl_xor_sync(0xffffffffu, nl_max, o));
-  if (c == 0 && live && q == 0) d.nlive0[(size_t)w * NP + p] = nl;
+  if (live && q == 0) d.nlive[((size_t)w * 4 + c) * NP + p] = nl;
 
   // B again (the Jacobi overwrote it) and the lambda-independent field G
   const float* fld = (c == 0) ? d.fld0 : (c == 3 ? d.fld1 : d.fld2);
@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(128, (svd_minblocks<RPL, NC, SM>()))
     if (c == 0 && live && use && d.U0) {
 #pragma unroll
       for (int r = 0; r < RPL; ++r)
-        if (roff[r] >= 0) d.U0[(((size_t)w * NCg + t) * g.M + q * RPL + r) * NP + p] = a[r];
+        if (roff[r] >= 0) d.U0[g.u_at(w, p) + (t * g.M + q * RPL + r) * 32] = a[r];
     }
     // v_t = B^T u_t / s_t and h_t = u_t^T G v_t = sum_k v_k (G_k . u_t),
     // the latter from the lanes' partial sums with one reduction
@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(128, (svd_minblocks<RPL, NC, SM>()))
       bu = lanes_sum<LANES>(bu);
       const float vk = bu * inv;
       if (c == 0 && live && use && (k % LANES) == q && d.V0)
-        d.V0[(((size_t)w * NCg + t) * nwin + k) * NP + p] = vk;
+        d.V0[g.v_at(w, p) + (t * nwin + k) * 32] = vk;
       if (fw_ && live && use) {
         const uint32_t pc = __ldg(posw + (size_t)k * g.P + posidx);
         const size_t base = (size_t)k * F + (pc & 0xffffu) + (size_t)(pc >> 16) * g.S;

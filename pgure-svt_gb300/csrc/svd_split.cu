@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(128) k_qr(Problem pb, DeviceBuffers d, int nit
 // ---- end of a sweep kernel: the column norms (the singular values) of one
 // patch per lane group, sorted, and the rotated columns of the triplets that
 // can survive the threshold, in that order: xq [item][rank][XR], the count in
-// xqn [item].  Lane q takes columns 4n + q: their sums come from a
+// nlive.  Lane q takes columns 4n + q: their sums come from a
 // reduce-scatter (the lanes added in lanes_sum's order), their ranks from
 // comparisons with every column (ties by index); sorting in the factors
 // kernels took more instructions there than the factors themselves.  `get`:
@@ -316,10 +316,7 @@ __device__ __forceinline__ void store_sorted(const Problem& pb, const DeviceBuff
         if (t >= nl) hvo[(size_t)t * NP] = 0.f;
       }
     }
-    if (q == 0) {
-      reinterpret_cast<int*>(d.xqn)[gid] = nl;
-      if (c == 0) d.nlive0[(size_t)w * NP + p] = nl;
-    }
+    if (q == 0) d.nlive[((size_t)w * 4 + c) * NP + p] = nl;
     float* xo = d.xq + (size_t)gid * NC * XR + q * RX;
 #pragma unroll
     for (int k = 0; k < NC - 1; ++k) {
@@ -379,9 +376,6 @@ __global__ void __launch_bounds__(128, 5) k_qr_out(Problem pb, DeviceBuffers d, 
   const bool live = gid < nitems;
   const int nwin = g.nwin, M = g.M;
   __shared__ __align__(16) float Vs[8][NC][kQT];  // v_t of the triplets at hand
-  const int nl = live ? reinterpret_cast<const int*>(d.xqn)[gid] : 0;
-  const int nl_max = max(nl, __shfl_xor_sync(0xffffffffu, nl, 16));
-  if (nl_max == 0) return;  // warp-uniform
   int p, c, w;
   {
     const int gg = live ? gid : 0;
@@ -390,6 +384,9 @@ __global__ void __launch_bounds__(128, 5) k_qr_out(Problem pb, DeviceBuffers d, 
     c = r % d.ncopies;
     w = r / d.ncopies;
   }
+  const int nl = live ? d.nlive[((size_t)w * 4 + c) * g.NP + p] : 0;
+  const int nl_max = max(nl, __shfl_xor_sync(0xffffffffu, nl, 16));
+  if (nl_max == 0) return;  // warp-uniform
   const float* X = d.xq + (size_t)(live ? gid : 0) * NC * D::XR;
   int roff[kQR];
 #pragma unroll
@@ -421,7 +418,7 @@ __global__ void __launch_bounds__(128, 5) k_qr_out(Problem pb, DeviceBuffers d, 
           const float v = (t0 + t < nl && l16 < nwin) ? X[(t0 + t) * D::XR + l16] * inv[t] : 0.f;
           Vs[slot][l16][t] = v;
           if (keep && t0 + t < nl && l16 < nwin)
-            d.V0[(((size_t)w * NCg + t0 + t) * nwin + l16) * NP + p] = v;
+            d.V0[g.v_at(w, p) + ((t0 + t) * nwin + l16) * 32] = v;
         }
       } else if (l16 < NC) {
         Vs[slot][l16][t] = 0.f;
@@ -455,7 +452,7 @@ __global__ void __launch_bounds__(128, 5) k_qr_out(Problem pb, DeviceBuffers d, 
       for (int r = 0; r < kQR; ++r) {
         a[t][r] *= inv[t];
         if (keep && t0 + t < nl && roff[r] >= 0)
-          d.U0[(((size_t)w * NCg + t0 + t) * g.M + l16 * kQR + r) * NP + p] = a[t][r];
+          d.U0[g.u_at(w, p) + ((t0 + t) * M + l16 * kQR + r) * 32] = a[t][r];
       }
     }
     if (fw_) {
@@ -551,9 +548,6 @@ __global__ void __launch_bounds__(128, 8) k_bout(Problem pb, DeviceBuffers d, in
   const int gid = blockIdx.x * 32 + (threadIdx.x >> 2);
   const bool live = gid < nitems;
   const int nwin = g.nwin, M = g.M;
-  const int nl = live ? reinterpret_cast<const int*>(d.xqn)[gid] : 0;
-  const int nl_max = __reduce_max_sync(0xffffffffu, nl);
-  if (nl_max == 0) return;  // warp-uniform
   int p, c, w;
   {
     const int gg = live ? gid : 0;
@@ -562,6 +556,9 @@ __global__ void __launch_bounds__(128, 8) k_bout(Problem pb, DeviceBuffers d, in
     c = r % d.ncopies;
     w = r / d.ncopies;
   }
+  const int nl = live ? d.nlive[((size_t)w * 4 + c) * g.NP + p] : 0;
+  const int nl_max = __reduce_max_sync(0xffffffffu, nl);
+  if (nl_max == 0) return;  // warp-uniform
   const float* X = d.xq + (size_t)(live ? gid : 0) * NC * XR + q * RX;
   int roff[RX];
 #pragma unroll
@@ -594,7 +591,7 @@ __global__ void __launch_bounds__(128, 8) k_bout(Problem pb, DeviceBuffers d, in
       for (int r = 0; r < RX; ++r) {
         a[t][r] = xp[r] * inv[t];
         if (keep && use && roff[r] >= 0)
-          d.U0[(((size_t)w * NCg + t0 + t) * g.M + q * RX + r) * NP + p] = a[t][r];
+          d.U0[g.u_at(w, p) + ((t0 + t) * M + q * RX + r) * 32] = a[t][r];
       }
     }
     // v_t = B^T u_t / s_t and h_t = u_t^T G v_t = sum_k v_k (G_k . u_t)
@@ -615,7 +612,7 @@ __global__ void __launch_bounds__(128, 8) k_bout(Problem pb, DeviceBuffers d, in
         for (int r = 0; r < RX; ++r) bu = fmaf(B[r], a[t][r], bu);
         const float vk = lanes_sum<4>(bu) * inv[t];
         if (keep && t0 + t < nl && (k & 3) == q)
-          d.V0[(((size_t)w * NCg + t0 + t) * nwin + k) * NP + p] = vk;
+          d.V0[g.v_at(w, p) + ((t0 + t) * nwin + k) * 32] = vk;
         float gu = 0.f;
 #pragma unroll
         for (int r = 0; r < RX; ++r) gu = fmaf(G[r], a[t][r], gu);
@@ -662,7 +659,7 @@ __global__ void __launch_bounds__(128, 4)
   const int NCg = g.NC;
   const float* svo = d.sv + (((size_t)w * 4 + c) * NCg) * NP + p;
   float* hvo = d.hv + (((size_t)w * 4 + c) * NCg) * NP + p;
-  const int nl = live ? reinterpret_cast<const int*>(d.xqn)[gid] : 0;
+  const int nl = live ? d.nlive[((size_t)w * 4 + c) * g.NP + p] : 0;
   const int nl_max = __reduce_max_sync(0xffffffffu, nl);
   const float* fld = (c == 0) ? d.fld0 : (c == 3 ? d.fld1 : d.fld2);
   const float* fw_ = (pb.optimize && fld) ? fld + (size_t)w * g.cube() : nullptr;
@@ -825,7 +822,7 @@ __global__ void __launch_bounds__(128, 4)
     if (c == 0 && live && use && d.U0 && d.V0) {
 #pragma unroll
       for (int r = 0; r < RX; ++r)
-        if (roff[r] >= 0) d.U0[(((size_t)w * NCg + t) * g.M + q * RX + r) * NP + p] = a[r];
+        if (roff[r] >= 0) d.U0[g.u_at(w, p) + (t * M + q * RX + r) * 32] = a[r];
     }
     // v_t = B^T u_t / s_t and h_t = u_t^T G v_t = sum_k v_k (G_k . u_t)
     float h = 0.f;
@@ -838,7 +835,7 @@ __global__ void __launch_bounds__(128, 4)
       bu = lanes_sum<4>(bu);
       const float vk = bu * inv;
       if (c == 0 && live && use && (k % 4) == q && d.V0)
-        d.V0[(((size_t)w * NCg + t) * nwin + k) * NP + p] = vk;
+        d.V0[g.v_at(w, p) + (t * nwin + k) * 32] = vk;
       if (fw_ && live && use) {
         const float4 g4 = *reinterpret_cast<const float4*>(gs + k * 4 * RX);
         const float* gp = &g4.x;
@@ -858,7 +855,7 @@ __global__ void __launch_bounds__(128, 4)
 
 template <int NC>
 cudaError_t run_svd_qr(const Problem& pb, const DeviceBuffers& d, cudaStream_t s) {
-  if (!d.xq || !d.xqn) return cudaErrorInvalidValue;
+  if (!d.xq) return cudaErrorInvalidValue;
   const int nitems = pb.W * d.ncopies * pb.g.NP;
   k_qr<NC><<<(nitems + 7) / 8, 128, 0, s>>>(pb, d, nitems);
   k_xsweep<NC><<<(nitems + 31) / 32, 128, 0, s>>>(pb, d, nitems);
@@ -910,7 +907,7 @@ bool frame_map(CUtensorMap* m, CUtensorMapDataType dt, size_t esize, const void*
 
 template <int NC>
 cudaError_t run_svd_split(const Problem& pb, const DeviceBuffers& d, cudaStream_t s, bool staged) {
-  if (!d.xq || !d.xqn) return cudaErrorInvalidValue;
+  if (!d.xq) return cudaErrorInvalidValue;
   const int nitems = pb.W * d.ncopies * pb.g.NP;
   const int S = pb.g.S, nwin = pb.g.nwin;
   k_bsweep<NC><<<(nitems + 31) / 32, 128, 0, s>>>(pb, d, nitems);

@@ -72,3 +72,25 @@ def test_qr_factors_of_every_triplet(capi, pkg, oracle, bs, T):
     Y, _, _ = capi.denoise(noisy, capi.default_params(autotune=5, **kw))
     Yo, _, _ = oracle.denoise(noisy, n_jobs=4, **kw)
     assert np.abs(Y - Yo).max() <= 2e-5 * np.abs(Yo).max()
+
+
+@pytest.mark.parametrize("bs,T,side", [(2, 3, 21), (3, 7, 30), (4, 15, 35), (5, 9, 29), (6, 21, 31),
+                                       (7, 15, 26), (8, 21, 33), (9, 9, 30), (16, 21, 40)])
+@pytest.mark.parametrize("nl", [1, 2, 9, 16])
+def test_eval_round_of_any_length(capi, pkg, oracle, bs, T, side, nl):
+    """Rounds of one to sixteen lambda values (single, paired, odd; the smaller
+    tiles of long rounds), every patch side's rows per pass, against the
+    oracle's risks (the tolerance of the risk tests)."""
+    noisy, _, _ = _noisy(pkg, side, T + 2, 60 + bs)
+    lams = np.geomspace(0.01, 20.0, nl)
+    noise = dict(alpha=0.01, mu=0.02, sigma=0.03)
+    p = capi.default_params(traj_length=T, block_size=bs, motion_window=5, median_size=-1,
+                            random_seed=3, **noise)
+    res, _ = capi.denoise_batch([dict(X=noisy, params=p, lambdas=lams)])
+    fw = min(T, bs * bs - 1) // 2
+    u = np.asarray(noisy[..., :2 * fw + 1], np.float64)
+    u = u / u.max()
+    rows, cols = oracle.arps_window(u, bs, 5, fw, fw, T + 2)
+    ro = oracle.risk_window(u, bs, 1, rows, cols, lams, *noise.values(), 3)
+    r = res[0]["risks"][fw]
+    assert np.abs(r - ro).max() <= 1e-4 * np.abs(ro).max()
