@@ -20,7 +20,8 @@
 // The epilogue needs no V accumulation: with u_i = a_i/s_i, the right vectors
 // are v_i = B^T u_i / s_i from a fresh gather of B, and the risk projections
 // h_i = u_i^T G v_i use the lambda-independent fields G (eval.cu).  Singular
-// triplets are stored sorted by decreasing s.
+// triplets are stored sorted by decreasing s; the factors go over the slices
+// with four surviving triplets side by side.
 #include "pgsvt_internal.h"
 
 namespace pgsvt {

@@ -180,20 +180,20 @@ __device__ __forceinline__ void store_rows(float* p, const float (&v)[RPL]) {
 // Shared-memory footprint of one patch: SM keeps the columns there during the
 // sweeps ([NC][MP] plus NC norms, the patch stride an odd multiple of 16
 // floats so the two 4-lane patches of a quarter-warp use disjoint banks);
-// otherwise the epilogue's staging copy ([NC][MP+1]).
+// otherwise the epilogue's staging copy ([NC][MP+1]).  Then the epilogue's
+// tables: the sorted singular values and the columns in that order.
 template <int RPL, int LANES, int NC, bool SM>
 struct SvdSmem {
   static constexpr int MP = RPL * LANES;
   static constexpr int CS = SM ? MP : MP + 1;  // column stride
   static constexpr int NRM = ((NC + 15) / 16) * 16;
-  static constexpr int BASE = NC * MP + NRM;
-  static constexpr int STRIDE = SM ? ((LANES == 4 && BASE % 32 == 0) ? BASE + 16 : BASE)
-                                   : NC * (MP + 1) + 4;
+  static constexpr int TAB = SM ? NC * MP + NRM : NC * (MP + 1) + 4;
+  static constexpr int BASE = TAB + 2 * NRM;
+  static constexpr int STRIDE = SM ? ((LANES == 4 && BASE % 32 == 0) ? BASE + 16 : BASE) : BASE;
 };
 
 // residency target: the shared-memory form holds a round's column pairs in
-// registers, (NC/2) * 2 * RPL floats; the register form holds RPL * NC
-// floats twice over (sweeps, then the epilogue's fresh gather)
+// registers, (NC/2) * 2 * RPL floats, the register form RPL * NC floats of columns
 template <int RPL, int NC, bool SM>
 constexpr int svd_minblocks() {
   return SM ? ((NC / 2) * 2 * RPL <= 64 ? PGSVT_SVD_MINBLOCKS_SM
@@ -397,16 +397,158 @@ __device__ int owner_sweeps(RegCols<4, NC>& A, float* As, int q, int nwin,
   return sweeps;
 }
 
+// The owner form for the other shapes (5x5 patches and larger, 8 or 16 lanes per
+// patch; 3 rows per lane): as owner_sweeps, lane q owning pairs q + LANES * i,
+// with the inner products, norms and convergence rules of register_sweeps'
+// replicated form below (a butterfly sum has the same bits in every lane, and a
+// reduce-scatter in its order the same as well).  The replicated rotations were
+// half of the instructions.  One round per loop iteration: three thrashed the
+// instruction cache (92 -> 120 ms for the 6 x 6 patches below).  With the epilogue
+// below, 21-frame windows of a batch of uneven sequences, GB300: 6 x 6 patches
+// 196.5 -> 92.2 ms, 8 x 8 patches 145.2 -> 64.2 ms; bound by instruction issue, a
+// fifth of it the column shift.
+template <int RPL, int LANES, int NC>
+constexpr bool kOwnerAny =
+#ifdef PGSVT_SVD_REPLICATED
+    false;
+#else
+    LANES >= 4 && LANES <= 16 && !kOwnerForm<RPL, LANES, NC>;
+#endif
+
+// One step of a reduce-scatter over an array of N partial sums: lanes whose
+// bit B of the lane number is set keep the odd ones, the others the even ones.
+template <int N, int B>
+__device__ __forceinline__ void scatter_step(float (&v)[N], int q) {
+  const bool odd = (q >> B) & 1;
+#pragma unroll
+  for (int j = 0; j < N / 2; ++j) {
+    const float keep = odd ? v[2 * j + 1] : v[2 * j];
+    const float send = odd ? v[2 * j] : v[2 * j + 1];
+    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 1 << B);
+  }
+}
+
+// Sums over the LANES lanes of v[0 .. LANES * S): the sum of entry q + LANES * i
+// ends in lane q's v[i] (lanes added in lanes_sum's order).
+template <int LANES, int S>
+__device__ __forceinline__ void reduce_scatter(float (&v)[LANES * S], int q) {
+  scatter_step<LANES * S, 0>(v, q);
+  if constexpr (LANES >= 4) scatter_step<LANES * S / 2, 1>(reinterpret_cast<float(&)[LANES * S / 2]>(v), q);
+  if constexpr (LANES >= 8) scatter_step<LANES * S / 4, 2>(reinterpret_cast<float(&)[LANES * S / 4]>(v), q);
+  if constexpr (LANES >= 16) scatter_step<LANES * S / 8, 3>(reinterpret_cast<float(&)[LANES * S / 8]>(v), q);
+}
+
+template <int RPL, int LANES, int NC, int CS>
+__device__ int owner_any_sweeps(RegCols<RPL, NC>& A, float* As, int q, int nwin,
+                                unsigned& fp64_tests) {
+  constexpr int NP = NC / 2;                      // pairs per round, pair 0 included
+  constexpr int SL = (NP + LANES - 1) / LANES;    // pairs owned by a lane
+  const int lane = threadIdx.x & 31, gbase = lane & ~(LANES - 1);
+  const int up = gbase | ((q + 1) & (LANES - 1)), dn = gbase | ((q + LANES - 1) & (LANES - 1));
+  // ballot bits of the lanes that own a pair = owner + LANES * i
+  constexpr unsigned kGroups = LANES == 4 ? 0x11111111u : (LANES == 8 ? 0x01010101u : 0x00010001u);
+  int sweeps = 0;
+#pragma unroll 1
+  for (; sweeps < kMaxSweeps; ++sweeps) {
+    float L[SL], R[SL];
+    {
+      float l[LANES * SL], r[LANES * SL];
+#pragma unroll
+      for (int p = 0; p < LANES * SL; ++p) {
+        l[p] = r[p] = 0.f;
+        if (p < NP) {
+#pragma unroll
+          for (int e = 0; e < RPL; ++e) l[p] = fmaf(A(e, p), A(e, p), l[p]);
+          if (p > 0)
+#pragma unroll
+            for (int e = 0; e < RPL; ++e) r[p] = fmaf(A(e, NC - 1 - p), A(e, NC - 1 - p), r[p]);
+        }
+      }
+      reduce_scatter<LANES, SL>(l, q);
+      reduce_scatter<LANES, SL>(r, q);
+#pragma unroll
+      for (int i = 0; i < SL; ++i) {
+        L[i] = l[i];
+        R[i] = r[i];
+      }
+    }
+    bool definite = false, band = false;
+#pragma unroll 1
+    for (int rd = 0; rd < NC - 1; ++rd) {
+      float g[LANES * SL];
+#pragma unroll
+      for (int p = 0; p < LANES * SL; ++p) {
+        g[p] = 0.f;
+        if (p >= 1 && p < NP)
+#pragma unroll
+          for (int r = 0; r < RPL; ++r) g[p] = fmaf(A(r, p), A(r, NC - 1 - p), g[p]);
+      }
+      reduce_scatter<LANES, SL>(g, q);
+      float cs_[SL], sn_[SL];
+      unsigned need_[SL];
+#pragma unroll
+      for (int i = 0; i < SL; ++i) {
+        const int po = q + LANES * i;
+        const float al = L[i], be = R[i], gv = g[i];
+        const float g2 = gv * gv, ab = al * be;
+        const bool need = po >= 1 && po < NP && g2 > (kTol * kTol) * ab;
+        cs_[i] = 1.f;
+        sn_[i] = 0.f;
+        if (need) {
+          rotation(al, be, gv, g2, ab, cs_[i], sn_[i], definite, band);
+          rotated_norms(al, be, gv, cs_[i], sn_[i], L[i], R[i]);
+        }
+        need_[i] = __ballot_sync(0xffffffffu, need);
+      }
+#pragma unroll
+      for (int pp = 1; pp < NP; ++pp) {
+        const int i = pp / LANES, o = pp % LANES;
+        if (!(need_[i] & (kGroups << o))) continue;  // warp-uniform
+        const float cs = __shfl_sync(0xffffffffu, cs_[i], gbase | o);
+        const float sn = __shfl_sync(0xffffffffu, sn_[i], gbase | o);
+        A.rotate(pp, NC - 1 - pp, cs, sn);
+      }
+      A.shift();
+      // the norms follow their columns (owner_sweeps)
+      float nl[SL], nr[SL];
+#pragma unroll
+      for (int i = 0; i < SL; ++i) {
+        const float vl = (q == 0) ? L[(i + 1) % SL] : L[i];
+        const float vr = (q == LANES - 1) ? (i == 0 ? 0.f : R[i > 0 ? i - 1 : 0])
+                                          : ((q == 0 && i == 0) ? L[0] : R[i]);
+        nl[i] = __shfl_sync(0xffffffffu, vl, up);
+        nr[i] = __shfl_sync(0xffffffffu, vr, dn);
+      }
+#pragma unroll
+      for (int i = 0; i < SL; ++i) {
+        L[i] = (q + LANES * i == NP - 1) ? R[i] : nl[i];
+        R[i] = nr[i];
+      }
+    }
+    if (__any_sync(0xffffffffu, definite)) continue;
+    if (!__any_sync(0xffffffffu, band)) break;
+#pragma unroll
+    for (int k = 0; k < NC; ++k)
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) As[k * CS + q * RPL + r] = A(r, k);
+    __syncwarp();
+    if (!fp64_check<RPL, LANES, CS>(As, q, nwin, fp64_tests)) break;
+  }
+  return sweeps;
+}
+
 // Jacobi sweeps with the columns in registers: the round-robin moves them one
 // position per round.  Column norms are recomputed exactly at every sweep's
 // start and updated in closed form after each rotation.  Returns the sweeps
 // with rotations; As ([NC][CS]) stages the columns for the FP64 check.
-// Patches of 4 lanes x 4 rows take the owner form above.
+// Patches of 4 lanes x 4 rows, and of 4 to 16 lanes, take the owner forms above.
 template <int RPL, int LANES, int NC, int CS, int U>
 __device__ int register_sweeps(RegCols<RPL, NC>& A, float* As, int q, int nwin,
                                unsigned& fp64_tests) {
   if constexpr (kOwnerForm<RPL, LANES, NC>)
     return owner_sweeps<NC, CS, kOwnerUnroll<NC>>(A, As, q, nwin, fp64_tests);
+  if constexpr (kOwnerAny<RPL, LANES, NC>)
+    return owner_any_sweeps<RPL, LANES, NC, CS>(A, As, q, nwin, fp64_tests);
   int sweeps = 0;
   float nrm[NC];
 #pragma unroll 1
@@ -696,7 +838,7 @@ __global__ void __launch_bounds__(128, (svd_minblocks<RPL, NC, SM>()))
   if (q == 0 && fp64_tests) atomicAdd(d.counters + 2, (unsigned long long)fp64_tests);
 
   // ---- epilogue
-  // singular values and their order
+  // singular values (in every lane), and the columns in shared memory
   float sv[NC];
 #pragma unroll
   for (int k = 0; k < NC; ++k) {
@@ -713,96 +855,123 @@ __global__ void __launch_bounds__(128, (svd_minblocks<RPL, NC, SM>()))
     }
     sv[k] = sqrtf(lanes_sum<LANES>(s));
   }
-  __syncwarp();
   float smax = sv[0];
 #pragma unroll
   for (int k = 1; k < NC; ++k) smax = fmaxf(smax, sv[k]);
-  const size_t NP = g.NP;
-  const int NCg = g.NC;
-  const int cslot = c;
-  float* svo = d.sv + (((size_t)w * 4 + cslot) * NCg) * NP + p;
-  float* hvo = d.hv + (((size_t)w * 4 + cslot) * NCg) * NP + p;
-  // column of rank t: walk the columns in decreasing order (ties by index)
+  // their order (ties by index), lane q ranking columns LANES * n + q; NaN ones
+  // have no rank, and a value without a column is -1
+  constexpr int CPL = (NC + LANES - 1) / LANES;
+  constexpr int NRM = SvdSmem<RPL, LANES, NC, SM>::NRM;
+  float* sorted = As + SvdSmem<RPL, LANES, NC, SM>::TAB;
+  int* order = reinterpret_cast<int*>(sorted + NRM);
   int nl = 0;
 #pragma unroll
-  for (int k = 0; k < NC; ++k) nl += can_survive(pb, sv[k], smax, (float)wc.upper);
-  int nl_max = nl;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) nl_max = max(nl_max, __shfl_xor_sync(0xffffffffu, nl_max, o));
-  if (live && q == 0) d.nlive[((size_t)w * 4 + c) * NP + p] = nl;
-
-  // B again (the Jacobi overwrote it) and the lambda-independent field G
-  const float* fld = (c == 0) ? d.fld0 : (c == 3 ? d.fld1 : d.fld2);
-  const float* fw_ = (pb.optimize && fld) ? fld + (size_t)w * g.cube() : nullptr;
-  float B[RPL][NC];
-#pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    size_t base = 0;
-    const bool colok = live && k < nwin && nl_max > 0;
-    if (colok) {
-      const uint32_t pc = __ldg(posw + (size_t)k * g.P + posidx);
-      base = (size_t)k * F + (pc & 0xffffu) + (size_t)(pc >> 16) * g.S;
+  for (int n = 0; n < CPL; ++n)
+    if (LANES * n + q < NC) {
+      sorted[LANES * n + q] = -1.f;
+      order[LANES * n + q] = 0;
     }
+  __syncwarp();
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) B[r][k] = (colok && roff[r] >= 0) ? value(base + roff[r]) : 0.f;
-  }
-  int prev = -1;
-  float prev_s = INFINITY;
-  for (int t = 0; t < NC; ++t) {
-    // next column in decreasing singular-value order
-    int ct = 0;
-    float st = -1.f;
+  for (int n = 0; n < CPL; ++n) {
+    const int k = LANES * n + q;
+    float s = 0.f;
 #pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      const float s = sv[k];
-      const bool after = (s < prev_s) || (s == prev_s && k > prev);
-      if (after && (s > st)) {
-        st = s;
-        ct = k;
+    for (int j = 0; j < LANES; ++j)
+      if (LANES * n + j < NC && q == j) s = sv[(LANES * n + j) % NC];
+    if (k < NC) {
+      nl += can_survive(pb, s, smax, (float)wc.upper);
+      int rank = 0;
+#pragma unroll
+      for (int j = 0; j < NC; ++j) rank += sv[j] > s || (sv[j] == s && j < k);
+      if (s == s) {
+        sorted[rank] = s;
+        order[rank] = k;
       }
     }
-    prev = ct;
-    prev_s = st;
-    const bool use = t < nl;
-    if (live && q == 0) {
-      svo[(size_t)t * NP] = st;
-      if (!use) hvo[(size_t)t * NP] = 0.f;
+  }
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) nl += __shfl_xor_sync(0xffffffffu, nl, o);
+  const int nl_max = __reduce_max_sync(0xffffffffu, nl);
+  __syncwarp();
+  const size_t NP = g.NP;
+  const int NCg = g.NC;
+  float* svo = d.sv + (((size_t)w * 4 + c) * NCg) * NP + p;
+  float* hvo = d.hv + (((size_t)w * 4 + c) * NCg) * NP + p;
+  if (live) {
+#pragma unroll
+    for (int n = 0; n < CPL; ++n) {
+      const int t = LANES * n + q;
+      if (t < NC) {
+        svo[(size_t)t * NP] = sorted[t];
+        if (t >= nl) hvo[(size_t)t * NP] = 0.f;
+      }
     }
-    if (t >= nl_max) continue;  // warp-uniform
-    const float inv = st > 0.f ? 1.f / st : 0.f;
-    float a[RPL];
+    if (q == 0) d.nlive[((size_t)w * 4 + c) * NP + p] = nl;
+  }
+
+  // the factors of the nl triplets that can survive, kFT side by side while
+  // one slice of B (again: the Jacobi overwrote it) and of the lambda-
+  // independent field G is in registers
+  constexpr int kFT = 4;
+  const float* fld = (c == 0) ? d.fld0 : (c == 3 ? d.fld1 : d.fld2);
+  const float* fw_ = (pb.optimize && fld) ? fld + (size_t)w * g.cube() : nullptr;
+  const bool keep = c == 0 && live && d.U0 && d.V0;
+  for (int t0 = 0; t0 < nl_max; t0 += kFT) {
+    const int nt = min(kFT, nl_max - t0);  // warp-uniform
+    float a[kFT][RPL], inv[kFT], h[kFT];   // u_t rows, 1 / s_t
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) a[r] = As[ct * CS + q * RPL + r] * inv;  // u_t rows
-    if (c == 0 && live && use && d.U0) {
+    for (int t = 0; t < kFT; ++t) {
+      const bool use = t0 + t < nl;
+      const float st = use ? sorted[t0 + t] : 0.f;
+      inv[t] = st > 0.f ? 1.f / st : 0.f;
+      h[t] = 0.f;
+      const float* col = As + (use ? order[t0 + t] : 0) * CS + q * RPL;
 #pragma unroll
-      for (int r = 0; r < RPL; ++r)
-        if (roff[r] >= 0) d.U0[g.u_at(w, p) + (t * g.M + q * RPL + r) * 32] = a[r];
+      for (int r = 0; r < RPL; ++r) {
+        a[t][r] = use ? col[r] * inv[t] : 0.f;
+        if (keep && use && roff[r] >= 0)
+          d.U0[g.u_at(w, p) + ((t0 + t) * g.M + q * RPL + r) * 32] = a[t][r];
+      }
     }
     // v_t = B^T u_t / s_t and h_t = u_t^T G v_t = sum_k v_k (G_k . u_t),
     // the latter from the lanes' partial sums with one reduction
-    float h = 0.f;
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      if (k >= nwin) break;  // uniform: keeps B[][k] in registers
-      float bu = 0.f;
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) bu = fmaf(B[r][k], a[r], bu);
-      bu = lanes_sum<LANES>(bu);
-      const float vk = bu * inv;
-      if (c == 0 && live && use && (k % LANES) == q && d.V0)
-        d.V0[g.v_at(w, p) + (t * nwin + k) * 32] = vk;
-      if (fw_ && live && use) {
+#pragma unroll 2
+    for (int k = 0; k < nwin; ++k) {
+      size_t base = 0;
+      if (live) {
         const uint32_t pc = __ldg(posw + (size_t)k * g.P + posidx);
-        const size_t base = (size_t)k * F + (pc & 0xffffu) + (size_t)(pc >> 16) * g.S;
+        base = (size_t)k * F + (pc & 0xffffu) + (size_t)(pc >> 16) * g.S;
+      }
+      float B[RPL], G[RPL];
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) {
+        B[r] = roff[r] >= 0 ? value(base + roff[r]) : 0.f;
+        G[r] = fw_ && roff[r] >= 0 ? __ldg(fw_ + base + roff[r]) : 0.f;
+      }
+#pragma unroll
+      for (int t = 0; t < kFT; ++t) {
+        if (t >= nt) break;
+        float bu = 0.f;
+#pragma unroll
+        for (int r = 0; r < RPL; ++r) bu = fmaf(B[r], a[t][r], bu);
+        const float vk = lanes_sum<LANES>(bu) * inv[t];
+        if (keep && t0 + t < nl && (k % LANES) == q)
+          d.V0[g.v_at(w, p) + ((t0 + t) * nwin + k) * 32] = vk;
         float gu = 0.f;
 #pragma unroll
-        for (int r = 0; r < RPL; ++r)
-          if (roff[r] >= 0) gu = fmaf(__ldg(fw_ + base + roff[r]), a[r], gu);
-        h = fmaf(vk, gu, h);
+        for (int r = 0; r < RPL; ++r) gu = fmaf(G[r], a[t][r], gu);
+        h[t] = fmaf(vk, gu, h[t]);
       }
     }
-    if (fw_) h = lanes_sum<LANES>(h);
-    if (live && use && q == 0) hvo[(size_t)t * NP] = h;
+    if (fw_) {
+#pragma unroll
+      for (int t = 0; t < kFT; ++t)
+        if (t < nt) {
+          const float hs = lanes_sum<LANES>(h[t]);
+          if (live && t0 + t < nl && q == 0) hvo[(size_t)(t0 + t) * NP] = hs;
+        }
+    }
   }
 }
 

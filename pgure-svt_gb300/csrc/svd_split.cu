@@ -295,13 +295,18 @@ __device__ __forceinline__ void store_sorted(const Problem& pb, const DeviceBuff
 #pragma unroll
     for (int n = 0; n < N4; ++n) rank[n] += sj > s[n] || (sj == s[n] && j < 4 * n + q);
   }
+  // (a NaN column has no rank, and a value without a column is -1)
   __syncwarp();
   int* ir = reinterpret_cast<int*>(slot + 16);
 #pragma unroll
+  for (int n = 0; n < N4; ++n) slot[4 * n + q] = -1.f;
+  __syncwarp();
+#pragma unroll
   for (int n = 0; n < N4; ++n)
     if (4 * n + q < NC) {
-      slot[rank[n]] = s[n];
-      ir[4 * n + q] = rank[n];
+      const bool num = s[n] == s[n];
+      if (num) slot[rank[n]] = s[n];
+      ir[4 * n + q] = num ? rank[n] : NC;
     }
   __syncwarp();
   if (live) {

@@ -94,3 +94,26 @@ def test_eval_round_of_any_length(capi, pkg, oracle, bs, T, side, nl):
     ro = oracle.risk_window(u, bs, 1, rows, cols, lams, *noise.values(), 3)
     r = res[0]["risks"][fw]
     assert np.abs(r - ro).max() <= 1e-4 * np.abs(ro).max()
+
+
+@pytest.mark.parametrize("bs,T", [(5, 7), (5, 15), (6, 21), (7, 9), (7, 21), (8, 21)])
+@pytest.mark.parametrize("expw", [0, 1])
+def test_owner_forms_are_identical(capi, pkg, bs, T, expw):
+    """The register forms whose pairs are owned by one of 8 or 16 lanes (one or
+    two pairs each) against the shared-memory form, whose rotations every lane
+    computes: bit for bit."""
+    noisy, _, (a, m, s) = _noisy(pkg, 31, T + 2, 70 + bs)
+    out = []
+    for form in (0, 3):
+        p = capi.default_params(traj_length=T, block_size=bs, motion_window=5, median_size=-1,
+                                random_seed=3, alpha=a / 300, mu=m / 300, sigma=s / 300,
+                                exp_weighting=expw, autotune=form)
+        if form == 0 and bs >= 7 and T <= 15:
+            p.autotune = 5  # the QR form is the default there; compare it loosely
+        Y, est, st, ex = capi.denoise_ex(noisy, p)
+        out.append((Y, est, ex["risk"], st.svd_variant))
+    if out[0][3] == 4:
+        assert np.abs(out[0][0] - out[1][0]).max() <= 2e-5 * np.abs(out[1][0]).max()
+        return
+    for x, y in zip(out[0][:3], out[1][:3]):
+        np.testing.assert_array_equal(x, y)
