@@ -23,27 +23,54 @@ constexpr float kStopRel = 1e-3f; // owner form: a sweep whose rotations were al
 // A lane's RPL rows of the NC columns in registers.  With an even RPL the rows
 // are packed in pairs (float2) so that a rotation updates two rows per
 // packed FP32x2 instruction; the results are those of the scalar FMAs.
+// The pairs are kept as 64-bit registers: as float2 values the compiler moved
+// their halves around for every packed instruction.
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 template <int RPL, int NC, bool PACK = (RPL % 2 == 0)>
 struct RegCols {
-  float2 v[RPL / 2][NC];
-  __device__ __forceinline__ float& operator()(int r, int k) {
-    return (r & 1) ? v[r >> 1][k].y : v[r >> 1][k].x;
+  uint64_t v[RPL / 2][NC];
+  __device__ __forceinline__ float operator()(int r, int k) const {
+    const float2 f = unpack2(v[r >> 1][k]);
+    return (r & 1) ? f.y : f.x;
+  }
+  __device__ __forceinline__ void put(int r, int k, float x) {  // rows in ascending order
+    v[r >> 1][k] = (r & 1) ? pack2(unpack2(v[r >> 1][k]).x, x) : pack2(x, 0.f);
   }
   // columns i, j <- (c a_i - s a_j, s a_i + c a_j)
   __device__ __forceinline__ void rotate(int i, int j, float cs, float sn) {
-    const float2 c2 = make_float2(cs, cs), s2 = make_float2(sn, sn), n2 = make_float2(-sn, -sn);
+    const uint64_t c2 = pack2(cs, cs), s2 = pack2(sn, sn), n2 = pack2(-sn, -sn);
 #pragma unroll
     for (int r = 0; r < RPL / 2; ++r) {
-      const float2 a = v[r][i], b = v[r][j];
-      v[r][i] = __ffma2_rn(c2, a, __fmul2_rn(n2, b));
-      v[r][j] = __ffma2_rn(s2, a, __fmul2_rn(c2, b));
+      const uint64_t a = v[r][i], b = v[r][j];
+      v[r][i] = fma2(c2, a, mul2(n2, b));
+      v[r][j] = fma2(s2, a, mul2(c2, b));
     }
   }
   // positions 0..NC-2 move down by one, position 0 to NC-2
   __device__ __forceinline__ void shift() {
 #pragma unroll
     for (int r = 0; r < RPL / 2; ++r) {
-      const float2 t = v[r][0];
+      const uint64_t t = v[r][0];
 #pragma unroll
       for (int k = 0; k < NC - 2; ++k) v[r][k] = v[r][k + 1];
       v[r][NC - 2] = t;
@@ -53,7 +80,8 @@ struct RegCols {
 template <int RPL, int NC>
 struct RegCols<RPL, NC, false> {
   float v[RPL][NC];
-  __device__ __forceinline__ float& operator()(int r, int k) { return v[r][k]; }
+  __device__ __forceinline__ float operator()(int r, int k) const { return v[r][k]; }
+  __device__ __forceinline__ void put(int r, int k, float x) { v[r][k] = x; }
   __device__ __forceinline__ void rotate(int i, int j, float cs, float sn) {
 #pragma unroll
     for (int r = 0; r < RPL; ++r) {
@@ -187,7 +215,7 @@ struct SvdSmem {
   static constexpr int MP = RPL * LANES;
   static constexpr int CS = SM ? MP : MP + 1;  // column stride
   static constexpr int NRM = ((NC + 15) / 16) * 16;
-  static constexpr int TAB = SM ? NC * MP + NRM : NC * (MP + 1) + 4;
+  static constexpr int TAB = SM ? NC * MP + NRM : (NC * (MP + 1) + 7) / 4 * 4;
   static constexpr int BASE = TAB + 2 * NRM;
   static constexpr int STRIDE = SM ? ((LANES == 4 && BASE % 32 == 0) ? BASE + 16 : BASE) : BASE;
 };
@@ -255,10 +283,11 @@ constexpr bool kOwnerForm =
 template <int NC>
 constexpr int kOwnerUnroll = ((NC - 1) % PGSVT_SVD_OWNER_UNROLL == 0) ? PGSVT_SVD_OWNER_UNROLL : 1;
 
-// Lane q's copy of one of four per-lane candidates (q = 0..3), from registers
-// with compile-time indices.
-__device__ __forceinline__ float sel4(int q, float a, float b, float c, float d) {
-  return (q & 2) ? ((q & 1) ? d : c) : ((q & 1) ? b : a);
+// rsqrtf of a value that is not denormal (rsqrtf's scaling left out, same result)
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
 // Jacobi sweeps for patches held by 4 lanes x 4 rows, with each pair's
@@ -266,44 +295,56 @@ __device__ __forceinline__ float sel4(int q, float a, float b, float c, float d)
 // reduce-scatter the round's inner products (two exchange steps) so that lane
 // q holds the complete inner products of pairs q and q + 4 (pair 0 is the
 // zero pad column's); it computes those pairs' rotations and rotated norms
-// and broadcasts them, and every lane applies every rotation to its rows.
-// The pairs, the rotation formulas and the convergence rules are those of
-// register_sweeps; pairs no patch of the warp needs to rotate are skipped
-// warp-uniformly (a patch that does not need a rotated pair applies the
-// identity, which leaves its columns and norms unchanged).
+// and hands them to the other lanes through shared memory as the packed
+// operands of the FP32x2 instructions (cs, cs, -sn, -sn and sn, sn), and every
+// lane applies every rotation to its rows.  The pairs, the rotation formulas
+// and the convergence rules are those of register_sweeps.  A pair that needs no
+// rotation gets the identity, which leaves its columns and norms unchanged: a
+// branch around each pair saved a fifth of the rotations and cost more than
+// that in register moves.  How a sweep ends (a definite, a near-degenerate, a
+// big rotation) is settled in the first rounds of all but the last sweeps, so
+// the flags are collected only while it is open.
+//
+// As: the patch's shared memory, 16-byte aligned (the FP64 check stages the
+// columns there as well).  Bound by instruction issue (68%) and the FP32 pipe
+// (49%).  256 x 256 x 100, GB300: 94.1 -> 81.3 ms in 13 launches.
 template <int NC, int CS, int U>
 __device__ int owner_sweeps(RegCols<4, NC>& A, float* As, int q, int nwin,
                             unsigned& fp64_tests) {
   constexpr int NP = NC / 2;  // pairs per round, pair 0 included
   static_assert(NP <= 8, "each lane owns two pairs");
-  const int gbase = (threadIdx.x & 31) & ~3;
+  const int lane = threadIdx.x & 31, gbase = lane & ~3;
   const int up = gbase | ((q + 1) & 3), dn = gbase | ((q + 3) & 3);
   const bool b1 = (q & 2) != 0, b0 = (q & 1) != 0;
+  // the round's rotations: 8 x float4, then 8 x float2; patches start on
+  // different banks (their stride is 16 mod 32 words)
+  float* xch = As + 4 * (lane >> 3);
   int sweeps = 0;
 #pragma unroll 1
   for (; sweeps < kMaxSweeps; ++sweeps) {
-    // squared norms of the owned pairs' columns: L[i] of position q + 4i,
-    // R[i] of position NC - 1 - q - 4i (the pad column's is 0)
+    // squared norms of the owned pairs' columns: L[i] of position q + 4i, R[i]
+    // of position NC - 1 - q - 4i (the pad column's is 0), reduce-scattered
+    // (the lanes added in lanes_sum's order)
     float L[2], R[2];
-    {
-      float nrm[NC];
 #pragma unroll
-      for (int k = 0; k < NC - 1; ++k) {
-        float t = 0.f;
+    for (int i = 0; i < 4; ++i) {
+      float t[4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) t = fmaf(A(r, k), A(r, k), t);
-        nrm[k] = lanes_sum<4>(t);
+      for (int j = 0; j < 4; ++j) {
+        const int k = i < 2 ? 4 * i + j : NC - 1 - 4 * (i - 2) - j;
+        t[j] = 0.f;
+        if (k < NC - 1)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) t[j] = fmaf(A(r, k), A(r, k), t[j]);
       }
-      nrm[NC - 1] = 0.f;
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        L[i] = sel4(q, nrm[(4 * i) % NC], nrm[(4 * i + 1) % NC], nrm[(4 * i + 2) % NC],
-                    nrm[(4 * i + 3) % NC]);
-        R[i] = sel4(q, nrm[NC - 1 - 4 * i], nrm[NC - 2 - 4 * i], nrm[NC - 3 - 4 * i],
-                    nrm[NC - 4 - 4 * i]);
-      }
+      const float u0 = (b0 ? t[1] : t[0]) + __shfl_xor_sync(0xffffffffu, b0 ? t[0] : t[1], 1);
+      const float u1 = (b0 ? t[3] : t[2]) + __shfl_xor_sync(0xffffffffu, b0 ? t[2] : t[3], 1);
+      const float v = (b1 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b1 ? u0 : u1, 2);
+      if (i < 2) L[i] = v;
+      else R[i - 2] = v;
     }
-    bool definite = false, band = false, big = false;
+    unsigned flags = 0u;  // 1: a definite rotation, 2: a near-degenerate one, 4: a big one
+    bool open = true;     // the sweep's outcome is not settled yet
 #pragma unroll U
     for (int rd = 0; rd < NC - 1; ++rd) {
       // this lane's partial inner products of the round's pairs
@@ -311,8 +352,8 @@ __device__ int owner_sweeps(RegCols<4, NC>& A, float* As, int q, int nwin,
 #pragma unroll
       for (int pp = 0; pp < 8; ++pp) {
         if (pp >= 1 && pp < NP) {
-          float2 t = __fmul2_rn(A.v[0][pp], A.v[0][NC - 1 - pp]);
-          t = __ffma2_rn(A.v[1][pp], A.v[1][NC - 1 - pp], t);
+          const float2 t = unpack2(fma2(A.v[1][pp], A.v[1][NC - 1 - pp],
+                                        mul2(A.v[0][pp], A.v[0][NC - 1 - pp])));
           gm[pp] = t.x + t.y;
         } else {
           gm[pp] = 0.f;
@@ -329,35 +370,56 @@ __device__ int owner_sweeps(RegCols<4, NC>& A, float* As, int q, int nwin,
         const float send = b1 ? gm[lo] : gm[lo + 2];
         h[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
       }
-      float cs_[2], sn_[2];
-      bool need_[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const float keep = b0 ? h[2 * i + 1] : h[2 * i];
         const float send = b0 ? h[2 * i] : h[2 * i + 1];
         const float gv = keep + __shfl_xor_sync(0xffffffffu, send, 1);
         const int po = q + 4 * i;  // the owned pair
+        const bool own = (i > 0 || q > 0) && (NP == 8 || po < NP);
         const float al = L[i], be = R[i];
         const float g2 = gv * gv, ab = al * be;
-        need_[i] = po >= 1 && po < NP && g2 > (kTol * kTol) * ab;
-        cs_[i] = 1.f;
-        sn_[i] = 0.f;
-        if (need_[i]) {
-          rotation(al, be, gv, g2, ab, cs_[i], sn_[i], definite, band);
-          big |= g2 > (kStopRel * kStopRel) * ab;
-          rotated_norms(al, be, gv, cs_[i], sn_[i], L[i], R[i]);
+        const bool need = own && g2 > (kTol * kTol) * ab;
+        const float dd = be - al;
+        if (open) {  // warp-uniform
+          const bool degen = fabsf(dd) <= kDegen * (al + be);
+          if (need) {
+            flags |= (degen && g2 <= (kBand * kBand * kTol * kTol) * ab) ? 2u : 1u;
+            if (g2 > (kStopRel * kStopRel) * ab) flags |= 4u;
+          }
+        }
+        // rotation(), rotated_norms(); the identity where it is not needed
+        const float ir = rsqrtf(fmaf(dd, dd, 4.f * g2));
+        const float hh = fmaf(0.5f * fabsf(dd), ir, 0.5f);
+        const float rh = rsqrt_normal(hh);
+        float cs = hh * rh;
+        float sn = (dd >= 0.f ? gv : -gv) * ir * rh;
+        float ni, nj;
+        rotated_norms(al, be, gv, cs, sn, ni, nj);
+        cs = need ? cs : 1.f;
+        sn = need ? sn : 0.f;
+        L[i] = need ? ni : al;
+        R[i] = need ? nj : be;
+        if (NP == 8 || po < NP) {
+          *reinterpret_cast<float4*>(xch + 4 * po) = make_float4(cs, cs, -sn, -sn);
+          *reinterpret_cast<float2*>(xch + 48 + 2 * po) = make_float2(sn, sn);
         }
       }
-      const unsigned m0 = __ballot_sync(0xffffffffu, need_[0]);
-      const unsigned m1 = __ballot_sync(0xffffffffu, need_[1]);
+      if (open) {
+        const unsigned f = __reduce_or_sync(0xffffffffu, flags);
+        open = !((f & 1u) && (f & 6u));
+      }
+      __syncwarp();
 #pragma unroll
       for (int pp = 1; pp < NP; ++pp) {
-        const int i = pp >> 2;
-        if (!((i ? m1 : m0) & (0x11111111u << (pp & 3)))) continue;  // warp-uniform
-        const int src = gbase | (pp & 3);
-        const float cs = __shfl_sync(0xffffffffu, cs_[i], src);
-        const float sn = __shfl_sync(0xffffffffu, sn_[i], src);
-        A.rotate(pp, NC - 1 - pp, cs, sn);
+        const ulonglong2 cn = *reinterpret_cast<const ulonglong2*>(xch + 4 * pp);
+        const uint64_t s2 = *reinterpret_cast<const uint64_t*>(xch + 48 + 2 * pp);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const uint64_t a = A.v[r][pp], b = A.v[r][NC - 1 - pp];
+          A.v[r][pp] = fma2(cn.x, a, mul2(cn.y, b));
+          A.v[r][NC - 1 - pp] = fma2(s2, a, mul2(cn.x, b));
+        }
       }
       A.shift();
       // the norms follow their columns to the next round's owners: the new
@@ -378,15 +440,17 @@ __device__ int owner_sweeps(RegCols<4, NC>& A, float* As, int q, int nwin,
         L[i] = (q + 4 * i == NP - 1) ? R[i] : nl[i];
         R[i] = nr[i];
       }
+      __syncwarp();  // the next round writes xch
     }
-    if (__any_sync(0xffffffffu, definite)) {
+    const unsigned f = __reduce_or_sync(0xffffffffu, flags);
+    if (f & 1u) {
       // every rotation of the sweep was smaller than kStopRel: convergence is
       // quadratic, so the inner products it leaves are of order kStopRel^2,
       // the rotation threshold, and the next sweep would be the last
-      if (!__any_sync(0xffffffffu, band) && !__any_sync(0xffffffffu, big)) break;
+      if (!(f & 6u)) break;
       continue;
     }
-    if (!__any_sync(0xffffffffu, band)) break;
+    if (!(f & 2u)) break;
 #pragma unroll
     for (int k = 0; k < NC; ++k)
 #pragma unroll
@@ -394,6 +458,7 @@ __device__ int owner_sweeps(RegCols<4, NC>& A, float* As, int q, int nwin,
     __syncwarp();
     if (!fp64_check<4, 4, CS>(As, q, nwin, fp64_tests)) break;
   }
+  __syncwarp();
   return sweeps;
 }
 
@@ -659,7 +724,7 @@ __global__ void __launch_bounds__(128, (svd_minblocks<RPL, NC, SM>()))
     return v;
   };
 
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   float* As = smem + (size_t)(wib * GROUPS + grp) * GSTRIDE;  // [NC][CS]
 
   // ---- gather B (svt.hpp:101-109)
@@ -676,7 +741,7 @@ __global__ void __launch_bounds__(128, (svd_minblocks<RPL, NC, SM>()))
     for (int r = 0; r < RPL; ++r) {
       const float v = (colok && roff[r] >= 0) ? value(base + roff[r]) : 0.f;
       if constexpr (SM) As[k * CS + q * RPL + r] = v;
-      else A(r, k) = v;
+      else A.put(r, k, v);
     }
   }
 

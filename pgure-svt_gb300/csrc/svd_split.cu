@@ -348,14 +348,14 @@ __global__ void __launch_bounds__(128, 4) k_xsweep(Problem pb, DeviceBuffers d, 
   const int slot = threadIdx.x >> 2;  // patch of the block (32 per block)
   const int gid = blockIdx.x * 32 + slot;
   const bool live = gid < nitems;
-  __shared__ float Xs[32][NC * CS];
+  __shared__ __align__(16) float Xs[32][(NC * CS + 3) / 4 * 4];
   float* X = Xs[slot];
   const float* xi = d.xq + (size_t)(live ? gid : 0) * NC * D::XR;
   RegCols<RX, NC> A;
 #pragma unroll
   for (int k = 0; k < NC; ++k)
 #pragma unroll
-    for (int r = 0; r < RX; ++r) A(r, k) = live ? __ldg(xi + k * D::XR + q * RX + r) : 0.f;
+    for (int r = 0; r < RX; ++r) A.put(r, k, live ? __ldg(xi + k * D::XR + q * RX + r) : 0.f);
   unsigned fp64_tests = 0;
   const int sweeps = register_sweeps<RX, 4, NC, CS, 1>(A, X, q, pb.g.nwin, fp64_tests);
   if (lane == 0) atomicAdd(d.counters + 1, (unsigned long long)(sweeps + 1));
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(128, 4) k_bsweep(Problem pb, DeviceBuffers d, 
   const int gid = blockIdx.x * 32 + slot;
   const bool live = gid < nitems;
   const int nwin = g.nwin, M = g.M;
-  __shared__ float Xs[32][NC * CS];
+  __shared__ __align__(16) float Xs[32][(NC * CS + 3) / 4 * 4];
   float* X = Xs[slot];
   PatchSrc src;
   {
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(128, 4) k_bsweep(Problem pb, DeviceBuffers d, 
     const bool colok = live && k < nwin;
     const size_t b = colok ? src.base(k) : 0;
 #pragma unroll
-    for (int r = 0; r < RX; ++r) A(r, k) = (colok && roff[r] >= 0) ? src.value(b + roff[r]) : 0.f;
+    for (int r = 0; r < RX; ++r) A.put(r, k, (colok && roff[r] >= 0) ? src.value(b + roff[r]) : 0.f);
   }
   unsigned fp64_tests = 0;
   const int sweeps = register_sweeps<RX, 4, NC, CS, 1>(A, X, q, nwin, fp64_tests);
