@@ -20,9 +20,9 @@ constexpr float kStopRel = 1e-3f; // owner form: a sweep whose rotations were al
 // paired; after each round positions 0..NC-2 shift by one.  NC-1 rounds pair
 // every two columns once and bring every column back to its position.
 
-// A lane's RPL rows of the NC columns in registers.  With an even RPL the rows
-// are packed in pairs (float2) so that a rotation updates two rows per
-// packed FP32x2 instruction; the results are those of the scalar FMAs.
+// A lane's RPL rows of the NC columns in registers.  The rows are packed in
+// pairs (the last of an odd number alone) so that a rotation updates two rows
+// per packed FP32x2 instruction; the results are those of the scalar FMAs.
 // The pairs are kept as 64-bit registers: as float2 values the compiler moved
 // their halves around for every packed instruction.
 __device__ __forceinline__ uint64_t pack2(float x, float y) {
@@ -46,57 +46,49 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   return d;
 }
 
-template <int RPL, int NC, bool PACK = (RPL % 2 == 0)>
+template <int RPL, int NC>
 struct RegCols {
-  uint64_t v[RPL / 2][NC];
+  static constexpr int H = RPL / 2;
+  uint64_t v[H > 0 ? H : 1][NC];
+  float w[NC];  // the last row of an odd number
   __device__ __forceinline__ float operator()(int r, int k) const {
+    if (r == 2 * H) return w[k];
     const float2 f = unpack2(v[r >> 1][k]);
     return (r & 1) ? f.y : f.x;
   }
   __device__ __forceinline__ void put(int r, int k, float x) {  // rows in ascending order
-    v[r >> 1][k] = (r & 1) ? pack2(unpack2(v[r >> 1][k]).x, x) : pack2(x, 0.f);
+    if (r == 2 * H) w[k] = x;
+    else v[r >> 1][k] = (r & 1) ? pack2(unpack2(v[r >> 1][k]).x, x) : pack2(x, 0.f);
   }
   // columns i, j <- (c a_i - s a_j, s a_i + c a_j)
   __device__ __forceinline__ void rotate(int i, int j, float cs, float sn) {
     const uint64_t c2 = pack2(cs, cs), s2 = pack2(sn, sn), n2 = pack2(-sn, -sn);
 #pragma unroll
-    for (int r = 0; r < RPL / 2; ++r) {
+    for (int r = 0; r < H; ++r) {
       const uint64_t a = v[r][i], b = v[r][j];
       v[r][i] = fma2(c2, a, mul2(n2, b));
       v[r][j] = fma2(s2, a, mul2(c2, b));
+    }
+    if constexpr (RPL % 2 == 1) {
+      const float a = w[i], b = w[j];
+      w[i] = fmaf(cs, a, -sn * b);
+      w[j] = fmaf(sn, a, cs * b);
     }
   }
   // positions 0..NC-2 move down by one, position 0 to NC-2
   __device__ __forceinline__ void shift() {
 #pragma unroll
-    for (int r = 0; r < RPL / 2; ++r) {
+    for (int r = 0; r < H; ++r) {
       const uint64_t t = v[r][0];
 #pragma unroll
       for (int k = 0; k < NC - 2; ++k) v[r][k] = v[r][k + 1];
       v[r][NC - 2] = t;
     }
-  }
-};
-template <int RPL, int NC>
-struct RegCols<RPL, NC, false> {
-  float v[RPL][NC];
-  __device__ __forceinline__ float operator()(int r, int k) const { return v[r][k]; }
-  __device__ __forceinline__ void put(int r, int k, float x) { v[r][k] = x; }
-  __device__ __forceinline__ void rotate(int i, int j, float cs, float sn) {
+    if constexpr (RPL % 2 == 1) {
+      const float t = w[0];
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const float a = v[r][i], b = v[r][j];
-      v[r][i] = fmaf(cs, a, -sn * b);
-      v[r][j] = fmaf(sn, a, cs * b);
-    }
-  }
-  __device__ __forceinline__ void shift() {
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const float t = v[r][0];
-#pragma unroll
-      for (int k = 0; k < NC - 2; ++k) v[r][k] = v[r][k + 1];
-      v[r][NC - 2] = t;
+      for (int k = 0; k < NC - 2; ++k) w[k] = w[k + 1];
+      w[NC - 2] = t;
     }
   }
 };
@@ -468,10 +460,11 @@ __device__ int owner_sweeps(RegCols<4, NC>& A, float* As, int q, int nwin,
 // replicated form below (a butterfly sum has the same bits in every lane, and a
 // reduce-scatter in its order the same as well).  The replicated rotations were
 // half of the instructions.  One round per loop iteration: three thrashed the
-// instruction cache (92 -> 120 ms for the 6 x 6 patches below).  With the epilogue
+// instruction cache (a third slower).  With the epilogue
 // below, 21-frame windows of a batch of uneven sequences, GB300: 6 x 6 patches
-// 196.5 -> 92.2 ms, 8 x 8 patches 145.2 -> 64.2 ms; bound by instruction issue, a
-// fifth of it the column shift.
+// 196.5 -> 80.1 ms, 8 x 8 patches 145.2 -> 59.9 ms (with branches around the pairs that
+// need no rotation 92.2 and 64.2); bound by instruction issue, a fifth of it the
+// column shift.
 template <int RPL, int LANES, int NC>
 constexpr bool kOwnerAny =
 #ifdef PGSVT_SVD_REPLICATED
@@ -510,8 +503,6 @@ __device__ int owner_any_sweeps(RegCols<RPL, NC>& A, float* As, int q, int nwin,
   constexpr int SL = (NP + LANES - 1) / LANES;    // pairs owned by a lane
   const int lane = threadIdx.x & 31, gbase = lane & ~(LANES - 1);
   const int up = gbase | ((q + 1) & (LANES - 1)), dn = gbase | ((q + LANES - 1) & (LANES - 1));
-  // ballot bits of the lanes that own a pair = owner + LANES * i
-  constexpr unsigned kGroups = LANES == 4 ? 0x11111111u : (LANES == 8 ? 0x01010101u : 0x00010001u);
   int sweeps = 0;
 #pragma unroll 1
   for (; sweeps < kMaxSweeps; ++sweeps) {
@@ -550,7 +541,6 @@ __device__ int owner_any_sweeps(RegCols<RPL, NC>& A, float* As, int q, int nwin,
       }
       reduce_scatter<LANES, SL>(g, q);
       float cs_[SL], sn_[SL];
-      unsigned need_[SL];
 #pragma unroll
       for (int i = 0; i < SL; ++i) {
         const int po = q + LANES * i;
@@ -563,12 +553,10 @@ __device__ int owner_any_sweeps(RegCols<RPL, NC>& A, float* As, int q, int nwin,
           rotation(al, be, gv, g2, ab, cs_[i], sn_[i], definite, band);
           rotated_norms(al, be, gv, cs_[i], sn_[i], L[i], R[i]);
         }
-        need_[i] = __ballot_sync(0xffffffffu, need);
       }
 #pragma unroll
       for (int pp = 1; pp < NP; ++pp) {
         const int i = pp / LANES, o = pp % LANES;
-        if (!(need_[i] & (kGroups << o))) continue;  // warp-uniform
         const float cs = __shfl_sync(0xffffffffu, cs_[i], gbase | o);
         const float sn = __shfl_sync(0xffffffffu, sn_[i], gbase | o);
         A.rotate(pp, NC - 1 - pp, cs, sn);
