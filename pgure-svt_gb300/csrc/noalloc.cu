@@ -73,6 +73,13 @@ std::mutex g_mu;
 void* g_addr[64];                // scratch address per device, resolved on first use ...
 unsigned long long g_ctx[64];    // ... in the context with this identifier
 
+int fail(int code, const std::string& m) {
+  set_last_error(m);  // read back with pgsvt_last_error()
+  return code;
+}
+
+}  // namespace
+
 // Identifier of the calling thread's current CUDA context (0: none yet).  A
 // device reset destroys the context that held the scratch and a new one gets
 // a new identifier, so the address is resolved again after a reset.  The
@@ -102,12 +109,6 @@ unsigned long long current_context_id() {
   return id;
 }
 
-int fail(int code, const std::string& m) {
-  set_last_error(m);  // read back with pgsvt_last_error()
-  return code;
-}
-
-}  // namespace
 }  // namespace pgsvt
 
 using namespace pgsvt;

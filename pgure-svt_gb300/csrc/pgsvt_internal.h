@@ -43,14 +43,16 @@ namespace pgsvt {
 // patch list here, so all of them keep the same patches in the same order.
 inline std::vector<int32_t> kept_patches(int S, int bs, int ov) {
   const int64_t nMbs = S - bs;
-  std::vector<int64_t> v;
+  std::vector<uint8_t> keep((size_t)((nMbs + 1) * (nMbs + 1)), 0);
   for (int64_t i = 0; i < 1 + nMbs; i += ov)
-    for (int64_t j = 0; j < 1 + nMbs; j += ov) v.push_back(i * nMbs + j);
-  for (int64_t i = 0; i < 1 + nMbs; i += ov) v.push_back((nMbs + 1) * i + nMbs);
-  for (int64_t i = 0; i < 1 + nMbs; i += ov) v.push_back((nMbs + 1) * nMbs + i);
-  std::sort(v.begin(), v.end());
-  v.erase(std::unique(v.begin(), v.end()), v.end());
-  return std::vector<int32_t>(v.begin(), v.end());
+    for (int64_t j = 0; j < 1 + nMbs; j += ov) keep[i * nMbs + j] = 1;
+  for (int64_t i = 0; i < 1 + nMbs; i += ov) keep[(nMbs + 1) * i + nMbs] = 1;
+  for (int64_t i = 0; i < 1 + nMbs; i += ov) keep[(nMbs + 1) * nMbs + i] = 1;
+  std::vector<int32_t> v;
+  v.reserve(keep.size());
+  for (size_t it = 0; it < keep.size(); ++it)
+    if (keep[it]) v.push_back((int32_t)it);
+  return v;
 }
 
 constexpr int kMaxK = 16;          // lambda values per evaluation round
@@ -316,6 +318,9 @@ cudaError_t lambda_grad(const float* m, const void* wbf, const float* feat, cons
 size_t lambda_act_floats(int n);
 cudaError_t lambda_train_epoch(const LambdaTrain& t, cudaStream_t s);
 cudaError_t lambda_attrs();
+
+// identifier of the calling thread's current CUDA context (0: none yet)
+unsigned long long current_context_id();
 
 // message returned by pgsvt_last_error() on the calling thread
 void set_last_error(const std::string& m);
