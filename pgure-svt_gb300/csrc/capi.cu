@@ -45,54 +45,75 @@ struct Fail : std::runtime_error {
   } while (0)
 
 // ---------------------------------------------------------------------------
-// Probes: pcg64 (O'Neill's PCG, 128-bit LCG with XSL-RR output, seeded as the
-// reference's RNG.seed(randomSeed), pgure.hpp:52-59) feeding
-// std::bernoulli_distribution semantics (one 64-bit draw scaled by 2^-64,
-// true when below p), in column-major cube order, delta1 then delta2
-// (pgure.hpp:167-186).
+// pcg64 (O'Neill's PCG, 128-bit LCG with XSL-RR output, seeded as the
+// reference's RNG.seed(randomSeed), pgure.hpp:52-59).
 class Pcg64 {
  public:
   using u128 = unsigned __int128;
-  explicit Pcg64(u128 seed) {
-    inc_ = ((u128)6364136223846793005ULL << 64) | 1442695040888963407ULL;
-    state_ = (seed + inc_) * mult() + inc_;
-  }
+  explicit Pcg64(u128 seed) { state_ = (seed + inc()) * mult() + inc(); }
   uint64_t operator()() {
-    state_ = state_ * mult() + inc_;
+    state_ = state_ * mult() + inc();
     const uint64_t hi = (uint64_t)(state_ >> 64), lo = (uint64_t)state_;
     const unsigned rot = (unsigned)(hi >> 58);
     const uint64_t x = hi ^ lo;
     return (x >> rot) | (x << ((64u - rot) & 63u));
   }
+  u128 state() const { return state_; }
+  static u128 mult() { return ((u128)2549297995355413924ULL << 64) | 4865540595714422341ULL; }
+  static u128 inc() { return ((u128)6364136223846793005ULL << 64) | 1442695040888963407ULL; }
 
  private:
-  static u128 mult() { return ((u128)2549297995355413924ULL << 64) | 4865540595714422341ULL; }
-  u128 state_, inc_;
+  u128 state_;
 };
-
-bool draw(Pcg64& g, double p) {
-  double u = (double)g() / 18446744073709551616.0;
-  if (u >= 1.0) u = std::nextafter(1.0, 0.0);
-  return u < p;
-}
 
 double probe_vp() {
   const double kappa = 1.0;
   return 0.5 + 0.5 * kappa / std::sqrt(kappa * kappa + 4);
 }
 
-void make_probes(int64_t seed, size_t n, int8_t* d1, int8_t* d2code) {
-  Pcg64::u128 s;
-  if (seed >= 0) {
-    s = (Pcg64::u128)(uint64_t)seed;
-  } else {
-    std::random_device rd;
-    s = ((Pcg64::u128)(((uint64_t)rd() << 32) | rd()) << 64) | (((uint64_t)rd() << 32) | rd());
+// std::bernoulli_distribution semantics: one 64-bit draw scaled by 2^-64 (and
+// kept below 1), true when below p.  The scaling is monotone, so the draws that
+// are true are those below one integer.
+uint64_t draws_below(double p) {
+  uint64_t lo = 0, hi = ~0ULL;  // the least draw that is not true lies in [lo, hi]
+  while (lo < hi) {
+    const uint64_t mid = lo + (hi - lo) / 2;
+    double u = (double)mid / 18446744073709551616.0;
+    if (u >= 1.0) u = std::nextafter(1.0, 0.0);
+    if (u < p) lo = mid + 1;
+    else hi = mid;
   }
-  Pcg64 g(s);
-  const double vP = probe_vp();
-  for (size_t i = 0; i < n; ++i) d1[i] = draw(g, 0.5) ? -1 : 1;
-  for (size_t i = 0; i < n; ++i) d2code[i] = draw(g, vP) ? 1 : 0;
+  return lo;
+}
+
+// The probe streams of `windows` windows: one seed, or fresh entropy per window
+// (pgure.hpp:54-55).
+ProbeStream probe_stream(int64_t seed, int windows) {
+  ProbeStream ps{};
+  for (int w = 0; w < windows; ++w) {
+    Pcg64::u128 s;
+    if (seed >= 0) {
+      s = (Pcg64::u128)(uint64_t)seed;
+    } else {
+      std::random_device rd;
+      s = ((Pcg64::u128)(((uint64_t)rd() << 32) | rd()) << 64) | (((uint64_t)rd() << 32) | rd());
+    }
+    const Pcg64::u128 st = Pcg64(s).state();
+    ps.hi[w] = (uint64_t)(st >> 64);
+    ps.lo[w] = (uint64_t)st;
+  }
+  Pcg64::u128 m = Pcg64::mult(), c = Pcg64::inc();
+  for (int b = 0; b < 40; ++b) {  // 2^b steps: x -> m x + c
+    ps.mul_hi[b] = (uint64_t)(m >> 64);
+    ps.mul_lo[b] = (uint64_t)m;
+    ps.add_hi[b] = (uint64_t)(c >> 64);
+    ps.add_lo[b] = (uint64_t)c;
+    c = (m + 1) * c;
+    m = m * m;
+  }
+  ps.below1 = draws_below(0.5);
+  ps.below2 = draws_below(probe_vp());
+  return ps;
 }
 
 // ---------------------------------------------------------------------------
@@ -501,7 +522,6 @@ struct Lane {
   cudaStream_t s = nullptr;
   bool own = false;
   DeviceBuffers d{};
-  std::vector<int8_t> hp1, hp2;
   int8_t* pd1 = nullptr;
   int8_t* pd2 = nullptr;
   std::unique_ptr<StageClock> clk;
@@ -750,14 +770,9 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
   int8_t* sp1 = nullptr;
   int8_t* sp2 = nullptr;
   if (pb.optimize && shared_probes) {  // one probe set for every window (pgure.hpp:52-59)
-    std::vector<int8_t> h1(C), h2(C);
-    make_probes(p.random_seed, C, h1.data(), h2.data());
     sp1 = mem.arr<int8_t>(C);
     sp2 = mem.arr<int8_t>(C);
-    PGSVT_CK(cudaMemcpyAsync(sp1, h1.data(), C, cudaMemcpyHostToDevice, s));
-    PGSVT_CK(cudaMemcpyAsync(sp2, h2.data(), C, cudaMemcpyHostToDevice, s));
-    PGSVT_CK(cudaStreamSynchronize(s));  // h1/h2 go out of scope
-    stats.h2d += 2 * C;
+    check_launch(launch_probes(probe_stream(p.random_seed, 1), 1, C, sp1, sp2, s), stats);
   }
   if (fb > 0 || fe < nimg) {
     PGSVT_CK(cudaMemsetAsync(Y_dev, 0, sizeof(double) * (size_t)nimg * F, s));
@@ -883,8 +898,6 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
       } else {  // fresh entropy per window (pgure.hpp:54-55)
         L.pd1 = mem.arr<int8_t>((size_t)W * C);
         L.pd2 = mem.arr<int8_t>((size_t)W * C);
-        L.hp1.resize((size_t)W * C);
-        L.hp2.resize((size_t)W * C);
         d.d1 = L.pd1;
         d.d2code = L.pd2;
         d.probe_stride = C;
@@ -901,15 +914,9 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     d.win0 = win0;
     d.chains = dch + (size_t)win0 * nchains;
     StageClock& clk = *L.clk;
-    if (pb.optimize && !shared_probes) {
-      PGSVT_CK(cudaStreamSynchronize(L.s));  // the lane's host buffers are reused
-      for (int w = 0; w < pbb.W; ++w)
-        make_probes(-1, C, L.hp1.data() + (size_t)w * C, L.hp2.data() + (size_t)w * C);
-      PGSVT_CK(cudaMemcpyAsync(L.pd1, L.hp1.data(), (size_t)pbb.W * C, cudaMemcpyHostToDevice, L.s));
-      PGSVT_CK(cudaMemcpyAsync(L.pd2, L.hp2.data(), (size_t)pbb.W * C, cudaMemcpyHostToDevice, L.s));
-      stats.h2d += 2 * (size_t)pbb.W * C;
-    }
-    clk.mark(7);  // probe uploads and other gaps
+    if (pb.optimize && !shared_probes)
+      check_launch(launch_probes(probe_stream(-1, pbb.W), pbb.W, C, L.pd1, L.pd2, L.s), stats);
+    clk.mark(7);  // per-window probes and gaps
     check_launch(launch_window_setup(pbb, d, L.s), stats, 2);
     if (estimate) check_launch(launch_noise_apply(pbb, d, est_win, fb, L.s), stats);
     clk.mark(1);
@@ -1712,12 +1719,9 @@ int pgsvt_risk_window(const double* u, uint32_t nrows, uint32_t nwin, uint32_t b
     ow.d.fld0 = ow.mem.arr<float>(C);
     ow.d.fld2 = ow.mem.arr<float>(C);
     ow.d.fld1 = ncopies == 4 ? ow.mem.arr<float>(C) : nullptr;
-    std::vector<int8_t> h1(C), h2(C);
-    make_probes(random_seed, C, h1.data(), h2.data());
     int8_t* d1 = ow.mem.arr<int8_t>(C);
     int8_t* d2 = ow.mem.arr<int8_t>(C);
-    PGSVT_CK(cudaMemcpyAsync(d1, h1.data(), C, cudaMemcpyHostToDevice, ow.s));
-    PGSVT_CK(cudaMemcpyAsync(d2, h2.data(), C, cudaMemcpyHostToDevice, ow.s));
+    PGSVT_CK(launch_probes(probe_stream(random_seed, 1), 1, C, d1, d2, ow.s));
     ow.d.d1 = d1;
     ow.d.d2code = d2;
     ow.d.probe_stride = 0;

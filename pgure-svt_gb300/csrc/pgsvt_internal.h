@@ -231,6 +231,18 @@ cudaError_t launch_frame_max(const float* xs, const double* x64, int nimg, size_
 cudaError_t launch_median(const float* xs, const double* x64, int nimg, int S, int r, float* zs,
                           cudaStream_t s);
 constexpr int kMaxMedian = 15;     // median pre-filter radius supported
+// Probe streams of up to kProbeWindows windows (prep.cu): the seeded generator
+// states, the LCG's 2^b-step multipliers and increments, and the least output
+// that is not below each probability.
+constexpr int kProbeWindows = 32;
+struct ProbeStream {
+  uint64_t hi[kProbeWindows], lo[kProbeWindows];
+  uint64_t mul_hi[40], mul_lo[40], add_hi[40], add_lo[40];
+  uint64_t below1, below2;
+};
+// delta1 (-1 / 1) and delta2 codes (1 / 0), n values per window each
+cudaError_t launch_probes(const ProbeStream& ps, int windows, size_t n, int8_t* d1, int8_t* d2,
+                          cudaStream_t s);
 cudaError_t launch_window_setup(const Problem& pb, const DeviceBuffers& d, cudaStream_t s);
 cudaError_t launch_window_norm_only(const Problem& pb, const DeviceBuffers& d, cudaStream_t s);
 cudaError_t launch_arps(const Problem& pb, const DeviceBuffers& d, cudaStream_t s);

@@ -225,4 +225,56 @@ cudaError_t launch_window_norm_only(const Problem& pb, const DeviceBuffers& d, c
   return cudaGetLastError();
 }
 
+// ---- PGURE probes (pgure.hpp:52-59,167-186)
+//
+// Draws 0 .. n-1 of a window's pcg64 stream give delta1, draws n .. 2n-1 delta2.
+// The generator is a 128-bit LCG, so any draw's state is reached in about
+// log2(draw) multiplications (F. Brown, "Random number generation with
+// arbitrary strides", 1994): a thread jumps to its 16 draws and writes them as
+// one 16-byte vector.  The draws on a host core and their upload took 17 ms of a
+// call on 512 x 512 frames (20 output frames of 60, GB300: 134.3 -> 117.6 ms).
+using u128 = unsigned __int128;
+
+__device__ __forceinline__ uint64_t pcg_out(u128 state) {  // XSL-RR
+  const uint64_t hi = (uint64_t)(state >> 64), lo = (uint64_t)state;
+  const unsigned rot = (unsigned)(hi >> 58);
+  const uint64_t x = hi ^ lo;
+  return (x >> rot) | (x << ((64u - rot) & 63u));
+}
+
+__global__ void __launch_bounds__(256) k_probes(ProbeStream ps, size_t n, int8_t* d1, int8_t* d2) {
+  const int w = blockIdx.z, second = blockIdx.y;
+  const size_t i0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 16;
+  if (i0 >= n) return;
+  u128 st = ((u128)ps.hi[w] << 64) | ps.lo[w];
+  size_t jump = i0 + (second ? n : 0);
+  for (int b = 0; jump; ++b, jump >>= 1)
+    if (jump & 1)
+      st = st * (((u128)ps.mul_hi[b] << 64) | ps.mul_lo[b]) +
+           (((u128)ps.add_hi[b] << 64) | ps.add_lo[b]);
+  const u128 mul = ((u128)ps.mul_hi[0] << 64) | ps.mul_lo[0];
+  const u128 add = ((u128)ps.add_hi[0] << 64) | ps.add_lo[0];
+  const uint64_t below = second ? ps.below2 : ps.below1;
+  const int8_t yes = second ? 1 : -1, no = second ? 0 : 1;
+  __align__(16) int8_t v[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    st = st * mul + add;
+    v[j] = pcg_out(st) < below ? yes : no;
+  }
+  int8_t* o = (second ? d2 : d1) + (size_t)w * n + i0;
+  if (i0 + 16 <= n && (((uintptr_t)o) & 15) == 0) {
+    *reinterpret_cast<int4*>(o) = *reinterpret_cast<const int4*>(v);
+  } else {
+    for (int j = 0; j < 16 && i0 + j < n; ++j) o[j] = v[j];
+  }
+}
+
+cudaError_t launch_probes(const ProbeStream& ps, int windows, size_t n, int8_t* d1, int8_t* d2,
+                          cudaStream_t s) {
+  const size_t threads = (n + 15) / 16;
+  k_probes<<<dim3((unsigned)((threads + 255) / 256), 2, windows), 256, 0, s>>>(ps, n, d1, d2);
+  return cudaGetLastError();
+}
+
 }  // namespace pgsvt

@@ -117,3 +117,22 @@ def test_owner_forms_are_identical(capi, pkg, bs, T, expw):
         return
     for x, y in zip(out[0][:3], out[1][:3]):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("side,nwin", [(8, 3), (17, 5), (21, 15), (32, 15)])
+@pytest.mark.parametrize("seed", [0, 11, 2 ** 63 - 1])
+def test_probe_streams(capi, oracle, side, nwin, seed):
+    """The probes are drawn on the device, 16 draws per thread: window sizes that
+    are and are not multiples of 16, both probe sets (without the integer-delta1
+    quirk the risk depends on delta1 as well), against the oracle's risk (the
+    tolerance of the risk tests)."""
+    rng = np.random.default_rng(side + nwin)
+    u = rng.uniform(0.2, 1.0, (side, side, nwin))
+    u /= u.max()
+    P = (side - 4 + 1) ** 2
+    rows = np.tile(np.arange(P) % (side - 3), (nwin, 1)).astype(np.int32)
+    cols = np.tile(np.arange(P) // (side - 3), (nwin, 1)).astype(np.int32)
+    for compat in (capi.COMPAT_ALL, capi.COMPAT_ALL & ~capi.COMPAT_INT_DELTA1):
+        args = (u, 4, 1, rows, cols, [0.5, 5.0], 0.02, 0.03, 0.05, seed, compat)
+        r, ro = capi.risk_window(*args), oracle.risk_window(*args)
+        assert np.abs(r - ro).max() <= 1e-4 * np.abs(ro).max()
