@@ -10,6 +10,8 @@
 // reference does (FP64 x/umax, FP64 squares, Armadillo's two-accumulator
 // accu(), no fused multiply-add) and the FP64 argmin is taken.  The decisions,
 // hence the motion vectors, are therefore the FP64 ones.
+#include <cstring>
+
 #include "pgsvt_internal.h"
 
 namespace pgsvt {
@@ -17,10 +19,19 @@ namespace pgsvt {
 namespace {
 
 
+// How a block cost is computed.  kFloat: FP32 with an error bound.  Integer-
+// valued input (at most 2^19) has exact sums of squared differences instead: in
+// FP32 where m * max^2 <= 2^24 (kIntF), else in 64-bit integers (kInt64).
+enum { kFloat, kIntF, kInt64 };
+
+template <int MODE>
+struct CostT { using type = float; };
+template <>
+struct CostT<kInt64> { using type = unsigned long long; };
+
 struct ArpsCtx {
-  bool integer;       // integer-valued input below 2^19: exact integer costs
-  const float* fa1;   // normalised window slice a1
-  const float* fa2;   // normalised window slice a2
+  const float* fa1;   // slices a1 and a2 that the costs read: the normalised
+  const float* fa2;   // window, or the raw integers
   const float* xa1;   // input frames (exact f32 values) for the FP64 path
   const float* xa2;
   const double* xa1d; // input frames when the input is f64
@@ -35,11 +46,13 @@ struct ArpsCtx {
 
 // The reference block of one position.  BS > 0: its values in registers;
 // BS == 0 (patch sides above 8): read from the frame where needed.
-template <int BS>
+template <int BS, int MODE>
 struct Block {
-  float ref[BS > 0 ? BS * BS : 1];  // normalised values, or the raw integers in integer mode
+  using T = typename CostT<MODE>::type;
+  float ref[BS > 0 ? BS * BS : 1];  // normalised values, or the raw integers
   const float* src = nullptr;       // BS == 0: the block's first element
   int S = 0;
+  float a2 = 0.f;                   // kFloat: the sum of its squares
 
   __device__ __forceinline__ float at(int e, int nb) const {
     if constexpr (BS > 0) return ref[e];
@@ -47,90 +60,99 @@ struct Block {
   }
 
   __device__ void load(const ArpsCtx& c, int i, int j) {
-    const float* sp = c.integer ? c.xa1 : c.fa1;
+    const float* sp = c.fa1 + (i + j * c.S);
     if constexpr (BS > 0) {
 #pragma unroll
       for (int cc = 0; cc < BS; ++cc)
 #pragma unroll
-        for (int r = 0; r < BS; ++r) ref[r + cc * BS] = __ldg(sp + (i + r) + (size_t)(j + cc) * c.S);
+        for (int r = 0; r < BS; ++r) ref[r + cc * BS] = __ldg(sp + r + cc * c.S);
     } else {
-      src = sp + i + (size_t)j * c.S;
+      src = sp;
       S = c.S;
+    }
+    if constexpr (MODE == kFloat) {
+      const int nb = BS > 0 ? BS : c.bs;
+      for (int e = 0; e < nb * nb; ++e) a2 = fmaf(at(e, nb), at(e, nb), a2);
     }
   }
 
-  // Integer mode: the exact sum of squared differences D.  The reference's
+  // Cost of the candidate at offset off (row + column * S), with a bound on its
+  // error.
+  //
+  // Integers: the exact sum of squared differences D.  The reference's
   // FP64 cost is D / (umax^2 m) up to an absolute error below
   // (m + 7) 2^-53 (values <= 1 after normalisation), while two different D
   // differ by at least 1 / (umax^2 m) > 2 (m + 7) 2^-53 for umax <= 2^19 and
   // m <= 64, or umax <= 2^17 and m <= 256 (the host enables the mode only
   // then): comparing D decides exactly as the reference does, except for
   // equal D.
-  __device__ unsigned long long ssd(const ArpsCtx& c, int y, int x) const {
+  //
+  // kFloat: a bound on |cost32 - cost64| (u = 2^-24, m = bs^2): the
+  // FP32 operands differ from the reference's FP64 ones by <= 2u|a| (the
+  // normalisation divides by the FP32-rounded maximum), so every difference
+  // by <= 3u(|a|+|b|) and every square by <= 6u(|a|+|b|)^2; the m-term FMA
+  // sum adds <= m u sum d^2 = m^2 u cost.  (|a|+|b|)^2 <= (2|a|+|d|)^2 <= 8a^2 + 2d^2
+  // bounds the first sum by the reference block's squares and the cost itself
+  // (adding the terms up per candidate took half of the arithmetic).  With
+  // margin:
+  //   err = u * (8 * (8 sum a^2 + 2 sum d^2) / m + (m + 4) * cost)
+  __device__ __forceinline__ void cost(const ArpsCtx& c, int off, T& cst, float& err) const {
     const int nb = BS > 0 ? BS : c.bs;
-    unsigned long long acc = 0ull;
+    const float* sp = c.fa2 + off;
+    if constexpr (MODE == kInt64) {
+      unsigned long long acc = 0ull;
 #pragma unroll
-    for (int cc = 0; cc < nb; ++cc)
+      for (int cc = 0; cc < nb; ++cc)
 #pragma unroll
-      for (int r = 0; r < nb; ++r) {
-        const int a = (int)at(r + cc * nb, nb);
-        const int b = (int)__ldg(c.xa2 + (y + r) + (size_t)(x + cc) * c.S);
-        const unsigned d = (unsigned)abs(a - b);  // < 2^19
-        acc += (unsigned long long)d * d;
+        for (int r = 0; r < nb; ++r) {
+          const float d = at(r + cc * nb, nb) - __ldg(sp + r + cc * c.S);  // exact, |d| <= 2^19
+          const int di = __float_as_int(d + 12582912.f) - 0x4B400000;      // 1.5 * 2^23
+          acc += (unsigned long long)((long long)di * di);
+        }
+      cst = acc;
+      err = 0.f;
+    } else {
+      float acc = 0.f;
+#pragma unroll
+      for (int cc = 0; cc < nb; ++cc)
+#pragma unroll
+        for (int r = 0; r < nb; ++r) {
+          const float d = at(r + cc * nb, nb) - __ldg(sp + r + cc * c.S);
+          acc = fmaf(d, d, acc);
+        }
+      if constexpr (MODE == kIntF) {
+        cst = acc;
+        err = 0.f;
+      } else {
+        const float m = (float)(nb * nb), oo = 1.0f / m;
+        cst = acc * oo;
+        err = 5.9604645e-8f * (8.f * (8.f * a2 + 2.f * acc) * oo + (m + 4.f) * cst);
       }
-    return acc;
+    }
   }
 
-  // the candidate block at (y, x) equals the one at (y2, x2), element by element
-  __device__ bool same(const ArpsCtx& c, int y, int x, int y2, int x2) const {
+  // the candidate block at offset o equals the one at o2, element by element
+  __device__ bool same(const ArpsCtx& c, int o, int o2) const {
     const int nb = BS > 0 ? BS : c.bs;
     bool eq = true;
 #pragma unroll
     for (int cc = 0; cc < nb; ++cc)
 #pragma unroll
       for (int r = 0; r < nb; ++r)
-        eq &= __ldg(c.xa2 + (y + r) + (size_t)(x + cc) * c.S) ==
-              __ldg(c.xa2 + (y2 + r) + (size_t)(x2 + cc) * c.S);
+        eq &= __ldg(c.fa2 + o + r + cc * c.S) == __ldg(c.fa2 + o2 + r + cc * c.S);
     return eq;
   }
+};
 
-  // cost of the candidate at (y, x): FP32 with an error bound, or exact D
-  __device__ void cost(const ArpsCtx& c, int y, int x, float& cf, float& err,
-                       unsigned long long& cd) const {
-    if (c.integer) {
-      cd = ssd(c, y, x);
-      cf = 0.f;
-      err = 0.f;
-    } else {
-      cost32(c, y, x, cf, err);
-      cd = 0ull;
-    }
+// Offset of slot k of a diamond of half-width st around the current position;
+// slot 5 is the predicted motion (mx, my).
+struct Diamond {
+  int st, mx, my;
+  __device__ __forceinline__ int dx(int k) const {
+    return k == 1 ? -st : (k == 3 ? st : (k == 5 ? mx : 0));
   }
-
-  // FP32 cost and a bound on |cost32 - cost64| (u = 2^-24, m = bs^2): the
-  // FP32 operands differ from the reference's FP64 ones by <= 2u|a| (the
-  // normalisation divides by the FP32-rounded maximum), so every difference
-  // by <= 3u(|a|+|b|) and every square by <= 6u(|a|+|b|)^2; the m-term FMA
-  // sum adds <= m u sum d^2 = m^2 u cost.  With margin:
-  //   err = u * (8 * sum_e (|a_e|+|b_e|)^2 / m + (m + 4) * cost)
-  __device__ void cost32(const ArpsCtx& c, int y, int x, float& cost, float& err) const {
-    const int nb = BS > 0 ? BS : c.bs;
-    float acc = 0.f, sb = 0.f;
-#pragma unroll
-    for (int cc = 0; cc < nb; ++cc)
-#pragma unroll
-      for (int r = 0; r < nb; ++r) {
-        const float a = at(r + cc * nb, nb);
-        const float b = __ldg(c.fa2 + (y + r) + (size_t)(x + cc) * c.S);
-        const float d = a - b;
-        acc = fmaf(d, d, acc);
-        const float s = fabsf(a) + fabsf(b);
-        sb = fmaf(s, s, sb);
-      }
-    const float m = (float)(nb * nb);
-    const float oo = 1.0f / m;
-    cost = acc * oo;
-    err = 5.9604645e-8f * (8.f * sb * oo + (m + 4.f) * cost);
+  __device__ __forceinline__ int dy(int k) const {
+    return k == 0 ? -st : (k == 4 ? st : (k == 5 ? my : 0));
   }
 };
 
@@ -160,8 +182,8 @@ struct ArpsWarp {
 // so this takes a small part of the FP64 instructions (and of the latency) of
 // per-thread evaluations.  Results in ws.cst[lane * 6 + slot].
 template <int BS>
-__device__ void warp_cost64(const ArpsCtx& c, ArpsWarp<BS>& ws, unsigned em, int i, int j,
-                            int y, int x, const int (*off)[2], int nslot) {
+__device__ __noinline__ void warp_cost64(const ArpsCtx& c, ArpsWarp<BS>& ws, unsigned em, int i,
+                                         int j, int y, int x, const Diamond dm, int nslot) {
   const int lane = threadIdx.x & 31;
   const int nb = BS > 0 ? BS : c.bs;
   const int m = nb * nb;
@@ -180,7 +202,7 @@ __device__ void warp_cost64(const ArpsCtx& c, ArpsWarp<BS>& ws, unsigned em, int
     int r = first;
     for (int k = 0; k < nslot; ++k) {
       if (!((em >> k) & 1u)) continue;
-      ws.pos[lane * 6 + k] = ((uint32_t)(y + off[k][1]) & 0xffffu) | ((uint32_t)(x + off[k][0]) << 16);
+      ws.pos[lane * 6 + k] = ((uint32_t)(y + dm.dy(k)) & 0xffffu) | ((uint32_t)(x + dm.dx(k)) << 16);
       ws.cand[r++] = (uint16_t)(lane * 6 + k);
     }
   }
@@ -239,174 +261,168 @@ __device__ int resolve_exact(bool integer, const double* cst, unsigned em, int n
   return 2;
 }
 
-// Integer mode: first index of the least D; equal D decided as the
+// The slot of a step from the costs of the evaluated slots (bits of ev, slot 2
+// always), or -1 with the slots to evaluate exactly in em.
+//
+// Integers: first index of the least D; equal D decided as the
 // reference does: identical candidate blocks have identical FP64 costs (the
-// first one wins), otherwise the FP64 costs of the tied candidates decide
-// (returns -1 with those slots in em).
-template <int BS>
-__device__ int decide_int(const ArpsCtx& c, const Block<BS>& blk, const unsigned long long* cd,
-                          const bool* ev, const int (*off)[2], int nslot, int y, int x,
-                          unsigned& em) {
+// first one wins; D = 0 are all copies of the reference block), otherwise the
+// FP64 costs of the tied candidates decide.
+//
+// kFloat: first index of the minimum when the FP32 decision is certain under the
+// error bounds, else every evaluated slot is to be evaluated exactly.
+template <int BS, int MODE, class T>
+__device__ __forceinline__ int decide(const ArpsCtx& c, const Block<BS, MODE>& blk, const T (&cs)[6],
+                                      const float (&es)[6], unsigned ev, const Diamond& dm, int off,
+                                      unsigned& em) {
   int ks = 2;
-  unsigned long long best = cd[2];
-  for (int k = 0; k < nslot; ++k)
-    if (ev[k] && (cd[k] < best || (cd[k] == best && k < ks))) {
-      best = cd[k];
-      ks = k;
-    }
-  unsigned tied = 1u << ks;
-  bool distinct = false;
-  for (int k = 0; k < nslot; ++k) {
-    if (!ev[k] || k == ks || cd[k] != best) continue;
-    tied |= 1u << k;
-    if (!blk.same(c, y + off[k][1], x + off[k][0], y + off[ks][1], x + off[ks][0])) distinct = true;
-  }
-  if (!distinct) return ks;
-  em = tied;
-  return -1;
-}
-
-// First index of the minimum among evaluated slots when the FP32 decision is
-// certain under the error bounds; else -1 with every evaluated slot in em.
-__device__ int decide_f32(const float* cs, const float* es, const bool* ev, int nslot,
-                          unsigned& em) {
-  int ks = 2;
-  float best = cs[2];
-  for (int k = 0; k < nslot; ++k)
-    if (ev[k] && (cs[k] < best || (cs[k] == best && k < ks))) {
+  T best = cs[2];
+  float ebest = es[2];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    if (k == 2) continue;
+    if (((ev >> k) & 1u) && (cs[k] < best || (cs[k] == best && k < ks))) {
       best = cs[k];
+      ebest = es[k];
       ks = k;
     }
-  bool certain = true;
-  const float hi = cs[ks] + es[ks];
-  for (int k = 0; k < nslot; ++k) {
-    if (!ev[k] || k == ks) continue;
-    const float lo = cs[k] - es[k];
-    if (k < ks ? !(lo > hi) : !(lo >= hi)) certain = false;
   }
-  if (certain) return ks;
-  em = 0u;
-  for (int k = 0; k < nslot; ++k)
-    if (ev[k]) em |= 1u << k;
-  return -1;
+  if constexpr (MODE == kFloat) {
+    bool certain = true;
+    const float hi = best + ebest;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      if (!((ev >> k) & 1u) || k == ks) continue;
+      const float lo = cs[k] - es[k];
+      if (k < ks ? !(lo > hi) : !(lo >= hi)) certain = false;
+    }
+    if (certain) return ks;
+    em = ev;
+    return -1;
+  } else {
+    unsigned tied = 0u;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      if (((ev >> k) & 1u) && cs[k] == best) tied |= 1u << k;
+    if (best == (T)0 || !(tied & (tied - 1u))) return ks;
+    bool distinct = false;
+    const int o2 = off + dm.dy(ks) + dm.dx(ks) * c.S;
+    for (unsigned t = tied & ~(1u << ks); t; t &= t - 1u) {
+      const int k = __ffs(t) - 1;
+      if (!blk.same(c, off + dm.dy(k) + dm.dx(k) * c.S, o2)) distinct = true;
+    }
+    if (!distinct) return ks;
+    em = tied;
+    return -1;
+  }
 }
 
 // ARPSMotionEstimation (arps.hpp:153-375) for one position of one frame pair.
 // (my, mx) holds the predictor slot on entry and the new motion on exit.
 // The lanes of a warp step through the diamond searches together (a lane
 // whose search ended, or that holds no position, idles), so that the exact
-// decisions any of them needs are taken by the whole warp.
-template <int BS>
+// decisions any of them needs are taken by the whole warp.  `seen`: this
+// thread's bitmap of visited cells, word q at seen[q * 128].
+template <int BS, int MODE>
 __device__ void arps_pair(const ArpsCtx& c, bool live, int it, int& my, int& mx, int& oy,
-                          int& ox, ArpsWarp<BS>& ws, unsigned& nexact) {
+                          int& ox, ArpsWarp<BS>& ws, uint32_t* seen, unsigned& nexact) {
+  using T = typename CostT<MODE>::type;
   const int lane = threadIdx.x & 31;
   const int S = c.S, M = c.mw, Wd = 2 * M + 1;
   const int nb = BS > 0 ? BS : c.bs;
   const int n1 = S - nb + 1;
   const int i = it % n1, j = it / n1;
-  Block<BS> blk;
+  Block<BS, MODE> blk;
   blk.load(c, i, j);
-  uint32_t seen[(2 * kMaxMW + 1) * (2 * kMaxMW + 1) / 32 + 1];
   const int nw = (Wd * Wd + 31) / 32;
-  for (int q = 0; q < nw; ++q) seen[q] = 0u;
-  auto mark = [&](int dy, int dx) {
-    if (dy < -M || dy > M || dx < -M || dx > M) return;  // cannot occur for mw >= 2
-    const int b = (dy + M) * Wd + (dx + M);
-    seen[b >> 5] |= 1u << (b & 31);
-  };
-  auto is_seen = [&](int dy, int dx) {
-    const int b = (dy + M) * Wd + (dx + M);
-    return (seen[b >> 5] >> (b & 31)) & 1u;
-  };
+  for (int q = 0; q < nw; ++q) seen[q * 128] = 0u;
   int x = j, y = i;
-  float cs[6], es[6];
-  unsigned long long cd[6];
-  bool ev[6];
-  float curC, curE;
-  unsigned long long curD;
-  blk.cost(c, i, j, curC, curE, curD);
-  mark(0, 0);
-  int step, nld;
-  int LD[6][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};
-  if (j == 0) {
-    step = 2;
-    nld = 5;
-  } else {
-    const int ay = abs(my), ax = abs(mx);
-    step = (ax <= ay) ? ay : ax;
-    if ((ay == 0 && ax == step) || (ax == 0 && ay == step)) {
-      nld = 5;
-    } else {
-      nld = 6;
-      LD[5][0] = mx;
-      LD[5][1] = my;
-    }
+  T cs[6];
+  float es[6];
+  blk.cost(c, i + j * S, cs[2], es[2]);
+  {
+    const int b = M * Wd + M;
+    seen[(b >> 5) * 128] |= 1u << (b & 31);
   }
-  LD[0][1] = -step;
-  LD[1][0] = -step;
-  LD[3][0] = step;
-  LD[4][1] = step;
-  // LDSP candidates (arps.hpp:247-287)
-  for (int k = 0; k < 6; ++k) ev[k] = false;
-  ev[2] = true;
-  cs[2] = curC;
-  es[2] = curE;
-  cd[2] = curD;
-  if (live)
-    for (int k = 0; k < nld; ++k) {
-      if (k == 2 || step == 0) continue;
-      const int vy = y + LD[k][1], hx = x + LD[k][0];
-      if (hx < 0 || vy < 0 || hx + nb - 1 >= S || vy + nb - 1 >= S) continue;
-      blk.cost(c, vy, hx, cs[k], es[k], cd[k]);
-      ev[k] = true;
-      mark(LD[k][1], LD[k][0]);
-    }
-  // step 0 decides the LDSP (arps.hpp:289-294), steps 1.. the SDSP
-  // (arps.hpp:299-368); every SDSP move enters an unvisited cell, so a search
-  // ends within Wd*Wd moves.
-  const int SD[5][2] = {{0, -1}, {-1, 0}, {0, 0}, {1, 0}, {0, 1}};
+  // step 0 is the LDSP (arps.hpp:247-294), steps 1.. the SDSP (arps.hpp:299-368):
+  // the same diamond, of the predictor's length and of 1, the first with the
+  // predicted motion as a sixth candidate when it is off the axes and without
+  // the search window's limits.  Every SDSP move enters an unvisited cell, so a
+  // search ends within Wd*Wd moves.
+  Diamond dm{2, 0, 0};
+  bool six = false;
+  if (j > 0) {
+    const int ay = abs(my), ax = abs(mx);
+    dm.st = (ax <= ay) ? ay : ax;
+    six = !((ay == 0 && ax == dm.st) || (ax == 0 && ay == dm.st));
+    dm.mx = mx;
+    dm.my = my;
+  }
   bool done = !live;
   for (int n = 0; n <= Wd * Wd + 1; ++n) {
-    const int (*off)[2] = (n == 0) ? LD : SD;
-    const int nslot = (n == 0) ? 6 : 5;
-    if (n > 0 && !done) {
-      for (int k = 0; k < 6; ++k) ev[k] = false;
-      ev[2] = true;
-      cs[2] = curC;
-      es[2] = curE;
-      cd[2] = curD;
-      for (int k = 0; k < 5; ++k) {
-        if (k == 2) continue;
-        const int vy = y + SD[k][1], hx = x + SD[k][0];
-        if (hx < 0 || vy < 0 || hx + nb - 1 >= S || vy + nb - 1 >= S) continue;
-        if (hx < j - M || hx > j + M || vy < i - M || vy > i + M) continue;
-        if (is_seen(vy - i, hx - j)) continue;
-        blk.cost(c, vy, hx, cs[k], es[k], cd[k]);
-        ev[k] = true;
-        mark(vy - i, hx - j);
+    unsigned ev = 4u;
+    if (!done) {
+      const int o = y + x * S;
+      auto slot = [&](int k, T& ck, float& ek) {  // cost of slot k, if it is a candidate
+        const int ddx = dm.dx(k), ddy = dm.dy(k);
+        const int hx = x + ddx, vy = y + ddy;
+        bool ok = hx >= 0 && vy >= 0 && hx + nb <= S && vy + nb <= S;
+        const int wy = vy - i, wx = hx - j;  // cell of the search window
+        const bool in = wy >= -M && wy <= M && wx >= -M && wx <= M;
+        const int b = (wy + M) * Wd + (wx + M);
+        if (n > 0) ok = ok && in && !((seen[(b >> 5) * 128] >> (b & 31)) & 1u);
+        if (!ok) return;
+        blk.cost(c, o + ddy + ddx * S, ck, ek);
+        ev |= 1u << k;
+        if (in) seen[(b >> 5) * 128] |= 1u << (b & 31);
+      };
+      if (dm.st != 0) {
+        if constexpr (BS > 0 && BS <= 4) {
+#pragma unroll
+          for (int k = 0; k < 5; ++k)
+            if (k != 2) slot(k, cs[k], es[k]);
+        } else {  // one copy of the cost code for the larger blocks
+#pragma unroll 1
+          for (int k = 0; k < 5; ++k) {
+            if (k == 2) continue;
+            T ck = (T)0;
+            float ek = 0.f;
+            slot(k, ck, ek);
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+              if (q != 2 && q == k) {
+                cs[q] = ck;
+                es[q] = ek;
+              }
+          }
+        }
       }
+      if (n == 0 && six) slot(5, cs[5], es[5]);
     }
     int ks = 2;
     unsigned em = 0u;
-    if (!done)
-      ks = c.integer ? decide_int<BS>(c, blk, cd, ev, off, nslot, y, x, em)
-                     : decide_f32(cs, es, ev, nslot, em);
+    if (!done) ks = decide<BS, MODE>(c, blk, cs, es, ev, dm, y + x * S, em);
     if (__any_sync(0xffffffffu, em != 0u)) {
-      warp_cost64<BS>(c, ws, em, i, j, y, x, off, nslot);
+      const int nslot = n == 0 ? 6 : 5;
+      warp_cost64<BS>(c, ws, em, i, j, y, x, dm, nslot);
       if (em) {
-        ks = resolve_exact(c.integer, ws.cst + lane * 6, em, nslot);
+        ks = resolve_exact(MODE != kFloat, ws.cst + lane * 6, em, nslot);
         ++nexact;
       }
       __syncwarp();
     }
     if (!done) {
-      x += off[ks][0];
-      y += off[ks][1];
-      curC = cs[ks];
-      curE = es[ks];
-      curD = cd[ks];
+      x += dm.dx(ks);
+      y += dm.dy(ks);
+#pragma unroll
+      for (int k = 0; k < 6; ++k)
+        if (k != 2 && k == ks) {
+          cs[2] = cs[k];
+          es[2] = es[k];
+        }
       if (n > 0 && ks == 2) done = true;
     }
+    dm.st = 1;
     if (!__any_sync(0xffffffffu, !done)) break;
   }
   my = y - i;
@@ -415,17 +431,30 @@ __device__ void arps_pair(const ArpsCtx& c, bool live, int it, int& my, int& mx,
   ox = x;
 }
 
-// five blocks per SM: 96 registers, no spills (128 at the default bound)
-template <int BS>
-__global__ void __launch_bounds__(128, 5) k_arps(Problem pb, DeviceBuffers d) {
+// Chain table of a batch in the kernel's parameters: its entries and the frame
+// addresses that follow from them are uniform over a block.
+struct ArpsTable {
+  ArpsChain c[kArpsChains];
+};
+
+// five blocks per SM: 96 registers.  Bound by the instructions of the costs and
+// their loads (nine tenths of them hit L1).  GB300, against one form with runtime
+// candidate lists, 64-bit integer sums and per-candidate error sums: 256 x 256 x
+// 100 floats 17.9 -> 11.2 ms; 256 x 256 x 24 bytes, 8 x 8 patches, 19.0 -> 6.6 ms; median-
+// filtered 512 x 512 x 40 (two thirds of it exact tie decisions) 115 -> 81 ms.
+template <int BS, int MODE>
+__global__ void __launch_bounds__(128, 5)
+    k_arps(Problem pb, DeviceBuffers d, const __grid_constant__ ArpsTable tab) {
   const Geometry& g = pb.g;
   const int it0 = blockIdx.x * blockDim.x + threadIdx.x;
   const int ch = blockIdx.y, w = blockIdx.z;
-  const ArpsChain cn = d.chains[w * d.nchains + ch];
-  if (cn.npairs == 0) return;  // uniform over the block
+  const ArpsChain& cn = tab.c[w * d.nchains + ch];
+  const int npairs = cn.npairs;
+  if (npairs == 0) return;  // uniform over the block
   const bool live = it0 < g.P;
   const int it = live ? it0 : 0;
   __shared__ ArpsWarp<BS> wsh[4];
+  extern __shared__ uint32_t seen[];  // [words][128]
   ArpsWarp<BS>& ws = wsh[threadIdx.x >> 5];
   const WinConst& wc = d.wc[w];
   const size_t F = g.F();
@@ -437,28 +466,47 @@ __global__ void __launch_bounds__(128, 5) k_arps(Problem pb, DeviceBuffers d) {
   const double* xd = med ? nullptr : d.x64;
   ArpsCtx c;
   c.bs = g.bs;
-  c.integer = med || d.int_input;
   c.umax = med ? wc.wnorm : wc.unorm;
   c.S = g.S;
   c.mw = g.mw;
   int my = 0, mx = 0;
   unsigned nexact = 0u;
-  for (int q = 0; q < cn.npairs; ++q) {
+  for (int q = 0; q < npairs; ++q) {
     const int a1 = cn.a1[q], a2 = cn.a2[q];
-    c.fa1 = fw + ((size_t)w * g.nwin + a1) * F;
-    c.fa2 = fw + ((size_t)w * g.nwin + a2) * F;
     c.xa1 = xw + (size_t)(wc.s0 + a1) * F;
     c.xa2 = xw + (size_t)(wc.s0 + a2) * F;
+    if constexpr (MODE == kFloat) {
+      c.fa1 = fw + ((size_t)w * g.nwin + a1) * F;
+      c.fa2 = fw + ((size_t)w * g.nwin + a2) * F;
+    } else {
+      c.fa1 = c.xa1;
+      c.fa2 = c.xa2;
+    }
     c.xa1d = xd ? xd + (size_t)(wc.s0 + a1) * F : nullptr;
     c.xa2d = xd ? xd + (size_t)(wc.s0 + a2) * F : nullptr;
     c.pa1 = d.w64 ? d.w64 + ((size_t)w * g.nwin + a1) * F : nullptr;
     c.pa2 = d.w64 ? d.w64 + ((size_t)w * g.nwin + a2) * F : nullptr;
     int oy, ox;
-    arps_pair<BS>(c, live, it, my, mx, oy, ox, ws, nexact);
+    arps_pair<BS, MODE>(c, live, it, my, mx, oy, ox, ws, seen + threadIdx.x, nexact);
     if (live) d.pos[((size_t)w * g.nwin + a2) * g.P + it] = (uint32_t)oy | ((uint32_t)ox << 16);
   }
   for (int o = 16; o > 0; o >>= 1) nexact += __shfl_xor_sync(0xffffffffu, nexact, o);
   if ((threadIdx.x & 31) == 0 && nexact) atomicAdd(d.counters, (unsigned long long)nexact);
+}
+
+template <int MODE>
+void launch_k_arps(dim3 grid, size_t shm, const Problem& pb, const DeviceBuffers& d,
+                   const ArpsTable& tab, cudaStream_t s) {
+  switch (pb.g.bs) {
+    case 2: k_arps<2, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;
+    case 3: k_arps<3, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;
+    case 4: k_arps<4, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;
+    case 5: k_arps<5, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;
+    case 6: k_arps<6, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;
+    case 7: k_arps<7, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;
+    case 8: k_arps<8, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;
+    default: k_arps<0, MODE><<<grid, 128, shm, s>>>(pb, d, tab); break;  // sides 9..16
+  }
 }
 
 // Reference slice (always) and, without motion estimation, the other slices:
@@ -487,16 +535,15 @@ cudaError_t launch_arps(const Problem& pb, const DeviceBuffers& d, cudaStream_t 
   k_grid<<<gg, threads, 0, s>>>(pb, d);
   if (!pb.motion || d.nchains == 0) return cudaGetLastError();
   dim3 ga((g.P + threads - 1) / threads, d.nchains, pb.W);
-  switch (g.bs) {
-    case 2: k_arps<2><<<ga, threads, 0, s>>>(pb, d); break;
-    case 3: k_arps<3><<<ga, threads, 0, s>>>(pb, d); break;
-    case 4: k_arps<4><<<ga, threads, 0, s>>>(pb, d); break;
-    case 5: k_arps<5><<<ga, threads, 0, s>>>(pb, d); break;
-    case 6: k_arps<6><<<ga, threads, 0, s>>>(pb, d); break;
-    case 7: k_arps<7><<<ga, threads, 0, s>>>(pb, d); break;
-    case 8: k_arps<8><<<ga, threads, 0, s>>>(pb, d); break;
-    default: k_arps<0><<<ga, threads, 0, s>>>(pb, d); break;  // sides 9..16
-  }
+  if (pb.W * d.nchains > kArpsChains) return cudaErrorInvalidValue;
+  ArpsTable tab;
+  std::memcpy(tab.c, d.chains, sizeof(ArpsChain) * pb.W * d.nchains);
+  const int wd = 2 * g.mw + 1;
+  const size_t shm = (size_t)((wd * wd + 31) / 32) * 128 * sizeof(uint32_t);
+  if (!d.zs && !d.int_input) launch_k_arps<kFloat>(ga, shm, pb, d, tab, s);
+  else if ((double)g.M * d.arps_max * d.arps_max <= 16777216.0)
+    launch_k_arps<kIntF>(ga, shm, pb, d, tab, s);
+  else launch_k_arps<kInt64>(ga, shm, pb, d, tab, s);
   return cudaGetLastError();
 }
 

@@ -619,6 +619,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
   for (int v : hint) int_input &= v;
   if (g.M > 64)
     for (double v : hmax) int_input &= (v <= 131072.0) ? 1 : 0;
+  const double vmax = *std::max_element(hmax.begin(), hmax.end());
   for (double v : hmax)
     if (v < 0) throw Fail(PGSVT_ERR_NONFINITE, "input holds negative, NaN or infinite values");
   // noise estimation tables per input frame (noise.cu)
@@ -760,9 +761,6 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     auto c = chains_for(t, g.fw, nimg, g.nwin);
     std::copy(c.begin(), c.end(), hch.begin() + (size_t)t * nchains);
   }
-  ArpsChain* dch = mem.arr<ArpsChain>(hch.size());
-  PGSVT_CK(cudaMemcpyAsync(dch, hch.data(), sizeof(ArpsChain) * hch.size(), cudaMemcpyHostToDevice, s));
-  stats.h2d += sizeof(ArpsChain) * hch.size();
   unsigned long long* counters = mem.arr<unsigned long long>(5);
   PGSVT_CK(cudaMemsetAsync(counters, 0, 5 * sizeof(unsigned long long), s));
   const double vP = probe_vp();
@@ -836,6 +834,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     d.zs = zs;
     d.zmax = zmx;
     d.int_input = int_input;
+    d.arps_max = zs ? std::min(vmax, 65535.0) : vmax;  // (the pre-filter works on uint16)
     if (zs) {
       d.wz = mem.arr<float>((size_t)W * C);
       d.w64 = mem.arr<double>((size_t)W * C);
@@ -912,7 +911,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     Problem pbb = pb;
     pbb.W = std::min(W, fe - win0);
     d.win0 = win0;
-    d.chains = dch + (size_t)win0 * nchains;
+    d.chains = hch.data() + (size_t)win0 * nchains;
     StageClock& clk = *L.clk;
     if (pb.optimize && !shared_probes)
       check_launch(launch_probes(probe_stream(-1, pbb.W), pbb.W, C, L.pd1, L.pd2, L.s), stats);
@@ -1598,9 +1597,7 @@ int pgsvt_arps_window(const double* w, uint32_t nrows, uint32_t nwin, uint32_t b
     OneWindow ow(w, nrows, nwin, p, ref, ref);
     const Geometry& g = ow.pb.g;
     auto ch = chains_for(t, tw, ni, (int)nwin);
-    ArpsChain* dch = ow.mem.arr<ArpsChain>(ch.size());
-    PGSVT_CK(cudaMemcpyAsync(dch, ch.data(), sizeof(ArpsChain) * ch.size(), cudaMemcpyHostToDevice, ow.s));
-    ow.d.chains = dch;
+    ow.d.chains = ch.data();
     PGSVT_CK(launch_arps(ow.pb, ow.d, ow.s));
     std::vector<uint32_t> h((size_t)g.nwin * g.P);
     PGSVT_CK(cudaMemcpyAsync(h.data(), ow.d.pos, h.size() * 4, cudaMemcpyDeviceToHost, ow.s));

@@ -124,6 +124,8 @@ struct ArpsChain {
   int8_t a1[2], a2[2];
 };
 
+constexpr int kArpsChains = 32 * 20;  // windows per batch x chains of a 21-frame window
+
 struct Geometry {
   int S;        // frame side
   int bs;       // patch side
@@ -200,7 +202,8 @@ struct DeviceBuffers {
   double* part_mse;        // [W][K][nblk_mse]
   WinConst* wc;
   SearchState* st;
-  const ArpsChain* chains; // [W][2*fw]
+  const ArpsChain* chains; // [W][2*fw], host memory (kernel parameters)
+  double arps_max;         // bound on the ARPS input's values (integer modes)
   int nchains;
   double* Y;               // output [nimg][S*S] (double)
   double* est;             // output estimates (nimg x 4)

@@ -136,3 +136,25 @@ def test_probe_streams(capi, oracle, side, nwin, seed):
         args = (u, 4, 1, rows, cols, [0.5, 5.0], 0.02, 0.03, 0.05, seed, compat)
         r, ro = capi.risk_window(*args), oracle.risk_window(*args)
         assert np.abs(r - ro).max() <= 1e-4 * np.abs(ro).max()
+
+
+@pytest.mark.parametrize("bs,vmax,dtype", [(4, 1023, "uint16"), (4, 1025, "uint16"), (8, 511, "uint16"),
+                                           (8, 513, "float32"), (9, 65535, "uint16"), (2, 2047, "uint16"),
+                                           (5, 524288, "float32"), (4, 524289, "float32"),
+                                           (3, 3, "uint8"), (6, 7, "uint8")])
+def test_arps_cost_forms(capi, oracle, bs, vmax, dtype):
+    """Exact FP32 sums up to m * max^2 = 2^24, 64-bit ones to values of 2^19, FP32
+    with error bounds beyond; few grey levels give many ties.  Motion vectors are
+    those of the oracle, so the output is too (the whole-sequence tolerance at
+    fixed lambda)."""
+    rng = np.random.default_rng(bs * 1000 + vmax % 97)
+    side, T = 34, 7 if bs > 2 else 3
+    base = rng.integers(0, vmax + 1, (side + 8, side + 8))
+    base[::3] = vmax
+    X = np.stack([base[2 + k % 3:2 + k % 3 + side, 4 - k % 4:4 - k % 4 + side] for k in range(T + 1)], -1)
+    X = np.asfortranarray(X.astype(dtype))
+    kw = dict(traj_length=T, block_size=bs, motion_window=7, median_size=-1, random_seed=3,
+              optimize_pgure=0, lambda_=0.05)
+    Y, _, _ = capi.denoise(X, capi.default_params(**kw))
+    Yo, _, _ = oracle.denoise(X, n_jobs=4, **kw)
+    assert np.abs(Y - Yo).max() <= 2e-5 * np.abs(Yo).max()
