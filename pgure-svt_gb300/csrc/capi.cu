@@ -854,6 +854,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
       d.fld0 = mem.arr<float>((size_t)W * C);
       d.fld2 = mem.arr<float>((size_t)W * C);
       d.fld1 = (ncopies == 4) ? mem.arr<float>((size_t)W * C) : nullptr;
+      d.ftab = mem.arr<float2>((size_t)W * 512);
     }
     d.U0 = mem.arr<float>((size_t)W * g.NC * g.M * g.NPB() * 32);
     d.V0 = mem.arr<float>((size_t)W * g.NC * g.nwin * g.NPB() * 32);
@@ -1716,6 +1717,7 @@ int pgsvt_risk_window(const double* u, uint32_t nrows, uint32_t nwin, uint32_t b
     ow.d.fld0 = ow.mem.arr<float>(C);
     ow.d.fld2 = ow.mem.arr<float>(C);
     ow.d.fld1 = ncopies == 4 ? ow.mem.arr<float>(C) : nullptr;
+    ow.d.ftab = ow.mem.arr<float2>(512);
     int8_t* d1 = ow.mem.arr<int8_t>(C);
     int8_t* d2 = ow.mem.arr<int8_t>(C);
     PGSVT_CK(launch_probes(probe_stream(random_seed, 1), 1, C, d1, d2, ow.s));
@@ -1723,6 +1725,7 @@ int pgsvt_risk_window(const double* u, uint32_t nrows, uint32_t nwin, uint32_t b
     ow.d.d2code = d2;
     ow.d.probe_stride = 0;
     PGSVT_CK(launch_fields(ow.pb, ow.d, ow.s));
+    PGSVT_CK(launch_search_init(ow.pb, ow.d, ow.s));  // sum(U)
     {  // the largest requested lambda bounds the thresholds the SVD must keep
       double upper = 0.0;
       for (uint32_t j = 0; j < nl; ++j) upper = std::max(upper, lambdas[j]);

@@ -36,55 +36,32 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// ---- coverage counts (weights in svt.hpp:157-159)
+// ---- lambda-independent fields and sum(U)
 //
-// A warp's 32 patches are half of an 8 x 8 tile of grid positions (the
-// processing order), so their blocks in slice k overlap: the warp counts them
-// in a shared-memory tile and adds the tile with one global atomic per
-// touched pixel (plain global atomics when the footprint does not fit).
-constexpr int kCountTile = 512;
+// With the integer-delta1 quirk a voxel's fields depend on its coverage and its
+// probe code only: k_field_table tabulates them in FP64 for the coverages below
+// kFieldTab (the FP64 pipe, at 1/64 of the FP32 rate, was what bounded the
+// kernel: a division and ten products per voxel); what is left in FP64 per voxel
+// is sum(U).  Two windows of 512 x 512 x 15, GB300: 0.27 -> 0.10 ms.
+constexpr int kFieldTab = 256;
 
-__global__ void __launch_bounds__(128) k_counts(Problem pb, DeviceBuffers d) {
-  const Geometry& g = pb.g;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y, w = blockIdx.z;
-  const int lane = threadIdx.x & 31;
-  __shared__ int tiles[4][kCountTile];
-  int* tile = tiles[threadIdx.x >> 5];
-  const bool live = p < g.NP;
-  int y = 0, x = 0;
-  if (live) {
-    const uint32_t pc = d.pos[((size_t)w * g.nwin + k) * g.P + d.plist[p]];
-    y = pc & 0xffffu;
-    x = pc >> 16;
-  }
-  const int y0 = __reduce_min_sync(0xffffffffu, live ? y : 0x7fffffff);
-  const int y1 = __reduce_max_sync(0xffffffffu, live ? y : -1);
-  const int x0 = __reduce_min_sync(0xffffffffu, live ? x : 0x7fffffff);
-  const int x1 = __reduce_max_sync(0xffffffffu, live ? x : -1);
-  if (y1 < 0) return;  // no live patch in this warp (warp-uniform)
-  int32_t* c = d.cnt + (size_t)w * g.cube() + (size_t)k * g.F();
-  const int th = y1 - y0 + g.bs, tw = x1 - x0 + g.bs;
-  if (th * tw > kCountTile) {  // warp-uniform
-    if (live)
-      for (int cc = 0; cc < g.bs; ++cc)
-        for (int r = 0; r < g.bs; ++r) atomicAdd(c + (y + r) + (size_t)(x + cc) * g.S, 1);
-    return;
-  }
-  for (int i = lane; i < th * tw; i += 32) tile[i] = 0;
-  __syncwarp();
-  if (live)
-    for (int cc = 0; cc < g.bs; ++cc)
-      for (int r = 0; r < g.bs; ++r) atomicAdd(tile + (y - y0 + r) + (x - x0 + cc) * th, 1);
-  __syncwarp();
-  for (int i = lane; i < th * tw; i += 32) {
-    const int v = tile[i];
-    if (v) atomicAdd(c + (y0 + i % th) + (size_t)(x0 + i / th) * g.S, v);
-  }
+// (field 0, field 2) of a voxel covered n times
+__device__ __forceinline__ float2 field_entry(const WinConst& wc, double dl2, int n) {
+  const double a = wc.alpha, m = wc.mu, s2 = wc.sigma * wc.sigma;
+  const double c2 = 2 * s2 * a / (wc.eps2 * wc.eps2);
+  const double ic = n > 0 ? 1.0 / n : 0.0;
+  const double l0 = 2 * c2 * dl2 + 2 * m;
+  return make_float2((float)(l0 * ic), (float)(-c2 * dl2 * ic));
 }
 
-// ---- lambda-independent fields and sum(U)
-__global__ void k_fields(Problem pb, DeviceBuffers d) {
+// [window][probe code][coverage]
+__global__ void __launch_bounds__(kFieldTab) k_field_table(Problem pb, DeviceBuffers d) {
+  const int w = blockIdx.y, code = blockIdx.x;
+  d.ftab[((size_t)w * 2 + code) * kFieldTab + threadIdx.x] =
+      field_entry(d.wc[w], code ? d.d2neg : d.d2pos, threadIdx.x);
+}
+
+__global__ void __launch_bounds__(256) k_fields(Problem pb, DeviceBuffers d) {
   const Geometry& g = pb.g;
   const int w = blockIdx.y;
   const size_t C = g.cube();
@@ -96,6 +73,7 @@ __global__ void k_fields(Problem pb, DeviceBuffers d) {
   const bool intd1 = pb.compat & 0x4;
   const int8_t* d1 = d.d1 + (size_t)w * d.probe_stride;
   const int8_t* d2c = d.d2code + (size_t)w * d.probe_stride;
+  const float2* tab = d.ftab + (size_t)w * 2 * kFieldTab;
   double su = 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < C;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -103,14 +81,19 @@ __global__ void k_fields(Problem pb, DeviceBuffers d) {
     su += uv;
     if (!pb.optimize) continue;
     const int n = cnt[i];
-    const double ic = n > 0 ? 1.0 / n : 0.0;
-    const double dl2 = d2c[i] ? d.d2neg : d.d2pos;
-    double l0 = 2 * c2 * dl2 + 2 * m;
-    if (!intd1) {
-      const double l1 = (2 / wc.eps1) * d1[i] * ((a * uv - a * m) + s2);
-      l0 -= l1;
-      d.fld1[(size_t)w * C + i] = (float)(l1 * ic);
+    const bool code = d2c[i] != 0;
+    if (intd1) {
+      const float2 f = n < kFieldTab ? __ldg(tab + code * kFieldTab + n)
+                                     : field_entry(wc, code ? d.d2neg : d.d2pos, n);
+      d.fld0[(size_t)w * C + i] = f.x;
+      d.fld2[(size_t)w * C + i] = f.y;
+      continue;
     }
+    const double ic = n > 0 ? 1.0 / n : 0.0;
+    const double dl2 = code ? d.d2neg : d.d2pos;
+    const double l1 = (2 / wc.eps1) * d1[i] * ((a * uv - a * m) + s2);
+    const double l0 = 2 * c2 * dl2 + 2 * m - l1;
+    d.fld1[(size_t)w * C + i] = (float)(l1 * ic);
     d.fld0[(size_t)w * C + i] = (float)(l0 * ic);
     d.fld2[(size_t)w * C + i] = (float)(-c2 * dl2 * ic);
   }
@@ -124,16 +107,9 @@ __global__ void k_fields(Problem pb, DeviceBuffers d) {
     d.part_mse[(size_t)w * gridDim.x + blockIdx.x] = t;  // reused as scratch
   }
 }
+constexpr int kFieldBlocks = 256;  // per window
 
-__global__ void k_sum_u(Problem pb, DeviceBuffers d, int nblk) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= pb.W) return;
-  double t = 0.0;
-  for (int b = 0; b < nblk; ++b) t += d.part_mse[(size_t)w * nblk + b];
-  d.wc[w].sum_u = t;
-}
-
-// ---- search state machine (one thread per window)
+// ---- search state machine (one block per window, thread 0 decides)
 //
 // Bracketed batch grid search, identical to the oracle's: round 0 places K
 // points geometrically over [lo, hi]; each later round places K/2 points
@@ -146,10 +122,13 @@ __global__ void k_sum_u(Problem pb, DeviceBuffers d, int nblk) {
 // and the better of the two results is kept.
 
 struct Sch {
+  // grid point j of K from lo to hi
+  __device__ static double point(int j, int K, double lo, double hi) {
+    return (K == 1) ? hi : lo * pow(hi / lo, (double)j / (double)(K - 1));
+  }
   __device__ static void grid(SearchState& s, double lo, double hi) {
     const int K = s.K;
-    for (int j = 0; j < K; ++j)
-      s.next[j] = (K == 1) ? hi : lo * pow(hi / lo, (double)j / (double)(K - 1));
+    for (int j = 0; j < K; ++j) s.next[j] = point(j, K, lo, hi);
     s.nnext = K;
     s.first = 1;
   }
@@ -183,60 +162,84 @@ struct Sch {
 // round also evaluates the plain grid's ends that it does not reach
 // (sentinels, kept out of the point list): one of them below the narrow
 // grid's best sends the search to the plain grid.
+// Called by the threads of a block; each point's pow() runs in its own thread.
 __device__ void start_narrow(SearchState& s, const Problem& pb, double upper, double hint) {
   const double h = fmin(hint, upper);
   const double lo = h / pb.hint_span, hi = fmin(upper, h * pb.hint_span);
-  Sch::phase(s, 1, pb.hint_K, pb.max_evals, pb.hint_rounds, lo <= upper * 1e-4 ? 1 : 0);
-  Sch::grid(s, lo, hi);
-  const int room = min(pb.K - s.nnext, pb.max_evals - s.nnext);
-  if (room > 0 && lo > upper * 1e-4) s.next[s.nnext + s.nsent++] = upper * 1e-4;
-  if (room > s.nsent && hi < upper) s.next[s.nnext + s.nsent++] = upper;
-  s.nnext += s.nsent;
+  if (threadIdx.x == 0) {
+    Sch::phase(s, 1, pb.hint_K, pb.max_evals, pb.hint_rounds, lo <= upper * 1e-4 ? 1 : 0);
+    s.nnext = s.K;
+    s.first = 1;
+    const int room = min(pb.K - s.nnext, pb.max_evals - s.nnext);
+    if (room > 0 && lo > upper * 1e-4) s.next[s.nnext + s.nsent++] = upper * 1e-4;
+    if (room > s.nsent && hi < upper) s.next[s.nnext + s.nsent++] = upper;
+    s.nnext += s.nsent;
+  }
+  __syncthreads();
+  if (threadIdx.x < s.K) s.next[threadIdx.x] = Sch::point(threadIdx.x, s.K, lo, hi);
 }
 
-__global__ void k_search_init(Problem pb, DeviceBuffers d) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= pb.W) return;
+// sum(U) of the window from k_fields' partials (in their order), the search's
+// bounds and its first round
+__global__ void __launch_bounds__(kFieldBlocks) k_search_init(Problem pb, DeviceBuffers d) {
+  const int w = blockIdx.x;
   const Geometry& g = pb.g;
   WinConst& wc = d.wc[w];
   SearchState& s = d.st[w];
-  s.npts = 0;
-  s.nnext = 0;
-  s.evals_total = 0;
-  s.best = 0;
-  s.final_lambda = pb.lambda_user;
-  s.final_risk = 0.0;
-  s.hint_lambda = s.hint_risk = 0.0;
-  s.nsent = 0;
-  s.sent_risk = INFINITY;
-  if (!pb.optimize) {
-    s.done = 1;
-    return;
+  __shared__ double part[kFieldBlocks];
+  __shared__ double s_upper;
+  part[threadIdx.x] = d.part_mse[(size_t)w * kFieldBlocks + threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+#pragma unroll 8
+    for (int b = 0; b < kFieldBlocks; ++b) t += part[b];
+    wc.sum_u = t;
+    s.npts = 0;
+    s.nnext = 0;
+    s.evals_total = 0;
+    s.best = 0;
+    s.final_lambda = pb.lambda_user;
+    s.final_risk = 0.0;
+    s.hint_lambda = s.hint_risk = 0.0;
+    s.nsent = 0;
+    s.sent_risk = INFINITY;
+    s.done = pb.optimize ? 0 : 1;
+    if (pb.optimize) {
+      // pguresvt.hpp:139-141
+      const double OoN = 1.0 / (double)((uint32_t)g.S * (uint32_t)g.S * (uint32_t)g.Ntc);
+      double start = (pb.lambda_user >= 0.0) ? pb.lambda_user : t * OoN;
+      start = fmax(0.0, start);
+      wc.start = start;
+      s_upper = wc.upper = fmax(100.0, start);
+    }
   }
-  // pguresvt.hpp:139-141
-  const double OoN = 1.0 / (double)((uint32_t)g.S * (uint32_t)g.S * (uint32_t)g.Ntc);
-  double start = (pb.lambda_user >= 0.0) ? pb.lambda_user : wc.sum_u * OoN;
-  start = fmax(0.0, start);
-  wc.start = start;
-  wc.upper = fmax(100.0, start);
-  s.done = 0;
+  __syncthreads();
+  if (!pb.optimize) return;
+  const double upper = s_upper;
   if (pb.nfixed > 0) {  // a given list: one round, no refinement
-    Sch::phase(s, 0, pb.nfixed, pb.nfixed, 0, 0);
-    for (int j = 0; j < pb.nfixed; ++j) s.next[j] = pb.fixed[j];
-    s.nnext = pb.nfixed;
-    s.first = 1;
+    if (threadIdx.x == 0) {
+      Sch::phase(s, 0, pb.nfixed, pb.nfixed, 0, 0);
+      for (int j = 0; j < pb.nfixed; ++j) s.next[j] = pb.fixed[j];
+      s.nnext = pb.nfixed;
+      s.first = 1;
+    }
   } else if (pb.hint > 0) {
-    start_narrow(s, pb, wc.upper, pb.hint);
+    start_narrow(s, pb, upper, pb.hint);
   } else {
-    Sch::phase(s, 0, pb.K, pb.max_evals, pb.rounds, 1);
-    Sch::grid(s, wc.upper * 1e-4, wc.upper);
+    if (threadIdx.x == 0) {
+      Sch::phase(s, 0, pb.K, pb.max_evals, pb.rounds, 1);
+      s.nnext = s.K;
+      s.first = 1;
+    }
+    __syncthreads();
+    if (threadIdx.x < s.K) s.next[threadIdx.x] = Sch::point(threadIdx.x, s.K, upper * 1e-4, upper);
   }
 }
 
 // Narrow searches around the learned proposals y = log10(lambda/upper).
-__global__ void k_search_hint(Problem pb, DeviceBuffers d) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= pb.W) return;
+__global__ void __launch_bounds__(32) k_search_hint(Problem pb, DeviceBuffers d) {
+  const int w = blockIdx.x;
   SearchState& s = d.st[w];
   if (s.done) return;
   const double upper = d.wc[w].upper;
@@ -258,41 +261,52 @@ __device__ void search_finish(SearchState& s, unsigned long long* counters) {
   s.nnext = 0;
 }
 
-// Risk of lambda slot j of window w (pgure.hpp:136) from the block
-// partials, reduced by the calling block in a fixed order.
-__device__ double block_sum(const double* v, int n, double* red) {
-  double t = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) t += v[i];
-  red[threadIdx.x] = t;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  const double r = red[0];
-  __syncthreads();
-  return r;
-}
-
 // Merge the risks of the pending round and schedule the next one.
-// One block per window: the partial sums are reduced in parallel, thread 0
-// advances the search state.
-__global__ void __launch_bounds__(256) k_search_step(Problem pb, DeviceBuffers d) {
+// One block per window: the partial sums of all its lambda values are reduced
+// side by side, in four groups of 256 threads (each sum in the order of a
+// 256-thread block: a strided sum per thread, then a tree), and thread 0 advances
+// the search state.  Latency-bound: 512 x 512 x 15, 4 to 6 values, GB300: 30 -> 10 us
+// (one sum after the other before).
+constexpr int kStepGroups = 4;
+
+__global__ void __launch_bounds__(256 * kStepGroups) k_search_step(Problem pb, DeviceBuffers d) {
   const int w = blockIdx.x;
   SearchState& s = d.st[w];
   if (s.done) return;
-  __shared__ double red[256];
+  __shared__ double red[kStepGroups][256];
+  __shared__ double sums[2 * kMaxK];
   __shared__ double risk[kMaxK];
   const Geometry& g = pb.g;
   const WinConst& wc = d.wc[w];
-  const double N = (double)g.S * g.S * g.nwin;
-  const double a = wc.alpha, m = wc.mu, s2 = wc.sigma * wc.sigma;
   const int nn = s.nnext;
-  for (int j = 0; j < nn; ++j) {
-    const double lin = block_sum(d.part_lin + ((size_t)w * pb.K + j) * d.nblk_eval, d.nblk_eval, red);
-    const double mse = block_sum(d.part_mse + ((size_t)w * pb.K + j) * d.nblk_mse, d.nblk_mse, red);
-    if (threadIdx.x == 0) risk[j] = (1.0 / N) * (mse + lin - (a + m) * wc.sum_u + m) - s2;  // pgure.hpp:136
+  const int grp = threadIdx.x >> 8, t = threadIdx.x & 255;
+  for (int q0 = 0; q0 < 2 * nn; q0 += kStepGroups) {  // uniform over the block
+    const int q = q0 + grp, j = q >> 1;
+    if (q < 2 * nn) {
+      const int n = (q & 1) ? d.nblk_mse : d.nblk_eval;
+      const double* v = ((q & 1) ? d.part_mse : d.part_lin) + ((size_t)w * pb.K + j) * n;
+      double x = 0.0;
+#pragma unroll 8
+      for (int i = t; i < n; i += 256) x += v[i];
+      red[grp][t] = x;
+    }
+    __syncthreads();
+    if (q < 2 * nn && t < 32) {
+      const double* r = red[grp];
+      double x = ((r[t] + r[t + 128]) + (r[t + 64] + r[t + 192])) +
+                 ((r[t + 32] + r[t + 160]) + (r[t + 96] + r[t + 224]));
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (t == 0) sums[q] = x;
+    }
+    __syncthreads();
   }
+  if (threadIdx.x < nn) {  // pgure.hpp:136
+    const double N = (double)g.S * g.S * g.nwin;
+    const double a = wc.alpha, m = wc.mu, s2 = wc.sigma * wc.sigma;
+    risk[threadIdx.x] = (1.0 / N) * (sums[2 * threadIdx.x + 1] + sums[2 * threadIdx.x] -
+                                     (a + m) * wc.sum_u + m) - s2;
+  }
+  __syncthreads();
   if (threadIdx.x != 0) return;
   const double prev_best = s.npts > 0 ? s.risk[s.best] : 0.0;
   for (int j = nn - s.nsent; j < nn; ++j) s.sent_risk = fmin(s.sent_risk, risk[j]);
@@ -735,6 +749,45 @@ __global__ void __launch_bounds__(128) k_eval_out(Problem pb, DeviceBuffers d) {
   }
 }
 
+// ---- coverage counts (weights in svt.hpp:157-159): as the scatter, a warp
+// counts its 32 patches' pixels in a tile and adds it with one atomic per pixel
+constexpr int kCountTile = 512;
+
+__global__ void __launch_bounds__(128) k_counts(Problem pb, DeviceBuffers d) {
+  const Geometry& g = pb.g;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = blockIdx.y, w = blockIdx.z;
+  const int lane = threadIdx.x & 31;
+  __shared__ __align__(16) int tiles[4][kCountTile];
+  int* tile = tiles[threadIdx.x >> 5];
+  const bool live = p < g.NP;
+  int y = 0, x = 0;
+  if (live) {
+    const uint32_t pc = d.pos[((size_t)w * g.nwin + k) * g.P + d.plist[p]];
+    y = pc & 0xffffu;
+    x = pc >> 16;
+  }
+  Footprint f;
+  f.init(live, y, x, g.bs, kCountTile);
+  if (f.th < g.bs) return;  // no live patch in this warp (warp-uniform)
+  int32_t* c = d.cnt + (size_t)w * g.cube() + (size_t)k * g.F();
+  if (!f.tile) {  // warp-uniform
+    if (live)
+      for (int cc = 0; cc < g.bs; ++cc)
+        for (int r = 0; r < g.bs; ++r) atomicAdd(c + (y + r) + (size_t)(x + cc) * g.S, 1);
+    return;
+  }
+  for (int i = lane * 4; i < kCountTile; i += 128) *reinterpret_cast<int4*>(tile + i) = make_int4(0, 0, 0, 0);
+  __syncwarp();
+  if (live) {
+    int* t = tile + (y - f.y0) + (x - f.x0) * f.ths;
+    for (int cc = 0; cc < g.bs; ++cc, t += f.ths)
+      for (int r = 0; r < g.bs; ++r) atomicAdd(t + r, 1);
+  }
+  __syncwarp();
+  flush<1>(f, tile, kCountTile, c, 0, 1, g.S, lane);
+}
+
 // ---- sum over voxels of (Uh - U)^2 for every lambda of the round; clears acc
 template <typename AccT, int KT>
 __global__ void __launch_bounds__(256) k_mse(Problem pb, DeviceBuffers d) {
@@ -959,19 +1012,18 @@ cudaError_t launch_fields(const Problem& pb, const DeviceBuffers& d, cudaStream_
   cudaMemsetAsync(d.cnt, 0, sizeof(int32_t) * g.cube() * pb.W, s);
   dim3 gc((g.NP + 127) / 128, g.nwin, pb.W);
   k_counts<<<gc, 128, 0, s>>>(pb, d);
-  const int nb = 256;
-  k_fields<<<dim3(nb, pb.W), 256, 0, s>>>(pb, d);
-  k_sum_u<<<(pb.W + 63) / 64, 64, 0, s>>>(pb, d, nb);
+  if (pb.optimize && (pb.compat & 0x4)) k_field_table<<<dim3(2, pb.W), kFieldTab, 0, s>>>(pb, d);
+  k_fields<<<dim3(kFieldBlocks, pb.W), 256, 0, s>>>(pb, d);
   return cudaGetLastError();
 }
 
 cudaError_t launch_search_init(const Problem& pb, const DeviceBuffers& d, cudaStream_t s) {
-  k_search_init<<<(pb.W + 63) / 64, 64, 0, s>>>(pb, d);
+  k_search_init<<<pb.W, kFieldBlocks, 0, s>>>(pb, d);
   return cudaGetLastError();
 }
 
 cudaError_t launch_search_hint(const Problem& pb, const DeviceBuffers& d, cudaStream_t s) {
-  k_search_hint<<<(pb.W + 63) / 64, 64, 0, s>>>(pb, d);
+  k_search_hint<<<pb.W, 32, 0, s>>>(pb, d);
   return cudaGetLastError();
 }
 
@@ -985,7 +1037,7 @@ cudaError_t launch_eval_round(const Problem& pb, const DeviceBuffers& d, int fin
   launch_k_eval(pb, d, final_pass, final_pass ? 1 : pb.K, s);
   if (final_pass) return cudaGetLastError();  // 2: every slice
   launch_k_mse(pb, d, s);
-  k_search_step<<<pb.W, 256, 0, s>>>(pb, d);
+  k_search_step<<<pb.W, 256 * kStepGroups, 0, s>>>(pb, d);
   return cudaGetLastError();
 }
 

@@ -187,6 +187,7 @@ struct DeviceBuffers {
   float* fld0;
   float* fld1;             // first-order field (only without the int-delta1 quirk)
   float* fld2;
+  float2* ftab;            // [W][2][256] fields by probe code and coverage (eval.cu)
   const int8_t* d1;        // probes, nwin*S*S per set
   const int8_t* d2code;    // 1 -> -sqrt(vQ/vP), 0 -> sqrt(vP/vQ)
   size_t probe_stride;     // 0: one set for all windows (seed >= 0), else per window
