@@ -635,7 +635,6 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     const size_t nn = (size_t)nimg * nf.maxNodes;
     nf.split = mem.arr<uint8_t>(std::max<size_t>(1, (size_t)nimg * B));
     nf.nodes = mem.arr<int4>(nn);
-    nf.isdel = mem.arr<uint8_t>(nn);
     nf.leaf = mem.arr<int4>(nn);
     nf.nleaf = mem.arr<int>(nimg);
     nf.big = mem.arr<int>(nn);
@@ -645,7 +644,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     nf.first = mem.arr<int>((size_t)nimg * noise_blocks(nf.nlev + 1));
     nf.err = mem.arr<int>(1);
     PGSVT_CK(cudaMemsetAsync(nf.err, 0, sizeof(int), s));
-    check_launch(launch_noise_frames(xs, x64, nimg, S, nf, s), stats, 6);
+    check_launch(launch_noise_frames(xs, x64, nimg, S, nf, s), stats, 5);
     int herr = 0;
     PGSVT_CK(cudaMemcpyAsync(&herr, nf.err, sizeof(int), cudaMemcpyDeviceToHost, s));
     PGSVT_CK(cudaStreamSynchronize(s));

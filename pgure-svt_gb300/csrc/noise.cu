@@ -25,7 +25,7 @@
 // absolute), so they run once per (frame, distinct window maximum) pair, and
 // every window then fits its own line:
 //   k_quad_decide   one CTA per (frame, block of side > 8): the F statistic
-//   k_quad_tree     one thread per frame: replays the reference's recursion
+//   k_quad_tree     one CTA per frame: a thread replays the reference's recursion
 //                   over the decision table, including its quirks (the
 //                   node that was last before a split is re-visited, the
 //                   fourth child is not; the smallest split index, the root,
@@ -167,12 +167,12 @@ __device__ void decide_block(const FrameSrc& src, int f, int b, int nlev, uint8_
   const size_t R = (size_t)N * N;
   const int lane = BLOCK ? threadIdx.x : (threadIdx.x & 31);
   const int step = BLOCK ? blockDim.x : 32;
-  const double sq30 = sqrt(30.0);  // sqrt(l*l + l), l = 5
+  const double isq30 = 1.0 / sqrt(30.0);  // 1 / sqrt(l*l + l), l = 5
   auto A = [&](int r, int c) { return src.at(f, i0 + r, j0 + c); };
   auto res = [&](size_t e) {
     const int y = (int)(e % N), x = (int)(e / N);
     const double s4 = ((A(nxt(y, N), x) + A(prv(y, N), x)) + A(y, prv(x, N))) + A(y, nxt(x, N));
-    return (5.0 * A(y, x) - s4) / sq30;
+    return (5.0 * A(y, x) - s4) * isq30;
   };
   auto sum = [&](double v) { return BLOCK ? block_sum(v, red) : warp_sum(v); };
   double sa = 0.0, sr = 0.0;
@@ -211,68 +211,131 @@ __global__ void __launch_bounds__(256) k_quad_decide_small(FrameSrc src, int nle
   decide_block<false>(src, blockIdx.y, b, nlev, split, nullptr);
 }
 
-// QuadTree (noise.hpp:411-453) replayed over the decision table; writes the
-// leaves (row, col, side) in the reference's order.
-__global__ void k_quad_tree(const uint8_t* split, int nimg, int S, int nlev, int maxNodes,
-                            int4* nodes, uint8_t* isdel, int4* leaf, int* nleaf, int* dup,
-                            int* first, int* err) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nimg) return;
-  const uint8_t* sp = split + (size_t)f * level_off(nlev);
-  int4* nd = nodes + (size_t)f * maxNodes;
-  uint8_t* dl = isdel + (size_t)f * maxNodes;
-  int len = 1, minDel = maxNodes, top = 0;
-  nd[0] = make_int4(0, 0, S, 0);
-  dl[0] = 0;
-  int stk_n[32], stk_it[32];
-  bool bad = false;
-  auto try_split = [&](int part) {
-    const int4 q = nd[part];
-    if (q.z <= kLeafMin) return;
-    const int l = 31 - __clz(S / q.z), nb = 1 << l;
-    if (!sp[level_off(l) + q.x / q.z + (q.y / q.z) * nb]) return;
-    if (len + 4 > maxNodes || top >= 32) {
-      bad = true;
-      return;
-    }
-    const int h = q.z / 2, n = len - 1;
-    nd[len] = make_int4(q.x, q.y, h, 0);
-    nd[len + 1] = make_int4(q.x + h, q.y, h, 0);
-    nd[len + 2] = make_int4(q.x, q.y + h, h, 0);
-    nd[len + 3] = make_int4(q.x + h, q.y + h, h, 0);
-    for (int k = 0; k < 4; ++k) dl[len + k] = 0;
-    len += 4;
-    dl[part] = 1;
-    minDel = min(minDel, part);
-    stk_n[top] = n;
-    stk_it[top] = n;
-    ++top;
-  };
-  try_split(0);
-  while (top > 0 && !bad) {
-    const int t = top - 1;
-    if (stk_it[t] > stk_n[t] + 3) {
-      --top;
-      continue;
-    }
-    try_split(stk_it[t]++);
+// QuadTree (noise.hpp:411-453) replayed over the decision table, one block per
+// frame; writes the leaves (row, col, side) in the reference's order.
+//
+// The replay is a chain of dependent reads, so thread 0 runs it on shared
+// memory: a node is one word (level, block column and row, a deleted flag), and
+// the decisions and the nodes of frames up to 1024 x 1024 fit (larger ones keep
+// their nodes in global memory).  The whole block then lists the leaves: the
+// recursion lists most blocks twice, and a repeated block (same row, column,
+// side) reuses the first one's statistics.  512 x 512 x 40, GB300: 15 ms with
+// one thread per frame on global memory, 1.04 ms now.
+constexpr int kTreeThreads = 256;
+constexpr uint32_t kNodeDel = 0x80000000u;
+
+// exclusive prefix sum of v over the block; *total receives the sum
+__device__ int block_scan(int v, int* sh, int* total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int inc = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
   }
-  // leaves in node order; the recursion lists most blocks twice, and a
-  // repeated block (same row, column, side) reuses the first one's statistics
-  int* fi = first + (size_t)f * level_off(nlev + 1);
-  for (int b = 0; b < level_off(nlev + 1); ++b) fi[b] = -1;
-  int nl = 0;
-  for (int k = 0; k < len; ++k) {
-    if (dl[k] && k != minDel) continue;
-    const int4 q = nd[k];
-    const int l = 31 - __clz(S / q.z);
-    const int id = level_off(l) + q.x / q.z + (q.y / q.z) * (1 << l);
-    dup[(size_t)f * maxNodes + nl] = fi[id];
-    if (fi[id] < 0) fi[id] = nl;
-    leaf[(size_t)f * maxNodes + nl++] = q;
+  __syncthreads();
+  if (lane == 31) sh[wid] = inc;
+  __syncthreads();
+  int before = 0, t = 0;
+  for (int q = 0; q < nw; ++q) {
+    if (q < wid) before += sh[q];
+    t += sh[q];
   }
-  nleaf[f] = bad ? 0 : nl;
-  if (bad) atomicExch(err, 1);
+  *total = t;
+  return before + inc - v;
+}
+
+__global__ void __launch_bounds__(kTreeThreads) k_quad_tree(
+    const uint8_t* split, int S, int nlev, int maxNodes, bool smem_nodes, int4* nodes, int4* leaf,
+    int* nleaf, int* dup, int* first, int* big, int* nbig, int* err, bool smem_split) {
+  extern __shared__ uint32_t tsm[];
+  __shared__ int s_len, s_min, s_bad, s_scan[kTreeThreads / 32];
+  const int f = blockIdx.x, tid = threadIdx.x;
+  const int nsplit = level_off(nlev), nids = level_off(nlev + 1);
+  uint32_t* nd = smem_nodes ? tsm : reinterpret_cast<uint32_t*>(nodes + (size_t)f * maxNodes);
+  const uint8_t* sp = split + (size_t)f * nsplit;
+  if (smem_split) {
+    uint8_t* sps = reinterpret_cast<uint8_t*>(tsm + (smem_nodes ? maxNodes : 0));
+    for (int i = tid; i < nsplit; i += kTreeThreads) sps[i] = sp[i];
+    sp = sps;
+  }
+  int* fi = first + (size_t)f * nids;
+  for (int i = tid; i < nids; i += kTreeThreads) fi[i] = 0x7fffffff;
+  __syncthreads();
+  if (tid == 0) {
+    int len = 1, minDel = maxNodes, top = 0;
+    bool bad = false;
+    int stk_n[32], stk_it[32];
+    nd[0] = 0;  // level 0, block (0, 0)
+    auto try_split = [&](int part) {
+      const uint32_t q = nd[part];
+      const int l = (int)((q >> 26) & 15u), bx = (int)(q & 8191u), by = (int)((q >> 13) & 8191u);
+      if ((S >> l) <= kLeafMin) return;
+      if (!sp[level_off(l) + bx + (by << l)]) return;
+      if (len + 4 > maxNodes || top >= 32) {
+        bad = true;
+        return;
+      }
+      const int n = len - 1;
+      const uint32_t c = ((uint32_t)(l + 1) << 26) | ((uint32_t)(2 * by) << 13) | (uint32_t)(2 * bx);
+      nd[len] = c;                      // (row, col), then one row block on,
+      nd[len + 1] = c + 1u;             // one column block on, both
+      nd[len + 2] = c + (1u << 13);
+      nd[len + 3] = c + (1u << 13) + 1u;
+      len += 4;
+      nd[part] = q | kNodeDel;
+      minDel = min(minDel, part);
+      stk_n[top] = n;
+      stk_it[top] = n;
+      ++top;
+    };
+    try_split(0);
+    while (top > 0 && !bad) {
+      const int t = top - 1;
+      if (stk_it[t] > stk_n[t] + 3) {
+        --top;
+        continue;
+      }
+      try_split(stk_it[t]++);
+    }
+    s_len = len;
+    s_min = minDel;
+    s_bad = bad;
+  }
+  __syncthreads();
+  const int len = s_len, minDel = s_min;
+  // leaves in node order (two passes: the first leaf of a block, then the lists)
+  int nl = 0, nb = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    nl = nb = 0;
+    for (int k0 = 0; k0 < len; k0 += kTreeThreads) {  // uniform over the block
+      const int k = k0 + tid;
+      const uint32_t q = k < len ? nd[k] : 0u;
+      const bool is_leaf = k < len && (!(q & kNodeDel) || k == minDel);
+      const int l = (int)((q >> 26) & 15u), bx = (int)(q & 8191u), by = (int)((q >> 13) & 8191u);
+      const int z = S >> l, id = level_off(l) + bx + (by << l);
+      int total, totalb;
+      const int at = nl + block_scan(is_leaf, s_scan, &total);
+      if (pass == 0) {
+        if (is_leaf) atomicMin(&fi[id], at);
+      } else {
+        const int ab = nb + block_scan(is_leaf && z > 32, s_scan, &totalb);
+        if (is_leaf) {
+          leaf[(size_t)f * maxNodes + at] = make_int4(bx * z, by * z, z, 0);
+          const int fa = fi[id];
+          dup[(size_t)f * maxNodes + at] = fa < at ? fa : -1;
+          if (z > 32) big[(size_t)f * maxNodes + ab] = at;
+        }
+        nb += totalb;
+      }
+      nl += total;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    nleaf[f] = s_bad ? 0 : nl;
+    nbig[f] = s_bad ? 0 : nb;
+    if (s_bad) atomicExch(err, 1);
+  }
 }
 
 // ConvolveFIR (noise.hpp:386-409) value at e = x + y*N of the N x N block:
@@ -378,6 +441,8 @@ struct ClusterSmem {
   unsigned t[2][kDigits];   // the cluster's
   int dg[2], kk[2];
   int scan[kClThreads / 32 + 1];
+  int slice, cnt[2], ln[2];            // cluster_select_near
+  unsigned long long res[2];
 };
 
 // Sums over the cluster of up to 8 values per thread; every thread of every
@@ -487,6 +552,121 @@ __device__ void cluster_select2(cg::cluster_group& cl, K key, int lo, int hi, in
   }
   v0 = pre[0];
   v1 = pre[1];
+}
+
+// The k0-th and k1-th smallest of the n keys key(i) when both are expected in
+// [vlo, vhi]: a histogram over 2,046 equal bins of that range (and one to either
+// side), then the exact order among the few keys of the two bins.  The CTAs share
+// the work of adding their histograms up, so a call takes 4 cluster barriers where
+// the radix selection takes 12 (6 passes).  False, in every thread of the cluster,
+// when a rank falls outside the range or into a bin of more than kNear keys.
+constexpr int kNear = 512;
+
+template <class K>
+__device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi, int k0, int k1,
+                                    double vlo, double vhi, ClusterSmem& sm,
+                                    unsigned long long& v0, unsigned long long& v1) {
+  constexpr int kSlice = kDigits / kCl;  // bins a CTA adds up
+  static_assert(kSlice <= kClThreads && 2 * kNear * 2 <= kDigits && kNear <= kClThreads, "sizes");
+  const int rank = (int)cl.block_rank(), tid = threadIdx.x;
+  if (!(vhi > vlo) || !isfinite(vlo) || !isfinite(vhi)) return false;
+  const double scale = (kDigits - 2) / (vhi - vlo);
+  auto bin = [&](double v) {  // monotone
+    if (!(v >= vlo)) return 0;
+    if (!(v < vhi)) return kDigits - 1;
+    return 1 + min(kDigits - 3, (int)((v - vlo) * scale));
+  };
+  for (int b = tid; b < kDigits; b += kClThreads) sm.h[0][b] = 0u;
+  if (tid < 2) sm.ln[tid] = 0;
+  __syncthreads();
+  for (int i = lo + tid; i < hi; i += kClThreads) atomicAdd(&sm.h[0][bin(ovalue(key(i)))], 1u);
+  cl.sync();
+  // this CTA's slice of the cluster's histogram
+  if (tid < kSlice) {
+    unsigned c = 0u;
+#pragma unroll
+    for (int r = 0; r < kCl; ++r) c += cl.map_shared_rank(&sm, r)->h[0][rank * kSlice + tid];
+    sm.t[0][tid] = c;
+  }
+  __syncthreads();
+  if (tid < 32) {
+    unsigned t = 0u;
+    for (int b = tid; b < kSlice; b += 32) t += sm.t[0][b];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (tid == 0) sm.slice = (int)t;
+  }
+  cl.sync();
+  int k[2] = {k0, k1}, owner[2];
+  {
+    int ss[kCl];
+#pragma unroll
+    for (int r = 0; r < kCl; ++r) ss[r] = cl.map_shared_rank(&sm, r)->slice;
+    for (int q = 0; q < 2; ++q) {
+      int o = 0;
+      while (o + 1 < kCl && k[q] >= ss[o]) k[q] -= ss[o++];
+      owner[q] = o;
+    }
+  }
+  for (int q = 0; q < 2; ++q)
+    if (owner[q] == rank) {  // uniform over the CTA
+      find_digit(sm.t[0], kSlice, k[q], &sm.dg[q], &sm.kk[q], sm.scan);
+      if (tid == 0) {
+        sm.cnt[q] = (int)sm.t[0][sm.dg[q]];
+        sm.dg[q] += rank * kSlice;
+      }
+      __syncthreads();
+    }
+  cl.sync();
+  int dg[2], kk[2], n[2];
+  bool ok = true;
+  for (int q = 0; q < 2; ++q) {
+    const ClusterSmem* os = cl.map_shared_rank(&sm, owner[q]);
+    dg[q] = os->dg[q];
+    kk[q] = os->kk[q];
+    n[q] = os->cnt[q];
+    ok = ok && dg[q] > 0 && dg[q] < kDigits - 1 && n[q] <= kNear;
+  }
+  if (!ok) {
+    cl.sync();  // the shared memory is used again
+    return false;
+  }
+  unsigned long long* list = reinterpret_cast<unsigned long long*>(sm.t[1]);  // [2][kNear]
+  for (int i = lo + tid; i < hi; i += kClThreads) {
+    const unsigned long long kv = key(i);
+    const int b = bin(ovalue(kv));
+    for (int q = 0; q < 2; ++q)
+      if (b == dg[q]) list[q * kNear + atomicAdd(&sm.ln[q], 1)] = kv;
+  }
+  cl.sync();
+  // every CTA ranks the keys of both bins
+  unsigned long long* all = reinterpret_cast<unsigned long long*>(sm.h[1]);  // [2][kNear]
+  for (int q = 0; q < 2; ++q)
+    if (tid < n[q]) {
+      int r = 0, j = tid;
+      for (; r + 1 < kCl; ++r) {
+        const int nr = cl.map_shared_rank(&sm, r)->ln[q];
+        if (j < nr) break;
+        j -= nr;
+      }
+      all[q * kNear + tid] =
+          reinterpret_cast<const unsigned long long*>(cl.map_shared_rank(&sm, r)->t[1])[q * kNear + j];
+    }
+  __syncthreads();
+  for (int q = 0; q < 2; ++q)
+    if (tid < n[q]) {
+      const unsigned long long kv = all[q * kNear + tid];
+      int less = 0;
+      for (int j = 0; j < n[q]; ++j) {
+        const unsigned long long o = all[q * kNear + j];
+        less += o < kv || (o == kv && j < tid);
+      }
+      if (less == kk[q]) sm.res[q] = kv;
+    }
+  __syncthreads();
+  v0 = sm.res[0];
+  v1 = sm.res[1];
+  __syncthreads();
+  return true;
 }
 
 // Armadillo median() from the two middle keys of an even count
@@ -637,17 +817,6 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
   if (rank == 0 && threadIdx.x == 0) a.mean[(size_t)pr * a.maxNodes + li] = m;
 }
 
-// Leaves of side > 32 of each frame.
-__global__ void k_big_leaves(const int4* leaf, const int* nleaf, int nimg, int maxNodes, int* big,
-                             int* nbig) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nimg) return;
-  int c = 0;
-  for (int li = 0; li < nleaf[f]; ++li)
-    if (leaf[(size_t)f * maxNodes + li].z > 32) big[(size_t)f * maxNodes + c++] = li;
-  nbig[f] = c;
-}
-
 struct FitArgs {
   const int* nleaf;
   const int* dup;
@@ -669,8 +838,14 @@ struct FitArgs {
 };
 
 // WLSFit (noise.hpp:302-358) and the method's mu / sigma for every window:
-// one cluster per window.
-__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads) k_noise_fit(FitArgs a) {
+// one cluster per window.  What bounds it is the latency of the cluster barriers
+// and of the two order statistics that every iteration takes of the residuals.
+// They move by at most max |x| |dp0| + |dp1| when the line moves by (dp0, dp1), so
+// after the first iteration they are looked for around the last ones
+// (cluster_select_near); two CTAs share an SM.  GB300: 8.0 -> 5.5 ms (128 x 128 x
+// 64 frames), 26 -> 24 ms (512 x 512 x 40).
+__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads, 2)
+    k_noise_fit(FitArgs a) {
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), w = blockIdx.y;
   __shared__ ClusterSmem sm;
@@ -703,6 +878,15 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads) k_nois
     Y[i] = a.stats[(f * a.maxNodes + src) * 3 + 2] / um2;
   }
   cl.sync();
+  double mn = 1e300, mx = -1e300;
+  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+    mn = fmin(mn, X[i]);
+    mx = fmax(mx, X[i]);
+  }
+  mn = -cluster_max(cl, -mn, sm);
+  mx = cluster_max(cl, mx, sm);
+  const double xabs = fmax(fabs(mn), fabs(mx));
+  unsigned long long r0 = 0, r1 = 0;
   const int mq = ((N + 1) / 2 + 1) / 2;
   double a0 = 1e12, b0 = 1e12, p0 = 0.0, p1 = 0.0, q0 = 0.0, q1 = 0.0, dd = 1.0;
   for (int it = 0; it < kMaxIter; ++it) {
@@ -733,21 +917,21 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads) k_nois
     if ((fabs(a0 - p0) < kTol && fabs(b0 - p1) < kTol) || se[0] / (double)N < kTol) break;
     a0 = p0;
     b0 = p1;
-    unsigned long long r0, r1;
-    cluster_select2(cl, [&](int i) { return K[i]; }, lo, hi, mq - 1, N - mq - 1, sm, r0, r1);
+    const auto key = [&](int i) { return K[i]; };
+    bool found = false;
+    if (it > 0) {  // q0, q1: the line that r0 and r1 belong to
+      const double u0 = ovalue(r0), u1 = ovalue(r1);
+      const double move = xabs * fabs(p0 - q0) + fabs(p1 - q1);
+      const double pad = 1.001 * move + 0.01 * (u1 - u0);
+      found = cluster_select_near(cl, key, lo, hi, mq - 1, N - mq - 1, u0 - pad, u1 + pad, sm, r0, r1);
+    }
+    if (!found) cluster_select2(cl, key, lo, hi, mq - 1, N - mq - 1, sm, r0, r1);
     q0 = p0;
     q1 = p1;
     dd = (ovalue(r1) - ovalue(r0)) + kEps;
   }
-  // mu: smallest leaf mean (method 4) or the mode of the leaf means (3)
-  double mn = 1e300, mx = -1e300;
-  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    mn = fmin(mn, X[i]);
-    mx = fmax(mx, X[i]);
-  }
-  mn = -cluster_max(cl, -mn, sm);
-  mx = cluster_max(cl, mx, sm);
-  // mu and sigma by the noise method (noise.hpp:115-147)
+  // mu and sigma by the noise method (noise.hpp:115-147): mn is the smallest leaf
+  // mean (method 4), mx bounds the modes
   int* h = a.hist + (size_t)w * (per + 1);
   unsigned long long* fk = a.fkey + (size_t)w * (per + 1);
   int* fi = a.fidx + (size_t)w * (per + 1);
@@ -920,11 +1104,16 @@ cudaError_t launch_noise_frames(const float* xs, const double* x64, int nimg, in
   if (lbig > 0) k_quad_decide_big<<<dim3(level_off(lbig), nimg), 256, 0, s>>>(src, nlev, nf.split);
   if (nsmall > 0)
     k_quad_decide_small<<<dim3((nsmall + 7) / 8, nimg), 256, 0, s>>>(src, nlev, lbig, nf.split);
-  k_quad_tree<<<(nimg + 63) / 64, 64, 0, s>>>(nf.split, nimg, S, nlev, nf.maxNodes, nf.nodes,
-                                              nf.isdel, nf.leaf, nf.nleaf, nf.dup, nf.first,
-                                              nf.err);
-  k_big_leaves<<<(nimg + 63) / 64, 64, 0, s>>>(nf.leaf, nf.nleaf, nimg, nf.maxNodes, nf.big,
-                                               nf.nbig);
+  constexpr size_t kTreeSmem = 200 * 1024;
+  const bool nodes_fit = (size_t)nf.maxNodes * 4 + level_off(nlev) <= kTreeSmem;
+  const bool split_fits = (size_t)level_off(nlev) <= kTreeSmem;  // sides up to 4096
+  const size_t shm = (nodes_fit ? (size_t)nf.maxNodes * 4 : 0) + (split_fits ? level_off(nlev) : 0);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_quad_tree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTreeSmem);
+  if (e != cudaSuccess) return e;
+  k_quad_tree<<<nimg, kTreeThreads, shm, s>>>(nf.split, S, nlev, nf.maxNodes, nodes_fit, nf.nodes,
+                                              nf.leaf, nf.nleaf, nf.dup, nf.first, nf.big, nf.nbig,
+                                              nf.err, split_fits);
   k_leaf_stats_small<<<dim3((nf.maxNodes + 3) / 4, nimg), 128, 0, s>>>(src, nf.leaf, nf.nleaf,
                                                                        nf.dup, nf.maxNodes,
                                                                        nf.stats);

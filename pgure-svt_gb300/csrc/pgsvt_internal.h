@@ -265,8 +265,7 @@ cudaError_t launch_risk_round(const Problem& pb, const DeviceBuffers& d, double*
 struct NoiseFrames {
   int nlev, maxNodes, maxBig;
   uint8_t* split;   // [nimg][blocks of side > 8] F-test decisions
-  int4* nodes;      // [nimg][maxNodes] quadtree replay scratch
-  uint8_t* isdel;   // [nimg][maxNodes]
+  int4* nodes;      // [nimg][maxNodes] quadtree replay scratch (large frames)
   int4* leaf;       // [nimg][maxNodes] leaves (row, col, side) in the reference's order
   int* nleaf;       // [nimg]
   int* big;         // [nimg][maxNodes] indices of leaves of side > 32

@@ -158,3 +158,34 @@ def test_arps_cost_forms(capi, oracle, bs, vmax, dtype):
     Y, _, _ = capi.denoise(X, capi.default_params(**kw))
     Yo, _, _ = oracle.denoise(X, n_jobs=4, **kw)
     assert np.abs(Y - Yo).max() <= 2e-5 * np.abs(Yo).max()
+
+
+def _noise_window(kind, side, T):
+    """Frames of the noise estimator's rare cases, maximum 1."""
+    rng = np.random.default_rng(side + T)
+    if kind == "random":
+        u = 1.0 + rng.random((side, side, 1)) * rng.random((side, side, T))
+    else:
+        # three quarters made of one 8 x 8 tile each: a few hundred equal leaves
+        u = 1.0 + 0.3 * rng.random((side, side, T))
+        y, x = np.mgrid[0:8, 0:8] / 7.0
+        h = side // 2
+        for q, (r, c) in enumerate(((0, 0), (0, h), (h, 0))):
+            tile = 0.5 + 0.7 * q + (x + q * y) ** 2 + 0.05 * (q + 1) * rng.random((8, 8))
+            u[r:r + h, c:c + h] = np.tile(tile, (h // 8, h // 8))[:, :, None]
+    return np.asfortranarray(u / u.max())
+
+
+@pytest.mark.parametrize("kind,side,T", [("random", 16, 5), ("random", 32, 15), ("random", 128, 5),
+                                         ("tiles", 64, 7), ("tiles", 256, 5)])
+def test_noise_estimates_of_equal_and_few_leaves(capi, oracle, kind, side, T):
+    """Frames of one to a thousand leaves; equal leaves have equal residuals,
+    which the bracketed order statistics must hand to the radix selection.
+    1e-4: the robust means stop on an absolute tolerance of 1e-6."""
+    u = _noise_window(kind, side, T)
+    for method in (1, 2, 3, 4):
+        p = capi.default_params(median_size=0, traj_length=T, noise_method=method, random_seed=3,
+                                search_points=4, search_rounds=1)
+        _, est, _ = capi.denoise(u, p)
+        ref = oracle.noise_estimate(u, method=method)
+        np.testing.assert_allclose(est[:, 1:], np.tile(ref, (T, 1)), rtol=1e-4)
