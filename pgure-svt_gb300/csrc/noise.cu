@@ -115,17 +115,6 @@ __device__ double block_sum(double v, double* red) {
   return t;
 }
 
-__device__ double block_max(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[wid] = v;
-  __syncthreads();
-  double t = red[0];
-  for (int q = 1; q < nw; ++q) t = fmax(t, red[q]);
-  return t;
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -338,22 +327,21 @@ __global__ void __launch_bounds__(kTreeThreads) k_quad_tree(
   }
 }
 
-// ConvolveFIR (noise.hpp:386-409) value at e = x + y*N of the N x N block:
+// ConvolveFIR (noise.hpp:386-409) value at (x, y) of the N x N block:
 // in(x, y) - (its 8 neighbours) / 8, in the order of the reference's 3x3
 // product with two interleaved accumulators.
 template <class A_t>
-__device__ __forceinline__ double lap_at(A_t A, int e, int N) {
-  const int x = e % N, y = e / N;
+__device__ __forceinline__ double lap_at(A_t A, int x, int y, int N) {
   const int xp = nxt(x, N), xm = prv(x, N), yp = nxt(y, N), ym = prv(y, N);
   const double nb[9] = {A(xm, ym), A(xm, y), A(xm, yp), A(x, ym), A(x, y),
                         A(x, yp), A(xp, ym), A(xp, y), A(xp, yp)};
   double v1 = 0.0, v2 = 0.0;
 #pragma unroll
-  for (int k = 0; k < 8; k += 2) {
-    v1 = __dadd_rn(v1, __dmul_rn(nb[k], k == 4 ? 1.0 : -0.125));
-    v2 = __dadd_rn(v2, __dmul_rn(nb[k + 1], -0.125));
+  for (int k = 0; k < 8; k += 2) {  // the products are exact
+    v1 = k == 4 ? __dadd_rn(v1, nb[k]) : __fma_rn(nb[k], -0.125, v1);
+    v2 = __fma_rn(nb[k + 1], -0.125, v2);
   }
-  v1 = __dadd_rn(v1, __dmul_rn(nb[8], -0.125));
+  v1 = __fma_rn(nb[8], -0.125, v1);
   return __dadd_rn(v1, v2);
 }
 
@@ -409,7 +397,7 @@ __global__ void __launch_bounds__(128) k_leaf_stats_small(FrameSrc src, const in
   const int m = iqd_m(n);
   const double alo = ovalue(buf[m - 1]), ahi = ovalue(buf[n - m - 1]);
   __syncwarp();
-  sort_vals([&](int e) { return lap_at(A, e, N); });
+  sort_vals([&](int e) { return lap_at(A, e % N, e / N, N); });
   const double med = median_sorted();
   __syncwarp();
   // |lap - med| of the sorted values (the order does not matter)
@@ -435,41 +423,66 @@ constexpr int kDigitBits = 11, kDigits = 1 << kDigitBits;
 namespace cg = cooperative_groups;
 
 struct ClusterSmem {
-  double red[32];
-  double part[8];
-  unsigned h[2][kDigits];   // this CTA's histograms
-  unsigned t[2][kDigits];   // the cluster's
+  double red[5][kClThreads / 32];
+  double part[2][5], tot[5];
+  double out[4];            // what the leading thread hands to its CTA
+  alignas(8) unsigned h[2][kDigits];   // this CTA's histograms
+  alignas(8) unsigned t[2][kDigits];   // the cluster's
   int dg[2], kk[2];
   int scan[kClThreads / 32 + 1];
-  int slice, cnt[2], ln[2];            // cluster_select_near
-  unsigned long long res[2];
+  int slice, cnt[2], ln[2], below[2], done;  // cluster_select_near, _list; the loops' ends
+  unsigned long long res[2], klo[2], khi[2];
 };
 
-// Sums over the cluster of up to 8 values per thread; every thread of every
-// CTA gets the same totals (the CTAs' partials added in rank order).
-template <int NV>
-__device__ void cluster_sums(cg::cluster_group& cl, double (&v)[NV], ClusterSmem& sm) {
+// Reductions over the cluster of up to 5 values per thread, by sum or maximum: every
+// CTA gets the same totals (the CTAs' partials combined in rank order) in sm.tot, and
+// its thread 0 runs lead() on them before the others go on.  One warp instruction of
+// FP64 holds an SM's unit for about 16 cycles, so what is the same for all threads is
+// computed by one.  `ph` alternates between two sets of partials, which makes one
+// cluster barrier per call enough; a kernel ends with one more.
+template <int NV, class Op, class F>
+__device__ void cluster_reduce(cg::cluster_group& cl, double (&v)[NV], ClusterSmem& sm, int& ph,
+                               Op op, F lead) {
+  const int tid = threadIdx.x, wid = tid >> 5;
+#pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const double b = block_sum(v[k], sm.red);
-    if (threadIdx.x == 0) sm.part[k] = b;
+    for (int o = 16; o > 0; o >>= 1) v[k] = op(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+    if ((tid & 31) == 0) sm.red[k][wid] = v[k];
+  }
+  __syncthreads();
+  if (tid < NV) {
+    double t = sm.red[tid][0];
+    for (int q = 1; q < kClThreads / 32; ++q) t = op(t, sm.red[tid][q]);
+    sm.part[ph][tid] = t;
   }
   cl.sync();
-  for (int k = 0; k < NV; ++k) {
-    double t = 0.0;
-    for (int r = 0; r < kCl; ++r) t += cl.map_shared_rank(sm.part, r)[k];
-    v[k] = t;
+  if (tid < 32) {
+    if (tid < NV) {
+      double t = cl.map_shared_rank(&sm, 0)->part[ph][tid];
+      for (int r = 1; r < kCl; ++r) t = op(t, cl.map_shared_rank(&sm, r)->part[ph][tid]);
+      sm.tot[tid] = t;
+    }
+    __syncwarp();
+    if (tid == 0) lead();
   }
-  cl.sync();  // the partials may be overwritten afterwards
+  ph ^= 1;
+  __syncthreads();
 }
 
-__device__ double cluster_max(cg::cluster_group& cl, double v, ClusterSmem& sm) {
-  const double b = block_max(v, sm.red);
-  if (threadIdx.x == 0) sm.part[0] = b;
-  cl.sync();
-  double t = *cl.map_shared_rank(sm.part, 0);
-  for (int r = 1; r < kCl; ++r) t = fmax(t, cl.map_shared_rank(sm.part, r)[0]);
-  cl.sync();
-  return t;
+struct AddOp {
+  __device__ double operator()(double a, double b) const { return a + b; }
+};
+struct MaxOp {
+  __device__ double operator()(double a, double b) const { return fmax(a, b); }
+};
+
+// smallest and largest value over the cluster
+__device__ void cluster_range(cg::cluster_group& cl, double& mn, double& mx, ClusterSmem& sm,
+                              int& ph) {
+  double v[2] = {-mn, mx};
+  cluster_reduce(cl, v, sm, ph, MaxOp(), [] {});
+  mn = -sm.tot[0];
+  mx = sm.tot[1];
 }
 
 // The digit of the k-th smallest key among the counts t[0..nb): a block-wide
@@ -554,92 +567,17 @@ __device__ void cluster_select2(cg::cluster_group& cl, K key, int lo, int hi, in
   v1 = pre[1];
 }
 
-// The k0-th and k1-th smallest of the n keys key(i) when both are expected in
-// [vlo, vhi]: a histogram over 2,046 equal bins of that range (and one to either
-// side), then the exact order among the few keys of the two bins.  The CTAs share
-// the work of adding their histograms up, so a call takes 4 cluster barriers where
-// the radix selection takes 12 (6 passes).  False, in every thread of the cluster,
-// when a rank falls outside the range or into a bin of more than kNear keys.
+// The kk[q]-th smallest of the n[q] keys that the CTAs of the cluster hold in their
+// lists (sm.t, sm.ln keys), ranked by every CTA for itself.  The lists of the other
+// CTAs are read until the caller's next cluster barrier.
 constexpr int kNear = 512;
+static_assert(kNear <= kClThreads && 2 * kNear * sizeof(unsigned long long) <= sizeof(ClusterSmem::t),
+              "lists");
 
-template <class K>
-__device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi, int k0, int k1,
-                                    double vlo, double vhi, ClusterSmem& sm,
-                                    unsigned long long& v0, unsigned long long& v1) {
-  constexpr int kSlice = kDigits / kCl;  // bins a CTA adds up
-  static_assert(kSlice <= kClThreads && 2 * kNear * 2 <= kDigits && kNear <= kClThreads, "sizes");
-  const int rank = (int)cl.block_rank(), tid = threadIdx.x;
-  if (!(vhi > vlo) || !isfinite(vlo) || !isfinite(vhi)) return false;
-  const double scale = (kDigits - 2) / (vhi - vlo);
-  auto bin = [&](double v) {  // monotone
-    if (!(v >= vlo)) return 0;
-    if (!(v < vhi)) return kDigits - 1;
-    return 1 + min(kDigits - 3, (int)((v - vlo) * scale));
-  };
-  for (int b = tid; b < kDigits; b += kClThreads) sm.h[0][b] = 0u;
-  if (tid < 2) sm.ln[tid] = 0;
-  __syncthreads();
-  for (int i = lo + tid; i < hi; i += kClThreads) atomicAdd(&sm.h[0][bin(ovalue(key(i)))], 1u);
-  cl.sync();
-  // this CTA's slice of the cluster's histogram
-  if (tid < kSlice) {
-    unsigned c = 0u;
-#pragma unroll
-    for (int r = 0; r < kCl; ++r) c += cl.map_shared_rank(&sm, r)->h[0][rank * kSlice + tid];
-    sm.t[0][tid] = c;
-  }
-  __syncthreads();
-  if (tid < 32) {
-    unsigned t = 0u;
-    for (int b = tid; b < kSlice; b += 32) t += sm.t[0][b];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (tid == 0) sm.slice = (int)t;
-  }
-  cl.sync();
-  int k[2] = {k0, k1}, owner[2];
-  {
-    int ss[kCl];
-#pragma unroll
-    for (int r = 0; r < kCl; ++r) ss[r] = cl.map_shared_rank(&sm, r)->slice;
-    for (int q = 0; q < 2; ++q) {
-      int o = 0;
-      while (o + 1 < kCl && k[q] >= ss[o]) k[q] -= ss[o++];
-      owner[q] = o;
-    }
-  }
-  for (int q = 0; q < 2; ++q)
-    if (owner[q] == rank) {  // uniform over the CTA
-      find_digit(sm.t[0], kSlice, k[q], &sm.dg[q], &sm.kk[q], sm.scan);
-      if (tid == 0) {
-        sm.cnt[q] = (int)sm.t[0][sm.dg[q]];
-        sm.dg[q] += rank * kSlice;
-      }
-      __syncthreads();
-    }
-  cl.sync();
-  int dg[2], kk[2], n[2];
-  bool ok = true;
-  for (int q = 0; q < 2; ++q) {
-    const ClusterSmem* os = cl.map_shared_rank(&sm, owner[q]);
-    dg[q] = os->dg[q];
-    kk[q] = os->kk[q];
-    n[q] = os->cnt[q];
-    ok = ok && dg[q] > 0 && dg[q] < kDigits - 1 && n[q] <= kNear;
-  }
-  if (!ok) {
-    cl.sync();  // the shared memory is used again
-    return false;
-  }
-  unsigned long long* list = reinterpret_cast<unsigned long long*>(sm.t[1]);  // [2][kNear]
-  for (int i = lo + tid; i < hi; i += kClThreads) {
-    const unsigned long long kv = key(i);
-    const int b = bin(ovalue(kv));
-    for (int q = 0; q < 2; ++q)
-      if (b == dg[q]) list[q * kNear + atomicAdd(&sm.ln[q], 1)] = kv;
-  }
-  cl.sync();
-  // every CTA ranks the keys of both bins
-  unsigned long long* all = reinterpret_cast<unsigned long long*>(sm.h[1]);  // [2][kNear]
+__device__ void rank_lists(cg::cluster_group& cl, const int (&n)[2], const int (&kk)[2],
+                           ClusterSmem& sm, unsigned long long& v0, unsigned long long& v1) {
+  const int tid = threadIdx.x;
+  unsigned long long* all = reinterpret_cast<unsigned long long*>(sm.h);  // [2][kNear]
   for (int q = 0; q < 2; ++q)
     if (tid < n[q]) {
       int r = 0, j = tid;
@@ -649,7 +587,7 @@ __device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi
         j -= nr;
       }
       all[q * kNear + tid] =
-          reinterpret_cast<const unsigned long long*>(cl.map_shared_rank(&sm, r)->t[1])[q * kNear + j];
+          reinterpret_cast<const unsigned long long*>(cl.map_shared_rank(&sm, r)->t)[q * kNear + j];
     }
   __syncthreads();
   for (int q = 0; q < 2; ++q)
@@ -666,6 +604,150 @@ __device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi
   v0 = sm.res[0];
   v1 = sm.res[1];
   __syncthreads();
+}
+
+// The k0-th and k1-th smallest of the n keys key(i) when both are expected in
+// [vlo, vhi]: a histogram over 2,046 equal bins of that range (and one to either
+// side), then the exact order among the few keys of the two bins.  The CTAs share
+// the work of adding their histograms up, so a call takes 4 cluster barriers where
+// the radix selection takes 12 (6 passes).  False, in every thread of the cluster,
+// when a rank falls outside the range or into a bin of more than kNear keys (in the
+// last of up to three rounds on ever smaller ranges, when the ranks are neighbours).
+template <class K>
+__device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi, int k0, int k1,
+                                    double vlo, double vhi, ClusterSmem& sm,
+                                    unsigned long long& v0, unsigned long long& v1) {
+  constexpr int kSlice = kDigits / kCl;  // bins a CTA adds up
+  static_assert(kSlice <= kClThreads, "one bin per thread");
+  const int rank = (int)cl.block_rank(), tid = threadIdx.x;
+  for (int round = 0; round < 3; ++round) {
+    if (!(vhi > vlo) || !isfinite(vlo) || !isfinite(vhi)) return false;
+    const double scale = (kDigits - 2) / (vhi - vlo);
+    auto bin = [&](double v) {  // monotone
+      if (!(v >= vlo)) return 0;
+      if (!(v < vhi)) return kDigits - 1;
+      return 1 + min(kDigits - 3, (int)((v - vlo) * scale));
+    };
+    for (int b = tid; b < kDigits; b += kClThreads) sm.h[0][b] = 0u;
+    if (tid < 2) sm.ln[tid] = 0;
+    __syncthreads();
+    for (int i = lo + tid; i < hi; i += kClThreads) atomicAdd(&sm.h[0][bin(ovalue(key(i)))], 1u);
+    cl.sync();
+    // this CTA's slice of the cluster's histogram
+    if (tid < kSlice) {
+      unsigned c = 0u;
+#pragma unroll
+      for (int r = 0; r < kCl; ++r) c += cl.map_shared_rank(&sm, r)->h[0][rank * kSlice + tid];
+      sm.t[0][tid] = c;
+    }
+    __syncthreads();
+    if (tid < 32) {
+      unsigned t = 0u;
+      for (int b = tid; b < kSlice; b += 32) t += sm.t[0][b];
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (tid == 0) sm.slice = (int)t;
+    }
+    cl.sync();
+    int k[2] = {k0, k1}, owner[2];
+    {
+      int ss[kCl];
+#pragma unroll
+      for (int r = 0; r < kCl; ++r) ss[r] = cl.map_shared_rank(&sm, r)->slice;
+      for (int q = 0; q < 2; ++q) {
+        int o = 0;
+        while (o + 1 < kCl && k[q] >= ss[o]) k[q] -= ss[o++];
+        owner[q] = o;
+      }
+    }
+    for (int q = 0; q < 2; ++q)
+      if (owner[q] == rank) {  // uniform over the CTA
+        find_digit(sm.t[0], kSlice, k[q], &sm.dg[q], &sm.kk[q], sm.scan);
+        if (tid == 0) {
+          sm.cnt[q] = (int)sm.t[0][sm.dg[q]];
+          sm.dg[q] += rank * kSlice;
+        }
+        __syncthreads();
+      }
+    cl.sync();
+    int dg[2], kk[2], n[2];
+    bool ok = true, inside = true;
+    for (int q = 0; q < 2; ++q) {
+      const ClusterSmem* os = cl.map_shared_rank(&sm, owner[q]);
+      dg[q] = os->dg[q];
+      kk[q] = os->kk[q];
+      n[q] = os->cnt[q];
+      inside = inside && dg[q] > 0 && dg[q] < kDigits - 1;
+      ok = ok && n[q] <= kNear;
+    }
+    if (!ok || !inside) {
+      cl.sync();  // the shared memory is used again
+      if (!inside || dg[1] - dg[0] > 1) return false;
+      // again on the bins' own range, with a bin to spare on either side
+      const double at = vlo;
+      vlo = at + (dg[0] - 2) / scale;
+      vhi = at + (dg[1] + 1) / scale;
+      continue;
+    }
+    unsigned long long* list = reinterpret_cast<unsigned long long*>(sm.t);  // [2][kNear]
+    for (int i = lo + tid; i < hi; i += kClThreads) {
+      const unsigned long long kv = key(i);
+      const int b = bin(ovalue(kv));
+      for (int q = 0; q < 2; ++q)
+        if (b == dg[q]) list[q * kNear + atomicAdd(&sm.ln[q], 1)] = kv;
+    }
+    cl.sync();
+    rank_lists(cl, n, kk, sm, v0, v1);
+    return true;
+  }
+  return false;
+}
+
+// The same for small brackets [klo, khi] of the keys, one for either rank: the keys
+// below are counted and the ones inside listed in a single pass of integer work, for
+// one cluster barrier.  False when a rank is not inside, or more than kNear keys are.
+template <class K>
+__device__ bool cluster_select_list(cg::cluster_group& cl, K key, int lo, int hi, int k0, int k1,
+                                    const unsigned long long (&klo)[2],
+                                    const unsigned long long (&khi)[2], ClusterSmem& sm,
+                                    unsigned long long& v0, unsigned long long& v1) {
+  const int tid = threadIdx.x;
+  if (tid < 2) sm.ln[tid] = sm.below[tid] = 0;
+  __syncthreads();
+  unsigned long long* list = reinterpret_cast<unsigned long long*>(sm.t);  // [2][kNear]
+  int below[2] = {0, 0};
+  for (int i = lo + tid; i < hi; i += kClThreads) {
+    const unsigned long long kv = key(i);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (kv < klo[q]) {
+        ++below[q];
+      } else if (kv <= khi[q]) {
+        const int at = atomicAdd(&sm.ln[q], 1);
+        if (at < kNear) list[q * kNear + at] = kv;
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int c = __reduce_add_sync(0xffffffffu, below[q]);
+    if ((tid & 31) == 0) atomicAdd(&sm.below[q], c);
+  }
+  cl.sync();
+  int k[2] = {k0, k1}, n[2] = {0, 0};
+  for (int r = 0; r < kCl; ++r) {
+    const ClusterSmem* rs = cl.map_shared_rank(&sm, r);
+    for (int q = 0; q < 2; ++q) {
+      k[q] -= rs->below[q];
+      n[q] += rs->ln[q];
+    }
+  }
+  bool ok = true;
+  for (int q = 0; q < 2; ++q) ok = ok && k[q] >= 0 && k[q] < n[q] && n[q] <= kNear;
+  if (!ok) {
+    cl.sync();  // the counts are used again
+    return false;
+  }
+  rank_lists(cl, n, k, sm, v0, v1);
   return true;
 }
 
@@ -677,8 +759,11 @@ __device__ __forceinline__ double median_from(unsigned long long lo, unsigned lo
 }
 
 // Per (frame, unique leaf of side > 32): the leaf statistics of
-// k_leaf_stats_small by one cluster per leaf.
-__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
+// k_leaf_stats_small by one cluster per leaf.  FP64 bounds it (the Laplacian is
+// evaluated anew in every pass), so the order statistics take three passes each,
+// the range, a histogram over it and a short list, where the radix selection takes
+// six.  512 x 512 x 40, GB300: 13.0 -> 7.5 ms.
+__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads, 2)
     k_leaf_stats_big(FrameSrc src, const int4* leaf, const int* big, const int* nbig,
                      const int* dup, int maxNodes, double* stats) {
   cg::cluster_group cl = cg::this_cluster();
@@ -689,18 +774,30 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
   const int li = big[(size_t)f * maxNodes + bi];
   if (dup[(size_t)f * maxNodes + li] >= 0) return;
   const int4 q = leaf[(size_t)f * maxNodes + li];
-  const int N = q.z, n = N * N;
+  const int N = q.z, n = N * N, sh = 31 - __clz(N);  // N > 32 is a power of two
   const int lo = (int)((long long)n * rank / kCl), hi = (int)((long long)n * (rank + 1) / kCl);
   auto A = [&](int r, int c) { return src.at(f, q.x + r, q.y + c); };
   const int m = iqd_m(n);
+  int ph = 0;
   unsigned long long a0, a1, l0, l1, d0, d1;
-  cluster_select2(cl, [&](int e) { return okey(A(e % N, e / N)); }, lo, hi, m - 1, n - m - 1, sm,
-                  a0, a1);
+  // the two keys by their range, or by radix when too many fall together
+  auto select = [&](auto value, int k0, int k1, unsigned long long& v0, unsigned long long& v1) {
+    const auto key = [&](int e) { return okey(value(e)); };
+    double mn = 1e300, mx = -1e300;
+    for (int e = lo + threadIdx.x; e < hi; e += kClThreads) {
+      const double v = value(e);
+      mn = fmin(mn, v);
+      mx = fmax(mx, v);
+    }
+    cluster_range(cl, mn, mx, sm, ph);
+    if (!cluster_select_near(cl, key, lo, hi, k0, k1, mn, mx, sm, v0, v1))
+      cluster_select2(cl, key, lo, hi, k0, k1, sm, v0, v1);
+  };
+  select([&](int e) { return A(e & (N - 1), e >> sh); }, m - 1, n - m - 1, a0, a1);
   const int mlo = n % 2 ? n / 2 : n / 2 - 1;
-  cluster_select2(cl, [&](int e) { return okey(lap_at(A, e, N)); }, lo, hi, mlo, n / 2, sm, l0, l1);
+  select([&](int e) { return lap_at(A, e & (N - 1), e >> sh, N); }, mlo, n / 2, l0, l1);
   const double med = median_from(l0, l1, n);
-  cluster_select2(cl, [&](int e) { return okey(fabs(lap_at(A, e, N) - med)); }, lo, hi, mlo,
-                  n / 2, sm, d0, d1);
+  select([&](int e) { return fabs(lap_at(A, e & (N - 1), e >> sh, N) - med); }, mlo, n / 2, d0, d1);
   const double mad = median_from(d0, d1, n);
   if (rank == 0 && threadIdx.x == 0) {
     const double sig = 1.4826 * mad;
@@ -709,6 +806,7 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
     o[1] = ovalue(a1);
     o[2] = sig * sig;
   }
+  cl.sync();  // no CTA ends while its lists are read
 }
 
 // RobustMeanEstimate (noise.hpp:239-270) of one leaf, run on the raw values
@@ -717,35 +815,80 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
 // so m_u = m_x / um without dividing every element.  The weights of an
 // iteration come from the previous (m, 1/d), so nothing is stored per
 // element; the IQD of r = x - m is (x_hi - m) - (x_lo - m) from the leaf's
-// order statistics.  `sum(a, b, c)` reduces three values over the
-// cooperating threads (a warp, or a cluster).
+// order statistics.  `red` reduces over the cooperating threads (a warp, or a
+// cluster) and evaluates what is the same for all of them; n is a power of 4 for
+// every leaf of a frame that can be split.
 template <class V, class R>
 __device__ double robust_mean(V val, int lo, int hi, int n, double xlo, double xhi, double um,
-                              int lane, int step, R sum) {
-  const double tol = kTol * um, eps = kEps * um;
-  double m = 0.0, m0 = 1e12 * um, mprev = 0.0, inv = 0.0;
+                              int lane, int step, R& red) {
+  const double tol = kTol * um, eps = kEps * um, ntol = tol * (double)n;
+  double m = 0.0, m0 = 1e12 * um, inv = 0.0;
   for (int it = 0; it < kMaxIter; ++it) {
     double sw = 0.0, swa = 0.0;
-    for (int e = lo + lane; e < hi; e += step) {
-      const double x = val(e);
-      const double w = it == 0 ? 1.0 : huber((x - mprev) * inv);
+    for (int e = lo + lane, j = 0; e < hi; e += step, ++j) {
+      const double x = val(e, j);
+      const double w = it == 0 ? 1.0 : huber((x - m) * inv);
       sw += w;
       swa += w * x;
     }
-    double se = 0.0;
+    m = red.two(sw, swa, [&](double a, double b) { return (fabs(a) < kEps) ? m0 : b / a; });
     // e = mean |x - m| needs m first: a second pass after the reduction
-    sum(sw, swa, se, false);
-    m = (fabs(sw) < kEps) ? m0 : swa / sw;
-    for (int e = lo + lane; e < hi; e += step) se += fabs(val(e) - m);
-    sum(sw, swa, se, true);
-    if (fabs(m0 - m) < tol || se / (double)n < tol) break;
+    double se = 0.0;
+    for (int e = lo + lane, j = 0; e < hi; e += step, ++j) se += fabs(val(e, j) - m);
+    bool stop;
+    inv = red.one(
+        se,
+        [&](double e, bool& end) {
+          end = fabs(m0 - m) < tol || e < ntol;
+          return end ? 0.0 : 1.0 / (((xhi - m) - (xlo - m)) + eps);
+        },
+        stop);
+    if (stop) break;
     m0 = m;
-    const double d = ((xhi - m) - (xlo - m)) + eps;
-    mprev = m;
-    inv = 1.0 / d;
   }
   return m / um;
 }
+
+// by a warp; two sums share the first step of the exchange, the lower half of the
+// warp going on with the one and the upper half with the other
+struct WarpRed {
+  template <class F>
+  __device__ double two(double a, double b, F f) {
+    const bool up = threadIdx.x & 16;
+    double v = up ? b : a;
+    v += __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return f(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 16));
+  }
+  template <class F>
+  __device__ double one(double e, F f, bool& stop) {
+    return f(warp_sum(e), stop);
+  }
+};
+
+// by a cluster
+struct ClusterRed {
+  cg::cluster_group& cl;
+  ClusterSmem& sm;
+  int ph;
+  template <class F>
+  __device__ double two(double a, double b, F f) {
+    double v[2] = {a, b};
+    cluster_reduce(cl, v, sm, ph, AddOp(), [&] { sm.out[0] = f(sm.tot[0], sm.tot[1]); });
+    return sm.out[0];
+  }
+  template <class F>
+  __device__ double one(double e, F f, bool& stop) {
+    double v[1] = {e};
+    cluster_reduce(cl, v, sm, ph, AddOp(), [&] {
+      bool end;
+      sm.out[1] = f(sm.tot[0], end);
+      sm.done = end;
+    });
+    stop = sm.done;
+    return sm.out[1];
+  }
+};
 
 struct PairArgs {
   FrameSrc src;
@@ -762,7 +905,9 @@ struct PairArgs {
 };
 
 // robust means of the leaves of side <= 32 of every (frame, normalisation)
-// pair: one warp per leaf
+// pair: one warp per leaf.  FP64 bounds it: the 8 x 8 leaves, most of them, stay in
+// registers, and the two sums of an iteration share their exchanges.  512 x 512 x
+// 40, GB300: 9.2 -> 7.3 ms.
 __global__ void __launch_bounds__(128) k_leaf_mean_warp(PairArgs a) {
   const int pr = blockIdx.y, lane = threadIdx.x & 31;
   const int li = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -773,16 +918,17 @@ __global__ void __launch_bounds__(128) k_leaf_mean_warp(PairArgs a) {
   const int N = q.z;
   const double um = a.pair_norm[pr];
   const double* st = a.stats + (f * a.maxNodes + li) * 3;
-  const double m = robust_mean(
-      [&](int e) { return a.src.at(f, q.x + e % N, q.y + e / N); }, 0, N * N, N * N, st[0], st[1],
-      um, lane, 32, [](double& x, double& y, double& z, bool zonly) {
-        if (zonly) {
-          z = warp_sum(z);
-        } else {
-          x = warp_sum(x);
-          y = warp_sum(y);
-        }
-      });
+  WarpRed red;
+  double m;
+  if (N == 8) {
+    const double v[2] = {a.src.at(f, q.x + (lane & 7), q.y + (lane >> 3)),
+                         a.src.at(f, q.x + (lane & 7), q.y + 4 + (lane >> 3))};
+    m = robust_mean([&](int, int j) { return j ? v[1] : v[0]; }, 0, 64, 64, st[0], st[1], um, lane,
+                    32, red);
+  } else {
+    m = robust_mean([&](int e, int) { return a.src.at(f, q.x + e % N, q.y + e / N); }, 0, N * N,
+                    N * N, st[0], st[1], um, lane, 32, red);
+  }
   if (lane == 0) a.mean[(size_t)pr * a.maxNodes + li] = m;
 }
 
@@ -797,24 +943,15 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads)
   if (a.dup[f * a.maxNodes + li] >= 0) return;
   __shared__ ClusterSmem sm;
   const int4 q = a.leaf[f * a.maxNodes + li];
-  const int N = q.z, n = N * N;
+  const int N = q.z, n = N * N, sh = 31 - __clz(N);  // N > 32 is a power of two
   const int lo = (int)((long long)n * rank / kCl), hi = (int)((long long)n * (rank + 1) / kCl);
   const double* st = a.stats + (f * a.maxNodes + li) * 3;
-  const double m = robust_mean(
-      [&](int e) { return a.src.at(f, q.x + e % N, q.y + e / N); }, lo, hi, n, st[0], st[1],
-      a.pair_norm[pr], threadIdx.x, blockDim.x, [&](double& x, double& y, double& z, bool zonly) {
-        if (zonly) {
-          double v[1] = {z};
-          cluster_sums(cl, v, sm);
-          z = v[0];
-        } else {
-          double v[2] = {x, y};
-          cluster_sums(cl, v, sm);
-          x = v[0];
-          y = v[1];
-        }
-      });
+  ClusterRed red{cl, sm, 0};
+  const double m = robust_mean([&](int e, int) { return a.src.at(f, q.x + (e & (N - 1)), q.y + (e >> sh)); },
+                               lo, hi, n, st[0], st[1], a.pair_norm[pr], threadIdx.x, blockDim.x,
+                               red);
   if (rank == 0 && threadIdx.x == 0) a.mean[(size_t)pr * a.maxNodes + li] = m;
+  cl.sync();  // no CTA ends while its partials are read
 }
 
 struct FitArgs {
@@ -838,12 +975,16 @@ struct FitArgs {
 };
 
 // WLSFit (noise.hpp:302-358) and the method's mu / sigma for every window:
-// one cluster per window.  What bounds it is the latency of the cluster barriers
-// and of the two order statistics that every iteration takes of the residuals.
-// They move by at most max |x| |dp0| + |dp1| when the line moves by (dp0, dp1), so
-// after the first iteration they are looked for around the last ones
-// (cluster_select_near); two CTAs share an SM.  GB300: 8.0 -> 5.5 ms (128 x 128 x
-// 64 frames), 26 -> 24 ms (512 x 512 x 40).
+// one cluster per window.  What bounds it is FP64 arithmetic, and the barriers of
+// the cluster on few leaves.  So the residuals and the weights, with their two
+// divisions, are computed once for the leaves that the recursion lists twice, and
+// the two order statistics of the residuals that every iteration takes are looked
+// for by their keys: they move by no more than the residuals do when the line moves
+// by (dp0, dp1), so after the first iteration they are found around the last ones
+// (cluster_select_list, and cluster_select_near while the line still moves far).
+// The sums go over all entries in their order.  GB300: 8.0 ms with 6 radix passes
+// per iteration and everything per entry and per thread, 2.2 ms now (128 x 128 x 40
+// frames); 26 and 16 ms (512 x 512 x 40).
 __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads, 2)
     k_noise_fit(FitArgs a) {
   cg::cluster_group cl = cg::this_cluster();
@@ -877,58 +1018,105 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads, 2)
     X[i] = a.mean[(size_t)a.win_pair[(size_t)w * nwin + k] * a.maxNodes + src];
     Y[i] = a.stats[(f * a.maxNodes + src) * 3 + 2] / um2;
   }
+  // the entries that repeat no other, in order: entry U[lo + j], slot lo + j
+  int* slot = a.hist + (size_t)w * (per + 1);            // of every entry
+  double* W2 = reinterpret_cast<double*>(a.fkey + (size_t)w * (per + 1));  // by slot, like K
+  int* U = a.fidx + (size_t)w * (per + 1);
+  int nu = 0;
+  for (int i0 = lo; i0 < hi; i0 += kClThreads) {  // uniform over the block
+    const int i = i0 + threadIdx.x;
+    int k = 0, total;
+    while (i < hi && k + 1 < nwin && i >= base[k + 1]) ++k;
+    const bool own = i < hi && a.dup[(size_t)(s0 + k) * a.maxNodes + i - base[k]] < 0;
+    const int at = lo + nu + block_scan(own, sm.scan, &total);
+    if (own) {
+      U[at] = i;
+      slot[i] = at;
+      W2[at] = 1.0;
+    }
+    nu += total;
+  }
+  __threadfence();
   cl.sync();
+  for (int i = lo + threadIdx.x; i < hi; i += kClThreads) {
+    int k = 0;
+    while (k + 1 < nwin && i >= base[k + 1]) ++k;
+    const int dp = a.dup[(size_t)(s0 + k) * a.maxNodes + i - base[k]];
+    if (dp >= 0) slot[i] = __ldcg(&slot[base[k] + dp]);
+  }
   double mn = 1e300, mx = -1e300;
   for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
     mn = fmin(mn, X[i]);
     mx = fmax(mx, X[i]);
   }
-  mn = -cluster_max(cl, -mn, sm);
-  mx = cluster_max(cl, mx, sm);
+  int ph = 0;
+  cluster_range(cl, mn, mx, sm, ph);
   const double xabs = fmax(fabs(mn), fabs(mx));
   unsigned long long r0 = 0, r1 = 0;
   const int mq = ((N + 1) / 2 + 1) / 2;
-  double a0 = 1e12, b0 = 1e12, p0 = 0.0, p1 = 0.0, q0 = 0.0, q1 = 0.0, dd = 1.0;
+  double a0 = 1e12, b0 = 1e12, p0 = 0.0, p1 = 0.0;
   for (int it = 0; it < kMaxIter; ++it) {
     double s[5] = {0, 0, 0, 0, 0};
     for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
       const double xi = X[i], yi = Y[i];
-      const double wt = it == 0 ? 1.0 : huber((yi - (xi * q0 + q1)) / dd);
-      const double w2 = wt * wt;
+      const double w2 = __ldcg(&W2[slot[i]]);
       s[0] += w2;
       s[1] += w2 * xi;
       s[2] += w2 * yi;
       s[3] += w2 * (xi * yi);
       s[4] += w2 * (xi * xi);
     }
-    cluster_sums(cl, s, sm);
-    p0 = s[0] * s[3] - s[1] * s[2];
-    const double aux = s[0] * s[4] - s[1] * s[1];
-    p0 = (fabs(aux) < kEps) ? a0 : p0 / aux;
-    p1 = s[2] - p0 * s[1];
-    p1 = (fabs(aux) < kEps) ? b0 : p1 / s[0];
-    double se[1] = {0.0};
-    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-      const double r = Y[i] - (X[i] * p0 + p1);
-      se[0] += fabs(r);
-      K[i] = okey(r);
+    const double q0 = p0, q1 = p1;  // the line that r0 and r1 belong to
+    cluster_reduce(cl, s, sm, ph, AddOp(), [&] {
+      const double* t = sm.tot;
+      double c0 = t[0] * t[3] - t[1] * t[2];
+      const double aux = t[0] * t[4] - t[1] * t[1];
+      c0 = (fabs(aux) < kEps) ? a0 : c0 / aux;
+      double c1 = t[2] - c0 * t[1];
+      c1 = (fabs(aux) < kEps) ? b0 : c1 / t[0];
+      sm.out[0] = c0;
+      sm.out[1] = c1;
+    });
+    p0 = sm.out[0];
+    p1 = sm.out[1];
+    for (int j = lo + threadIdx.x; j < lo + nu; j += blockDim.x) {
+      const int i = U[j];
+      K[j] = okey(Y[i] - (X[i] * p0 + p1));
     }
-    cluster_sums(cl, se, sm);  // its syncs also publish K
-    if ((fabs(a0 - p0) < kTol && fabs(b0 - p1) < kTol) || se[0] / (double)N < kTol) break;
+    __threadfence();
+    cl.sync();
+    const auto key = [&](int i) { return __ldcg(&K[slot[i]]); };
+    double se[1] = {0.0};
+    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) se[0] += fabs(ovalue(key(i)));
+    cluster_reduce(cl, se, sm, ph, AddOp(), [&] {
+      sm.done = (fabs(a0 - p0) < kTol && fabs(b0 - p1) < kTol) || sm.tot[0] / (double)N < kTol;
+      // a residual moves by -(x dp0 + dp1), and an order statistic within the range
+      const double u0 = ovalue(r0), u1 = ovalue(r1);
+      const double ma = mn * (p0 - q0) + (p1 - q1), mb = mx * (p0 - q0) + (p1 - q1);
+      const double eps = 1e-12 * (fabs(u0) + fabs(u1) + xabs * fabs(p0) + fabs(p1));
+      const double down = fmax(ma, mb) + eps, up = eps - fmin(ma, mb);
+      sm.out[2] = u0 - down;
+      sm.out[3] = u1 + up;
+      sm.klo[0] = okey(u0 - down);
+      sm.klo[1] = okey(u1 - down);
+      sm.khi[0] = okey(u0 + up);
+      sm.khi[1] = okey(u1 + up);
+    });
+    if (sm.done) break;
     a0 = p0;
     b0 = p1;
-    const auto key = [&](int i) { return K[i]; };
-    bool found = false;
-    if (it > 0) {  // q0, q1: the line that r0 and r1 belong to
-      const double u0 = ovalue(r0), u1 = ovalue(r1);
-      const double move = xabs * fabs(p0 - q0) + fabs(p1 - q1);
-      const double pad = 1.001 * move + 0.01 * (u1 - u0);
-      found = cluster_select_near(cl, key, lo, hi, mq - 1, N - mq - 1, u0 - pad, u1 + pad, sm, r0, r1);
-    }
+    const bool found =
+        it > 0 && (cluster_select_list(cl, key, lo, hi, mq - 1, N - mq - 1, sm.klo, sm.khi, sm, r0, r1) ||
+                   cluster_select_near(cl, key, lo, hi, mq - 1, N - mq - 1, sm.out[2], sm.out[3], sm,
+                                       r0, r1));
     if (!found) cluster_select2(cl, key, lo, hi, mq - 1, N - mq - 1, sm, r0, r1);
-    q0 = p0;
-    q1 = p1;
-    dd = (ovalue(r1) - ovalue(r0)) + kEps;
+    const double dd = (ovalue(r1) - ovalue(r0)) + kEps;
+    for (int j = lo + threadIdx.x; j < lo + nu; j += blockDim.x) {
+      const double wt = huber(ovalue(K[j]) / dd);
+      W2[j] = wt * wt;
+    }
+    __threadfence();
+    cl.sync();
   }
   // mu and sigma by the noise method (noise.hpp:115-147): mn is the smallest leaf
   // mean (method 4), mx bounds the modes
@@ -1043,7 +1231,8 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads, 2)
   } else if (a.method == 2) {
     double ymx = -1e300;
     for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) ymx = fmax(ymx, Y[t]);
-    ymx = cluster_max(cl, ymx, sm);
+    double ymn = 0.0;
+    cluster_range(cl, ymn, ymx, sm, ph);
     const double mmode = mode_all([&](int t) { return X[t]; }, mx, true);
     const double dSi = mode_all([&](int t) { return Y[t]; }, ymx, false);
     if (mu < 0) mu = mmode;
@@ -1062,6 +1251,7 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads, 2)
     a.est[(size_t)w * 3 + 1] = mu;
     a.est[(size_t)w * 3 + 2] = sigma;
   }
+  cl.sync();  // no CTA ends while its lists are read
 }
 
 // The estimates of a window batch into its window constants: caller-side
