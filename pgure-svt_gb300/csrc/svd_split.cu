@@ -11,8 +11,8 @@
 // singular vectors of B directly (R = W S U_X^T, so B = (Q W) S U_X^T):
 // v_t = U_X e_t, and the left ones follow from B itself, u_t = B v_t / s_t.
 // Q and W are never formed.
-//   k_qr      16 lanes per patch: B staged in shared memory, Householder
-//             reflections in a runtime loop; X = R^T to a scratch array
+//   k_qr      16 lanes per patch: Householder reflections on four columns at a
+//             time in registers; X = R^T to a scratch array
 //   k_xsweep  4 lanes x (NC/4) rows per patch, eight patches per warp: the
 //             register-form Jacobi sweeps of svd_kernel.cuh (same rotations,
 //             same convergence rules) on X; the singular values, sorted, and
@@ -49,7 +49,6 @@ struct QrDims {
   static constexpr int RX = (NC + 3) / 4;  // rows of X per lane in the sweeps
   static constexpr int XR = 4 * RX;        // rows of X (NC rounded up to 4)
   static constexpr int CS = XR + 1;        // column stride of X staged in shared memory
-  static constexpr int MS = 68;            // column stride of B in shared memory (64 rows)
 };
 
 // One patch's source: window, trajectory and the perturbation of its copy.
@@ -143,19 +142,43 @@ __device__ __forceinline__ void tma_tile3(uint32_t dst, const CUtensorMap* map, 
 }
 
 // ---- Householder QR of every patch's Casorati matrix, X = R^T to xq
-// ([item][NC][XR]; column k of X = row k of R).  B in shared memory, one
-// reflection per column in a runtime loop, four rows per lane.
+// ([item][NC][XR]; column k of X = row k of R).  Four rows per lane, four columns
+// at a time in registers: the reflections of the earlier columns come from shared
+// memory, one after the other, and their four dot products share one exchange
+// over the lanes (each in half_sum's order).  What bounds it is the L1 data pipe
+// (80% busy: gathers, shuffles and shared memory), and all columns in shared memory
+// with one exchange per dot product took four times the last two.  256 x 256 x 24, 8 x 8 patches, GB300:
+// 22.4 -> 14.3 ms in 3 launches.
+
+// f[i] = beta * half_sum(t[i])
+__device__ __forceinline__ void half_sums4(const float (&t)[4], float beta, float (&f)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool b0 = lane & 1, b1 = lane & 2;
+  float k0 = b0 ? t[2] : t[0], k1 = b0 ? t[3] : t[1];
+  k0 += __shfl_xor_sync(0xffffffffu, b0 ? t[0] : t[2], 1);
+  k1 += __shfl_xor_sync(0xffffffffu, b0 ? t[1] : t[3], 1);
+  float v = b1 ? k1 : k0;
+  v += __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 8);
+  v *= beta;  // lanes 0, 2, 1, 3 of every four hold t[0..3]'s
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = __shfl_sync(0xffffffffu, v, (i >> 1) | ((i & 1) << 1), 4);
+}
+
 template <int NC>
-__global__ void __launch_bounds__(128) k_qr(Problem pb, DeviceBuffers d, int nitems) {
+__global__ void __launch_bounds__(128, 8) k_qr(Problem pb, DeviceBuffers d, int nitems) {
   using D = QrDims<NC>;
+  constexpr int kRows = kQL * kQR;
   const Geometry& g = pb.g;
   const int lane = threadIdx.x & 31, l16 = lane & (kQL - 1);
   const int slot = threadIdx.x >> 4;  // patch of the block (8 per block)
   const int gid = blockIdx.x * 8 + slot;
   const bool live = gid < nitems;
   const int nwin = g.nwin, M = g.M;
-  __shared__ __align__(16) float Bs[8][NC * D::MS];
-  float* B = Bs[slot];
+  constexpr int kKept = D::XR - 4;  // reflections that a later column needs
+  __shared__ __align__(16) float Hs[8][kKept * kRows];  // their vectors
+  __shared__ float Bt[8][kKept];                        // and factors
   int p, c, w;
   {
     const int gg = live ? gid : 0;
@@ -166,75 +189,94 @@ __global__ void __launch_bounds__(128) k_qr(Problem pb, DeviceBuffers d, int nit
   }
   PatchSrc src;
   src.init(pb, d, p, c, w);
-  // gather B (svt.hpp:101-109): rows l16*4 .. +3 of every column
-  for (int k = 0; k < NC; ++k) {
-    const bool colok = live && k < nwin;
-    const size_t b = colok ? src.base(k) : 0;
-    float4 v;
-    float* vp = &v.x;
-#pragma unroll
-    for (int r = 0; r < kQR; ++r) {
-      const int e = l16 * kQR + r;
-      vp[r] = (colok && e < M) ? src.value(b + (e % g.bs) + (size_t)(e / g.bs) * g.S) : 0.f;
-    }
-    *reinterpret_cast<float4*>(B + k * D::MS + l16 * kQR) = v;
-  }
-  __syncwarp();
   const int r0 = l16 * kQR;
-  for (int jj = 0; jj < nwin; ++jj) {
-    const float4 x4 = *reinterpret_cast<const float4*>(B + jj * D::MS + r0);
-    const float* xp = &x4.x;
-    float ss = 0.f;  // |rows >= jj of column jj|^2
+  int roff[kQR];
 #pragma unroll
-    for (int r = 0; r < kQR; ++r)
-      if (r0 + r >= jj) ss = fmaf(xp[r], xp[r], ss);
-    ss = half_sum(ss);
-    const float xj = B[jj * D::MS + jj];
-    const float alpha = xj >= 0.f ? -sqrtf(ss) : sqrtf(ss);
-    const float vtv = 2.f * (ss - xj * alpha);  // |x - alpha e_jj|^2
-    const float beta = vtv > 0.f ? 2.f / vtv : 0.f;
-    float v[kQR];
+  for (int r = 0; r < kQR; ++r)
+    roff[r] = r0 + r < M ? ((r0 + r) % g.bs) + ((r0 + r) / g.bs) * g.S : -1;
+  float* H = Hs[slot] + r0;
+  float* xo = d.xq + ((size_t)gid * NC + r0) * D::XR;
+  for (int j0 = 0; j0 < D::XR; j0 += 4) {
+    float b[4][kQR];  // columns j0 .. j0 + 3 (svt.hpp:101-109)
 #pragma unroll
-    for (int r = 0; r < kQR; ++r) {
-      const int e = r0 + r;
-      v[r] = e > jj ? xp[r] : (e == jj ? xj - alpha : 0.f);
+    for (int i = 0; i < 4; ++i) {
+      const bool colok = live && j0 + i < nwin;
+      const size_t at = colok ? src.base(j0 + i) : 0;
+#pragma unroll
+      for (int r = 0; r < kQR; ++r)
+        b[i][r] = (colok && roff[r] >= 0) ? src.value(at + roff[r]) : 0.f;
     }
-#pragma unroll 4
-    for (int kk = jj + 1; kk < nwin; ++kk) {
-      float4 b4 = *reinterpret_cast<const float4*>(B + kk * D::MS + r0);
-      float* bp = &b4.x;
-      float t = 0.f;
+    const int jn = min(j0, nwin);
+    for (int j = 0; j < jn; ++j) {
+      const float4 v4 = *reinterpret_cast<const float4*>(H + j * kRows);
+      const float* v = &v4.x;
+      float t[4], f[4];
 #pragma unroll
-      for (int r = 0; r < kQR; ++r) t = fmaf(v[r], bp[r], t);
-      const float f = beta * half_sum(t);
+      for (int i = 0; i < 4; ++i) {
+        t[i] = 0.f;
 #pragma unroll
-      for (int r = 0; r < kQR; ++r) bp[r] = fmaf(-f, v[r], bp[r]);
-      *reinterpret_cast<float4*>(B + kk * D::MS + r0) = b4;
+        for (int r = 0; r < kQR; ++r) t[i] = fmaf(v[r], b[i][r], t[i]);
+      }
+      half_sums4(t, Bt[slot][j], f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int r = 0; r < kQR; ++r) b[i][r] = fmaf(-f[i], v[r], b[i][r]);
     }
-    __syncwarp();
-    float4 o4 = x4;
-    float* op = &o4.x;
 #pragma unroll
-    for (int r = 0; r < kQR; ++r) {
-      const int e = r0 + r;
-      if (e == jj) op[r] = alpha;
-      else if (e > jj) op[r] = 0.f;
-    }
-    *reinterpret_cast<float4*>(B + jj * D::MS + r0) = o4;
-    __syncwarp();
-  }
-  // X column k = row k of R (rows >= nwin of R are zero)
-  if (live && l16 < NC) {
-    float* xo = d.xq + ((size_t)gid * NC + l16) * D::XR;
+    for (int i = 0; i < 4; ++i) {
+      const int jj = j0 + i;
+      if (jj >= nwin) break;  // warp-uniform
+      float ss = 0.f;         // |rows >= jj of column jj|^2
 #pragma unroll
-    for (int j = 0; j < D::XR; j += 4) {
-      float4 t;
-      t.x = j + 0 < NC ? B[(j + 0) * D::MS + l16] : 0.f;
-      t.y = j + 1 < NC ? B[(j + 1) * D::MS + l16] : 0.f;
-      t.z = j + 2 < NC ? B[(j + 2) * D::MS + l16] : 0.f;
-      t.w = j + 3 < NC ? B[(j + 3) * D::MS + l16] : 0.f;
-      *reinterpret_cast<float4*>(xo + j) = t;
+      for (int r = 0; r < kQR; ++r)
+        if (r0 + r >= jj) ss = fmaf(b[i][r], b[i][r], ss);
+      ss = half_sum(ss);
+      const float xj = __shfl_sync(0xffffffffu, b[i][i], j0 >> 2, kQL);  // row jj
+      const float alpha = xj >= 0.f ? -sqrtf(ss) : sqrtf(ss);
+      const float vtv = 2.f * (ss - xj * alpha);  // |x - alpha e_jj|^2
+      const float beta = vtv > 0.f ? 2.f / vtv : 0.f;
+      float4 v4;
+      float* v = &v4.x;
+#pragma unroll
+      for (int r = 0; r < kQR; ++r) {
+        const int e = r0 + r;
+        v[r] = e > jj ? b[i][r] : (e == jj ? xj - alpha : 0.f);
+        if (e == jj) b[i][r] = alpha;
+        else if (e > jj) b[i][r] = 0.f;
+      }
+      if (jj < kKept) {
+        *reinterpret_cast<float4*>(H + jj * kRows) = v4;
+        if (l16 == 0) Bt[slot][jj] = beta;
+      }
+      float t[4] = {0.f, 0.f, 0.f, 0.f}, f[4];
+#pragma unroll
+      for (int n = i + 1; n < 4; ++n)
+#pragma unroll
+        for (int r = 0; r < kQR; ++r) t[n] = fmaf(v[r], b[n][r], t[n]);
+      if (i < 2) {
+        half_sums4(t, beta, f);
+      } else if (i == 2) {
+        f[3] = beta * half_sum(t[3]);
+      }
+#pragma unroll
+      for (int n = i + 1; n < 4; ++n)
+#pragma unroll
+        for (int r = 0; r < kQR; ++r) b[n][r] = fmaf(-f[n], v[r], b[n][r]);
     }
+    __syncwarp();  // Bt
+    // X column k = row k of R (rows >= nwin of R are zero)
+    if (live)
+#pragma unroll
+      for (int r = 0; r < kQR; ++r)
+        if (r0 + r < NC) {
+          float4 t;
+          t.x = j0 + 0 < nwin ? b[0][r] : 0.f;
+          t.y = j0 + 1 < nwin ? b[1][r] : 0.f;
+          t.z = j0 + 2 < nwin ? b[2][r] : 0.f;
+          t.w = j0 + 3 < nwin ? b[3][r] : 0.f;
+          *reinterpret_cast<float4*>(xo + r * D::XR + j0) = t;
+        }
   }
 }
 
