@@ -788,9 +788,40 @@ __global__ void __launch_bounds__(128) k_counts(Problem pb, DeviceBuffers d) {
   flush<1>(f, tile, kCountTile, c, 0, 1, g.S, lane);
 }
 
-// ---- sum over voxels of (Uh - U)^2 for every lambda of the round; clears acc
+// The warp's sums of KT values per thread in FP64, each in warp_sum_d's order: while
+// more than one value is left, the halves of the lanes go on with half of the values
+// each, so 8 values take 9 FP64 additions instead of 40 (an SM needs 16 cycles for
+// one).  Value `j` is this lane's; lanes that differ in the last steps' bits agree.
+template <int KT>
+__device__ __forceinline__ double warp_sums_d(const float (&v)[KT], int n, int& j) {
+  const int lane = threadIdx.x & 31;
+  double x[KT];
+#pragma unroll
+  for (int t = 0; t < KT; ++t) x[t] = t < n ? (double)v[t] : 0.0;
+  j = 0;
+#pragma unroll
+  for (int o = 16, m = KT / 2; o > 0; o >>= 1, m >>= 1) {
+    if (m > 0) {
+      const bool up = lane & o;
+      j += up ? m : 0;
+#pragma unroll
+      for (int t = 0; t < m; ++t) {
+        const double give = up ? x[t] : x[t + m];
+        x[t] = (up ? x[t + m] : x[t]) + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    } else {
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+    }
+  }
+  return x[0];
+}
+
+// ---- sum over voxels of (Uh - U)^2 for every lambda of the round; clears acc.
+// Bound by DRAM, so a thread has the loads of two voxels in flight.  Eight windows of
+// 256 x 256 x 15, GB300: 166 -> 126 us a round (one voxel at a time, and five FP64
+// additions per warp and lambda).
 template <typename AccT, int KT>
-__global__ void __launch_bounds__(256) k_mse(Problem pb, DeviceBuffers d) {
+__global__ void __launch_bounds__(256, sizeof(AccT) * KT <= 32 ? 3 : 1) k_mse(Problem pb, DeviceBuffers d) {
   const Geometry& g = pb.g;
   const int w = blockIdx.y;
   const SearchState& st = d.st[w];
@@ -800,34 +831,44 @@ __global__ void __launch_bounds__(256) k_mse(Problem pb, DeviceBuffers d) {
   const float* u = d.u + (size_t)w * C;
   const int32_t* cnt = d.cnt + (size_t)w * C;
   AccT* acc = (AccT*)d.acc + (size_t)w * pb.K * C;
+  constexpr int U = sizeof(AccT) * KT <= 64 ? 2 : 1;  // voxels side by side
+  const size_t step = (size_t)gridDim.x * blockDim.x;
   float part[KT];  // a thread sees about 16 voxels: FP32 partials, FP64 beyond
 #pragma unroll
   for (int j = 0; j < KT; ++j) part[j] = 0.f;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < C;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int n = __ldg(cnt + i);
-    const float uv = __ldg(u + i);
-    const float inv = n > 0 ? 1.f / (float)n : 0.f;
-    AccT av[KT];  // every load first: the clears below could alias them
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < C; i += U * step) {
+    int n[U];
+    float uv[U];
+    AccT av[U][KT];  // every load first: the clears below could alias them
+    const bool two = U > 1 && i + step < C;
 #pragma unroll
-    for (int j = 0; j < KT; ++j) av[j] = (j < nl) ? __ldcs(acc + (size_t)j * C + i) : (AccT)0;
+    for (int v = 0; v < U; ++v) {
+      const size_t at = v > 0 && two ? i + step : i;
+      n[v] = __ldg(cnt + at);
+      uv[v] = __ldg(u + at);
 #pragma unroll
-    for (int j = 0; j < KT; ++j)
-      if (j < nl) __stcs(acc + (size_t)j * C + i, (AccT)0);
+      for (int j = 0; j < KT; ++j)
+        av[v][j] = (j < nl) ? __ldcs(acc + (size_t)j * C + at) : (AccT)0;
+    }
 #pragma unroll
-    for (int j = 0; j < KT; ++j) {
-      const float df = Acc<AccT>::unfix(av[j]) * inv - uv;
-      if (j < nl) part[j] = fmaf(df, df, part[j]);
+    for (int v = 0; v < U; ++v) {
+      const size_t at = v > 0 && two ? i + step : i;
+      const bool use = v == 0 || two;
+      const float inv = n[v] > 0 ? 1.f / (float)n[v] : 0.f;
+#pragma unroll
+      for (int j = 0; j < KT; ++j) {
+        if (j < nl) __stcs(acc + (size_t)j * C + at, (AccT)0);
+        const float df = Acc<AccT>::unfix(av[v][j]) * inv - uv[v];
+        const float add = fmaf(df, df, part[j]);
+        if (j < nl) part[j] = use ? add : part[j];
+      }
     }
   }
   __shared__ double sm[KT][8];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int j = 0; j < KT; ++j) {
-    if (j >= nl) break;
-    const double t = warp_sum_d((double)part[j]);
-    if (lane == 0) sm[j][wid] = t;
-  }
+  const int wid = threadIdx.x >> 5;
+  int jw;
+  const double t = warp_sums_d<KT>(part, nl, jw);
+  sm[jw][wid] = t;  // the lanes of one value write the same
   __syncthreads();
   if (threadIdx.x < nl) {
     const int j = threadIdx.x;
