@@ -437,13 +437,23 @@ struct ArpsTable {
   ArpsChain c[kArpsChains];
 };
 
-// five blocks per SM: 96 registers.  Bound by the instructions of the costs and
-// their loads (nine tenths of them hit L1).  GB300, against one form with runtime
-// candidate lists, 64-bit integer sums and per-candidate error sums: 256 x 256 x
-// 100 floats 17.9 -> 11.2 ms; 256 x 256 x 24 bytes, 8 x 8 patches, 19.0 -> 6.6 ms; median-
-// filtered 512 x 512 x 40 (two thirds of it exact tie decisions) 115 -> 81 ms.
+// Resident blocks per SM.  The walks of a warp diverge, so more warps hide more of
+// their latency until the costs spill: patches of up to 4 x 4 pixels take 6 blocks
+// (80 registers; 256 x 256 x 100 floats 11.1 -> 10.8 ms, 7 blocks 11.9) and, with
+// integer costs, 7 (72; median-filtered 512 x 512 x 40 80.1 -> 69.4 ms, 6 blocks 74.4,
+// 8 blocks 77.9), larger ones 5 (8 x 8 patches, bytes, 6.6 ms; 6 blocks 7.7).
 template <int BS, int MODE>
-__global__ void __launch_bounds__(128, 5)
+constexpr int arps_blocks() {
+  return BS >= 1 && BS <= 4 && MODE != kInt64 ? (MODE == kIntF ? 7 : 6) : 5;
+}
+
+// Bound by the instructions of the costs and their loads (nine tenths of them hit
+// L1).  GB300, against one form with runtime candidate lists, 64-bit integer sums
+// and per-candidate error sums: 256 x 256 x 100 floats 17.9 -> 10.8 ms; 256 x 256 x
+// 24 bytes, 8 x 8 patches, 19.0 -> 6.6 ms; median-filtered 512 x 512 x 40 (two thirds
+// of it exact tie decisions) 115 -> 69 ms.
+template <int BS, int MODE>
+__global__ void __launch_bounds__(128, arps_blocks<BS, MODE>())
     k_arps(Problem pb, DeviceBuffers d, const __grid_constant__ ArpsTable tab) {
   const Geometry& g = pb.g;
   const int it0 = blockIdx.x * blockDim.x + threadIdx.x;
