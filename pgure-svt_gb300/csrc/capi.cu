@@ -921,7 +921,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     clk.mark(1);
     check_launch(launch_arps(pbb, d, L.s), stats, pbb.motion ? 2 : 1);
     clk.mark(2);
-    check_launch(launch_fields(pbb, d, L.s), stats, 4);
+    check_launch(launch_fields(pbb, d, L.s), stats, pb.optimize ? 4 : 2);
     check_launch(launch_search_init(pbb, d, L.s), stats);  // sets the lambda range
     clk.mark(3);
     if (tune) {

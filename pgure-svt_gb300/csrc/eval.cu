@@ -42,7 +42,8 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 // probe code only: k_field_table tabulates them in FP64 for the coverages below
 // kFieldTab (the FP64 pipe, at 1/64 of the FP32 rate, was what bounded the
 // kernel: a division and ten products per voxel); what is left in FP64 per voxel
-// is sum(U).  Two windows of 512 x 512 x 15, GB300: 0.27 -> 0.10 ms.
+// is sum(U).  Two windows of 512 x 512 x 15, GB300: 0.27 -> 0.10 ms.  Without the risk
+// there are no fields, and nothing reads sum(U).
 constexpr int kFieldTab = 256;
 
 // (field 0, field 2) of a voxel covered n times
@@ -68,8 +69,6 @@ __global__ void __launch_bounds__(256) k_fields(Problem pb, DeviceBuffers d) {
   const WinConst& wc = d.wc[w];
   const float* u = d.u + (size_t)w * C;
   const int32_t* cnt = d.cnt + (size_t)w * C;
-  const double a = wc.alpha, m = wc.mu, s2 = wc.sigma * wc.sigma;
-  const double c2 = 2 * s2 * a / (wc.eps2 * wc.eps2);
   const bool intd1 = pb.compat & 0x4;
   const int8_t* d1 = d.d1 + (size_t)w * d.probe_stride;
   const int8_t* d2c = d.d2code + (size_t)w * d.probe_stride;
@@ -79,7 +78,6 @@ __global__ void __launch_bounds__(256) k_fields(Problem pb, DeviceBuffers d) {
        i += (size_t)gridDim.x * blockDim.x) {
     const double uv = u[i];
     su += uv;
-    if (!pb.optimize) continue;
     const int n = cnt[i];
     const bool code = d2c[i] != 0;
     if (intd1) {
@@ -89,6 +87,8 @@ __global__ void __launch_bounds__(256) k_fields(Problem pb, DeviceBuffers d) {
       d.fld2[(size_t)w * C + i] = f.y;
       continue;
     }
+    const double a = wc.alpha, m = wc.mu, s2 = wc.sigma * wc.sigma;
+    const double c2 = 2 * s2 * a / (wc.eps2 * wc.eps2);
     const double ic = n > 0 ? 1.0 / n : 0.0;
     const double dl2 = code ? d.d2neg : d.d2pos;
     const double l1 = (2 / wc.eps1) * d1[i] * ((a * uv - a * m) + s2);
@@ -188,12 +188,14 @@ __global__ void __launch_bounds__(kFieldBlocks) k_search_init(Problem pb, Device
   SearchState& s = d.st[w];
   __shared__ double part[kFieldBlocks];
   __shared__ double s_upper;
-  part[threadIdx.x] = d.part_mse[(size_t)w * kFieldBlocks + threadIdx.x];
+  part[threadIdx.x] = pb.optimize ? d.part_mse[(size_t)w * kFieldBlocks + threadIdx.x] : 0.0;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
+    if (pb.optimize) {
 #pragma unroll 8
-    for (int b = 0; b < kFieldBlocks; ++b) t += part[b];
+      for (int b = 0; b < kFieldBlocks; ++b) t += part[b];
+    }
     wc.sum_u = t;
     s.npts = 0;
     s.nnext = 0;
@@ -1053,7 +1055,8 @@ cudaError_t launch_fields(const Problem& pb, const DeviceBuffers& d, cudaStream_
   cudaMemsetAsync(d.cnt, 0, sizeof(int32_t) * g.cube() * pb.W, s);
   dim3 gc((g.NP + 127) / 128, g.nwin, pb.W);
   k_counts<<<gc, 128, 0, s>>>(pb, d);
-  if (pb.optimize && (pb.compat & 0x4)) k_field_table<<<dim3(2, pb.W), kFieldTab, 0, s>>>(pb, d);
+  if (!pb.optimize) return cudaGetLastError();
+  if (pb.compat & 0x4) k_field_table<<<dim3(2, pb.W), kFieldTab, 0, s>>>(pb, d);
   k_fields<<<dim3(kFieldBlocks, pb.W), 256, 0, s>>>(pb, d);
   return cudaGetLastError();
 }
