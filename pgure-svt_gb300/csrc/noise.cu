@@ -32,8 +32,9 @@
 //                   stays a leaf), and lists the leaves in its order
 //   k_leaf_stats    per (frame, unique leaf): order statistics (IQD bounds,
 //                   Laplacian median and MAD) by warp bitonic sorts in shared
-//                   memory (sides <= 32) or by a cluster of 8 CTAs with
-//                   11-bit radix selection over distributed shared memory
+//                   memory (sides <= 32) or by a cluster of 8 CTAs over
+//                   distributed shared memory: a histogram of the values'
+//                   range and a short list, 11-bit radix selection in general
 //   k_leaf_mean     per (frame, window maximum) pair: one warp per leaf of
 //                   side <= 32, one cluster of 8 CTAs per larger leaf: the
 //                   IRLS robust mean, on the raw values with the absolute
@@ -42,7 +43,7 @@
 //                   the first one's results
 //   k_noise_fit     one cluster of 8 CTAs per window, all windows in one
 //                   launch (distributed shared memory for the sums and the
-//                   radix selections): the IRLS fit, mu, sigma; modes over
+//                   order statistics): the IRLS fit, mu, sigma; modes over
 //                   all leaves by a histogram of the n + 1 rounded values
 //                   with first-occurrence keys, method 1's few leaves by
 //                   a radix selection and the reference's O(n^2) count
@@ -621,9 +622,11 @@ __device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi
   static_assert(kSlice <= kClThreads, "one bin per thread");
   const int rank = (int)cl.block_rank(), tid = threadIdx.x;
   for (int round = 0; round < 3; ++round) {
-    if (!(vhi > vlo) || !isfinite(vlo) || !isfinite(vhi)) return false;
+    if (k0 < 0 || k1 < 0 || !(vhi > vlo) || !isfinite(vlo) || !isfinite(vhi)) return false;
     const double scale = (kDigits - 2) / (vhi - vlo);
-    auto bin = [&](double v) {  // monotone
+    auto bin = [&](unsigned long long kv) {  // monotone in the key, NaN too
+      const double v = ovalue(kv);
+      if (kv > okey(INFINITY)) return kDigits - 1;
       if (!(v >= vlo)) return 0;
       if (!(v < vhi)) return kDigits - 1;
       return 1 + min(kDigits - 3, (int)((v - vlo) * scale));
@@ -631,7 +634,7 @@ __device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi
     for (int b = tid; b < kDigits; b += kClThreads) sm.h[0][b] = 0u;
     if (tid < 2) sm.ln[tid] = 0;
     __syncthreads();
-    for (int i = lo + tid; i < hi; i += kClThreads) atomicAdd(&sm.h[0][bin(ovalue(key(i)))], 1u);
+    for (int i = lo + tid; i < hi; i += kClThreads) atomicAdd(&sm.h[0][bin(key(i))], 1u);
     cl.sync();
     // this CTA's slice of the cluster's histogram
     if (tid < kSlice) {
@@ -691,7 +694,7 @@ __device__ bool cluster_select_near(cg::cluster_group& cl, K key, int lo, int hi
     unsigned long long* list = reinterpret_cast<unsigned long long*>(sm.t);  // [2][kNear]
     for (int i = lo + tid; i < hi; i += kClThreads) {
       const unsigned long long kv = key(i);
-      const int b = bin(ovalue(kv));
+      const int b = bin(kv);
       for (int q = 0; q < 2; ++q)
         if (b == dg[q]) list[q * kNear + atomicAdd(&sm.ln[q], 1)] = kv;
     }
