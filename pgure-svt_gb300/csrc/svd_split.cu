@@ -583,12 +583,12 @@ __global__ void __launch_bounds__(128, 4) k_bsweep(Problem pb, DeviceBuffers d, 
 // side while one slice of B and G is in registers.  Nothing is held across
 // slices (the earlier form kept all of B and G, at 16 warps per SM, and was
 // bound by the latency of its loads and by sorting the columns).  256 x 256 x
-// 100, GB300: 35.0 -> 15.1 ms in 13 launches, still bound by the latency of the
-// gathers.
+// 100, GB300: 35.0 -> 15.3 ms in 13 launches, still bound by the latency of the
+// gathers: 7 blocks per SM (72 registers), where 8 took 16.6 and 6 or 10 16.8 ms.
 constexpr int kBT = 4;
 
 template <int NC>
-__global__ void __launch_bounds__(128, 8) k_bout(Problem pb, DeviceBuffers d, int nitems) {
+__global__ void __launch_bounds__(128, 7) k_bout(Problem pb, DeviceBuffers d, int nitems) {
   constexpr int RX = 4, XR = 16;
   const Geometry& g = pb.g;
   const int lane = threadIdx.x & 31, q = lane & 3;
