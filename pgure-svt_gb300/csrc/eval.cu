@@ -402,19 +402,7 @@ struct Acc<unsigned long long> {  // 2^-32
 // slice overlap heavily, so the warp sums them in a shared-memory tile in
 // int32 fixed point (2^-20, order-free) and adds the tile to the accumulator
 // with one atomic per touched pixel.
-// Pixels of a tile: the 32 blocks of an 8 x 4 half tile cover (7 + side) x (3 +
-// side) pixels when they move together, and a few more rows and columns as a
-// rule (simulated on the benchmark's trajectories: 4 x 4 patches fit 256 pixels
-// in 85% of the cases and 384 in 98%, 8 x 8 ones 256 in 62% and 512 in 97%; the
-// rest straddle two columns of tiles).  A footprint that does not fit costs a
-// global atomic per pixel and patch.  The int64 accumulators round values of the
-// tile and others differently, so they keep one size.
-// Patches of at most 16 rows with more than 8 lambda values in a round have no
-// room for more than 256 at two blocks per SM.
-template <int BS, typename AccT>
-__host__ __device__ constexpr int tile_pixels(int nl) {
-  return sizeof(AccT) == 8 ? 256 : (BS >= 1 && BS <= 4 ? (nl <= 8 ? 384 : 256) : 512);
-}
+// Its size is a launch's choice (eval_layout.h).
 constexpr float kTileBound = 60.f;  // |value| above this bypasses the tile (32 x 60 < 2048)
 constexpr float kMagicBound = 4.f;  // and below this value * 2^20 + 1.5 * 2^23 is exact
 
@@ -533,12 +521,6 @@ __device__ __forceinline__ float shrink(int expw, float s, float smax, float lam
 // pixels, divisions in the flush, conversions on the XU pipe, every triplet
 // shrunk, one lambda value per pass for the larger patches).
 
-// left vectors staged in shared memory for patches of at most 16 rows:
-// [triplet][lane][e], a lane's rows as 16-byte vectors that start on
-// different banks
-template <int M>
-constexpr int kUStride = M == 16 ? 20 : M;
-
 // Rows of a patch rebuilt per pass: all of a small patch, else whole columns, few
 // enough that the left vectors of a pass are loaded together within 64 registers
 // (16 rows of an 8 x 8 patch: the loads were made one by one, 62 instead of 34 ms).
@@ -569,12 +551,12 @@ __global__ void __launch_bounds__(32 * MAXW, MAXW <= 16 ? 2 : 1)
   extern __shared__ __align__(16) float sg[];  // left vectors, g of copy 0 [nl][NC][PB],
                                                // lin [nl][4][PB], tiles
   constexpr bool kStage = BS > 0 && BS * BS <= 16;
-  constexpr int US = kUStride<BS * BS>;
+  constexpr int US = eval_ustride(BS * BS);
   float* Us = sg;
-  float* sgv = kStage ? sg + NC * PB * US : sg;
-  const int T = tile_pixels<BS, AccT>(nl);
+  float* sgv = sg + eval_staged(BS, NC);
+  const int T = eval_tile(BS, sizeof(AccT) == 8, NC, nwarps, final_pass ? 1 : pb.K, nl);
   float* slin = sgv + (size_t)nl * NC * PB;
-  int* tiles = (int*)(slin + (size_t)nl * 4 * PB);
+  int* tiles = (int*)(sg + eval_tiles_at(BS, NC, nl));
   __shared__ int srmax[kMaxK];
   int* tile = tiles + (size_t)k * (2 * T);
   for (int i = lane * 4; i < 2 * T; i += 128) *reinterpret_cast<int4*>(tile + i) = make_int4(0, 0, 0, 0);
@@ -702,7 +684,7 @@ __global__ void __launch_bounds__(128) k_eval_out(Problem pb, DeviceBuffers d) {
   const Geometry& g = pb.g;
   const int w = blockIdx.y;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  constexpr int T = tile_pixels<BS, AccT>(1);
+  constexpr int T = eval_alloc_tile(BS, sizeof(AccT) == 8, 1);
   __shared__ int tiles[4][T];
   int* tile = tiles[wib];
   for (int i = lane; i < T; i += 32) tile[i] = 0;
@@ -953,14 +935,6 @@ __global__ void k_risk_collect(Problem pb, DeviceBuffers d, double* out) {
   }
 }
 
-// shared memory of a k_eval block (110 KB at most for windows up to 16 frames)
-template <int BS, typename AccT>
-size_t eval_smem(const Geometry& g, int nl) {
-  const int us = BS >= 1 && BS <= 4 ? g.NC * kUStride<BS * BS> : 0;  // staged left vectors
-  return ((size_t)nl * (g.NC + 4) + us) * kEvalPatches * sizeof(float) +
-         (size_t)g.nwin * 2 * tile_pixels<BS, AccT>(nl) * sizeof(int);
-}
-
 // Raise, never lower, a kernel's dynamic shared-memory limit on the current
 // device.  k_eval's footprint depends on the lambda count of the round, and
 // concurrent callers (pgsvt_denoise_batch runs sequences on several host
@@ -980,7 +954,9 @@ void allow_dynamic_smem(const void* kernel, size_t shm) {
 template <int BS, typename AccT>
 void launch_k_eval_bs(dim3 grid, int threads, int nl, cudaStream_t s, const Problem& pb,
                       const DeviceBuffers& d, int final_pass) {
-  const size_t shm = eval_smem<BS, AccT>(pb.g, nl);
+  // (110 KB at most for windows up to 16 frames)
+  const size_t shm =
+      (size_t)eval_alloc_words(BS, sizeof(AccT) == 8, pb.g.NC, pb.g.nwin, nl) * sizeof(int);
   if constexpr (BS > 0 && BS * BS <= 16) {  // windows of at most 15 frames
     allow_dynamic_smem((const void*)k_eval<BS, AccT, 16>, shm);
     k_eval<BS, AccT, 16><<<grid, threads, shm, s>>>(pb, d, final_pass);

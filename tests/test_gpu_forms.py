@@ -119,6 +119,44 @@ def test_owner_forms_are_identical(capi, pkg, bs, T, expw):
         np.testing.assert_array_equal(x, y)
 
 
+@pytest.mark.parametrize("points", [9, 10, 11, 12, 13, 16])
+@pytest.mark.parametrize("bs,T", [(3, 7), (4, 9), (4, 13), (4, 15)])
+@pytest.mark.parametrize("mode", ["plain", "hint", "learned", "budget"])
+def test_rounds_shorter_than_the_grid(capi, pkg, oracle, points, bs, T, mode):
+    """Searches of 9 to 16 grid points whose later rounds hold fewer values than
+    their launch allocates for: refinements of half the points, narrow searches of
+    4 to 6, a budget of 8 evaluations.  Against the oracle's risk at the returned
+    lambda (the tolerance of the risk tests), and its own search from the same
+    proposals (that of the search tests)."""
+    noisy, _, _ = _noisy(pkg, 32, T + 1, 80 + bs)
+    X = noisy.astype(np.float64)
+    fw = min(T, bs * bs - 1) // 2
+    noise = dict(alpha=0.01, mu=0.02, sigma=0.03)
+    kw = dict(traj_length=T, block_size=bs, motion_window=5, median_size=-1, random_seed=3,
+              search_points=points, frame_begin=fw, frame_end=fw + 1, **noise)
+    hints = None
+    if mode == "hint":
+        kw["lambda_hint"] = 1.0
+    elif mode == "budget":
+        kw["max_iter"] = 8
+    elif mode == "learned":
+        model = pkg.learned.load_model()
+        kw["lambda_model"] = model.ctypes.data
+    _, est, _, ex = capi.denoise_ex(X, capi.default_params(**kw), proposals=True)
+    if mode == "learned":
+        kw.pop("lambda_model")
+        hints = 100.0 * 10.0 ** np.clip(ex["proposals"].astype(np.float64), -6, 0)
+        hints = np.nan_to_num(hints, nan=1.0)  # frames out of range have no proposal
+    _, est0, rep = oracle.denoise(X, lambda_hints=hints, n_jobs=4, **kw)
+    u = X[:, :, :2 * fw + 1] / X[:, :, :2 * fw + 1].max()
+    rows, cols = oracle.arps_window(u, bs, 5, fw, fw, T + 1)
+    r = oracle.risk_window(u, bs, 1, rows, cols, [est[fw, 0], est0[fw, 0]], *noise.values(), 3)
+    assert abs(ex["risk"][fw] - r[0]) <= 1e-4 * abs(r[0])
+    assert (r[0] - r[1]) / abs(r[1]) < 0.01
+    if mode == "budget":
+        assert ex["evals"][fw] <= 8
+
+
 @pytest.mark.parametrize("side,nwin", [(8, 3), (17, 5), (21, 15), (32, 15)])
 @pytest.mark.parametrize("seed", [0, 11, 2 ** 63 - 1])
 def test_probe_streams(capi, oracle, side, nwin, seed):
