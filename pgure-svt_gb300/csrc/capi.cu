@@ -1171,7 +1171,9 @@ struct OneWindow {
     check_launch(launch_window_norm_only(pb, d, s), stats);
   }
   ~OneWindow() {
-    if (s) cudaStreamDestroy(s);
+    if (!s) return;
+    cudaStreamSynchronize(s);  // nothing may use the arrays when mem gives them back
+    cudaStreamDestroy(s);
   }
 
   void set_positions(const int32_t* rows, const int32_t* cols) {
@@ -1711,6 +1713,7 @@ int pgsvt_risk_window(const double* u, uint32_t nrows, uint32_t nwin, uint32_t b
     const Geometry& g = ow.pb.g;
     const size_t C = g.cube();
     ow.set_positions(rows, cols);
+    if (nl == 0) return;  // no risk to compute
     const int ncopies = (compat_flags & PGSVT_COMPAT_INT_DELTA1) ? 3 : 4;
     ow.alloc_factors(ncopies);
     ow.d.fld0 = ow.mem.arr<float>(C);

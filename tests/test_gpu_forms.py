@@ -227,3 +227,23 @@ def test_noise_estimates_of_equal_and_few_leaves(capi, oracle, kind, side, T):
         _, est, _ = capi.denoise(u, p)
         ref = oracle.noise_estimate(u, method=method)
         np.testing.assert_allclose(est[:, 1:], np.tile(ref, (T, 1)), rtol=1e-4)
+
+
+def test_risk_window_without_lambdas(capi, oracle):
+    """No lambda value: an empty result, and nothing of the call is left running on
+    memory that the next call gets (its results are those of a call before)."""
+    rng = np.random.default_rng(5)
+    u = rng.uniform(0.2, 1.0, (64, 64, 15))
+    u /= u.max()
+    P = 61 * 61
+    rows = np.tile(np.arange(P) % 61, (15, 1)).astype(np.int32)
+    cols = np.tile(np.arange(P) // 61, (15, 1)).astype(np.int32)
+    args = (0.02, 0.03, 0.05, 7)
+    r0 = capi.risk_window(u, 4, 1, rows, cols, [0.5, 5.0], *args)
+    ro = oracle.risk_window(u, 4, 1, rows, cols, [0.5, 5.0], *args)
+    assert np.abs(r0 - ro).max() <= 1e-4 * np.abs(ro).max()
+    for _ in range(8):
+        assert capi.risk_window(u, 4, 1, rows, cols, [], *args).size == 0
+        np.testing.assert_array_equal(capi.risk_window(u, 4, 1, rows, cols, [0.5, 5.0], *args), r0)
+    with pytest.raises(RuntimeError):  # the other arguments are still checked
+        capi.risk_window(u, 4, 1, rows + 61, cols, [], *args)
