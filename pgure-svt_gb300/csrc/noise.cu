@@ -157,12 +157,15 @@ __device__ void decide_block(const FrameSrc& src, int f, int b, int nlev, uint8_
   const size_t R = (size_t)N * N;
   const int lane = BLOCK ? threadIdx.x : (threadIdx.x & 31);
   const int step = BLOCK ? blockDim.x : 32;
-  const double isq30 = 1.0 / sqrt(30.0);  // 1 / sqrt(l*l + l), l = 5
+  const double sq30 = sqrt(30.0);  // sqrt(l*l + l), l = 5
   auto A = [&](int r, int c) { return src.at(f, i0 + r, j0 + c); };
+  // divided as the reference divides: a product with 1 / sqrt(30) differs by a
+  // rounding, and fused with the subtraction of the mean it leaves flat blocks a
+  // variance, which splits them
   auto res = [&](size_t e) {
     const int y = (int)(e % N), x = (int)(e / N);
     const double s4 = ((A(nxt(y, N), x) + A(prv(y, N), x)) + A(y, prv(x, N))) + A(y, nxt(x, N));
-    return (5.0 * A(y, x) - s4) * isq30;
+    return (5.0 * A(y, x) - s4) / sq30;
   };
   auto sum = [&](double v) { return BLOCK ? block_sum(v, red) : warp_sum(v); };
   double sa = 0.0, sr = 0.0;

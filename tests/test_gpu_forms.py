@@ -247,3 +247,30 @@ def test_risk_window_without_lambdas(capi, oracle):
         np.testing.assert_array_equal(capi.risk_window(u, 4, 1, rows, cols, [0.5, 5.0], *args), r0)
     with pytest.raises(RuntimeError):  # the other arguments are still checked
         capi.risk_window(u, 4, 1, rows + 61, cols, [], *args)
+
+
+@pytest.mark.parametrize("side,flat", [(32, 403.0), (32, 777.0), (32, 835.0), (32, 3943.0),
+                                       (64, 835.0), (128, 3943.0)])
+def test_flat_blocks_are_not_split(capi, oracle, side, flat):
+    """A quadrant of one value: its variance and its residuals' variance are both
+    zero, which is no split.  The values are chosen so that flat / sqrt(30) in FP64
+    ends in zero bits enough for the quadrant's residuals to add up exactly in any
+    order (and the maximum is a power of two, so that the oracle's normalised frames
+    behave the same): a residual off by one rounding makes the block split, which
+    changes the estimates by a tenth to a factor of three."""
+    rng = np.random.default_rng(1)
+    h = side // 2
+    y, x = np.mgrid[0:side, 0:side] * 32.0 / side
+    u = rng.poisson(200 + 20 * x + 9 * y, (3, side, side)).astype(np.float64).transpose(1, 2, 0)
+    u = np.minimum(u, 4000.0)
+    u[h:, h:] = flat
+    u[0, 0] = 4096.0
+    u = np.asfortranarray(u)
+    res = flat / np.sqrt(30.0)
+    assert (np.cumsum(np.full(h * h, res)) == np.arange(1, h * h + 1) * res).all()
+    for method in (1, 2, 3, 4):
+        p = capi.default_params(median_size=0, traj_length=3, noise_method=method, random_seed=3,
+                                search_points=4, search_rounds=1)
+        _, est, _ = capi.denoise(u, p)
+        ref = oracle.noise_estimate(u / 4096.0, method=method)
+        np.testing.assert_allclose(est[:, 1:], np.tile(ref, (3, 1)), rtol=1e-4)
