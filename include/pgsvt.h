@@ -383,6 +383,16 @@ int pgsvt_svd_window_noalloc(const float* u_dev, uint32_t nrows, uint32_t nwin,
                              const int32_t* rows_dev, const int32_t* cols_dev,
                              float* S_dev, uint32_t* npatch, void* stream);
 
+/* Give the device memory that the library keeps between calls back to the
+ * device.  The calls above (all but pgsvt_svd_window_noalloc) take their arrays
+ * from blocks that stay allocated when a call ends, at most 16 GiB per process, so
+ * that the next call need not allocate; a call frees them when an allocation
+ * of its own fails or when it leaves less than an eighth of the device's memory free.
+ * Another allocator in the process does not see them: call this before it needs
+ * the memory.  From any thread, also while other calls run (their blocks are
+ * theirs until they end).                                                    */
+int pgsvt_release_memory(void);
+
 /* Message of the last failing call on this thread ("" if none). */
 const char* pgsvt_last_error(void);
 

@@ -31,8 +31,8 @@ EXPORTS = ("pgsvt_default_params", "pgsvt_denoise", "pgsvt_denoise_device",
            "pgsvt_median_filter", "pgsvt_hot_pixel_filter",
            "pgsvt_arps_window", "pgsvt_svd_window", "pgsvt_svd_window_ex",
            "pgsvt_reconstruct_window",
-           "pgsvt_risk_window", "pgsvt_svd_window_noalloc", "pgsvt_last_error",
-           "pgsvt_version")
+           "pgsvt_risk_window", "pgsvt_svd_window_noalloc", "pgsvt_release_memory",
+           "pgsvt_last_error", "pgsvt_version")
 LAMBDA_FEATURES = 67
 LAMBDA_HIDDEN = 128
 LAMBDA_SAMPLES = 4096
@@ -158,6 +158,11 @@ def _check(rc):
 
 def _ptr(a):
     return ctypes.c_void_p(a.ctypes.data)
+
+
+def release_memory():
+    """pgsvt_release_memory: free the device memory kept between calls."""
+    _check(load().pgsvt_release_memory())
 
 
 def version():

@@ -335,9 +335,6 @@ size_t lambda_act_floats(int n);
 cudaError_t lambda_train_epoch(const LambdaTrain& t, cudaStream_t s);
 cudaError_t lambda_attrs();
 
-// identifier of the calling thread's current CUDA context (0: none yet)
-unsigned long long current_context_id();
-
 // message returned by pgsvt_last_error() on the calling thread
 void set_last_error(const std::string& m);
 
