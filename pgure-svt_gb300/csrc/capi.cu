@@ -836,6 +836,7 @@ int guarded(pgsvt_status* st, Fn&& fn) {
     code = f.code;
     cuda = f.cuda;
     g_err = f.what();
+    if (cuda) cudaGetLastError();  // reported here: the next call's launches must not see it
   } catch (const std::exception& e) {
     code = PGSVT_ERR_CUDA;
     g_err = e.what();

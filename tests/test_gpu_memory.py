@@ -1,5 +1,6 @@
 """Device memory kept between calls (csrc/device_memory.h) on the GPU: reuse by calls
-of other sizes, and giving it back."""
+of other sizes, a failed call, and giving it back."""
+import ctypes
 import threading
 
 import numpy as np
@@ -32,6 +33,16 @@ def test_results_do_not_depend_on_what_ran_before(capi, pkg):
     for _ in range(2):  # on blocks with other calls' contents
         for x, y in zip(_calls(capi, pkg), first):
             np.testing.assert_array_equal(x, y)
+
+
+def test_calls_after_a_failed_one(capi, pkg):
+    """One impossible allocation (575 GB) ends a call in the middle of its arrays."""
+    first = _calls(capi, pkg)
+    one = np.zeros(capi.LAMBDA_MODEL_FLOATS, np.float32)
+    ptr = ctypes.c_void_p(one.ctypes.data)  # not read: the allocation comes first
+    assert capi.load().pgsvt_lambda_predict(ptr, ptr, 2 ** 31, ptr) == capi.ERR_OOM
+    for x, y in zip(_calls(capi, pkg), first):
+        np.testing.assert_array_equal(x, y)
 
 
 def test_memory_is_given_back(capi, pkg):
