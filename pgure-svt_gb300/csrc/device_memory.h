@@ -60,6 +60,7 @@ class BlockCache {
     n = std::max(kBlock, (n + kBlock / 2 - 1) / (kBlock / 2) * (kBlock / 2));
     int dev = 0;
     PGSVT_CK(cudaGetDevice(&dev));
+    if (current_context_id() == 0) PGSVT_CK(cudaSetDevice(dev));  // a thread's first CUDA call
     const unsigned long long ctx = current_context_id();
     {
       std::lock_guard<std::mutex> lk(mu_);

@@ -139,6 +139,13 @@ CASES = {
   call({100 * MiB, 7 * MiB});  // and used again
   CHECK(live > 0);
 """,
+    # every call from a new thread: its first array too comes from the cache
+    "threads": r"""
+  call({30 * MiB, 7 * MiB, 50 * MiB});
+  const int m = mallocs;
+  for (int k = 0; k < 5; ++k) std::thread([] { call({30 * MiB, 7 * MiB, 50 * MiB}); }).join();
+  CHECK(mallocs == m && block_cache().cached() == live);
+""",
     # blocks of a context that a device reset destroyed are neither reused nor freed
     "reset": r"""
   call({100 * MiB});
