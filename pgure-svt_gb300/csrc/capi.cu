@@ -831,7 +831,10 @@ int guarded(pgsvt_status* st, Fn&& fn) {
   int code = PGSVT_OK, cuda = 0;
   g_err.clear();
   try {
-    fn(stats);
+    with_retry([&] {
+      stats = Stats();
+      fn(stats);
+    });
   } catch (const Fail& f) {
     code = f.code;
     cuda = f.cuda;

@@ -182,6 +182,23 @@ struct DevMem {
   ~DevMem() { release(); }
 };
 
+// Run a call, once more if it failed for lack of device memory.  The blocks that a
+// call reuses are up to twice as large as it needs; the second run has an empty
+// cache and allocates no more than its arrays.  (A call allocates before it writes
+// any output.)
+template <typename Fn>
+void with_retry(Fn&& fn) {
+  try {
+    fn();
+    return;
+  } catch (const Fail& f) {
+    if (f.cuda != (int)cudaErrorMemoryAllocation) throw;
+    cudaGetLastError();
+  }
+  block_cache().trim(0);
+  fn();
+}
+
 }  // namespace pgsvt
 
 #endif

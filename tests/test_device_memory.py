@@ -158,6 +158,34 @@ CASES = {
   block_cache().trim(0);
   CHECK(live == 0 && bad_frees == 0);
 """,
+    # arrays that fit the device one by one, after calls that left larger blocks: the
+    # reused blocks take what is missing, so the call starts again without them
+    "tight": r"""
+  kTotal = 10 * GiB;
+  call({3 * GiB, 3 * GiB});
+  int tries = 0;
+  try {
+    call({1600 * MiB, 1600 * MiB, 5 * GiB});
+    CHECK(!"fits without a second try");
+  } catch (const Fail&) {
+    cudaGetLastError();
+  }
+  with_retry([&] { ++tries; call({1600 * MiB, 1600 * MiB, 5 * GiB}); });
+  CHECK(tries == 2 && bad_frees == 0 && cudaGetLastError() == cudaSuccess);
+  tries = 0;
+  try {
+    with_retry([&] { ++tries; call({11 * GiB}); });
+  } catch (const Fail& f) {
+    CHECK(f.code == PGSVT_ERR_OOM);
+  }
+  CHECK(tries == 2);
+  tries = 0;
+  try {  // other failures are not tried again
+    with_retry([&] { ++tries; throw Fail(PGSVT_ERR_OOM, "not from an allocation"); });
+  } catch (const Fail&) {
+  }
+  CHECK(tries == 1);
+""",
     # little memory left on the device: a finished call keeps nothing
     "scarce": r"""
   kTotal = 10 * GiB;
