@@ -417,11 +417,12 @@ struct Footprint {
     x0 = __reduce_min_sync(0xffffffffu, live ? x : 1 << 30);
     const int y1 = __reduce_max_sync(0xffffffffu, live ? y : -1);
     const int x1 = __reduce_max_sync(0xffffffffu, live ? x : -1);
-    const int tw = x1 - x0 + nb;
-    th = y1 - y0 + nb;
+    const bool any = y1 >= 0;  // a lane holds a patch
+    const int tw = any ? x1 - x0 + nb : 0;
+    th = any ? y1 - y0 + nb : 0;
     ths = th <= 8 ? 8 : 8 + 16 * ((th - 8 + 15) / 16);
-    if (y1 >= 0 && ths * tw > tile_max) ths = th;
-    tile = y1 >= 0 && ths * tw <= tile_max;
+    if (ths * tw > tile_max) ths = th;
+    tile = any && ths * tw <= tile_max;
     area = th * tw;
   }
 };
