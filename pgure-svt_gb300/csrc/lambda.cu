@@ -186,7 +186,7 @@ __device__ void forward(const float* m, Smem& sm) {
 // Forward pass and the gradients of the pre-activations of the samples of one
 // batch (r0 .. n of the permuted order, rows padded to a multiple of 32): the
 // activations, gradients, output gradients and errors of every row to device
-// memory.  One block per GS rows; a batch of 256 fills 64 of the 152 SMs, and
+// memory.  One block per GS rows; a batch of 256 fills 64 SMs, and
 // its chains of dependent FMAs, not its 14 MFLOP, are what takes the time.
 // One training step (batch 256), GB300: 177 -> 11.7 us here and 8.5 us in
 // k_mlp_update (before, one block of 128 threads did everything for 32 samples).
@@ -475,7 +475,12 @@ cudaError_t lambda_shadow(const float* m, void* wbf, cudaStream_t s) {
 }
 
 // blocks of a pass over n rows: at most two per SM (their shared memory)
-static int pass_blocks(int n) { return std::min((n + lam::GS - 1) / lam::GS, 2 * 152); }
+static int pass_blocks(int n) {
+  int dev = 0, sms = 1;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return std::min((n + lam::GS - 1) / lam::GS, 2 * sms);
+}
 
 size_t lambda_rows(int n) { return ((size_t)n + 31) / 32 * 32; }
 size_t lambda_act_floats(int n) { return lambda_rows(n) * (lam::ACT_N * lam::H + 2); }
