@@ -74,37 +74,6 @@ __device__ __forceinline__ double ovalue(unsigned long long k) {
   return __longlong_as_double((long long)b);
 }
 
-// k-th smallest (0-based) of the n values val(i), by 8-bit radix digits of
-// their ordered bit patterns.  Called by every thread of the block.
-template <class F>
-__device__ double block_select(F val, int n, int k, unsigned* hist, int* sh) {
-  unsigned long long prefix = 0ull, mask = 0ull;
-  for (int shift = 56; shift >= 0; shift -= 8) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0u;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const unsigned long long kv = okey(val(i));
-      if ((kv & mask) == prefix) atomicAdd(&hist[(unsigned)(kv >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = 0, dg = 0;
-      for (; dg < 255; ++dg) {
-        if (acc + (int)hist[dg] > k) break;
-        acc += (int)hist[dg];
-      }
-      sh[0] = dg;
-      sh[1] = k - acc;
-    }
-    __syncthreads();
-    prefix |= (unsigned long long)sh[0] << shift;
-    mask |= 255ull << shift;
-    k = sh[1];
-    __syncthreads();
-  }
-  return ovalue(prefix);
-}
-
 __device__ double block_sum(double v, double* red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
