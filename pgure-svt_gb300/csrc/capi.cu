@@ -354,7 +354,7 @@ size_t window_bytes(const Problem& pb) {
   if (svd_split_scratch(g.M, g.NC)) b += 4 * NP * NC * 16 * 4;  // xq
   b += (size_t)pb.K * C * (pb.acc64 ? 8 : 4);  // acc
   b += (size_t)pb.K * ((NP + 31) / 32 + mse_blocks(g)) * 8 + 256 * 8;  // partials
-  b += sizeof(WinConst) + sizeof(SearchState) + 2 * (size_t)g.fw * sizeof(ArpsChain);
+  b += sizeof(WinConst) + sizeof(SearchState);
   return b;
 }
 
@@ -475,7 +475,7 @@ void run_sequence(const void* X_dev, int dtype, int S, int nimg, double* Y_dev, 
     nf.maxBig = 1 + 8 * noise_blocks(lbig);
     const size_t nn = (size_t)nimg * nf.maxNodes;
     nf.split = mem.arr<uint8_t>(std::max<size_t>(1, (size_t)nimg * B));
-    nf.nodes = mem.arr<int4>(nn);
+    nf.nodes = mem.arr<uint32_t>(nimg * noise_node_words(nf.nlev, nf.maxNodes));
     nf.leaf = mem.arr<int4>(nn);
     nf.nleaf = mem.arr<int>(nimg);
     nf.big = mem.arr<int>(nn);

@@ -207,13 +207,13 @@ __device__ int block_scan(int v, int* sh, int* total) {
 }
 
 __global__ void __launch_bounds__(kTreeThreads) k_quad_tree(
-    const uint8_t* split, int S, int nlev, int maxNodes, bool smem_nodes, int4* nodes, int4* leaf,
+    const uint8_t* split, int S, int nlev, int maxNodes, bool smem_nodes, uint32_t* nodes, int4* leaf,
     int* nleaf, int* dup, int* first, int* big, int* nbig, int* err, bool smem_split) {
   extern __shared__ uint32_t tsm[];
   __shared__ int s_len, s_min, s_bad, s_scan[kTreeThreads / 32];
   const int f = blockIdx.x, tid = threadIdx.x;
   const int nsplit = level_off(nlev), nids = level_off(nlev + 1);
-  uint32_t* nd = smem_nodes ? tsm : reinterpret_cast<uint32_t*>(nodes + (size_t)f * maxNodes);
+  uint32_t* nd = smem_nodes ? tsm : nodes + (size_t)f * maxNodes;
   const uint8_t* sp = split + (size_t)f * nsplit;
   if (smem_split) {
     uint8_t* sps = reinterpret_cast<uint8_t*>(tsm + (smem_nodes ? maxNodes : 0));
@@ -1261,6 +1261,15 @@ int noise_levels(int S) {
 }
 int noise_blocks(int nlev) { return level_off(nlev); }
 
+namespace {
+constexpr size_t kTreeSmem = 200 * 1024;
+bool nodes_fit(int nlev, int maxNodes) {
+  return (size_t)maxNodes * 4 + level_off(nlev) <= kTreeSmem;
+}
+}  // namespace
+// words of quadtree scratch per frame: none where the nodes stay in shared memory
+size_t noise_node_words(int nlev, int maxNodes) { return nodes_fit(nlev, maxNodes) ? 0 : maxNodes; }
+
 cudaError_t launch_noise_frames(const float* xs, const double* x64, int nimg, int S,
                                 const NoiseFrames& nf, cudaStream_t s) {
   const FrameSrc src{xs, x64, S};
@@ -1269,14 +1278,13 @@ cudaError_t launch_noise_frames(const float* xs, const double* x64, int nimg, in
   if (lbig > 0) k_quad_decide_big<<<dim3(level_off(lbig), nimg), 256, 0, s>>>(src, nlev, nf.split);
   if (nsmall > 0)
     k_quad_decide_small<<<dim3((nsmall + 7) / 8, nimg), 256, 0, s>>>(src, nlev, lbig, nf.split);
-  constexpr size_t kTreeSmem = 200 * 1024;
-  const bool nodes_fit = (size_t)nf.maxNodes * 4 + level_off(nlev) <= kTreeSmem;
+  const bool fit = nodes_fit(nlev, nf.maxNodes);
   const bool split_fits = (size_t)level_off(nlev) <= kTreeSmem;  // sides up to 4096
-  const size_t shm = (nodes_fit ? (size_t)nf.maxNodes * 4 : 0) + (split_fits ? level_off(nlev) : 0);
+  const size_t shm = (fit ? (size_t)nf.maxNodes * 4 : 0) + (split_fits ? level_off(nlev) : 0);
   const cudaError_t e =
       cudaFuncSetAttribute(k_quad_tree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTreeSmem);
   if (e != cudaSuccess) return e;
-  k_quad_tree<<<nimg, kTreeThreads, shm, s>>>(nf.split, S, nlev, nf.maxNodes, nodes_fit, nf.nodes,
+  k_quad_tree<<<nimg, kTreeThreads, shm, s>>>(nf.split, S, nlev, nf.maxNodes, fit, nf.nodes,
                                               nf.leaf, nf.nleaf, nf.dup, nf.first, nf.big, nf.nbig,
                                               nf.err, split_fits);
   k_leaf_stats_small<<<dim3((nf.maxNodes + 3) / 4, nimg), 128, 0, s>>>(src, nf.leaf, nf.nleaf,

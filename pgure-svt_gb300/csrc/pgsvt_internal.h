@@ -266,7 +266,7 @@ cudaError_t launch_risk_round(const Problem& pb, const DeviceBuffers& d, double*
 struct NoiseFrames {
   int nlev, maxNodes, maxBig;
   uint8_t* split;   // [nimg][blocks of side > 8] F-test decisions
-  int4* nodes;      // [nimg][maxNodes] quadtree replay scratch (large frames)
+  uint32_t* nodes;  // [nimg][noise_node_words()] quadtree replay scratch (large frames)
   int4* leaf;       // [nimg][maxNodes] leaves (row, col, side) in the reference's order
   int* nleaf;       // [nimg]
   int* big;         // [nimg][maxNodes] indices of leaves of side > 32
@@ -296,6 +296,7 @@ struct NoisePass {
 };
 int noise_levels(int S);
 int noise_blocks(int nlev);
+size_t noise_node_words(int nlev, int maxNodes);
 cudaError_t launch_noise_frames(const float* xs, const double* x64, int nimg, int S,
                                 const NoiseFrames& nf, cudaStream_t s);
 cudaError_t launch_noise_pass(const NoiseFrames& nf, const NoisePass& np, const float* xs,

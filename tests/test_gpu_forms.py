@@ -274,3 +274,18 @@ def test_flat_blocks_are_not_split(capi, oracle, side, flat):
         _, est, _ = capi.denoise(u, p)
         ref = oracle.noise_estimate(u / 4096.0, method=method)
         np.testing.assert_allclose(est[:, 1:], np.tile(ref, (3, 1)), rtol=1e-4)
+
+
+@pytest.mark.parametrize("side", [1024, 2048])
+def test_noise_of_large_frames(capi, oracle, side):
+    """The largest frames whose quadtree nodes stay in shared memory, and frames
+    whose nodes do not; every level splits somewhere."""
+    rng = np.random.default_rng(side)
+    y, x = np.mgrid[0:side, 0:side] / side
+    u = rng.poisson(50 + 40 * np.sin(9 * x) * np.cos(7 * y)) + rng.normal(0, 3, (side, side))
+    u = np.maximum(u, 0.0)[:, :, None]
+    u = np.asfortranarray(u / u.max())
+    p = capi.default_params(median_size=0, traj_length=1, random_seed=3, search_points=4,
+                            search_rounds=1)
+    _, est, _ = capi.denoise(u, p)
+    np.testing.assert_allclose(est[0, 1:], oracle.noise_estimate(u), rtol=1e-4)
