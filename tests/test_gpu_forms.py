@@ -289,3 +289,34 @@ def test_noise_of_large_frames(capi, oracle, side):
                             search_rounds=1)
     _, est, _ = capi.denoise(u, p)
     np.testing.assert_allclose(est[0, 1:], oracle.noise_estimate(u), rtol=1e-4)
+
+
+def test_fresh_probes_of_every_window(capi, pkg):
+    """A negative seed draws new probes for each window of a batch.  On equal windows
+    one shared set gives equal risks; fresh sets give risks that all differ, spread
+    as those of 24 seeds are (7 windows: within a factor of 10 of their deviation, and
+    6 deviations of their mean)."""
+    noisy, _, _ = _noisy(pkg, 32, 1, 91)
+    X = np.asfortranarray(np.repeat(noisy[:, :, :1], 13, axis=2))
+    kw = dict(traj_length=7, motion_window=5, median_size=-1, alpha=0.01, mu=0.02, sigma=0.03,
+              window_batch=4)
+
+    def risks(seed, **more):
+        p = capi.default_params(random_seed=seed, **kw, **more)
+        res, _ = capi.denoise_batch([dict(X=X, params=p, lambdas=[1.0])])
+        return res[0]["risks"][3:10, 0]
+
+    seeded = []
+    for seed in range(24):
+        r = risks(seed)
+        assert (r == r[0]).all()
+        seeded.append(r[0])
+    m, sd = np.mean(seeded), np.std(seeded)
+    assert sd > 0 and len(set(seeded)) == 24
+    for compat in (capi.COMPAT_ALL, capi.COMPAT_ALL & ~capi.COMPAT_INT_DELTA1):
+        r = risks(-1, compat_flags=compat)
+        assert len(set(r)) == 7  # windows of three batches
+        if compat == capi.COMPAT_ALL:
+            assert np.abs(r - m).max() < 6 * sd
+            assert sd / 10 < np.std(r) < 10 * sd
+    assert set(risks(-1)) != set(risks(-1))
