@@ -1254,6 +1254,7 @@ int pgsvt_lambda_grad(const float* model, const float* features, const float* ta
     float* f = mem.arr<float>((size_t)n * PGSVT_LAMBDA_FEATURES);
     float* t = mem.arr<float>(n);
     float* act = mem.arr<float>(lambda_act_floats((int)n));
+    float* part = mem.arr<float>(lambda_part_floats((int)n));
     float* pl = mem.arr<float>(nblk);
     float* g = mem.arr<float>(PGSVT_LAMBDA_PARAMS);
     PGSVT_CK(cudaMemcpyAsync(m, model, sizeof(float) * PGSVT_LAMBDA_MODEL_FLOATS, cudaMemcpyHostToDevice, s));
@@ -1262,7 +1263,8 @@ int pgsvt_lambda_grad(const float* model, const float* features, const float* ta
     PGSVT_CK(cudaMemcpyAsync(t, targets, sizeof(float) * n, cudaMemcpyHostToDevice, s));
     PGSVT_CK(lambda_attrs());
     check_launch(lambda_shadow(m, wbf, s), stats);
-    check_launch(lambda_grad(m, wbf, f, t, (int)n, act, pl, g, s), stats, 2);
+    check_launch(lambda_grad(m, wbf, f, t, (int)n, act, part, pl, g, s), stats,
+                 1 + lambda_update_launches((int)n));
     std::vector<float> hl(nblk);
     PGSVT_CK(cudaMemcpyAsync(grad, g, sizeof(float) * PGSVT_LAMBDA_PARAMS, cudaMemcpyDeviceToHost, s));
     PGSVT_CK(cudaMemcpyAsync(hl.data(), pl, sizeof(float) * nblk, cudaMemcpyDeviceToHost, s));
@@ -1314,6 +1316,7 @@ int pgsvt_lambda_train(float* model, const float* features, const float* targets
     t.perm = perm;
     t.epoch = mem.arr<int>(1);
     t.act = mem.arr<float>(lambda_act_floats(batch));
+    t.part = mem.arr<float>(lambda_part_floats(batch));
     t.loss_acc = mem.arr<float>((size_t)t.steps * nblk);
     t.epoch_loss = mem.arr<float>(tp->epochs);
     // sample order of every epoch: Fisher-Yates shuffles from a pcg64 stream
@@ -1358,7 +1361,7 @@ int pgsvt_lambda_train(float* model, const float* features, const float* targets
     PGSVT_CK(cudaGraphInstantiate(&exec, graph, 0));
     for (uint32_t e = 0; e < tp->epochs; ++e) {
       PGSVT_CK(cudaGraphLaunch(exec, s));
-      stats.launches += 2 * (uint64_t)t.steps + 1;
+      stats.launches += (1 + lambda_update_launches(batch)) * (uint64_t)t.steps + 1;
     }
     PGSVT_CK(cudaMemcpyAsync(model, t.m, sizeof(float) * PGSVT_LAMBDA_MODEL_FLOATS, cudaMemcpyDeviceToHost, s));
     if (epoch_loss)

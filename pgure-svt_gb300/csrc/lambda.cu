@@ -9,9 +9,9 @@
 // bf16 shadow that the passes read.  What bounds a step is latency: 14 MFLOP
 // over chains of 128 dependent FMAs per layer.  So it is spread thin: k_mlp_pass
 // runs four samples per block (the samples are independent), with the weights in
-// shared memory, and k_mlp_update forms every weight's gradient, sums it in
-// a fixed order (chains of 32 samples, then the chains) and applies AdamW in
-// the same thread, so training is deterministic.
+// shared memory, and k_mlp_update (many rows: k_mlp_chains and k_mlp_sum) forms
+// every weight's gradient, sums it in a fixed order (chains of 32 samples, then
+// the chains) and applies AdamW in the same thread, so training is deterministic.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -394,6 +394,102 @@ __global__ void __launch_bounds__(H * NCH) k_mlp_update(
   else grad[i] = g[0];
 }
 
+// The same in two kernels for many rows: a block of k_mlp_chains forms the sums of one
+// chain of 32 rows for a whole layer, 8 x 8 of them per thread from rows in shared
+// memory, and k_mlp_sum adds the chains up in their order.  k_mlp_update walks the
+// chains in every block, so its time goes with the rows.  A step's update, GB300:
+// 256 rows 8.6 us there, 8.9 + 4.6 us here; 512 rows 12.0 and 9.1 + 2.9; 1,024 rows
+// 23.6 and 9.3 + 3.3; 8,192 rows 175 and 35.4 + 9.6, bound by the FMAs of the chains.
+constexpr int CT = 256;  // threads of k_mlp_chains
+
+__global__ void __launch_bounds__(CT) k_mlp_chains(const float* __restrict__ act,
+                                                   const float* __restrict__ dO,
+                                                   const float* __restrict__ err, int rows_pad,
+                                                   float* __restrict__ part,
+                                                   float* __restrict__ loss) {
+  __shared__ __align__(16) float xs[32][H], ds[32][H];
+  const int ch = blockIdx.x, layer = blockIdx.y, tid = threadIdx.x;
+  const size_t plane = (size_t)rows_pad * H, row0 = (size_t)ch * 32 * H;
+  float* out = part + (size_t)ch * NPARAM;
+  if (layer == 3) {  // the biases, the output layer and the squared error
+    if (tid < H) {
+      float b[3] = {0.f, 0.f, 0.f}, w = 0.f;
+      for (int s = 0; s < 32; ++s) {
+#pragma unroll
+        for (int l = 0; l < 3; ++l) b[l] += act[(ACT_Z1 + l) * plane + row0 + s * H + tid];
+        w = fmaf(dO[ch * 32 + s], act[ACT_A3 * plane + row0 + s * H + tid], w);
+      }
+      out[OFF_B1 - OFF_W1 + tid] = b[0];
+      out[OFF_B2 - OFF_W1 + tid] = b[1];
+      out[OFF_B3 - OFF_W1 + tid] = b[2];
+      out[OFF_W4 - OFF_W1 + tid] = w;
+    } else if (tid < H + 32) {
+      const float e = err[ch * 32 + tid - H];
+      float sq = e * e;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if (tid == H) {
+        float t = 0.f;
+        for (int s = 0; s < 32; ++s) t += dO[ch * 32 + s];
+        out[OFF_B4 - OFF_W1] = t;
+        loss[ch] = sq;
+      }
+    }
+    return;
+  }
+  // (inputs beyond the features are not set in layer 0, and not stored below)
+  const float4* in = reinterpret_cast<const float4*>(act + (ACT_X0 + layer) * plane + row0);
+  const float4* dz = reinterpret_cast<const float4*>(act + (ACT_Z1 + layer) * plane + row0);
+  for (int i = tid; i < 32 * H / 4; i += CT) {
+    reinterpret_cast<float4*>(xs)[i] = in[i];
+    reinterpret_cast<float4*>(ds)[i] = dz[i];
+  }
+  __syncthreads();
+  const int k0 = (tid & 15) * 4, j0 = (tid >> 4) * 8;  // inputs k0.., 64 + k0.., outputs j0..
+  float g[8][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) g[j][k] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < 32; ++s) {
+    float x[8], d[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      *reinterpret_cast<float4*>(x + 4 * h) = *reinterpret_cast<const float4*>(&xs[s][k0 + 64 * h]);
+      *reinterpret_cast<float4*>(d + 4 * h) = *reinterpret_cast<const float4*>(&ds[s][j0 + 4 * h]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) g[j][k] = fmaf(d[j], x[k], g[j][k]);
+  }
+  const int kin = layer == 0 ? NF : H;
+  out += (layer == 0 ? OFF_W1 : (layer == 1 ? OFF_W2 : OFF_W3)) - OFF_W1;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int kk = k0 + (k & 3) + 64 * (k >> 2);
+      if (kk < kin) out[(j0 + j) * kin + kk] = g[j][k];
+    }
+}
+
+template <bool ADAM>
+__global__ void __launch_bounds__(128) k_mlp_sum(float* __restrict__ m, Shadow* __restrict__ wbf,
+                                                 float* __restrict__ mom1, float* __restrict__ mom2,
+                                                 const float* __restrict__ part, int nch,
+                                                 const int* __restrict__ epoch, int step, AdamCfg c,
+                                                 float* __restrict__ grad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= NPARAM) return;
+  float g = 0.f;
+#pragma unroll 16
+  for (int k = 0; k < nch; ++k) g += part[(size_t)k * NPARAM + i];
+  if constexpr (ADAM) adam(m, wbf, mom1, mom2, i, g, *epoch * c.steps_per_epoch + step + 1, c);
+  else grad[i] = g;
+}
+
 // Mean loss of the epoch; advances the device epoch counter.
 __global__ void k_mlp_epoch_end(const float* __restrict__ loss_acc, int nsteps, int nblk, int n,
                                 int* __restrict__ epoch, float* __restrict__ epoch_loss) {
@@ -492,18 +588,44 @@ cudaError_t lambda_forward(const float* m, const void* wbf, const float* feat, i
   return cudaGetLastError();
 }
 
-// Gradient over n samples: act holds lambda_act_floats(n) floats, part_loss
-// the squared error of each 32 samples.
+// Gradients of the rows of a pass into grad, or with ADAM the parameter update.
+// By chains from where two launches are faster than one (equal at 512 rows; 4
+// epochs of 8 steps of 8,192 rows 9.4 -> 5.5 ms).
+static bool by_chains(size_t rows) { return rows > 512; }
+
+template <bool ADAM>
+static void launch_update(float* m, lam::Shadow* wbf, float* mom1, float* mom2, const float* act,
+                          const float* dO, const float* err, int rows_pad, float* part,
+                          const int* epoch, int step, const lam::AdamCfg& c, float* grad,
+                          float* loss, cudaStream_t s) {
+  if (by_chains(rows_pad)) {
+    lam::k_mlp_chains<<<dim3(rows_pad / 32, 4), lam::CT, 0, s>>>(act, dO, err, rows_pad, part, loss);
+    lam::k_mlp_sum<ADAM><<<(lam::NPARAM + 127) / 128, 128, 0, s>>>(m, wbf, mom1, mom2, part,
+                                                                   rows_pad / 32, epoch, step, c, grad);
+  } else {
+    lam::k_mlp_update<ADAM><<<lam::kUpdateBlocks, lam::H * lam::NCH, 0, s>>>(
+        m, wbf, mom1, mom2, act, dO, err, rows_pad, epoch, step, c, grad, loss);
+  }
+}
+// floats of the chains' sums of n rows (0: not needed)
+size_t lambda_part_floats(int n) {
+  const size_t r = lambda_rows(n);
+  return by_chains(r) ? r / 32 * lam::NPARAM : 0;
+}
+int lambda_update_launches(int n) { return by_chains(lambda_rows(n)) ? 2 : 1; }
+
+// Gradient over n samples: act holds lambda_act_floats(n) floats, part
+// lambda_part_floats(n), part_loss the squared error of each 32 samples.
 cudaError_t lambda_grad(const float* m, const void* wbf, const float* feat, const float* target,
-                        int n, float* act, float* part_loss, float* grad, cudaStream_t s) {
+                        int n, float* act, float* part, float* part_loss, float* grad,
+                        cudaStream_t s) {
   const int rp = (int)lambda_rows(n);
   float* dO = act + (size_t)rp * lam::ACT_N * lam::H;
   lam::k_mlp_pass<<<pass_blocks(rp), lam::PT, lambda_smem(), s>>>(
       m, (const lam::Shadow*)wbf, feat, target, nullptr, nullptr, 0, 0, n, rp, 1.f / (float)n, act,
       dO, dO + rp);
-  lam::k_mlp_update<false><<<lam::kUpdateBlocks, lam::H * lam::NCH, 0, s>>>(
-      nullptr, nullptr, nullptr, nullptr, act, dO, dO + rp, rp, nullptr, 0, lam::AdamCfg{}, grad,
-      part_loss);
+  launch_update<false>(nullptr, nullptr, nullptr, nullptr, act, dO, dO + rp, rp, part, nullptr, 0,
+                       lam::AdamCfg{}, grad, part_loss, s);
   return cudaGetLastError();
 }
 
@@ -518,16 +640,15 @@ cudaError_t lambda_attrs() {
 // One epoch of training (stream-capturable: launches only; lambda_attrs()
 // must have run).
 cudaError_t lambda_train_epoch(const LambdaTrain& t, cudaStream_t s) {
-  const int nblk = t.batch / 32;
+  const int nblk = t.batch / 32, blocks = pass_blocks(t.batch);
   float* dO = t.act + (size_t)t.batch * lam::ACT_N * lam::H;
   lam::AdamCfg c{t.lr, t.lr_final, t.wd, t.b1, t.b2, t.eps, t.steps, t.total_steps};
   for (int st = 0; st < t.steps; ++st) {
-    lam::k_mlp_pass<<<pass_blocks(t.batch), lam::PT, lambda_smem(), s>>>(
+    lam::k_mlp_pass<<<blocks, lam::PT, lambda_smem(), s>>>(
         t.m, (const lam::Shadow*)t.wbf, t.feat, t.target, t.perm, t.epoch, t.n, st * t.batch,
         t.n, t.batch, 1.f / (float)t.batch, t.act, dO, dO + t.batch);
-    lam::k_mlp_update<true><<<lam::kUpdateBlocks, lam::H * lam::NCH, 0, s>>>(
-        t.m, (lam::Shadow*)t.wbf, t.mom1, t.mom2, t.act, dO, dO + t.batch, t.batch, t.epoch, st, c,
-        nullptr, t.loss_acc + (size_t)st * nblk);
+    launch_update<true>(t.m, (lam::Shadow*)t.wbf, t.mom1, t.mom2, t.act, dO, dO + t.batch, t.batch,
+                        t.part, t.epoch, st, c, nullptr, t.loss_acc + (size_t)st * nblk, s);
   }
   lam::k_mlp_epoch_end<<<1, 32, 0, s>>>(t.loss_acc, t.steps, nblk, t.steps * t.batch, t.epoch,
                                         t.epoch_loss);

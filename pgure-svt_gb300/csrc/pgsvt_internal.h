@@ -319,6 +319,7 @@ struct LambdaTrain {
   const int32_t* perm; // [epochs][n] sample order
   int* epoch;          // device epoch counter
   float* act;          // lambda_act_floats(batch): the rows of a pass
+  float* part;         // lambda_part_floats(batch): the sums of their chains
   float* loss_acc;     // [steps][batch/32]
   float* epoch_loss;   // [epochs]
   int n, batch, steps, total_steps;
@@ -331,8 +332,11 @@ cudaError_t lambda_shadow(const float* m, void* wbf, cudaStream_t s);
 cudaError_t lambda_forward(const float* m, const void* wbf, const float* feat, int n, float* y,
                            cudaStream_t s);
 cudaError_t lambda_grad(const float* m, const void* wbf, const float* feat, const float* target,
-                        int n, float* act, float* part_loss, float* grad, cudaStream_t s);
+                        int n, float* act, float* part, float* part_loss, float* grad,
+                        cudaStream_t s);
 size_t lambda_act_floats(int n);
+size_t lambda_part_floats(int n);
+int lambda_update_launches(int n);
 cudaError_t lambda_train_epoch(const LambdaTrain& t, cudaStream_t s);
 cudaError_t lambda_attrs();
 
