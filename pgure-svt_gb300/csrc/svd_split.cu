@@ -150,6 +150,11 @@ __device__ __forceinline__ void tma_tile3(uint32_t dst, const CUtensorMap* map, 
 // with one exchange per dot product took four times the last two.  256 x 256 x 24, 8 x 8 patches, GB300:
 // 22.4 -> 14.3 ms in 3 launches.
 
+// |v|^2 of a reflection below which it is left out: its column has no norm left
+// (equal columns, as of saturated pixels, leave 1e-7 of the norm each time), and
+// 2 / |v|^2 would overflow and make the patch's columns NaN.
+constexpr float kTinyColumn = 1e-36f;
+
 // f[i] = beta * half_sum(t[i])
 __device__ __forceinline__ void half_sums4(const float (&t)[4], float beta, float (&f)[4]) {
   const int lane = threadIdx.x & 31;
@@ -235,7 +240,7 @@ __global__ void __launch_bounds__(128, 8) k_qr(Problem pb, DeviceBuffers d, int 
       const float xj = __shfl_sync(0xffffffffu, b[i][i], j0 >> 2, kQL);  // row jj
       const float alpha = xj >= 0.f ? -sqrtf(ss) : sqrtf(ss);
       const float vtv = 2.f * (ss - xj * alpha);  // |x - alpha e_jj|^2
-      const float beta = vtv > 0.f ? 2.f / vtv : 0.f;
+      const float beta = vtv > kTinyColumn ? 2.f / vtv : 0.f;
       float4 v4;
       float* v = &v4.x;
 #pragma unroll

@@ -328,3 +328,33 @@ def test_fresh_probes_of_every_window(capi, pkg):
             assert np.abs(r - m).max() < 6 * sd
             assert sd / 10 < np.std(r) < 10 * sd
     assert set(risks(-1)) != set(risks(-1))
+
+
+def _saturated(kind, side, nt):
+    """Byte frames with clipped highlights, or flat 16 x 16 tiles in noise: patches
+    whose columns are equal in many frames."""
+    rng = np.random.default_rng(side + nt)
+    y, x = np.mgrid[0:side, 0:side]
+    f = []
+    for k in range(nt):
+        b = 40 + 30 * np.sin((x + k) / 5.0) * np.cos((y - k) / 7.0)
+        v = (np.minimum(rng.poisson(2 * b), 90) if kind == "clipped" else
+             np.where((x // 16 + 2 * (y // 16) + k) % 3 == 0, 3.0 + (x // 16) * 7 + k, rng.poisson(b)))
+        f.append(v)
+    return np.asfortranarray(np.stack(f, -1).astype(np.uint8))
+
+
+@pytest.mark.parametrize("bs,T,form", [(4, 15, 0), (4, 9, 3), (5, 9, 0), (5, 9, 5), (6, 15, 5),
+                                       (7, 7, 0), (8, 9, 0), (8, 15, 3), (8, 21, 0)])
+@pytest.mark.parametrize("kind", ["clipped", "flat"])
+@pytest.mark.parametrize("lam,expw", [(0.49, 0), (0.01, 0), (1e-4, 0), (0.3, 1)])
+def test_patches_of_equal_columns(capi, oracle, kind, bs, T, form, lam, expw):
+    """Each equal column leaves 1e-7 of the norm in the QR form, so the fourth has
+    a squared norm that FP32 cannot invert; every form against the oracle at a fixed
+    threshold (the whole-sequence tolerance at fixed lambda)."""
+    X = _saturated(kind, 64, T)
+    kw = dict(traj_length=T, block_size=bs, block_overlap=2, motion_window=3, median_size=-1,
+              random_seed=11, optimize_pgure=0, exp_weighting=expw, lambda_=lam)
+    Y, _, _ = capi.denoise(X, capi.default_params(autotune=form, frame_begin=2, frame_end=4, **kw))
+    Yo, _, _ = oracle.denoise(X, n_jobs=8, frame_begin=2, frame_end=4, **kw)
+    assert np.abs(Y - Yo).max() <= 2e-5 * np.abs(Yo).max()
