@@ -118,9 +118,13 @@ __device__ __forceinline__ double lanes_sum_d(double v) {
 // Can singular value s (largest smax) survive the threshold for some lambda
 // of the search (svt.hpp:135-143)?  Conservative: columns reported dead have
 // g = 0 for every lambda the search evaluates, with margin for FP32 rounding.
+// Or they are rounding noise (below 1e-7 of the largest) too small for the rotation
+// test, whose squares underflow below s smax = 1e-13: such a column need not be
+// orthogonal to the large ones, and with a threshold near 0 it would count them twice.
 __device__ __forceinline__ bool can_survive(const Problem& pb, float s, float smax,
                                             float upper) {
   if (!(s > 0.f)) return false;
+  if (s < 1e-7f * smax && s * smax < 1e-13f) return false;
   if (!pb.optimize) {
     const float lam = (float)pb.lambda_user;
     const float th = pb.expw ? fabsf(smax * expf(-0.5f * lam * (s * s))) : lam;

@@ -347,10 +347,11 @@ def _saturated(kind, side, nt):
 @pytest.mark.parametrize("bs,T,form", [(4, 15, 0), (4, 9, 3), (5, 9, 0), (5, 9, 5), (6, 15, 5),
                                        (7, 7, 0), (8, 9, 0), (8, 15, 3), (8, 21, 0)])
 @pytest.mark.parametrize("kind", ["clipped", "flat"])
-@pytest.mark.parametrize("lam,expw", [(0.49, 0), (0.01, 0), (1e-4, 0), (0.3, 1)])
+@pytest.mark.parametrize("lam,expw", [(0.49, 0), (0.01, 0), (1e-4, 0), (1e-7, 0), (0.0, 0), (0.3, 1)])
 def test_patches_of_equal_columns(capi, oracle, kind, bs, T, form, lam, expw):
     """Each equal column leaves 1e-7 of the norm in the QR form, so the fourth has
-    a squared norm that FP32 cannot invert; every form against the oracle at a fixed
+    a squared norm that FP32 cannot invert; and singular values of rounding noise,
+    which a threshold near 0 keeps.  Every form against the oracle at a fixed
     threshold (the whole-sequence tolerance at fixed lambda)."""
     X = _saturated(kind, 64, T)
     kw = dict(traj_length=T, block_size=bs, block_overlap=2, motion_window=3, median_size=-1,
