@@ -413,16 +413,16 @@ struct Footprint {
   int y0, x0, th, ths, area;  // corner, rows, column stride, pixels
   bool tile;              // it fits the tile
   __device__ __forceinline__ void init(bool live, int y, int x, int nb, int tile_max) {
-    y0 = __reduce_min_sync(0xffffffffu, live ? y : 1 << 30);
-    x0 = __reduce_min_sync(0xffffffffu, live ? x : 1 << 30);
+    // (frame sides are below 0x7fff; without a live lane the products stay in range)
+    y0 = __reduce_min_sync(0xffffffffu, live ? y : 0x7fff);
+    x0 = __reduce_min_sync(0xffffffffu, live ? x : 0x7fff);
     const int y1 = __reduce_max_sync(0xffffffffu, live ? y : -1);
     const int x1 = __reduce_max_sync(0xffffffffu, live ? x : -1);
-    const bool any = y1 >= 0;  // a lane holds a patch
-    const int tw = any ? x1 - x0 + nb : 0;
-    th = any ? y1 - y0 + nb : 0;
+    const int tw = x1 - x0 + nb;
+    th = y1 - y0 + nb;
     ths = th <= 8 ? 8 : 8 + 16 * ((th - 8 + 15) / 16);
-    if (ths * tw > tile_max) ths = th;
-    tile = any && ths * tw <= tile_max;
+    if (y1 >= 0 && ths * tw > tile_max) ths = th;
+    tile = y1 >= 0 && ths * tw <= tile_max;
     area = th * tw;
   }
 };
@@ -534,7 +534,7 @@ __host__ __device__ constexpr int chunk_rows() {
 // windows up to 16 frames run two blocks per SM
 template <int BS, typename AccT, int MAXW>
 __global__ void __launch_bounds__(32 * MAXW, MAXW <= 16 ? 2 : 1)
-    k_eval(Problem pb, DeviceBuffers d, int final_pass) {
+    k_eval(Problem pb, DeviceBuffers d, int final_pass, int large_rounds) {
   const int nb = BS > 0 ? BS : pb.g.bs;  // BS == 0: any side (9..16)
   const int M = nb * nb;
   constexpr int PB = kEvalPatches;  // patches per block
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(32 * MAXW, MAXW <= 16 ? 2 : 1)
   constexpr int US = eval_ustride(BS * BS);
   float* Us = sg;
   float* sgv = sg + eval_staged(BS, NC);
-  const int T = eval_tile(BS, sizeof(AccT) == 8, NC, nwarps, final_pass ? 1 : pb.K, nl);
+  const int T = eval_tile(BS, sizeof(AccT) == 8, large_rounds, nl);
   float* slin = sgv + (size_t)nl * NC * PB;
   int* tiles = (int*)(sg + eval_tiles_at(BS, NC, nl));
   __shared__ int srmax[kMaxK];
@@ -958,15 +958,16 @@ void launch_k_eval_bs(dim3 grid, int threads, int nl, cudaStream_t s, const Prob
   // (110 KB at most for windows up to 16 frames)
   const size_t shm =
       (size_t)eval_alloc_words(BS, sizeof(AccT) == 8, pb.g.NC, pb.g.nwin, nl) * sizeof(int);
+  const int large = eval_large_rounds(BS, sizeof(AccT) == 8, pb.g.NC, pb.g.nwin, nl);
   if constexpr (BS > 0 && BS * BS <= 16) {  // windows of at most 15 frames
     allow_dynamic_smem((const void*)k_eval<BS, AccT, 16>, shm);
-    k_eval<BS, AccT, 16><<<grid, threads, shm, s>>>(pb, d, final_pass);
+    k_eval<BS, AccT, 16><<<grid, threads, shm, s>>>(pb, d, final_pass, large);
   } else if (threads <= 32 * 16) {  // two blocks per SM
     allow_dynamic_smem((const void*)k_eval<BS, AccT, 16>, shm);
-    k_eval<BS, AccT, 16><<<grid, threads, shm, s>>>(pb, d, final_pass);
+    k_eval<BS, AccT, 16><<<grid, threads, shm, s>>>(pb, d, final_pass, large);
   } else {
     allow_dynamic_smem((const void*)k_eval<BS, AccT, 21>, shm);
-    k_eval<BS, AccT, 21><<<grid, threads, shm, s>>>(pb, d, final_pass);
+    k_eval<BS, AccT, 21><<<grid, threads, shm, s>>>(pb, d, final_pass, large);
   }
 }
 

@@ -53,11 +53,17 @@ PGSVT_HD constexpr int eval_alloc_tile(int bs, bool wide, int points) {
 PGSVT_HD constexpr int eval_alloc_words(int bs, bool wide, int NC, int nwin, int points) {
   return eval_words(bs, NC, nwin, points, eval_alloc_tile(bs, wide, points));
 }
-// The tile of a round of nl <= points values: the allocation's, or the larger one
-// of short launches where the values that the round does without leave room for it.
-PGSVT_HD constexpr int eval_tile(int bs, bool wide, int NC, int nwin, int points, int nl) {
-  const int T = eval_alloc_tile(bs, wide, points), T8 = eval_alloc_tile(bs, wide, 1);
-  return eval_words(bs, NC, nwin, nl, T8) <= eval_alloc_words(bs, wide, NC, nwin, points) ? T8 : T;
+// The most values of a round that leave room for the larger tile of short launches
+// (the whole launch, where that is its tile).
+PGSVT_HD constexpr int eval_large_rounds(int bs, bool wide, int NC, int nwin, int points) {
+  const int words = eval_alloc_words(bs, wide, NC, nwin, points);
+  int nl = points;
+  while (nl > 0 && eval_words(bs, NC, nwin, nl, eval_alloc_tile(bs, wide, 1)) > words) --nl;
+  return nl;
+}
+// The tile of a round of nl <= points values.
+PGSVT_HD constexpr int eval_tile(int bs, bool wide, int large_rounds, int nl) {
+  return eval_alloc_tile(bs, wide, nl <= large_rounds ? 1 : 16);
 }
 
 }  // namespace pgsvt

@@ -19,13 +19,14 @@ int main() {
         for (int points = 1; points <= 16; ++points) {
           const int words = eval_alloc_words(bs, wide, NC, nwin, points);
           for (int nl = 1; nl <= points; ++nl, ++rounds) {
-            const int T = eval_tile(bs, wide, NC, nwin, points, nl);
+            const int T = eval_tile(bs, wide, eval_large_rounds(bs, wide, NC, nwin, points), nl);
             // 16-byte clears of whole tiles; tiles large enough for one patch
             bool ok = T % 4 == 0 && T >= side * side && eval_tiles_at(bs, NC, nl) % 4 == 0;
             // the tiles are the last thing in the block's shared memory
             ok = ok && eval_tiles_at(bs, NC, nl) + nwin * 2 * T <= words;
             ok = ok && words * 4 <= 227 * 1024;
             if (wide) ok = ok && T == 256;  // rounding depends on the size
+            if (points <= 8) ok = ok && T == eval_alloc_tile(bs, wide, 1);
             if (!ok && bad++ < 5)
               std::printf("side %d nwin %d wide %d points %d nl %d\n", side, nwin, wide, points, nl);
           }
