@@ -36,7 +36,7 @@ struct Fail : std::runtime_error {
   } while (0)
 
 // Device memory of a call.  A call needs 25 to 90 arrays; allocating and freeing
-// each took 1.0 of 1.5 ms on a 32 x 32 x 16 sequence and 11 of 203 ms on 256 x
+// each took 0.9 of 1.8 ms on a 32 x 32 x 16 sequence and 11 of 203 ms on 256 x
 // 256 x 100, so arrays are carved out of blocks, and the blocks of a finished
 // call stay in a process-wide cache for the next one.  The cache is bounded
 // (kCacheBytes over all devices, the blocks longest unused are freed first) and

