@@ -60,3 +60,33 @@ def test_memory_is_given_back(capi, pkg):
     assert torch.cuda.mem_get_info()[0] >= free0
     for x, y in zip(_calls(capi, pkg), first):
         np.testing.assert_array_equal(x, y)
+
+
+def test_concurrent_calls_and_releases(capi, pkg):
+    """Calls of different sizes on four threads, blocks changing hands between them,
+    while a fifth keeps giving the memory back: every result is that of a call alone."""
+    first = _calls(capi, pkg)
+    wrong, stop = [], threading.Event()
+
+    def work():
+        try:
+            for _ in range(3):
+                for k, (x, y) in enumerate(zip(_calls(capi, pkg), first)):
+                    if not np.array_equal(x, y):
+                        wrong.append(k)
+        except Exception as e:  # reported by the main thread
+            wrong.append(e)
+
+    def give_back():
+        while not stop.wait(0.002):
+            capi.release_memory()
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    giver = threading.Thread(target=give_back)
+    for t in threads + [giver]:
+        t.start()
+    for t in threads:
+        t.join()
+    stop.set()
+    giver.join()
+    assert not wrong
