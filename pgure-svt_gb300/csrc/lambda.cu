@@ -405,12 +405,12 @@ constexpr int CT = 256;  // threads of k_mlp_chains
 __global__ void __launch_bounds__(CT) k_mlp_chains(const float* __restrict__ act,
                                                    const float* __restrict__ dO,
                                                    const float* __restrict__ err, int rows_pad,
-                                                   float* __restrict__ part,
+                                                   int ch0, float* __restrict__ part,
                                                    float* __restrict__ loss) {
   __shared__ __align__(16) float xs[32][H], ds[32][H];
-  const int ch = blockIdx.x, layer = blockIdx.y, tid = threadIdx.x;
+  const int ch = ch0 + blockIdx.x, layer = blockIdx.y, tid = threadIdx.x;
   const size_t plane = (size_t)rows_pad * H, row0 = (size_t)ch * 32 * H;
-  float* out = part + (size_t)ch * NPARAM;
+  float* out = part + (size_t)blockIdx.x * NPARAM;
   if (layer == 3) {  // the biases, the output layer and the squared error
     if (tid < H) {
       float b[3] = {0.f, 0.f, 0.f}, w = 0.f;
@@ -475,15 +475,16 @@ __global__ void __launch_bounds__(CT) k_mlp_chains(const float* __restrict__ act
     }
 }
 
+// (more: to the sums in grad of the chains before)
 template <bool ADAM>
 __global__ void __launch_bounds__(128) k_mlp_sum(float* __restrict__ m, Shadow* __restrict__ wbf,
                                                  float* __restrict__ mom1, float* __restrict__ mom2,
-                                                 const float* __restrict__ part, int nch,
+                                                 const float* __restrict__ part, int nch, bool more,
                                                  const int* __restrict__ epoch, int step, AdamCfg c,
                                                  float* __restrict__ grad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NPARAM) return;
-  float g = 0.f;
+  float g = !ADAM && more ? grad[i] : 0.f;
 #pragma unroll 16
   for (int k = 0; k < nch; ++k) g += part[(size_t)k * NPARAM + i];
   if constexpr (ADAM) adam(m, wbf, mom1, mom2, i, g, *epoch * c.steps_per_epoch + step + 1, c);
@@ -592,6 +593,9 @@ cudaError_t lambda_forward(const float* m, const void* wbf, const float* feat, i
 // By chains from where two launches are faster than one (equal at 512 rows; 4
 // epochs of 8 steps of 8,192 rows 9.4 -> 5.5 ms).
 static bool by_chains(size_t rows) { return rows > 512; }
+// The sums of at most kSlab chains (65,536 rows, 343 MB) are held at a time; a batch of
+// training has no more than 256.
+constexpr size_t kSlab = 2048;
 
 template <bool ADAM>
 static void launch_update(float* m, lam::Shadow* wbf, float* mom1, float* mom2, const float* act,
@@ -599,9 +603,12 @@ static void launch_update(float* m, lam::Shadow* wbf, float* mom1, float* mom2, 
                           const int* epoch, int step, const lam::AdamCfg& c, float* grad,
                           float* loss, cudaStream_t s) {
   if (by_chains(rows_pad)) {
-    lam::k_mlp_chains<<<dim3(rows_pad / 32, 4), lam::CT, 0, s>>>(act, dO, err, rows_pad, part, loss);
-    lam::k_mlp_sum<ADAM><<<(lam::NPARAM + 127) / 128, 128, 0, s>>>(m, wbf, mom1, mom2, part,
-                                                                   rows_pad / 32, epoch, step, c, grad);
+    for (int c0 = 0; c0 < rows_pad / 32; c0 += (int)kSlab) {
+      const int nch = std::min((int)kSlab, rows_pad / 32 - c0);
+      lam::k_mlp_chains<<<dim3(nch, 4), lam::CT, 0, s>>>(act, dO, err, rows_pad, c0, part, loss);
+      lam::k_mlp_sum<ADAM><<<(lam::NPARAM + 127) / 128, 128, 0, s>>>(
+          m, wbf, mom1, mom2, part, nch, c0 > 0, epoch, step, c, grad);
+    }
   } else {
     lam::k_mlp_update<ADAM><<<lam::kUpdateBlocks, lam::H * lam::NCH, 0, s>>>(
         m, wbf, mom1, mom2, act, dO, err, rows_pad, epoch, step, c, grad, loss);
@@ -610,9 +617,12 @@ static void launch_update(float* m, lam::Shadow* wbf, float* mom1, float* mom2, 
 // floats of the chains' sums of n rows (0: not needed)
 size_t lambda_part_floats(int n) {
   const size_t r = lambda_rows(n);
-  return by_chains(r) ? r / 32 * lam::NPARAM : 0;
+  return by_chains(r) ? std::min(r / 32, kSlab) * lam::NPARAM : 0;
 }
-int lambda_update_launches(int n) { return by_chains(lambda_rows(n)) ? 2 : 1; }
+int lambda_update_launches(int n) {
+  const size_t r = lambda_rows(n);
+  return by_chains(r) ? 2 * (int)((r / 32 + kSlab - 1) / kSlab) : 1;
+}
 
 // Gradient over n samples: act holds lambda_act_floats(n) floats, part
 // lambda_part_floats(n), part_loss the squared error of each 32 samples.

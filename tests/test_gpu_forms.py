@@ -39,11 +39,11 @@ def test_mlp_gradient_rows(capi, pkg, oracle, n):
     assert np.abs(capi.lambda_predict(m, f) - y0).max() <= 1e-4 * (1 + np.abs(y0).max())
 
 
-@pytest.mark.parametrize("n", [480, 512, 513, 1024, 1025, 9000])
+@pytest.mark.parametrize("n", [480, 512, 513, 1024, 1025, 9000, 65536, 65537, 131105])
 def test_mlp_gradient_of_many_rows(capi, pkg, oracle, n):
     """Either side of the number of rows from which the chains have a kernel of
-    their own, full and cut last chains; the tolerances are those of the fixed-size
-    test."""
+    their own, full and cut last chains, one to three slabs of chains; the tolerances
+    are those of the fixed-size test."""
     test_mlp_gradient_rows(capi, pkg, oracle, n)
 
 
